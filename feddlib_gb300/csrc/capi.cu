@@ -20,6 +20,7 @@ struct fedd_assembler {
     int64_t nn = 0, ne = 0, nn_p = 0;
     DBuf<double> xyz;
     DBuf<int32_t> conn, conn_p;
+    DBuf<float> geo;        // B^-1 and det B of every element (launch_geometry)
     Graph g, gp;
     DBuf<int32_t> vmap;     // Taylor-Hood: P2 vertex -> P1 node (-1 for edge nodes)
     DBuf<unsigned long long> work;  // the velocity-row kernel's position counter (device path)
@@ -222,7 +223,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
             if (!h->has_mlp) FEDD_FAIL(FEDD_ERR_STATE, "surrogate requested but no network set (fedd_set_surrogate)");
             const int64_t nqp = h->ne * h->htab.nq;
             stage(h, "qp_invariants", s, [&] {
-                launch_hyper_invariants(h->xyz.p, h->conn.p, h->ne, d_u, h->law, h->htab, h->qp_inv.p, h->d_err.p,
+                launch_hyper_invariants(h->geo.p, h->conn.p, h->ne, d_u, h->law, h->htab, h->qp_inv.p, h->d_err.p,
                                         s, lc);
             });
             FEDD_CUDA(cudaMemsetAsync(h->d_fb.p, 0, sizeof(int), s));
@@ -234,7 +235,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
             h->last_nqp = nqp;
         }
         stage(h, "hyper_elem", s, [&] {
-            launch_hyper_elem(h->xyz.p, h->conn.p, h->ne, d_u, h->law, h->htab, qpd, qfb, h->stage_f.p,
+            launch_hyper_elem(h->geo.p, h->conn.p, h->ne, d_u, h->law, h->htab, qpd, qfb, h->stage_f.p,
                               res && d_u != nullptr, h->d_err.p, s, lc);
         });
         stage(h, "hyper_rows", s, [&] {
@@ -250,12 +251,12 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         const float vd = h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density);
         const float dn = (float)h->prm.density;
         stage(h, "ns_record", s, [&] {
-            launch_ns_record(h->xyz.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab, vd, dn, h->stage_f.p,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab, vd, dn, h->stage_f.p,
                              h->d_err.p, s, lc);
         });
         if (h->gn_on)
             stage(h, "gn_elem", s, [&] {
-                launch_gn_elem(h->xyz.p, h->conn.p, h->ne, d_u, h->gn, h->prm.linearization, h->stage_gn.p,
+                launch_gn_elem(h->xyz.p, h->geo.p, h->conn.p, h->ne, d_u, h->gn, h->prm.linearization, h->stage_gn.p,
                                h->d_err.p, s, lc, 0, -1, h->outflow());
             });
         // with a verified vertex map the velocity-row warps of the vertices
@@ -360,6 +361,11 @@ fedd_status fedd_create(const fedd_mesh *mesh, const fedd_params *params, int de
         load_conn(h->conn, mesh->elements, h->npe);
         FEDD_CUDA(cudaStreamSynchronize(s));
         build_graph(h->g, h->ne, h->conn.p, h->npe, h->nn, h->conn.p, h->npe, h->nn, 0, h->d_err.p, s);
+        // build_graph has checked the node indices
+        if (prob != FEDD_LAPLACE) {
+            h->geo.alloc((size_t)h->ne * 10);
+            launch_geometry(h->xyz.p, h->conn.p, h->ne, h->geo.p, s);
+        }
         if (prob == FEDD_LAPLACE) {
             build_csr(h->csr[0], h->g.adj_ptr, h->g.adj, h->nn, h->nn, 1, 1, s);
             h->stage_d.alloc((size_t)h->ne * (h->order == 1 ? kLapStrideP1 : kLapStrideP2));
@@ -541,19 +547,19 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
     for (int k = 0; k < K; k++) {
         const int64_t n0 = h->cut[k], n1 = h->cut[k + 1], e0 = h->ecut[k], e1 = h->ecut[k + 1];
         if (ns) {
-            launch_ns_record(h->xyz.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab, vd_ns, (float)h->prm.density,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab, vd_ns, (float)h->prm.density,
                              h->stage_f.p, h->d_err.p, s, lc, e0, e1);
             if (h->gn_on)
-                launch_gn_elem(h->xyz.p, h->conn.p, h->ne, du, h->gn, h->prm.linearization, h->stage_gn.p, h->d_err.p,
+                launch_gn_elem(h->xyz.p, h->geo.p, h->conn.p, h->ne, du, h->gn, h->prm.linearization, h->stage_gn.p, h->d_err.p,
                                s, lc, e0, e1, h->outflow());
         } else {
             if (mlp && e1 > e0) {  // the points of elements [e0, e1): QPs [e0 nq, e1 nq)
-                launch_hyper_invariants(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p, s,
+                launch_hyper_invariants(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p, s,
                                         lc, e0, e1);
                 launch_mlp_qp(h->mlp, h->law, h->qp_inv.p + 4 * e0 * nq, (e1 - e0) * nq, h->qp_der.p + e0 * nq,
                               h->qp_fb.p + e0 * nq, h->d_fb.p, h->d_err.p, s, lc);
             }
-            launch_hyper_elem(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p,
+            launch_hyper_elem(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p,
                               res && du != nullptr, h->d_err.p, s, lc, e0, e1);
         }
         if (ns) {
@@ -738,11 +744,11 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
                             h->d_err.p, s, lc);
         } else if (prob == FEDD_NAVIER_STOKES) {
             nd = 34;
-            launch_ns_record(h->xyz.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
                              h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density), (float)h->prm.density,
                              h->stage_f.p, h->d_err.p, s, lc);
             if (h->gn_on)
-                launch_gn_elem(h->xyz.p, h->conn.p, h->ne, du, h->gn, h->prm.linearization, h->stage_gn.p, h->d_err.p,
+                launch_gn_elem(h->xyz.p, h->geo.p, h->conn.p, h->ne, du, h->gn, h->prm.linearization, h->stage_gn.p, h->d_err.p,
                                s, lc, 0, -1, h->outflow());
         } else {
             nd = 30;
@@ -750,7 +756,7 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
             const uint8_t *qfb = nullptr;
             if (h->law.kind == kLawMLP) {
                 if (!h->has_mlp) FEDD_FAIL(FEDD_ERR_STATE, "surrogate requested but no network set");
-                launch_hyper_invariants(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p, s,
+                launch_hyper_invariants(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p, s,
                                         lc);
                 FEDD_CUDA(cudaMemsetAsync(h->d_fb.p, 0, sizeof(int), s));
                 launch_mlp_qp(h->mlp, h->law, h->qp_inv.p, h->ne * h->htab.nq, h->qp_der.p, h->qp_fb.p, h->d_fb.p, h->d_err.p, s,
@@ -758,7 +764,7 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
                 qpd = h->qp_der.p;
                 qfb = h->qp_fb.p;
             }
-            launch_hyper_elem(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p, du != nullptr,
+            launch_hyper_elem(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p, du != nullptr,
                               h->d_err.p, s, lc);
         }
         if (count == 0) return;
@@ -853,7 +859,7 @@ fedd_status fedd_qp_invariants(fedd_assembler *h, const double *u, float *out) {
         inv.alloc((size_t)h->ne * h->htab.nq * 4);
         LaunchCounter lc;
         FEDD_CUDA(cudaMemsetAsync(h->d_err.p, 0, sizeof(int), s));
-        launch_hyper_invariants(h->xyz.p, h->conn.p, h->ne, du.p, h->law, h->htab, inv.p, h->d_err.p, s, lc);
+        launch_hyper_invariants(h->geo.p, h->conn.p, h->ne, du.p, h->law, h->htab, inv.p, h->d_err.p, s, lc);
         FEDD_CUDA(cudaMemcpyAsync(out, inv.p, inv.n * sizeof(float), cudaMemcpyDeviceToHost, s));
         read_dev_error(h, s);
     });
@@ -1139,7 +1145,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
                 launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, h->stage_d.p,
                                 h->d_err.p, s, lc, e0, e1);
             } else if (prob == FEDD_NAVIER_STOKES) {
-                launch_ns_record(h->xyz.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
+                launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
                                  (float)(h->prm.viscosity * h->prm.density), (float)h->prm.density, h->stage_f.p,
                                  h->d_err.p, s, lc, e0, e1);
             } else {
@@ -1148,7 +1154,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
                 if (h->law.kind == kLawMLP) {
                     if (!h->has_mlp) FEDD_FAIL(FEDD_ERR_STATE, "surrogate requested but no network set");
                     const int nq = h->htab.nq;
-                    launch_hyper_invariants(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p,
+                    launch_hyper_invariants(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, h->qp_inv.p, h->d_err.p,
                                             s, lc, e0, e1);
                     FEDD_CUDA(cudaMemsetAsync(h->d_fb.p, 0, sizeof(int), s));
                     launch_mlp_qp(h->mlp, h->law, h->qp_inv.p + 4 * e0 * nq, count * nq, h->qp_der.p + e0 * nq,
@@ -1156,7 +1162,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
                     qpd = h->qp_der.p;
                     qfb = h->qp_fb.p;
                 }
-                launch_hyper_elem(h->xyz.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p,
+                launch_hyper_elem(h->geo.p, h->conn.p, h->ne, du, h->law, h->htab, qpd, qfb, h->stage_f.p,
                                   du != nullptr, h->d_err.p, s, lc, e0, e1);
             }
             double *sK = scratch, *sr = scratch + (size_t)count * nd * nd;

@@ -89,6 +89,13 @@ __device__ __forceinline__ double geometry_fp64(const double *__restrict__ xyz, 
     return det;
 }
 
+// element e of the geometry table (launch_geometry): B^-1 into Bi, returns det B
+__device__ __forceinline__ float load_geometry(const float *__restrict__ geo, int64_t ne, int64_t e, float *Bi) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) Bi[k] = __ldg(geo + k * ne + e);
+    return __ldg(geo + 9 * ne + e);
+}
+
 __device__ __forceinline__ float ld_nc(const float *p) { return __ldg(p); }
 
 // streaming (evict-first) store of the write-once CSR values

@@ -18,7 +18,7 @@
 //
 // One warp per element, elements taken in batches of 32 per warp; lane
 // 3 b + l owns column (b, l) of the dense 30 x 30 matrix and row (b, l) of
-// the residual.  Geometry is FP64, one element of the batch per lane; the
+// the residual.  The geometry comes from the mesh's table, formed in FP64; the
 // rest is FP32.
 #include <cmath>
 
@@ -34,7 +34,6 @@ struct GNTab {
     float w15[15];
     float d15[15][10][3];
 };
-__constant__ GNTab c_gn;
 
 constexpr int kGNWarps = 4;
 
@@ -98,16 +97,17 @@ struct __align__(16) GNWarpSmem {
     float sF[15][36];       // Newton points: F_a^k at index 3 a + k (rows 16-byte aligned)
 };
 
-__global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const double *__restrict__ xyz,
+__global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__restrict__ geo,
                                                           const int32_t *__restrict__ conn, int64_t ne,
                                                           const double *__restrict__ u, ViscLaw L, int newton,
-                                                          float *stage, int *err, int64_t e_begin, int64_t e_end) {
+                                                          float *stage, int *err, int64_t e_begin, int64_t e_end,
+                                                          const __grid_constant__ GNTab rules) {
     __shared__ GNWarpSmem smem[kGNWarps];
     // the rule tables in shared memory: phase 1 reads a different point per
     // lane, which constant memory would serialise
     __shared__ GNTab tab;
     for (int t = threadIdx.x; t < (int)(sizeof(GNTab) / sizeof(float)); t += blockDim.x)
-        reinterpret_cast<float *>(&tab)[t] = reinterpret_cast<const float *>(&c_gn)[t];
+        reinterpret_cast<float *>(&tab)[t] = reinterpret_cast<const float *>(&rules)[t];
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     GNWarpSmem &S = smem[w];
@@ -118,14 +118,10 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const double *__re
     const float c0a = cy2 ? powf(L.prm[0], L.prm[4]) : 0.0f;
     for (int64_t e0 = e_begin + ((int64_t)blockIdx.x * kGNWarps + w) * 32; e0 < e_end;
          e0 += (int64_t)gridDim.x * kGNWarps * 32) {
-        // FP64 geometry of a batch of 32 elements, one element per lane (the
-        // FP64 pipe is narrow: one lane per element per warp would occupy it
-        // 32 times as long)
+        // geometry of a batch of 32 elements, one element per lane
         if (e0 + lane < e_end) {
-            int32_t v[4];
-            for (int k = 0; k < 4; k++) v[k] = conn[(int64_t)k * ne + e0 + lane];
             float gB[9];
-            const float gdet = fabsf(d2f_rn(geometry_fp64(xyz, v[0], v[1], v[2], v[3], gB)));
+            const float gdet = fabsf(load_geometry(geo, ne, e0 + lane, gB));
             if (!(gdet > 0.0f) || !isfinite(gdet)) set_dev_error(err, kDevBadDet);
 #pragma unroll
             for (int k = 0; k < 9; k++) S.sgeo[lane][k] = gB[k];
@@ -289,7 +285,7 @@ __global__ void k_gn_dense_add(const float *__restrict__ stage, int64_t first, i
         re[e * 34 + (k - 900)] += cuu * (double)S[kGNRes + (k - 900)];  // the viscous residual is part of ANB_uu u
 }
 
-void upload_gn_tables(cudaStream_t s) {
+GNTab make_gn_tables() {
     GNTab t{};
     Rule r5 = make_rule(5), r15 = make_rule(15);
     for (int q = 0; q < 5; q++) {
@@ -306,7 +302,7 @@ void upload_gn_tables(cudaStream_t s) {
         for (int a = 0; a < 10; a++)
             for (int c = 0; c < 3; c++) t.d15[q][a][c] = (float)d[3 * a + c];
     }
-    FEDD_CUDA(cudaMemcpyToSymbolAsync(c_gn, &t, sizeof t, 0, cudaMemcpyHostToDevice, s));
+    return t;
 }
 
 // ---- outflow Neumann boundary term ----------------------------------------
@@ -467,14 +463,14 @@ __global__ void __launch_bounds__(128) k_gn_outflow(const double *__restrict__ x
 
 }  // namespace
 
-void launch_gn_elem(const double *xyz, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
+void launch_gn_elem(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
                     int newton, float *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin,
                     int64_t e_end, const GNOutflow &outflow) {
-    upload_gn_tables(s);
+    static const GNTab rules = make_gn_tables();
     if (e_end < 0) e_end = ne;
     if (e_end <= e_begin) return;
     k_gn_elem<<<(unsigned)ceil_div(e_end - e_begin, 32 * kGNWarps), 32 * kGNWarps, 0, s>>>(
-        xyz, conn, ne, u, law, newton, stage, d_err, e_begin, e_end);
+        geo, conn, ne, u, law, newton, stage, d_err, e_begin, e_end, rules);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
     if (outflow.n > 0) {

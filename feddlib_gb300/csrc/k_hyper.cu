@@ -14,8 +14,8 @@
 //                  + sum_f 2 psi_4f (a_f.G_a)(a_f.G_b))
 //                  + (psi_J / J) (c_a,i c_b,j - c_b,i c_a,j)
 //     D_1 = 2 F G,  D_J = c = cof(F) G,  D_4f = 2 (F a_f)(a_f . G).
-// Geometry (B, det B, cofactors) is computed in FP64, one thread per
-// element; everything else is FP32.
+// The geometry (B^-1, det B) comes from the mesh's table, formed in FP64;
+// everything else is FP32.
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
@@ -25,7 +25,6 @@ namespace fedd {
 namespace {
 
 constexpr int kWarps = 4;
-__constant__ HyperTables c_htab;
 
 // ---- laws ----------------------------------------------------------------
 __device__ __forceinline__ void nh_matrix(int kind, float mu, float lam, float J, QPDerivs &d) {
@@ -103,7 +102,7 @@ __device__ __forceinline__ void cof3(const float *F, float *C) {
 
 // ---- element stage ----------------------------------------------------
 // One warp per element, elements taken in batches of 32 per warp:
-//   phase 1  FP64 geometry, one element of the batch per lane;
+//   phase 1  the geometry table's entries, one element of the batch per lane;
 // then for each element of the batch:
 //   phase Q  lane q < nq: F_q, cof F_q and the law's derivatives at F_q,
 //            folded with the weight w_q det B into the scalars below;
@@ -264,12 +263,13 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
 // that one; without the bound the register allocation of these instances
 // drifts between 72 and 160 with unrelated edits.
 template <int LAW, bool HAS_U>
-__global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_elem(const double *__restrict__ xyz,
+__global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_elem(const float *__restrict__ geo,
                                                             const int32_t *__restrict__ conn, int64_t ne,
                                                             const double *__restrict__ u, LawParams L,
                                                             const QPDerivs *__restrict__ qpd,
                                                             const uint8_t *__restrict__ qpfb, float *stage,
-                                                            int want_res, int *err, int64_t e_begin, int64_t e_end) {
+                                                            int want_res, int *err, int64_t e_begin, int64_t e_end,
+                                                            const __grid_constant__ HyperTables tab) {
     constexpr bool kFibre = (LAW == kLawAniso || LAW == kLawMLP || LAW == kLawMLPF);
     __shared__ __align__(16) float sdphi[5][36];  // per point: grad_ref phi of the 10 nodes, zero padded
     __shared__ float sw[5];
@@ -277,12 +277,12 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
     __shared__ __align__(16) float sU[kWarps][2][36];  // nodal u of the element pair of phase Q
     __shared__ __align__(16) float sBuf[kWarps][kImage + 5 * kQS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nq = c_htab.nq;
+    const int nq = tab.nq;
     for (int i = threadIdx.x; i < 5 * 36; i += blockDim.x) {
         const int q = i / 36, k = i - 36 * q;
-        (&sdphi[0][0])[i] = (q < nq && k < 30) ? (&c_htab.dphi[0][0][0])[30 * q + k] : 0.0f;
+        (&sdphi[0][0])[i] = (q < nq && k < 30) ? (&tab.dphi[0][0][0])[30 * q + k] : 0.0f;
     }
-    if (threadIdx.x < 5) sw[threadIdx.x] = (int)threadIdx.x < nq ? c_htab.w[threadIdx.x] : 0.0f;
+    if (threadIdx.x < 5) sw[threadIdx.x] = (int)threadIdx.x < nq ? tab.w[threadIdx.x] : 0.0f;
     if (lane < 12) sU[w][lane / 6][30 + lane % 6] = 0.0f;
     __syncthreads();
 
@@ -302,11 +302,11 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
 
     for (int64_t e0 = e_begin + ((int64_t)blockIdx.x * kWarps + w) * 32; e0 < e_end;
          e0 += (int64_t)gridDim.x * kWarps * 32) {
-        {  // phase 1: FP64 geometry, one element per lane
+        {  // phase 1: geometry, one element per lane
             int64_t e = e0 + lane;
             if (e < e_end) {
                 float Bi[9];
-                float det = d2f_rn(geometry_fp64(xyz, conn[e], conn[ne + e], conn[2 * ne + e], conn[3 * ne + e], Bi));
+                const float det = load_geometry(geo, ne, e, Bi);
 #pragma unroll
                 for (int k = 0; k < 9; k++) sBi[w][lane][k] = Bi[k];
                 // det B, times the element's E_e / E when a modulus field is set (the
@@ -621,14 +621,13 @@ __global__ void __launch_bounds__(256) k_hyper_rows(const int64_t *__restrict__ 
 }
 
 // ---- surrogate path: invariants at every quadrature point ---------------
-__global__ void k_hyper_invariants(const double *__restrict__ xyz, const int32_t *__restrict__ conn, int64_t ne,
+__global__ void k_hyper_invariants(const float *__restrict__ geo, const int32_t *__restrict__ conn, int64_t ne,
                                    const double *__restrict__ u, LawParams L, float *inv, int *err, int64_t e_begin,
-                                   int64_t e_end) {
+                                   int64_t e_end, const __grid_constant__ HyperTables tab) {
     int64_t e = e_begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= e_end) return;
     float Bi[9];
-    float det = d2f_rn(geometry_fp64(xyz, conn[e], conn[ne + e], conn[2 * ne + e], conn[3 * ne + e], Bi));
-    (void)det;
+    load_geometry(geo, ne, e, Bi);
     float ue[30];
 #pragma unroll
     for (int a = 0; a < 10; a++) {
@@ -636,7 +635,7 @@ __global__ void k_hyper_invariants(const double *__restrict__ xyz, const int32_t
 #pragma unroll
         for (int i = 0; i < 3; i++) ue[3 * a + i] = u ? d2f_rn(u[3 * (int64_t)node + i]) : 0.0f;
     }
-    const int nq = c_htab.nq;
+    const int nq = tab.nq;
     for (int q = 0; q < nq; q++) {
         float Hr[9];
 #pragma unroll
@@ -645,7 +644,7 @@ __global__ void k_hyper_invariants(const double *__restrict__ xyz, const int32_t
             for (int c = 0; c < 3; c++) {
                 float h = 0.0f;
 #pragma unroll
-                for (int a = 0; a < 10; a++) h = fmaf(ue[3 * a + i], c_htab.dphi[q][a][c], h);
+                for (int a = 0; a < 10; a++) h = fmaf(ue[3 * a + i], tab.dphi[q][a][c], h);
                 Hr[3 * i + c] = h;
             }
         float F[9];
@@ -795,10 +794,6 @@ __global__ void k_law_eval(LawParams L, MLPDev m, int use_mlp, int64_t n, const 
 }
 
 // ---- launchers --------------------------------------------------------------
-static void upload_htab(const HyperTables &tab, cudaStream_t s) {
-    FEDD_CUDA(cudaMemcpyToSymbolAsync(c_htab, &tab, sizeof tab, 0, cudaMemcpyHostToDevice, s));
-}
-
 static int sm_count() {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
@@ -806,11 +801,10 @@ static int sm_count() {
     return n > 0 ? n : 1;
 }
 
-void launch_hyper_elem(const double *xyz, const int32_t *conn, int64_t ne, const double *u, const LawParams &law,
+void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const double *u, const LawParams &law,
                        const HyperTables &tab, const QPDerivs *qpd, const uint8_t *qp_fallback, float *stage,
                        int want_res, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin,
                        int64_t e_end) {
-    upload_htab(tab, s);
     if (e_end < 0) e_end = ne;
     int64_t warps = (e_end - e_begin + 31) / 32;
     unsigned grid = (unsigned)std::min<int64_t>((warps + kWarps - 1) / kWarps, (int64_t)sm_count() * 16);
@@ -819,11 +813,11 @@ void launch_hyper_elem(const double *xyz, const int32_t *conn, int64_t ne, const
 #define FEDD_HYPER(LAWK)                                                                                 \
     do {                                                                                                 \
         if (hu)                                                                                          \
-            k_hyper_elem<LAWK, true><<<grid, 32 * kWarps, 0, s>>>(xyz, conn, ne, u, law, qpd, qp_fallback, \
-                                                                  stage, want_res, d_err, e_begin, e_end); \
+            k_hyper_elem<LAWK, true><<<grid, 32 * kWarps, 0, s>>>(geo, conn, ne, u, law, qpd, qp_fallback, \
+                                                                  stage, want_res, d_err, e_begin, e_end, tab); \
         else                                                                                             \
-            k_hyper_elem<LAWK, false><<<grid, 32 * kWarps, 0, s>>>(xyz, conn, ne, u, law, qpd, qp_fallback, \
-                                                                   stage, want_res, d_err, e_begin, e_end); \
+            k_hyper_elem<LAWK, false><<<grid, 32 * kWarps, 0, s>>>(geo, conn, ne, u, law, qpd, qp_fallback, \
+                                                                   stage, want_res, d_err, e_begin, e_end, tab); \
     } while (0)
     switch (law.kind) {
     case kLawSKR2: FEDD_HYPER(kLawSKR2); break;
@@ -856,14 +850,13 @@ void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr
 }
 
 
-void launch_hyper_invariants(const double *xyz, const int32_t *conn, int64_t ne, const double *u,
+void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, const double *u,
                              const LawParams &law, const HyperTables &tab, float *inv, int *d_err, cudaStream_t s,
                              LaunchCounter &lc, int64_t e_begin, int64_t e_end) {
-    upload_htab(tab, s);
     if (e_end < 0) e_end = ne;
     if (e_end <= e_begin) return;
-    k_hyper_invariants<<<ceil_div(e_end - e_begin, 128), 128, 0, s>>>(xyz, conn, ne, u, law, inv, d_err, e_begin,
-                                                                        e_end);
+    k_hyper_invariants<<<ceil_div(e_end - e_begin, 128), 128, 0, s>>>(geo, conn, ne, u, law, inv, d_err, e_begin,
+                                                                        e_end, tab);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

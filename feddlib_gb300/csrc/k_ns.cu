@@ -12,7 +12,7 @@
 //   N_ab  = sum_{c,k} uT[c][k] T[c][a][b][k], uT = |det B| B^-1 u_k
 //   W_(ai)(bj) = sum_m g[j][m][i] R[a][b][m],  g = |det B| grad u at vertex m
 //   Bd_p(bd) = sum_c Bs[d][c] Y[b][p][c],     Bs = |det B| B^-1
-// A record kernel (one thread per element, FP64 geometry) writes these
+// A record kernel (one thread per element) writes these
 // coefficients; the row kernels (one warp per node) contract them for the
 // node's row and accumulate in shared memory, then write each CSR value once.
 #include "kernels.cuh"
@@ -54,8 +54,7 @@ __constant__ float c_dv[4][10][3];
 //   X_e = (uT[c][k] at kk = 10 c + k for c < 3, k < 10; Gs[s] at kk = 30 + s)
 //   Y   = (rho T[c][a][b][k]; nu rho KS[a][b][s])
 // is a GEMM of (elements x 36) by (36 x 100), K padded to 40 and N to 112.
-// One kernel computes each element's record (one thread per element, FP64
-// geometry) and, for every tile of 128 elements (M = 128, element i of the
+// One kernel computes each element's record (one thread per element) and, for every tile of 128 elements (M = 128, element i of the
 // tile in TMEM lane i), that tile's NA: the threads split X into TF32 hi +
 // lo parts and write them to shared memory as K-major operands, one thread
 // issues tcgen05.mma kind::tf32 for hi hi + hi lo + lo hi (5 K steps of 8,
@@ -105,7 +104,7 @@ __device__ __forceinline__ bool group_sync_or(int g, bool v) {
 }
 
 // elements [e_begin, e_end)
-__global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const double *__restrict__ xyz, const int32_t *__restrict__ conn2,
+__global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__restrict__ geo, const int32_t *__restrict__ conn2,
                                                              const int32_t *__restrict__ conn1, int64_t ne,
                                                              const double *__restrict__ u, const double *__restrict__ p,
                                                              float *rec, int *err, int64_t e_begin, int64_t e_end,
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const double *__re
         const int64_t e_lane = e_begin + tile * kRecTile + gt;
         const int64_t e = e_lane < e_end ? e_lane : e_end - 1;
         float Bi[9];
-        const float det = d2f_rn(geometry_fp64(xyz, conn2[e], conn2[ne + e], conn2[2 * ne + e], conn2[3 * ne + e], Bi));
+        const float det = load_geometry(geo, ne, e, Bi);
         if (!(det > 0.0f) && !(det < 0.0f)) set_dev_error(err, kDevBadDet);
         const float ad = fabsf(det);
         float ue[30];
@@ -790,7 +789,7 @@ void ns_upload_tables(const NSTables &t, float **d_tables) {
 
 }
 
-void launch_ns_record(const double *xyz, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
+void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
                       const double *p, const float *d_tables, float visc_dens, float dens, float *rec, int *d_err,
                       cudaStream_t s, LaunchCounter &lc, int64_t e_begin, int64_t e_end) {
     if (e_end < 0) e_end = ne;
@@ -799,7 +798,7 @@ void launch_ns_record(const double *xyz, const int32_t *conn2, const int32_t *co
     // persistent CTAs, one per SM (shared memory, all 512 TMEM columns)
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)kRecTile * kRecGroups), (int64_t)sm_count_ns());
     FEDD_CUDA(cudaFuncSetAttribute(k_ns_record, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmem));
-    k_ns_record<<<grid, kRecThreads, kRecSmem, s>>>(xyz, conn2, conn1, ne, u, p, rec, d_err, e_begin, e_end, d_tables,
+    k_ns_record<<<grid, kRecThreads, kRecSmem, s>>>(geo, conn2, conn1, ne, u, p, rec, d_err, e_begin, e_end, d_tables,
                                                   visc_dens, dens);
     FEDD_CUDA(cudaGetLastError());
     lc.n += 1;

@@ -83,17 +83,21 @@ struct LaunchCounter {
     int64_t n = 0;
 };
 
+// Element geometry table, ten planes of ne floats: B^-1 row-major (0-8) and
+// det B (9), exactly geometry_fp64 rounded to FP32.  Built once per mesh.
+void launch_geometry(const double *xyz, const int32_t *conn, int64_t ne, float *geo, cudaStream_t s);
+
 // The element-stage launchers take an element range [e_begin, e_end) (e_end
 // -1: ne); ne stays the stride of the connectivity arrays.
 // hyperelastic / elasticity
-void launch_hyper_elem(const double *xyz, const int32_t *conn, int64_t ne, const double *u, const LawParams &law,
+void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const double *u, const LawParams &law,
                        const HyperTables &tab, const QPDerivs *qpd, const uint8_t *qp_fallback, float *stage,
                        int want_res, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                        int64_t e_end = -1);
 void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr, double *vals, double *res,
                        int64_t nnodes, cudaStream_t s, LaunchCounter &lc,
                        int64_t n_begin = 0);
-void launch_hyper_invariants(const double *xyz, const int32_t *conn, int64_t ne, const double *u,
+void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, const double *u,
                              const LawParams &law, const HyperTables &tab, float *inv, int *d_err, cudaStream_t s,
                              LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);
 void launch_mlp_qp(const MLPDev &m, const LawParams &law, const float *inv, int64_t nqp, QPDerivs *out,
@@ -106,7 +110,7 @@ void launch_hyper_dense(const float *stage, int64_t first, int64_t count, double
 
 // Navier-Stokes
 void ns_upload_tables(const NSTables &t, float **d_tables);
-void launch_ns_record(const double *xyz, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
+void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
                       const double *p, const float *d_tables, float visc_dens, float dens, float *rec, int *d_err,
                       cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);
 // per velocity-row node: first incidence, vertex P1 node, neighbour and
@@ -185,7 +189,7 @@ struct GNOutflow {
 // Viscous part (stress term, and its derivative with Newton) of every
 // element into the element stage (kGNStride floats per element), then the
 // outflow Neumann term of the flagged elements into their residual rows.
-void launch_gn_elem(const double *xyz, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
+void launch_gn_elem(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
                     int newton, float *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                     int64_t e_end = -1, const GNOutflow &outflow = GNOutflow{});
 void launch_gn_dense(const float *stage, int64_t first, int64_t count, double *Ke, double *re, cudaStream_t s,
