@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <unordered_map>
 
 #include "kernels.cuh"
@@ -18,6 +19,9 @@ struct fedd_assembler {
     fedd_params prm{};
     int order = 2, npe = 10;
     int64_t nn = 0, ne = 0, nn_p = 0;
+    // the arrays whose sizes the mesh gives, and those whose sizes the pattern
+    // gives; the members below view them
+    Arena mesh_mem, pattern_mem;
     DBuf<double> xyz;
     DBuf<int32_t> conn, conn_p;
     DBuf<float> geo;        // B^-1 and det B of every element (launch_geometry)
@@ -34,7 +38,7 @@ struct fedd_assembler {
     DBuf<float> stage_f;
     DBuf<double> stage_d;
     DBuf<double> lap_tab;
-    float *ns_tab = nullptr;
+    DBuf<float> ns_tab;
     HyperTables htab{};
     LawParams law{};
     // surrogate
@@ -93,7 +97,6 @@ struct fedd_assembler {
     std::vector<cudaEvent_t> ev;  // kProfCalls * kProfStages * 2
     std::vector<std::string> stage_names;
     ~fedd_assembler() {
-        if (ns_tab) cudaFree(ns_tab);
         for (auto e : ev) cudaEventDestroy(e);
         for (auto e : chunk_ev)
             if (e) cudaEventDestroy(e);
@@ -126,13 +129,6 @@ template <class F> fedd_status guarded(fedd_assembler *h, F &&f) {
         if (h) h->err = "unexpected exception";
         return FEDD_ERR_CUDA;
     }
-}
-
-std::vector<int32_t> to_soa(const int32_t *aos, int64_t ne, int npe) {
-    std::vector<int32_t> s((size_t)ne * npe);
-    for (int64_t e = 0; e < ne; e++)
-        for (int a = 0; a < npe; a++) s[(size_t)a * ne + e] = aos[(size_t)e * npe + a];
-    return s;
 }
 
 int quad_points(const fedd_assembler *h) {
@@ -251,7 +247,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         const float vd = h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density);
         const float dn = (float)h->prm.density;
         stage(h, "ns_record", s, [&] {
-            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab, vd, dn, h->stage_f.p,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab.p, vd, dn, h->stage_f.p,
                              h->d_err.p, s, lc);
         });
         if (h->gn_on)
@@ -262,7 +258,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         // with a verified vertex map the velocity-row warps of the vertices
         // assemble the pressure rows as well
         stage(h, "ns_vel_rows", s, [&] {
-            launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
+            launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab.p, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
                                v00, v01, res ? ru : nullptr, vd, dn, h->prm.linearization, jac, h->g.max_adj,
                                h->max_padj, h->ns_fused ? h->vmap.p : nullptr, h->csr[2].rowptr.p, v10,
                                res ? rp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, 0, -1, h->work.p,
@@ -270,7 +266,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         });
         if (!h->ns_fused)
             stage(h, "ns_pres_rows", s, [&] {
-                launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab, h->csr[2].rowptr.p, v10, res ? rp : nullptr, jac,
+                launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, v10, res ? rp : nullptr, jac,
                                     h->gp.max_adj, s, lc, h->coeff);
             });
         break;
@@ -338,78 +334,169 @@ fedd_status fedd_create(const fedd_mesh *mesh, const fedd_params *params, int de
         h->nn = mesh->num_nodes;
         h->ne = mesh->num_elements;
         cudaStream_t s = 0;
-        h->d_err.alloc(1);
-        h->d_err.zero(s);
-        // device-resident meshes are copied and transposed on the device
-        const bool dev_mesh = mesh->flags & FEDD_MESH_DEVICE;
-        auto load_conn = [&](DBuf<int32_t> &dst, const int32_t *src, int npe) {
-            if (dev_mesh) {
-                dst.alloc((size_t)h->ne * npe);
-                device_aos_to_soa(src, h->ne, npe, dst.p, s);
-            } else {
-                std::vector<int32_t> soa = to_soa(src, h->ne, npe);
-                dst.upload(soa.data(), soa.size(), s);
+        const bool ns = prob == FEDD_NAVIER_STOKES, lap = prob == FEDD_LAPLACE;
+        const int64_t nn = h->nn, ne = h->ne, n_inc = ne * h->npe, dofs = lap ? 1 : 3;
+        const int nq = quad_points(h);
+        if (!ns && !lap && nq != 4 && nq != 5) FEDD_FAIL(FEDD_ERR_UNSUPPORTED, "hyperelastic rules: 4 or 5 points");
+        if (ns) h->nn_p = mesh->num_nodes_p;
+        const int64_t nn1 = h->nn_p;
+        // every array whose size the mesh gives: a first pass over the list
+        // adds the sizes up, a second hands the memory out
+        size_t total = 0;
+        bool hand_out = false;
+        auto put = [&](auto &buf, int64_t count) {
+            using T = std::remove_reference_t<decltype(*buf.p)>;
+            if (hand_out)
+                buf.view(h->mesh_mem.take<T>((size_t)count), (size_t)count);
+            else
+                total += Arena::bytes<T>((size_t)count);
+        };
+        auto lay_out = [&] {
+            put(h->d_err, 1);
+            put(h->xyz, nn * 3);
+            put(h->conn, n_inc);
+            put(h->g.inc_ptr, nn + 1);
+            put(h->g.inc, n_inc);
+            put(h->g.slots, n_inc * kSlotStride);
+            put(h->g.adj_ptr, nn + 1);
+            put(h->csr[0].rowptr, nn * dofs + 1);
+            if (lap) {
+                put(h->stage_d, ne * (h->order == 1 ? kLapStrideP1 : kLapStrideP2));
+                put(h->lap_tab, kLapTab);
+                return;
+            }
+            put(h->geo, ne * 10);
+            put(h->stage_f, ne * (ns ? kNSRecord : kElemStride));
+            if (ns) {
+                put(h->conn_p, ne * 4);
+                put(h->gp.inc_ptr, nn1 + 1);
+                put(h->gp.inc, ne * 4);
+                put(h->gp.slots, ne * 4 * kSlotStride);
+                put(h->gp.adj_ptr, nn1 + 1);
+                put(h->padj_ptr, nn + 1);
+                put(h->csr[1].rowptr, nn * 3 + 1);
+                put(h->csr[2].rowptr, nn1 + 1);
+                put(h->csr[3].rowptr, nn1 + 1);
+                put(h->vmap, nn);
+                put(h->ninfo, nn);
+                put(h->work, 1);
+                put(h->ns_tab, kNSTab);
+            } else if (prob == FEDD_ANISO_FIBER) {
+                put(h->qp_inv, ne * nq * 4);
+                put(h->qp_der, ne * nq);
+                put(h->qp_fb, ne * nq);
+                put(h->d_fb, 1);
             }
         };
-        if (dev_mesh) {
-            h->xyz.alloc((size_t)h->nn * 3);
-            FEDD_CUDA(cudaMemcpyAsync(h->xyz.p, mesh->coords, (size_t)h->nn * 3 * sizeof(double),
-                                      cudaMemcpyDeviceToDevice, s));
-        } else {
-            h->xyz.upload(mesh->coords, (size_t)h->nn * 3, s);
+        lay_out();
+        h->mesh_mem.reserve(total);
+        hand_out = true;
+        lay_out();
+        FEDD_CUDA(cudaMemsetAsync(h->d_err.p, 0, sizeof(int), s));
+        // temporaries of this call: a host mesh's element arrays, the build's
+        // counts and its report
+        const bool dev_mesh = mesh->flags & FEDD_MESH_DEVICE;
+        Arena tmp;
+        tmp.reserve(Arena::bytes<GraphStats>(1) + Arena::bytes<int>(1) + graph_scratch(std::max(nn, nn1)) +
+                    (dev_mesh ? 0 : Arena::bytes<int32_t>(n_inc) + Arena::bytes<int32_t>(ns ? ne * 4 : 0)));
+        GraphStats *stats = tmp.take<GraphStats>(1);
+        int *vmap_bad = tmp.take<int>(1);
+        FEDD_CUDA(cudaMemsetAsync(stats, 0, sizeof(GraphStats), s));
+        FEDD_CUDA(cudaMemsetAsync(vmap_bad, 0, sizeof(int), s));
+        // the element arrays as the caller lays them out (the graph build reads
+        // those), and transposed for the element kernels
+        auto load_conn = [&](DBuf<int32_t> &dst, const int32_t *src, int npe) {
+            const int32_t *aos = src;
+            if (!dev_mesh) {
+                int32_t *up = tmp.take<int32_t>((size_t)ne * npe);
+                FEDD_CUDA(cudaMemcpyAsync(up, src, (size_t)ne * npe * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+                aos = up;
+            }
+            device_aos_to_soa(aos, ne, npe, dst.p, s);
+            return aos;
+        };
+        FEDD_CUDA(cudaMemcpyAsync(h->xyz.p, mesh->coords, (size_t)nn * 3 * sizeof(double),
+                                  dev_mesh ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
+        const int32_t *el = load_conn(h->conn, mesh->elements, h->npe);
+        const int32_t *el_p = ns ? load_conn(h->conn_p, mesh->elements_p, 4) : nullptr;
+        // graphs: velocity (or scalar, displacement) rows towards the same
+        // nodes; Navier-Stokes also velocity rows towards pressure columns and
+        // pressure rows towards velocity columns
+        Graph &g = h->g, &gp = h->gp;
+        g.nrow_nodes = g.ncol_nodes = nn;
+        build_incidences(g, ne, el, h->npe, stats, tmp, s);
+        if (ns) {
+            gp.nrow_nodes = nn1;
+            gp.ncol_nodes = nn;
+            build_incidences(gp, ne, el_p, 4, stats, tmp, s);
         }
-        load_conn(h->conn, mesh->elements, h->npe);
-        FEDD_CUDA(cudaStreamSynchronize(s));
-        build_graph(h->g, h->ne, h->conn.p, h->npe, h->nn, h->conn.p, h->npe, h->nn, 0, h->d_err.p, s);
-        // build_graph has checked the node indices
-        if (prob != FEDD_LAPLACE) {
-            h->geo.alloc((size_t)h->ne * 10);
-            launch_geometry(h->xyz.p, h->conn.p, h->ne, h->geo.p, s);
+        count_adjacency(g, true, el, h->npe, g.adj_ptr.p, &stats->max_inc[0], &stats->max_adj[0], stats, tmp, s);
+        if (ns) {
+            count_adjacency(g, false, el_p, 4, h->padj_ptr.p, nullptr, &stats->max_adj[1], stats, tmp, s);
+            count_adjacency(gp, true, el, 10, gp.adj_ptr.p, &stats->max_inc[1], &stats->max_adj[2], stats, tmp, s);
         }
-        if (prob == FEDD_LAPLACE) {
-            build_csr(h->csr[0], h->g.adj_ptr, h->g.adj, h->nn, h->nn, 1, 1, s);
-            h->stage_d.alloc((size_t)h->ne * (h->order == 1 ? kLapStrideP1 : kLapStrideP2));
-            std::vector<double> t;
-            lap_make_tables(h->order, t);
-            h->lap_tab.upload(t.data(), t.size(), s);
-        } else if (prob == FEDD_NAVIER_STOKES) {
-            h->nn_p = mesh->num_nodes_p;
-            load_conn(h->conn_p, mesh->elements_p, 4);
-            FEDD_CUDA(cudaStreamSynchronize(s));
-            build_graph_extra(h->g, h->ne, h->conn_p.p, 4, h->nn_p, 10, h->padj_ptr, h->padj, h->max_padj, h->n_padj,
-                              h->d_err.p, s);
-            build_graph(h->gp, h->ne, h->conn_p.p, 4, h->nn_p, h->conn.p, 10, h->nn, 0, h->d_err.p, s);
-            build_csr(h->csr[0], h->g.adj_ptr, h->g.adj, h->nn, h->nn, 3, 3, s);
-            build_csr(h->csr[1], h->padj_ptr, h->padj, h->nn, h->nn_p, 3, 1, s);
-            build_csr(h->csr[2], h->gp.adj_ptr, h->gp.adj, h->nn_p, h->nn, 1, 3, s);
-            h->ns_fused = build_vertex_map(h->conn.p, h->conn_p.p, h->ne, h->nn, h->nn_p, h->g, h->gp, h->vmap, s);
-            h->ninfo.alloc(h->nn);
-            launch_ns_node_info(h->g, h->padj_ptr.p, h->ns_fused ? h->vmap.p : nullptr, h->ninfo.p, s);
+        const GraphStats gs = read_graph_stats(stats, g.adj_ptr.p + nn, ns ? h->padj_ptr.p + nn : nullptr,
+                                               ns ? gp.adj_ptr.p + nn1 : nullptr, s);
+        // node indices and capacities are checked from here on
+        g.max_inc = gs.max_inc[0];
+        g.max_adj = gs.max_adj[0];
+        g.n_adj = gs.n_adj[0];
+        h->max_padj = gs.max_adj[1];
+        h->n_padj = gs.n_adj[1];
+        gp.max_inc = gs.max_inc[1];
+        gp.max_adj = gs.max_adj[2];
+        gp.n_adj = gs.n_adj[2];
+        auto shape = [&](Csr &c, int64_t nrows, int64_t ncols, int64_t nnz) {
+            c.nrows = nrows;
+            c.ncols = ncols;
+            c.nnz = nnz;
+        };
+        shape(h->csr[0], nn * dofs, nn * dofs, g.n_adj * dofs * dofs);
+        if (ns) {
+            shape(h->csr[1], nn * 3, nn1, h->n_padj * 3);
+            shape(h->csr[2], nn1, nn * 3, gp.n_adj * 3);
             // block (1,1): P1-P1 entries are all zero and FEDDLib inserts only
             // |v| > 1e-13 (FE_def.hpp:1024), so the block is empty
-            h->csr[3].nrows = h->nn_p;
-            h->csr[3].ncols = h->nn_p;
-            h->csr[3].nnz = 0;
-            h->csr[3].rowptr.alloc(h->nn_p + 1);
-            h->csr[3].rowptr.zero(s);
-            h->stage_f.alloc((size_t)h->ne * kNSRecord);
-            h->work.alloc(1);
-            NSTables tabs;
-            make_ns_tables(&tabs);
-            ns_upload_tables(tabs, &h->ns_tab);
+            shape(h->csr[3], nn1, nn1, 0);
+        }
+        const int nblk = ns ? 3 : 1;
+        int64_t n_col[3], n_adj[3] = {g.n_adj, h->n_padj, gp.n_adj};
+        DBuf<int32_t> *adj[3] = {&g.adj, &h->padj, &gp.adj};
+        total = 0;
+        for (int b = 0; b < nblk; b++) {
+            n_adj[b] = std::max<int64_t>(n_adj[b], 1);
+            n_col[b] = std::max<int64_t>(h->csr[b].nnz, 1);
+            total += Arena::bytes<int32_t>(n_adj[b]) + Arena::bytes<int32_t>(n_col[b]);
+        }
+        h->pattern_mem.reserve(total);
+        for (int b = 0; b < nblk; b++) {
+            adj[b]->view(h->pattern_mem.take<int32_t>(n_adj[b]), n_adj[b]);
+            h->csr[b].colind.view(h->pattern_mem.take<int32_t>(n_col[b]), n_col[b]);
+        }
+        fill_adjacency(g, el, h->npe, 0, g.adj_ptr.p, g.adj.p, s);
+        fill_csr(h->csr[0], g.adj_ptr.p, g.adj.p, nn, (int)dofs, (int)dofs, s);
+        if (!lap) launch_geometry(h->xyz.p, h->conn.p, ne, h->geo.p, s);
+        if (lap) {
+            std::vector<double> t;
+            lap_make_tables(h->order, t);
+            FEDD_CUDA(cudaMemcpyAsync(h->lap_tab.p, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+            FEDD_CUDA(cudaStreamSynchronize(s));  // t dies here
+        } else if (ns) {
+            fill_adjacency(g, el_p, 4, 10, h->padj_ptr.p, h->padj.p, s);
+            fill_adjacency(gp, el, 10, 0, gp.adj_ptr.p, gp.adj.p, s);
+            fill_csr(h->csr[1], h->padj_ptr.p, h->padj.p, nn, 3, 1, s);
+            fill_csr(h->csr[2], gp.adj_ptr.p, gp.adj.p, nn1, 1, 3, s);
+            FEDD_CUDA(cudaMemsetAsync(h->csr[3].rowptr.p, 0, (nn1 + 1) * sizeof(int64_t), s));
+            launch_vertex_map(h->conn.p, h->conn_p.p, ne, nn, nn1, g, gp, h->vmap.p, vmap_bad, tmp, s);
+            ns_upload_tables(h->ns_tab.p, s);
+            int bad = 0;
+            FEDD_CUDA(cudaMemcpyAsync(&bad, vmap_bad, sizeof bad, cudaMemcpyDeviceToHost, s));
+            FEDD_CUDA(cudaStreamSynchronize(s));
+            h->ns_fused = bad == 0;
+            launch_ns_node_info(g, h->padj_ptr.p, h->ns_fused ? h->vmap.p : nullptr, h->ninfo.p, s);
         } else {
-            build_csr(h->csr[0], h->g.adj_ptr, h->g.adj, h->nn, h->nn, 3, 3, s);
-            h->stage_f.alloc((size_t)h->ne * kElemStride);
-            int nq = quad_points(h);
-            if (nq != 4 && nq != 5) FEDD_FAIL(FEDD_ERR_UNSUPPORTED, "hyperelastic rules: 4 or 5 points");
             make_hyper_tables(nq, &h->htab);
             set_law(h);
-            if (prob == FEDD_ANISO_FIBER) {
-                h->qp_inv.alloc((size_t)h->ne * nq * 4);
-                h->qp_der.alloc((size_t)h->ne * nq);
-                h->qp_fb.alloc((size_t)h->ne * nq);
-                h->d_fb.alloc(1);
-            }
         }
         FEDD_CUDA(cudaStreamSynchronize(s));
     });
@@ -547,7 +634,7 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
     for (int k = 0; k < K; k++) {
         const int64_t n0 = h->cut[k], n1 = h->cut[k + 1], e0 = h->ecut[k], e1 = h->ecut[k + 1];
         if (ns) {
-            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab, vd_ns, (float)h->prm.density,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab.p, vd_ns, (float)h->prm.density,
                              h->stage_f.p, h->d_err.p, s, lc, e0, e1);
             if (h->gn_on)
                 launch_gn_elem(h->xyz.p, h->geo.p, h->conn.p, h->ne, du, h->gn, h->prm.linearization, h->stage_gn.p, h->d_err.p,
@@ -563,7 +650,7 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
                               res && du != nullptr, h->d_err.p, s, lc, e0, e1);
         }
         if (ns) {
-            launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
+            launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab.p, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
                                dv[0], dv[1], res ? dru : nullptr, vd_ns, (float)h->prm.density, h->prm.linearization,
                                1, h->g.max_adj, h->max_padj, h->ns_fused ? h->vmap.p : nullptr, h->csr[2].rowptr.p,
                                dv[2], res ? drp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, n0, n1,
@@ -584,7 +671,7 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
     }
     if (ns) {
         if (!h->ns_fused)
-            launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab, h->csr[2].rowptr.p, dv[2], res ? drp : nullptr, 1,
+            launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, dv[2], res ? drp : nullptr, 1,
                                 h->gp.max_adj, s, lc, h->coeff);
         FEDD_CUDA(cudaEventRecord(h->chunk_ev[K], s));
         FEDD_CUDA(cudaStreamWaitEvent(cs, h->chunk_ev[K], 0));
@@ -744,7 +831,7 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
                             h->d_err.p, s, lc);
         } else if (prob == FEDD_NAVIER_STOKES) {
             nd = 34;
-            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
+            launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab.p,
                              h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density), (float)h->prm.density,
                              h->stage_f.p, h->d_err.p, s, lc);
             if (h->gn_on)
@@ -773,7 +860,7 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
         if (prob == FEDD_LAPLACE)
             launch_lap_dense(h->stage_d.p, h->order, first, count, tK.p, tr.p, s);
         else if (prob == FEDD_NAVIER_STOKES) {
-            launch_ns_dense(h->stage_f.p, h->ns_tab, first, count,
+            launch_ns_dense(h->stage_f.p, h->ns_tab.p, first, count,
                             h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density), (float)h->prm.density,
                             h->prm.linearization, tK.p, tr.p, s, h->coeff);
             if (h->gn_on) launch_gn_dense(h->stage_gn.p, first, count, tK.p, tr.p, s, h->coeff.uu);
@@ -1145,7 +1232,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
                 launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, h->stage_d.p,
                                 h->d_err.p, s, lc, e0, e1);
             } else if (prob == FEDD_NAVIER_STOKES) {
-                launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab,
+                launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab.p,
                                  (float)(h->prm.viscosity * h->prm.density), (float)h->prm.density, h->stage_f.p,
                                  h->d_err.p, s, lc, e0, e1);
             } else {
@@ -1169,7 +1256,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
             if (prob == FEDD_LAPLACE)
                 launch_lap_dense(h->stage_d.p, h->order, first, count, sK, sr, s);
             else if (prob == FEDD_NAVIER_STOKES)
-                launch_ns_dense(h->stage_f.p, h->ns_tab, first, count, (float)(h->prm.viscosity * h->prm.density),
+                launch_ns_dense(h->stage_f.p, h->ns_tab.p, first, count, (float)(h->prm.viscosity * h->prm.density),
                                 (float)h->prm.density, h->prm.linearization, sK, sr, s, h->coeff);
             else
                 launch_hyper_dense(h->stage_f.p, first, count, sK, sr, s);

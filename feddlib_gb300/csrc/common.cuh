@@ -184,17 +184,26 @@ struct Status {
 
 #define FEDD_FAIL(code, msg) throw ::fedd::Status{code, msg}
 
+// device array: owns its memory, or views a part of an Arena
 template <class T> struct DBuf {
     T *p = nullptr;
     size_t n = 0;
+    bool own = true;
     DBuf() {}
     DBuf(const DBuf &) = delete;
     DBuf &operator=(const DBuf &) = delete;
     ~DBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p && own) cudaFree(p);
         p = nullptr;
         n = 0;
+        own = true;
+    }
+    void view(T *q, size_t count) {
+        release();
+        p = q;
+        n = count;
+        own = false;
     }
     void alloc(size_t count) {
         release();
@@ -213,6 +222,26 @@ template <class T> struct DBuf {
     }
     void zero(cudaStream_t s = 0) {
         if (n) FEDD_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
+    }
+};
+
+// One device allocation handed out piece by piece (256-byte aligned).  An
+// allocation and its release take about 65 us together whatever their size,
+// so arrays of one lifetime share one.
+struct Arena {
+    DBuf<char> mem;
+    size_t used = 0;
+    template <class T> static size_t bytes(size_t count) { return (count * sizeof(T) + 255) & ~(size_t)255; }
+    void reserve(size_t total) {
+        mem.alloc(total);
+        used = 0;
+    }
+    template <class T> T *take(size_t count) {
+        const size_t need = bytes<T>(count);
+        if (used + need > mem.n) FEDD_FAIL(FEDD_ERR_NOMEM, "device arena exhausted");
+        T *q = reinterpret_cast<T *>(mem.p + used);
+        used += need;
+        return q;
     }
 };
 

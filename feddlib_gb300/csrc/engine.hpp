@@ -23,7 +23,6 @@ void basis_dphi(int order, const double *p, double *g);   // Helper::gradPhi, 3D
 //   T[c][a][b][k]  = sum_q w_q phi_a phi_k dc phi_b        (advection)
 //   R[a][b][m]     = sum_q w_q lambda_m phi_a phi_b          (Newton term)
 //   Y[c][p][b]     = sum_q5 w_q psi_p dc phi_b               (divergence)
-//   DV[m][k][c]    = dc phi_k at vertex m                    (grad u at vertices)
 //   WPHI, DQ, PHIQ = weights x basis, reference gradients and basis at the
 //                    15 points (advection evaluated at the quadrature points)
 struct NSTables {
@@ -31,7 +30,6 @@ struct NSTables {
     float T[3][10][10][10];
     float R[10][10][4];
     float Y[3][4][10];
-    float DV[4][10][3];
     // quadrature-point form of the advection term (15-point rule):
     float WPHI[10][16];    // w_q phi_a(q)
     float DQ[10][3][16];   // d_c phi_b(q) (reference gradients)
@@ -64,17 +62,34 @@ struct Graph {
     int64_t n_inc = 0, n_adj = 0;
 };
 
-// Builds incidences of `row_conn` (SoA, npe_row x ne) and the adjacency
-// towards `col_conn` (SoA, npe_col x ne).  Slots land at `slot_off`.
-void build_graph(Graph &g, int64_t ne, const int32_t *row_conn, int npe_row, int64_t nrow_nodes,
-                 const int32_t *col_conn, int npe_col, int64_t ncol_nodes, int slot_off,
-                 int *d_err, cudaStream_t s);
-// Adds a second adjacency (e.g. velocity rows -> pressure columns) that
-// reuses g's incidences: fills adj2/adj2_ptr and slots at slot_off.
-void build_graph_extra(const Graph &g, int64_t ne, const int32_t *col_conn, int npe_col,
-                       int64_t ncol_nodes, int slot_off, DBuf<int64_t> &adj2_ptr,
-                       DBuf<int32_t> &adj2, int &max_adj2, int64_t &n_adj2, int *d_err,
-                       cudaStream_t s);
+// What the graph build reports back in one copy: the device error word, and
+// per incidence graph / adjacency the maxima and totals.
+struct GraphStats {
+    int err;
+    int max_inc[2];
+    int max_adj[3];
+    int64_t n_adj[3];
+};
+
+// The build, in stream order and without a host round trip until
+// read_graph_stats.  Element arrays are num_elements x npe as the caller lays
+// them out; the destination arrays are allocated by the caller (inc:
+// num_elements * npe_row entries); tmp provides graph_scratch bytes.
+//   build_incidences   inc_ptr and inc (in no fixed order yet)
+//   count_adjacency    adj_ptr of the row nodes towards col_conn; the first
+//                      call of a graph (sort) also puts the incidences in order
+//   read_graph_stats   totals from the ends of up to three adj_ptr arrays,
+//                      synchronises, throws on a bad node index or capacity
+//   fill_adjacency     adj, and the slots at byte slot_off
+size_t graph_scratch(int64_t nnodes);
+void build_incidences(Graph &g, int64_t ne, const int32_t *row_conn, int npe_row, GraphStats *st, Arena &tmp,
+                      cudaStream_t s);
+void count_adjacency(const Graph &g, bool sort, const int32_t *col_conn, int npe_col, int64_t *adj_ptr, int *maxinc,
+                     int *maxadj, GraphStats *st, Arena &tmp, cudaStream_t s);
+GraphStats read_graph_stats(GraphStats *st, const int64_t *end0, const int64_t *end1, const int64_t *end2,
+                            cudaStream_t s);
+void fill_adjacency(const Graph &g, const int32_t *col_conn, int npe_col, int slot_off, const int64_t *adj_ptr,
+                    int32_t *adj, cudaStream_t s);
 
 // CSR of a block whose rows are (row node, dr) for dr < dofs_r and whose
 // columns are (adjacent node, dc) for dc < dofs_c, node-wise numbering.
@@ -83,18 +98,19 @@ struct Csr {
     DBuf<int64_t> rowptr;
     DBuf<int32_t> colind;
 };
-void build_csr(Csr &c, const DBuf<int64_t> &adj_ptr, const DBuf<int32_t> &adj, int64_t nrow_nodes,
-               int64_t ncol_nodes, int dofs_r, int dofs_c, cudaStream_t s);
+// fills rowptr and colind (allocated by the caller)
+void fill_csr(const Csr &c, const int64_t *adj_ptr, const int32_t *adj, int64_t nrow_nodes, int dofs_r, int dofs_c,
+              cudaStream_t s);
 
 // Taylor-Hood vertex map: vmap[v] = the P1 node at P2 vertex v (-1 for edge
 // nodes), built from the elements' first four P2 nodes and the P1 element
-// nodes at the same local positions.  Returns true when the map is
+// nodes at the same local positions.  *bad (zero before) stays zero when the map is
 // consistent element by element, one-to-one onto the P1 nodes, no mapped
 // node appears at an edge position, and each mapped vertex's adjacency row in
 // g2 equals its P1 node's row in g1: the velocity-row kernel may then
 // assemble the pressure rows of the vertices as well.
-bool build_vertex_map(const int32_t *conn2, const int32_t *conn1, int64_t ne, int64_t nn2, int64_t nn1,
-                      const Graph &g2, const Graph &g1, DBuf<int32_t> &vmap, cudaStream_t s);
+void launch_vertex_map(const int32_t *conn2, const int32_t *conn1, int64_t ne, int64_t nn2, int64_t nn1,
+                       const Graph &g2, const Graph &g1, int32_t *vmap, int *bad, Arena &tmp, cudaStream_t s);
 
 // For K node ranges [bounds[k], bounds[k + 1]) of g's row nodes (bounds on
 // the host): the largest element index among each range's incidences (-1 for
@@ -108,8 +124,8 @@ void device_aos_to_soa(const int32_t *aos, int64_t ne, int npe, int32_t *soa, cu
 // message slot of handle-less C-ABI calls (per host thread)
 std::string &thread_error();
 
-// exclusive scan helpers (device)
-void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t s);
-void exclusive_scan_i32_to_i64(const int32_t *in, int64_t *out, int64_t n, cudaStream_t s);
+// exclusive scan (device), its block sums from tmp (scan_scratch bytes)
+size_t scan_scratch(int64_t n);
+void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, Arena &tmp, cudaStream_t s);
 
 }  // namespace fedd

@@ -5,25 +5,32 @@
 // addFeBlockMatrix insert every dof pair of every node pair of an element
 // (feddlib/core/FE/FE_def.hpp:1419-1442, 982-1062) and fillComplete sorts the
 // columns and merges duplicates (Matrix_decl.hpp:133-138).  Here: per row
-// node, the union of the column nodes of its incident elements, sorted and
-// made unique by one warp (segmented bitonic sort in shared memory); the
-// scalar CSR follows as node pattern x (dofs_r x dofs_c) blocks.
+// node, the union of the column nodes of its incident elements, made unique
+// by one warp in a shared-memory hash table and put in order by counting
+// ranks; the scalar CSR follows as node pattern x (dofs_r x dofs_c) blocks.
+//
+// The element arrays are read as the caller lays them out (num_elements x
+// npe): the ten column nodes of an incidence are then one or two 32-byte
+// sectors, where the transposed layout touches ten.  Against a bitonic sort
+// of all candidates (240 of a P2 vertex for 65 distinct nodes), run once to
+// count and once to fill, adjacency counting (with the sort of the incidences) went from 210 to 75 us
+// and filling from 267 to 99 us on a 24^3 x 6 mesh in file order (P2
+// rows, P2 columns).
 #include "engine.hpp"
 
 namespace fedd {
 
 namespace {
 
-constexpr int kCand = 1024;  // candidate buffer per warp (>= kMaxIncidence * 10)
-constexpr int kGraphWarps = 4;
+constexpr int kMaxCand = kMaxIncidence * 10;  // candidates of one row node at most
+constexpr int kHash = 512;                    // hash table entries per warp (at most 255 + 32 are ever inserted)
+constexpr int kGraphWarps = 8;
 
 __global__ void k_count_inc(const int32_t *__restrict__ conn, int npe, int64_t ne, int64_t nnodes,
                             int32_t *cnt, int *err) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= ne * npe) return;
-    int a = (int)(t / ne);
-    int64_t e = t - (int64_t)a * ne;
-    int32_t n = conn[(int64_t)a * ne + e];
+    int32_t n = conn[t];
     if (n < 0 || n >= nnodes) {
         set_dev_error(err, kDevMesh);
         return;
@@ -31,149 +38,176 @@ __global__ void k_count_inc(const int32_t *__restrict__ conn, int npe, int64_t n
     atomicAdd(&cnt[n], 1);
 }
 
+// counts each node's cursor down to zero: entry ptr[n] + cursor
 __global__ void k_fill_inc(const int32_t *__restrict__ conn, int npe, int64_t ne, int64_t nnodes,
                            const int64_t *__restrict__ ptr, int32_t *cursor, uint32_t *inc) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= ne * npe) return;
-    int a = (int)(t / ne);
-    int64_t e = t - (int64_t)a * ne;
-    int32_t n = conn[(int64_t)a * ne + e];
+    int32_t n = conn[t];
     if (n < 0 || n >= nnodes) return;
-    int pos = atomicAdd(&cursor[n], 1);
+    const int64_t e = t / npe;
+    const int a = (int)(t - e * npe);
+    int pos = atomicSub(&cursor[n], 1) - 1;
     inc[ptr[n] + pos] = ((uint32_t)e << 4) | (uint32_t)a;
 }
 
-// the fill order above depends on atomic timing: sort each list so that the
-// incidence order (and with it the summation order) is fixed: by the node's
-// local index in the element, then by element, so that a row kernel meets the
-// incidences sharing a local index (and its rows of the reference tables) in
-// one run
+// the fill order above depends on atomic timing: each list is sorted so that
+// the incidence order (and with it the summation order) is fixed: by the
+// node's local index in the element, then by element, so that a row kernel
+// meets the incidences sharing a local index (and its rows of the reference
+// tables) in one run
 __device__ __forceinline__ uint32_t inc_key(uint32_t v) { return ((v & 15u) << 28) | (v >> 4); }
 
-__global__ void k_sort_inc(const int64_t *__restrict__ ptr, uint32_t *inc, int64_t nnodes, int *err,
-                           int *maxinc) {
-    int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (n >= nnodes) return;
-    int64_t b = ptr[n], m = ptr[n + 1] - b;
-    if (m > kMaxIncidence) {
-        set_dev_error(err, kDevCapacity);
-        return;
-    }
-    atomicMax(maxinc, (int)m);
-    uint32_t v[kMaxIncidence];
-    for (int i = 0; i < m; i++) v[i] = inc[b + i];
-    for (int i = 1; i < m; i++) {
-        uint32_t x = v[i];
-        int j = i - 1;
-        while (j >= 0 && inc_key(v[j]) > inc_key(x)) {
-            v[j + 1] = v[j];
-            j--;
-        }
-        v[j + 1] = x;
-    }
-    for (int i = 0; i < m; i++) inc[b + i] = v[i];
-}
-
-// warp-level bitonic sort of buf[0..np) (np a power of two >= 32)
-__device__ void warp_bitonic(int32_t *buf, int np, int lane) {
-    for (int k = 2; k <= np; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < np; i += 32) {
-                int p = i ^ j;
-                if (p > i) {
-                    int32_t x = buf[i], y = buf[p];
-                    bool up = (i & k) == 0;
-                    if ((x > y) == up) {
-                        buf[i] = y;
-                        buf[p] = x;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-}
-
-// gathers the column nodes of node n's incidences, sorts them and makes them
-// unique into uniq[]; returns the number of unique nodes (or -1 on overflow)
-__device__ int node_union(int64_t n, const int64_t *__restrict__ ptr, const uint32_t *__restrict__ inc,
-                          const int32_t *__restrict__ col_conn, int npe_col, int64_t ne, int32_t *buf,
-                          int32_t *uniq, int lane) {
-    int64_t b = ptr[n];
-    int m = (int)(ptr[n + 1] - b);
-    int cnt = m * npe_col;
-    if (cnt > kCand) return -1;
-    int np = 32;
-    while (np < cnt) np <<= 1;
-    for (int i = lane; i < np; i += 32) {
-        int32_t v = 0x7fffffff;
-        if (i < cnt) {
-            int k = i / npe_col, j = i - k * npe_col;
-            uint32_t e = inc[b + k] >> 4;
-            v = col_conn[(int64_t)j * ne + e];
-        }
-        buf[i] = v;
+// one warp sorts its node's m <= 64 incidences (lane k holds entries k and
+// k + 32): every entry's rank is the number of smaller keys (keys differ)
+__device__ __forceinline__ void warp_sort_incidences(uint32_t *inc, int m, int lane) {
+    const uint32_t lo = lane < m ? inc[lane] : 0xffffffffu, hi = lane + 32 < m ? inc[lane + 32] : 0xffffffffu;
+    const uint32_t klo = inc_key(lo), khi = inc_key(hi);
+    int rlo = 0, rhi = 0;
+    for (int t = 0; t < m; t++) {
+        const uint32_t k = __shfl_sync(0xffffffffu, t < 32 ? klo : khi, t & 31);
+        rlo += k < klo;
+        rhi += k < khi;
     }
     __syncwarp();
-    warp_bitonic(buf, np, lane);
+    if (lane < m) inc[rlo] = lo;
+    if (lane + 32 < m) inc[rhi] = hi;
+    __syncwarp();
+}
+
+// per-warp shared memory of the node union
+struct __align__(16) UnionSmem {
+    int32_t key[kHash];       // hash table: node ids, -1 empty
+    int32_t list[256];        // distinct nodes in order of first occurrence (padded to a multiple of 4)
+    uint16_t at[256];         // their places in the table
+    uint8_t rank[kHash];      // place -> position in the sorted adjacency row
+    uint16_t cand[kMaxCand];  // place of every candidate
+};
+
+// Enters the column nodes of a node's m incidences into the hash table key;
+// with LIST also the list of distinct ones and every candidate's place into
+// S (key is S->key then).  Returns
+// the number of distinct nodes, or -1 when they exceed kMaxAdjacency.
+// Negative node ids do not occur: the caller has counted, and so checked,
+// every element array (an array with bad ids is reported before the result
+// is used; its entries are only compared here).
+template <bool LIST>
+__device__ __forceinline__ int node_union(int32_t *key, UnionSmem *S, const uint32_t *__restrict__ inc, int m,
+                                          const int32_t *__restrict__ col_conn, int npe, int lane) {
+    const int cnt = m * npe;
+    int bits = 6;
+    while (bits < 9 && (1 << bits) < 2 * cnt) bits++;
+    const int mask = (1 << bits) - 1;
+    for (int i = lane; i <= mask; i += 32) key[i] = -1;
+    __syncwarp();
     int K = 0;
     for (int base = 0; base < cnt; base += 32) {
-        int i = base + lane;
-        bool f = i < cnt && (i == 0 || buf[i] != buf[i - 1]);
-        unsigned bal = __ballot_sync(0xffffffffu, f);
-        int pos = K + __popc(bal & ((1u << lane) - 1u));
-        if (f && pos < kMaxAdjacency) uniq[pos] = buf[i];
+        const int i = base + lane;
+        bool fresh = false;
+        int32_t v = 0;
+        int h = 0;
+        if (i < cnt) {
+            const int k = i / npe, j = i - k * npe;
+            v = __ldg(col_conn + (int64_t)(inc[k] >> 4) * npe + j);
+            h = (int)(((uint32_t)v * 2654435769u) >> (32 - bits));
+            // at most 255 + 32 of the 512 places are taken, or cnt of 2 cnt
+            for (;;) {
+                const int32_t old = atomicCAS(&key[h], -1, v);
+                fresh = old == -1;
+                if (fresh || old == v) break;
+                h = (h + 1) & mask;
+            }
+            if (LIST) S->cand[i] = (uint16_t)h;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, fresh);
+        if (LIST && fresh) {
+            const int pos = K + __popc(bal & ((1u << lane) - 1u));
+            if (pos < 256) {
+                S->list[pos] = v;
+                S->at[pos] = (uint16_t)h;
+            }
+        }
         K += __popc(bal);
+        if (K > kMaxAdjacency) return -1;
     }
     __syncwarp();
     return K;
 }
 
-__global__ void k_adj_count(const int64_t *__restrict__ ptr, const uint32_t *__restrict__ inc,
-                            const int32_t *__restrict__ col_conn, int npe_col, int64_t ne, int64_t nnodes,
-                            int64_t *cnt, int *err, int *maxadj) {
-    __shared__ int32_t sbuf[kGraphWarps][kCand];
-    __shared__ int32_t suni[kGraphWarps][kMaxAdjacency + 1];
-    int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int64_t n = blockIdx.x * (int64_t)kGraphWarps + w;
-    if (n >= nnodes) return;
-    int K = node_union(n, ptr, inc, col_conn, npe_col, ne, sbuf[w], suni[w], lane);
+// SORT: the first adjacency of a graph also puts its incidences in order
+template <bool SORT>
+__global__ void __launch_bounds__(32 * kGraphWarps) k_adj_count(const int64_t *__restrict__ ptr, uint32_t *inc,
+                                                                const int32_t *__restrict__ col_conn, int npe_col,
+                                                                int64_t nnodes, int64_t *cnt, int *err, int *maxinc,
+                                                                int *maxadj) {
+    __shared__ int32_t key[kGraphWarps][kHash];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t n = blockIdx.x * (int64_t)kGraphWarps + w;
+    if (n > nnodes) return;
+    if (n == nnodes) {  // the scan's last entry
+        if (lane == 0) cnt[n] = 0;
+        return;
+    }
+    const int64_t b = ptr[n];
+    const int64_t m = ptr[n + 1] - b;
+    int K = -1;
+    if (m <= kMaxIncidence) {
+        if (SORT) warp_sort_incidences(inc + b, (int)m, lane);
+        K = node_union<false>(key[w], nullptr, inc + b, (int)m, col_conn, npe_col, lane);
+    }
     if (lane == 0) {
-        if (K < 0 || K > kMaxAdjacency) {
-            set_dev_error(err, kDevCapacity);
-            K = 0;
-        }
-        cnt[n] = K;
-        atomicMax(maxadj, K);
+        if (K < 0) set_dev_error(err, kDevCapacity);
+        cnt[n] = K < 0 ? 0 : K;
+        // the maxima settle after a few nodes: most warps only read them
+        if (SORT && m <= kMaxIncidence && (int)m > *(volatile int *)maxinc) atomicMax(maxinc, (int)m);
+        if (K > *(volatile int *)maxadj) atomicMax(maxadj, K);
     }
 }
 
-__global__ void k_adj_fill(const int64_t *__restrict__ ptr, const uint32_t *__restrict__ inc,
-                           const int32_t *__restrict__ col_conn, int npe_col, int64_t ne, int64_t nnodes,
-                           const int64_t *__restrict__ adj_ptr, int32_t *adj, uint8_t *slots, int slot_off) {
-    __shared__ int32_t sbuf[kGraphWarps][kCand];
-    __shared__ int32_t suni[kGraphWarps][kMaxAdjacency + 1];
-    int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int64_t n = blockIdx.x * (int64_t)kGraphWarps + w;
+__global__ void __launch_bounds__(32 * kGraphWarps) k_adj_fill(const int64_t *__restrict__ ptr,
+                                                               const uint32_t *__restrict__ inc,
+                                                               const int32_t *__restrict__ col_conn, int npe_col,
+                                                               int64_t nnodes, const int64_t *__restrict__ adj_ptr,
+                                                               int32_t *adj, uint8_t *slots, int slot_off) {
+    __shared__ UnionSmem smem[kGraphWarps];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t n = blockIdx.x * (int64_t)kGraphWarps + w;
     if (n >= nnodes) return;
-    int K = node_union(n, ptr, inc, col_conn, npe_col, ne, sbuf[w], suni[w], lane);
-    if (K < 0 || K > kMaxAdjacency) return;
-    int64_t a0 = adj_ptr[n];
-    for (int i = lane; i < K; i += 32) adj[a0 + i] = suni[w][i];
-    int64_t b = ptr[n];
-    int m = (int)(ptr[n + 1] - b);
-    for (int i = lane; i < m * npe_col; i += 32) {
-        int k = i / npe_col, j = i - k * npe_col;
-        uint32_t e = inc[b + k] >> 4;
-        int32_t v = col_conn[(int64_t)j * ne + e];
-        int lo = 0, hi = K - 1;
-        while (lo < hi) {
-            int mid = (lo + hi) >> 1;
-            if (suni[w][mid] < v) lo = mid + 1; else hi = mid;
+    UnionSmem &S = smem[w];
+    const int64_t b = ptr[n];
+    const int m = (int)(ptr[n + 1] - b);
+    const int K = node_union<true>(S.key, &S, inc + b, m, col_conn, npe_col, lane);
+    if (K <= 0) return;
+    // pad the list to whole 16-byte reads with ids above every node's
+    if (lane < 4 && K + lane < 256) S.list[K + lane] = 0x7fffffff;
+    __syncwarp();
+    // every node's position is the number of smaller ids in the list
+    const int64_t a0 = adj_ptr[n];
+    for (int i = lane; i < K; i += 32) {
+        const int32_t v = S.list[i];
+        int r = 0;
+        for (int t = 0; t < K; t += 4) {
+            const int4 x = *reinterpret_cast<const int4 *>(S.list + t);
+            r += (x.x < v) + (x.y < v) + (x.z < v) + (x.w < v);
         }
-        slots[(b + k) * kSlotStride + slot_off + j] = (uint8_t)lo;
+        adj[a0 + r] = v;
+        S.rank[S.at[i]] = (uint8_t)r;
+    }
+    __syncwarp();
+    for (int i = lane; i < m * npe_col; i += 32) {
+        const int k = i / npe_col, j = i - k * npe_col;
+        slots[(b + k) * kSlotStride + slot_off + j] = S.rank[S.cand[i]];
     }
     if (slot_off == 0)  // the row node's local index, for the row kernels' staged slot maps
         for (int k = lane; k < m; k += 32) slots[(b + k) * kSlotStride + kSlotLocal] = (uint8_t)(inc[b + k] & 15u);
+}
+
+// the totals of up to three adjacencies next to the maxima, so that one copy
+// to the host brings everything the build needs
+__global__ void k_collect(GraphStats *st, const int64_t *a0, const int64_t *a1, const int64_t *a2) {
+    if (a0) st->n_adj[0] = *a0;
+    if (a1) st->n_adj[1] = *a1;
+    if (a2) st->n_adj[2] = *a2;
 }
 
 __global__ void k_csr(const int64_t *__restrict__ adj_ptr, const int32_t *__restrict__ adj, int64_t nnodes,
@@ -229,115 +263,89 @@ __global__ void k_scan_add(int64_t *out, const int64_t *boff, int64_t n) {
 }
 
 template <class TIn>
-void scan_impl(const TIn *in, int64_t *out, int64_t n, cudaStream_t s) {
+void scan_impl(const TIn *in, int64_t *out, int64_t n, Arena &tmp, cudaStream_t s) {
     if (n <= 0) return;
     int64_t nb = (n + 1023) / 1024;
     if (nb == 1) {
         k_scan_block<TIn><<<1, 1024, 0, s>>>(in, out, nullptr, n);
         return;
     }
-    DBuf<int64_t> bsum, boff;
-    bsum.alloc(nb);
-    boff.alloc(nb);
-    k_scan_block<TIn><<<(unsigned)nb, 1024, 0, s>>>(in, out, bsum.p, n);
-    scan_impl<int64_t>(bsum.p, boff.p, nb, s);
-    k_scan_add<<<(unsigned)nb, 1024, 0, s>>>(out, boff.p, n);
-    FEDD_CUDA(cudaStreamSynchronize(s));  // temporaries die at scope exit
+    const size_t mark = tmp.used;
+    int64_t *bsum = tmp.take<int64_t>(nb), *boff = tmp.take<int64_t>(nb);
+    k_scan_block<TIn><<<(unsigned)nb, 1024, 0, s>>>(in, out, bsum, n);
+    scan_impl<int64_t>(bsum, boff, nb, tmp, s);
+    k_scan_add<<<(unsigned)nb, 1024, 0, s>>>(out, boff, n);
+    tmp.used = mark;  // whoever takes this memory next uses it behind these kernels on s
 }
 
 }  // namespace
 
-void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t s) {
-    scan_impl<int64_t>(in, out, n, s);
-}
-void exclusive_scan_i32_to_i64(const int32_t *in, int64_t *out, int64_t n, cudaStream_t s) {
-    scan_impl<int32_t>(in, out, n, s);
-}
-
-static int64_t read_i64(const int64_t *d, cudaStream_t s) {
-    int64_t v = 0;
-    FEDD_CUDA(cudaMemcpyAsync(&v, d, sizeof v, cudaMemcpyDeviceToHost, s));
-    FEDD_CUDA(cudaStreamSynchronize(s));
-    return v;
+size_t scan_scratch(int64_t n) {
+    size_t bytes = 0;
+    for (int64_t nb = (n + 1023) / 1024; nb > 1; nb = (nb + 1023) / 1024) bytes += 2 * Arena::bytes<int64_t>(nb);
+    return bytes;
 }
 
-static void check_err(int *d_err, cudaStream_t s, const char *what) {
-    int e = 0;
-    FEDD_CUDA(cudaMemcpyAsync(&e, d_err, sizeof e, cudaMemcpyDeviceToHost, s));
+void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, Arena &tmp, cudaStream_t s) {
+    scan_impl<int64_t>(in, out, n, tmp, s);
+}
+
+size_t graph_scratch(int64_t nnodes) {
+    // incidence counts, then adjacency counts (never at the same time), and the scans over them
+    return Arena::bytes<int64_t>(nnodes + 1) + scan_scratch(nnodes + 1);
+}
+
+void build_incidences(Graph &g, int64_t ne, const int32_t *row_conn, int npe_row, GraphStats *st, Arena &tmp,
+                      cudaStream_t s) {
+    const int64_t nn = g.nrow_nodes, nt = ne * npe_row;
+    const size_t mark = tmp.used;
+    int32_t *cnt = tmp.take<int32_t>(nn + 1);
+    FEDD_CUDA(cudaMemsetAsync(cnt, 0, (nn + 1) * sizeof(int32_t), s));
+    k_count_inc<<<ceil_div(nt, 256), 256, 0, s>>>(row_conn, npe_row, ne, nn, cnt, &st->err);
+    scan_impl<int32_t>(cnt, g.inc_ptr.p, nn + 1, tmp, s);
+    k_fill_inc<<<ceil_div(nt, 256), 256, 0, s>>>(row_conn, npe_row, ne, nn, g.inc_ptr.p, cnt, g.inc.p);
+    FEDD_CUDA(cudaGetLastError());
+    g.n_inc = nt;
+    tmp.used = mark;
+}
+
+void count_adjacency(const Graph &g, bool sort, const int32_t *col_conn, int npe_col, int64_t *adj_ptr, int *maxinc,
+                     int *maxadj, GraphStats *st, Arena &tmp, cudaStream_t s) {
+    const int64_t nn = g.nrow_nodes;
+    const size_t mark = tmp.used;
+    int64_t *cnt = tmp.take<int64_t>(nn + 1);
+    const unsigned nb = ceil_div(nn + 1, kGraphWarps);
+    if (sort)
+        k_adj_count<true><<<nb, 32 * kGraphWarps, 0, s>>>(g.inc_ptr.p, g.inc.p, col_conn, npe_col, nn, cnt, &st->err,
+                                                          maxinc, maxadj);
+    else
+        k_adj_count<false><<<nb, 32 * kGraphWarps, 0, s>>>(g.inc_ptr.p, g.inc.p, col_conn, npe_col, nn, cnt, &st->err,
+                                                           maxinc, maxadj);
+    FEDD_CUDA(cudaGetLastError());
+    scan_impl<int64_t>(cnt, adj_ptr, nn + 1, tmp, s);
+    tmp.used = mark;
+}
+
+GraphStats read_graph_stats(GraphStats *st, const int64_t *end0, const int64_t *end1, const int64_t *end2,
+                            cudaStream_t s) {
+    k_collect<<<1, 1, 0, s>>>(st, end0, end1, end2);
+    FEDD_CUDA(cudaGetLastError());
+    GraphStats h{};
+    FEDD_CUDA(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s));
     FEDD_CUDA(cudaStreamSynchronize(s));
-    if (e == kDevMesh) FEDD_FAIL(FEDD_ERR_MESH, std::string(what) + ": element node index out of range");
-    if (e == kDevCapacity)
-        FEDD_FAIL(FEDD_ERR_CAPACITY, std::string(what) + ": a node exceeds " + std::to_string(kMaxIncidence) +
+    if (h.err == kDevMesh) FEDD_FAIL(FEDD_ERR_MESH, "incidence count: element node index out of range");
+    if (h.err == kDevCapacity)
+        FEDD_FAIL(FEDD_ERR_CAPACITY, "adjacency: a node exceeds " + std::to_string(kMaxIncidence) +
                                          " incident elements or " + std::to_string(kMaxAdjacency) + " neighbours");
-    if (e) FEDD_FAIL(FEDD_ERR_CUDA, std::string(what) + ": device error " + std::to_string(e));
+    if (h.err) FEDD_FAIL(FEDD_ERR_CUDA, "graph build: device error " + std::to_string(h.err));
+    return h;
 }
 
-// node-level adjacency count + fill for a given incidence structure
-static void adjacency(int64_t nnodes, const int64_t *ptr, const uint32_t *inc, int64_t ne, const int32_t *col_conn,
-                      int npe_col, int slot_off, uint8_t *slots, DBuf<int64_t> &adj_ptr, DBuf<int32_t> &adj,
-                      int &max_adj, int64_t &n_adj, int *d_err, cudaStream_t s) {
-    DBuf<int64_t> cnt;
-    DBuf<int> dmax;
-    cnt.alloc(nnodes + 1);
-    cnt.zero(s);
-    dmax.alloc(1);
-    dmax.zero(s);
-    unsigned nb = ceil_div(nnodes, kGraphWarps);
-    k_adj_count<<<nb, 32 * kGraphWarps, 0, s>>>(ptr, inc, col_conn, npe_col, ne, nnodes, cnt.p, d_err, dmax.p);
+void fill_adjacency(const Graph &g, const int32_t *col_conn, int npe_col, int slot_off, const int64_t *adj_ptr,
+                    int32_t *adj, cudaStream_t s) {
+    k_adj_fill<<<ceil_div(g.nrow_nodes, kGraphWarps), 32 * kGraphWarps, 0, s>>>(
+        g.inc_ptr.p, g.inc.p, col_conn, npe_col, g.nrow_nodes, adj_ptr, adj, g.slots.p, slot_off);
     FEDD_CUDA(cudaGetLastError());
-    check_err(d_err, s, "adjacency");
-    adj_ptr.alloc(nnodes + 1);
-    exclusive_scan_i64(cnt.p, adj_ptr.p, nnodes + 1, s);
-    n_adj = read_i64(adj_ptr.p + nnodes, s);
-    int mx = 0;
-    FEDD_CUDA(cudaMemcpyAsync(&mx, dmax.p, sizeof mx, cudaMemcpyDeviceToHost, s));
-    FEDD_CUDA(cudaStreamSynchronize(s));
-    max_adj = mx;
-    adj.alloc(n_adj > 0 ? n_adj : 1);
-    k_adj_fill<<<nb, 32 * kGraphWarps, 0, s>>>(ptr, inc, col_conn, npe_col, ne, nnodes, adj_ptr.p, adj.p, slots,
-                                                slot_off);
-    FEDD_CUDA(cudaGetLastError());
-    FEDD_CUDA(cudaStreamSynchronize(s));
-}
-
-void build_graph(Graph &g, int64_t ne, const int32_t *row_conn, int npe_row, int64_t nrow_nodes,
-                 const int32_t *col_conn, int npe_col, int64_t ncol_nodes, int slot_off, int *d_err,
-                 cudaStream_t s) {
-    g.nrow_nodes = nrow_nodes;
-    g.ncol_nodes = ncol_nodes;
-    DBuf<int32_t> cnt, cursor;
-    DBuf<int> dmax;
-    cnt.alloc(nrow_nodes + 1);
-    cnt.zero(s);
-    cursor.alloc(nrow_nodes);
-    cursor.zero(s);
-    dmax.alloc(1);
-    dmax.zero(s);
-    int64_t nt = ne * npe_row;
-    k_count_inc<<<ceil_div(nt, 256), 256, 0, s>>>(row_conn, npe_row, ne, nrow_nodes, cnt.p, d_err);
-    FEDD_CUDA(cudaGetLastError());
-    check_err(d_err, s, "incidence count");
-    g.inc_ptr.alloc(nrow_nodes + 1);
-    exclusive_scan_i32_to_i64(cnt.p, g.inc_ptr.p, nrow_nodes + 1, s);
-    g.n_inc = read_i64(g.inc_ptr.p + nrow_nodes, s);
-    g.inc.alloc(g.n_inc);
-    k_fill_inc<<<ceil_div(nt, 256), 256, 0, s>>>(row_conn, npe_row, ne, nrow_nodes, g.inc_ptr.p, cursor.p, g.inc.p);
-    k_sort_inc<<<ceil_div(nrow_nodes, 128), 128, 0, s>>>(g.inc_ptr.p, g.inc.p, nrow_nodes, d_err, dmax.p);
-    FEDD_CUDA(cudaGetLastError());
-    check_err(d_err, s, "incidence sort");
-    FEDD_CUDA(cudaMemcpyAsync(&g.max_inc, dmax.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    g.slots.alloc(g.n_inc * kSlotStride);
-    g.slots.zero(s);
-    adjacency(nrow_nodes, g.inc_ptr.p, g.inc.p, ne, col_conn, npe_col, slot_off, g.slots.p, g.adj_ptr, g.adj,
-              g.max_adj, g.n_adj, d_err, s);
-}
-
-void build_graph_extra(const Graph &g, int64_t ne, const int32_t *col_conn, int npe_col, int64_t ncol_nodes,
-                       int slot_off, DBuf<int64_t> &adj2_ptr, DBuf<int32_t> &adj2, int &max_adj2, int64_t &n_adj2,
-                       int *d_err, cudaStream_t s) {
-    (void)ncol_nodes;
-    adjacency(g.nrow_nodes, g.inc_ptr.p, g.inc.p, ne, col_conn, npe_col, slot_off, g.slots.p, adj2_ptr, adj2,
-              max_adj2, n_adj2, d_err, s);
 }
 
 // ---- Taylor-Hood vertex map ------------------------------------------------
@@ -388,27 +396,19 @@ __global__ void k_vmap_cover(const int *__restrict__ cnt, int64_t nn1, int *bad)
     if (q < nn1 && cnt[q] != 1) atomicOr(bad, 32);
 }
 
-bool build_vertex_map(const int32_t *conn2, const int32_t *conn1, int64_t ne, int64_t nn2, int64_t nn1,
-                      const Graph &g2, const Graph &g1, DBuf<int32_t> &vmap, cudaStream_t s) {
-    if (ne == 0 || nn2 == 0 || nn1 == 0) return false;
-    vmap.alloc(nn2);
-    FEDD_CUDA(cudaMemsetAsync(vmap.p, 0xff, nn2 * sizeof(int32_t), s));  // -1
-    DBuf<int> cnt, bad;
-    cnt.alloc(nn1);
-    cnt.zero(s);
-    bad.alloc(1);
-    bad.zero(s);
-    k_vmap_fill<<<ceil_div(ne, 256), 256, 0, s>>>(conn2, conn1, ne, vmap.p);
-    k_vmap_check_elems<<<ceil_div(ne, 256), 256, 0, s>>>(conn2, conn1, ne, vmap.p, bad.p);
-    k_vmap_count<<<ceil_div(nn2, 256), 256, 0, s>>>(vmap.p, nn2, nn1, cnt.p, bad.p);
-    k_vmap_rows<<<ceil_div(nn2, 8), 256, 0, s>>>(vmap.p, nn2, cnt.p, g2.adj_ptr.p, g2.adj.p, g1.adj_ptr.p, g1.adj.p,
-                                                  bad.p);
-    k_vmap_cover<<<ceil_div(nn1, 256), 256, 0, s>>>(cnt.p, nn1, bad.p);
+void launch_vertex_map(const int32_t *conn2, const int32_t *conn1, int64_t ne, int64_t nn2, int64_t nn1,
+                       const Graph &g2, const Graph &g1, int32_t *vmap, int *bad, Arena &tmp, cudaStream_t s) {
+    const size_t mark = tmp.used;
+    int *cnt = tmp.take<int>(nn1);
+    FEDD_CUDA(cudaMemsetAsync(vmap, 0xff, nn2 * sizeof(int32_t), s));  // -1
+    FEDD_CUDA(cudaMemsetAsync(cnt, 0, nn1 * sizeof(int), s));
+    k_vmap_fill<<<ceil_div(ne, 256), 256, 0, s>>>(conn2, conn1, ne, vmap);
+    k_vmap_check_elems<<<ceil_div(ne, 256), 256, 0, s>>>(conn2, conn1, ne, vmap, bad);
+    k_vmap_count<<<ceil_div(nn2, 256), 256, 0, s>>>(vmap, nn2, nn1, cnt, bad);
+    k_vmap_rows<<<ceil_div(nn2, 8), 256, 0, s>>>(vmap, nn2, cnt, g2.adj_ptr.p, g2.adj.p, g1.adj_ptr.p, g1.adj.p, bad);
+    k_vmap_cover<<<ceil_div(nn1, 256), 256, 0, s>>>(cnt, nn1, bad);
     FEDD_CUDA(cudaGetLastError());
-    int b = 0;
-    FEDD_CUDA(cudaMemcpyAsync(&b, bad.p, sizeof b, cudaMemcpyDeviceToHost, s));
-    FEDD_CUDA(cudaStreamSynchronize(s));
-    return b == 0;
+    tmp.used = mark;
 }
 
 // largest element index among the incidences of each node range
@@ -445,20 +445,12 @@ void node_range_max_elem(const Graph &g, const int64_t *bounds, int K, int64_t *
     for (int k = 0; k < K; k++) out[k] = m[(size_t)k];
 }
 
-void build_csr(Csr &c, const DBuf<int64_t> &adj_ptr, const DBuf<int32_t> &adj, int64_t nrow_nodes,
-               int64_t ncol_nodes, int dofs_r, int dofs_c, cudaStream_t s) {
-    int64_t n_adj = read_i64(adj_ptr.p + nrow_nodes, s);
-    c.nrows = nrow_nodes * dofs_r;
-    c.ncols = ncol_nodes * dofs_c;
-    c.nnz = n_adj * dofs_r * dofs_c;
-    c.rowptr.alloc(c.nrows + 1);
-    c.colind.alloc(c.nnz > 0 ? c.nnz : 1);
-    if (nrow_nodes > 0) {
-        k_csr<<<ceil_div(nrow_nodes, 8), 256, 0, s>>>(adj_ptr.p, adj.p, nrow_nodes, dofs_r, dofs_c, c.rowptr.p,
-                                                       c.colind.p, c.nnz);
-        FEDD_CUDA(cudaGetLastError());
-    }
-    FEDD_CUDA(cudaStreamSynchronize(s));
+void fill_csr(const Csr &c, const int64_t *adj_ptr, const int32_t *adj, int64_t nrow_nodes, int dofs_r, int dofs_c,
+              cudaStream_t s) {
+    if (nrow_nodes <= 0) return;
+    k_csr<<<ceil_div(nrow_nodes, 8), 256, 0, s>>>(adj_ptr, adj, nrow_nodes, dofs_r, dofs_c, c.rowptr.p, c.colind.p,
+                                                   c.nnz);
+    FEDD_CUDA(cudaGetLastError());
 }
 
 }  // namespace fedd

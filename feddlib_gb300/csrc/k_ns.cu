@@ -42,11 +42,17 @@ constexpr int kTabT = 0;        // T[a][kc][lane][4]  3840
 constexpr int kTabKS = 3840;    // KS[a][b][6]        600
 constexpr int kTabR = 4440;     // R[a][b][4]         400
 constexpr int kTabY = 4840;     // Y[b][p][4] (c < 3) 160
-constexpr int kTabSize = 5000;
+static_assert(kTabY + 160 == kNSTab, "table size");
 constexpr int kVelTab = 560;    // floats of tables the velocity-row kernel keeps in shared memory (R, Y)
 
-__constant__ float c_dv[4][10][3];
-
+// reference P2 gradients at the vertices, d_c phi_k at vertex m: with the
+// barycentric gradients L, (4 [k = m] - 1) L_k for the vertex functions and
+// 4 ([a = m] L_b + [b = m] L_a) for the function of edge (a, b)
+__constant__ float c_dv[4][10][3] = {
+    {{-3, -3, -3}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1}, {4, 0, 0}, {0, 0, 0}, {0, 4, 0}, {0, 0, 4}, {0, 0, 0}, {0, 0, 0}},
+    {{1, 1, 1}, {3, 0, 0}, {0, -1, 0}, {0, 0, -1}, {-4, -4, -4}, {0, 4, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 4}, {0, 0, 0}},
+    {{1, 1, 1}, {-1, 0, 0}, {0, 3, 0}, {0, 0, -1}, {0, 0, 0}, {4, 0, 0}, {-4, -4, -4}, {0, 0, 0}, {0, 0, 0}, {0, 0, 4}},
+    {{1, 1, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, 3}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {-4, -4, -4}, {4, 0, 0}, {0, 4, 0}}};
 
 
 // ---- the record stage: coefficients, and NA on the fifth-generation tensor cores
@@ -768,25 +774,27 @@ int sm_count_ns() {
 
 }  // namespace
 
-void ns_upload_tables(const NSTables &t, float **d_tables) {
-    std::vector<float> h(kTabSize, 0.0f);
-    for (int c = 0; c < 3; c++)
+void ns_upload_tables(float *d_tables, cudaStream_t s) {
+    // constants of the element, the same for every handle
+    static const std::vector<float> tab = [] {
+        NSTables t;
+        make_ns_tables(&t);
+        std::vector<float> h(kNSTab, 0.0f);
+        for (int c = 0; c < 3; c++)
+            for (int a = 0; a < 10; a++)
+                for (int b = 0; b < 10; b++)
+                    for (int k = 0; k < 10; k++) h[kTabT + ((a * 3 + k / 4) * 32 + 3 * b + c) * 4 + k % 4] = t.T[c][a][b][k];
         for (int a = 0; a < 10; a++)
-            for (int b = 0; b < 10; b++)
-                for (int k = 0; k < 10; k++) h[kTabT + ((a * 3 + k / 4) * 32 + 3 * b + c) * 4 + k % 4] = t.T[c][a][b][k];
-    for (int a = 0; a < 10; a++)
-        for (int b = 0; b < 10; b++) {
-            for (int s = 0; s < 6; s++) h[kTabKS + (a * 10 + b) * 6 + s] = t.KS[a][b][s];
-            for (int m = 0; m < 4; m++) h[kTabR + (a * 10 + b) * 4 + m] = t.R[a][b][m];
-        }
-    for (int b = 0; b < 10; b++)
-        for (int p = 0; p < 4; p++)
-            for (int c = 0; c < 3; c++) h[kTabY + (b * 4 + p) * 4 + c] = t.Y[c][p][b];
-    FEDD_CUDA(cudaMalloc(d_tables, kTabSize * sizeof(float)));
-    FEDD_CUDA(cudaMemcpy(*d_tables, h.data(), kTabSize * sizeof(float), cudaMemcpyHostToDevice));
-    FEDD_CUDA(cudaMemcpyToSymbol(c_dv, t.DV, sizeof t.DV));
-
-
+            for (int b = 0; b < 10; b++) {
+                for (int s = 0; s < 6; s++) h[kTabKS + (a * 10 + b) * 6 + s] = t.KS[a][b][s];
+                for (int m = 0; m < 4; m++) h[kTabR + (a * 10 + b) * 4 + m] = t.R[a][b][m];
+            }
+        for (int b = 0; b < 10; b++)
+            for (int p = 0; p < 4; p++)
+                for (int c = 0; c < 3; c++) h[kTabY + (b * 4 + p) * 4 + c] = t.Y[c][p][b];
+        return h;
+    }();
+    FEDD_CUDA(cudaMemcpyAsync(d_tables, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice, s));
 }
 
 void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,

@@ -75,6 +75,8 @@ constexpr int kElemResCol = 30;    // column of each row holding its residual en
 constexpr int kGNStride = 992;     // floats per element
 constexpr int kGNRes = 960;        // offset of the residual row
 constexpr int kNSRecord = 228;     // floats per element record (Navier-Stokes): 128 + NA[10][10]
+constexpr int kNSTab = 5000;      // floats of the Navier-Stokes device tables
+constexpr int kLapTab = 610;      // doubles of the Laplace device tables
 constexpr int kLapStrideP1 = 16;   // doubles: 10 packed K + 4 load + pad
 constexpr int kLapStrideP2 = 72;   // doubles: 55 packed K + 10 load + pad
 
@@ -109,7 +111,8 @@ void launch_law_eval(const LawParams &law, const MLPDev *m, int64_t n, const dou
 void launch_hyper_dense(const float *stage, int64_t first, int64_t count, double *Ke, double *re, cudaStream_t s);
 
 // Navier-Stokes
-void ns_upload_tables(const NSTables &t, float **d_tables);
+// the reference tensors into d_tables (kNSTab floats)
+void ns_upload_tables(float *d_tables, cudaStream_t s);
 void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
                       const double *p, const float *d_tables, float visc_dens, float dens, float *rec, int *d_err,
                       cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);

@@ -287,7 +287,7 @@ fedd_status fedd_p2_of_p1(int64_t num_nodes, int64_t num_elements, const double 
         cudaStream_t s = 0;
         const bool dev = flags & FEDD_MESH_DEVICE;
         DBuf<double> xyz1;
-        DBuf<int32_t> aos, soa;
+        DBuf<int32_t> aos;
         const double *x1 = coords;
         const int32_t *c1 = elements;
         if (!dev) {
@@ -296,33 +296,46 @@ fedd_status fedd_p2_of_p1(int64_t num_nodes, int64_t num_elements, const double 
             x1 = xyz1.p;
             c1 = aos.p;
         }
-        soa.alloc((size_t)num_elements * 4);
-        device_aos_to_soa(c1, num_elements, 4, soa.p, s);
-        DBuf<int> err;
-        err.alloc(1);
-        err.zero(s);
+        // the P1 node graph and the edge offsets, in one allocation
+        const int64_t n_inc = num_elements * 4;
+        const size_t fixed = Arena::bytes<GraphStats>(1) + 3 * Arena::bytes<int64_t>(num_nodes + 1) +
+                             Arena::bytes<uint32_t>(n_inc) + Arena::bytes<uint8_t>(n_inc * kSlotStride) +
+                             Arena::bytes<int64_t>(num_nodes + 1) + graph_scratch(num_nodes);
+        Arena mem;
+        mem.reserve(fixed);
+        GraphStats *st = mem.take<GraphStats>(1);
+        FEDD_CUDA(cudaMemsetAsync(st, 0, sizeof(GraphStats), s));
         Graph g;
-        build_graph(g, num_elements, soa.p, 4, num_nodes, soa.p, 4, num_nodes, 0, err.p, s);
-        DBuf<int64_t> cnt, eoff;
-        cnt.alloc(num_nodes + 1);
-        eoff.alloc(num_nodes + 1);
-        k_edge_count<<<(unsigned)ceil_div(num_nodes + 1, 256), 256, 0, s>>>(g.adj_ptr.p, g.adj.p, num_nodes, cnt.p);
+        g.nrow_nodes = g.ncol_nodes = num_nodes;
+        g.inc_ptr.view(mem.take<int64_t>(num_nodes + 1), num_nodes + 1);
+        g.adj_ptr.view(mem.take<int64_t>(num_nodes + 1), num_nodes + 1);
+        g.inc.view(mem.take<uint32_t>(n_inc), n_inc);
+        g.slots.view(mem.take<uint8_t>(n_inc * kSlotStride), n_inc * kSlotStride);
+        int64_t *eoff = mem.take<int64_t>(num_nodes + 1);
+        build_incidences(g, num_elements, c1, 4, st, mem, s);
+        count_adjacency(g, true, c1, 4, g.adj_ptr.p, &st->max_inc[0], &st->max_adj[0], st, mem, s);
+        const GraphStats hs = read_graph_stats(st, g.adj_ptr.p + num_nodes, nullptr, nullptr, s);
+        g.n_adj = hs.n_adj[0];
+        g.adj.alloc(g.n_adj > 0 ? g.n_adj : 1);
+        fill_adjacency(g, c1, 4, 0, g.adj_ptr.p, g.adj.p, s);
+        int64_t *cnt = mem.take<int64_t>(num_nodes + 1);
+        k_edge_count<<<(unsigned)ceil_div(num_nodes + 1, 256), 256, 0, s>>>(g.adj_ptr.p, g.adj.p, num_nodes, cnt);
         FEDD_CUDA(cudaGetLastError());
-        exclusive_scan_i64(cnt.p, eoff.p, num_nodes + 1, s);
+        exclusive_scan_i64(cnt, eoff, num_nodes + 1, mem, s);
         int64_t nedges = 0;
-        FEDD_CUDA(cudaMemcpyAsync(&nedges, eoff.p + num_nodes, sizeof nedges, cudaMemcpyDeviceToHost, s));
+        FEDD_CUDA(cudaMemcpyAsync(&nedges, eoff + num_nodes, sizeof nedges, cudaMemcpyDeviceToHost, s));
         FEDD_CUDA(cudaStreamSynchronize(s));
         m->nn2 = num_nodes + nedges;
         if (m->nn2 >= (1LL << 31)) FEDD_FAIL(FEDD_ERR_ARG, "P2 mesh exceeds 2^31 nodes");
         m->xyz2.alloc((size_t)m->nn2 * 3);
         m->conn2.alloc((size_t)num_elements * 10);
-        k_edge_nodes<<<(unsigned)ceil_div(num_nodes, 256), 256, 0, s>>>(g.adj_ptr.p, g.adj.p, eoff.p, x1, num_nodes,
+        k_edge_nodes<<<(unsigned)ceil_div(num_nodes, 256), 256, 0, s>>>(g.adj_ptr.p, g.adj.p, eoff, x1, num_nodes,
                                                                         m->xyz2.p);
         k_p2_elems<<<(unsigned)ceil_div(num_elements, 256), 256, 0, s>>>(c1, num_elements, g.adj_ptr.p, g.adj.p,
-                                                                         eoff.p, num_nodes, m->conn2.p, err.p);
+                                                                         eoff, num_nodes, m->conn2.p, &st->err);
         FEDD_CUDA(cudaGetLastError());
         int e = 0;
-        FEDD_CUDA(cudaMemcpyAsync(&e, err.p, sizeof e, cudaMemcpyDeviceToHost, s));
+        FEDD_CUDA(cudaMemcpyAsync(&e, &st->err, sizeof e, cudaMemcpyDeviceToHost, s));
         FEDD_CUDA(cudaStreamSynchronize(s));
         if (e) FEDD_FAIL(FEDD_ERR_MESH, "P2 of P1: an element edge is missing from the node graph");
         *num_nodes_p2 = m->nn2;

@@ -139,13 +139,6 @@ void make_ns_tables(NSTables *t) {
         }
     for (int q = 0; q < 15; q++)
         for (int k = 0; k < 10; k++) t->PHIQ[q][k] = (float)phi[q][k];
-    const double V[4][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
-    for (int m = 0; m < 4; m++) {
-        double dp[10][3];
-        basis_dphi(2, V[m], &dp[0][0]);
-        for (int k = 0; k < 10; k++)
-            for (int c = 0; c < 3; c++) t->DV[m][k][c] = (float)dp[k][c];
-    }
 }
 
 void make_hyper_tables(int npts, HyperTables *t) {
