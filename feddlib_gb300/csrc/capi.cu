@@ -230,6 +230,13 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
             qfb = h->qp_fb.p;
             h->last_nqp = nqp;
         }
+        if (!jac) {  // no tangents, no rows of matrices
+            stage(h, "hyper_residual", s, [&] {
+                launch_hyper_residual(h->g, h->geo.p, h->conn.p, h->ne, d_u, h->law, h->htab, qpd, qfb, h->stage_f.p, ru,
+                                      h->d_err.p, s, lc);
+            });
+            break;
+        }
         stage(h, "hyper_elem", s, [&] {
             launch_hyper_elem(h->geo.p, h->conn.p, h->ne, d_u, h->law, h->htab, qpd, qfb, h->stage_f.p,
                               res && d_u != nullptr, h->d_err.p, s, lc);
@@ -246,6 +253,22 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         // its rows into their accumulation
         const float vd = h->gn_on ? 0.0f : (float)(h->prm.viscosity * h->prm.density);
         const float dn = (float)h->prm.density;
+        if (!jac) {  // smaller records, nothing scattered
+            stage(h, "ns_record", s, [&] {
+                launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab.p, vd, dn, h->stage_f.p,
+                                 h->d_err.p, s, lc, 0, -1, true);
+            });
+            if (h->gn_on)
+                stage(h, "gn_residual", s, [&] {
+                    launch_gn_residual(h->xyz.p, h->geo.p, h->conn.p, h->ne, d_u, h->gn, h->stage_gn.p, h->d_err.p, s, lc,
+                                       h->outflow());
+                });
+            stage(h, "ns_residual", s, [&] {
+                launch_ns_residual(h->g, h->gp, h->ninfo.p, h->stage_f.p, h->ns_tab.p,
+                                   h->gn_on ? h->stage_gn.p : nullptr, ru, rp, s, lc, h->coeff);
+            });
+            break;
+        }
         stage(h, "ns_record", s, [&] {
             launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, d_u, d_p, h->ns_tab.p, vd, dn, h->stage_f.p,
                              h->d_err.p, s, lc);

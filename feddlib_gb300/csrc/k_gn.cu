@@ -270,6 +270,71 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
     }
 }
 
+// The viscous residual rows alone: one thread per element takes k_gn_elem's
+// residual operations in the same order.  res: 32 floats per element.
+__global__ void __launch_bounds__(128) k_gn_residual(const float *__restrict__ geo, const int32_t *__restrict__ conn,
+                                                     int64_t ne, const double *__restrict__ u, ViscLaw L,
+                                                     float *__restrict__ res, int *err,
+                                                     const __grid_constant__ GNTab rules) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= ne) return;
+    const bool cy2 = L.model == 0 && abs_int(L.prm[4] - 2.0f) < 2.220446049250313e-16f;
+    const float e_eta = (L.prm[1] - 1.0f) / L.prm[4];
+    float Bi[9];
+    const float adet = fabsf(load_geometry(geo, ne, e, Bi));
+    if (!(adet > 0.0f) || !isfinite(adet)) set_dev_error(err, kDevBadDet);
+    float su[30], r[30];
+#pragma unroll
+    for (int b = 0; b < 10; b++) {
+        const double *up = u + 3 * (int64_t)conn[(int64_t)b * ne + e];
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+            su[3 * b + l] = d2f_rn(up[l]);
+            r[3 * b + l] = 0.0f;
+        }
+    }
+#pragma unroll 1
+    for (int q = 0; q < 5; q++) {
+        float g[30], du[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        const float(*d)[3] = rules.d5[q];
+#pragma unroll
+        for (int k = 0; k < 10; k++) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) g[3 * k + c] = d[k][0] * Bi[c] + d[k][1] * Bi[3 + c] + d[k][2] * Bi[6 + c];
+#pragma unroll
+            for (int a1 = 0; a1 < 3; a1++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) du[3 * a1 + c] = fmaf(su[3 * k + a1], g[3 * k + c], du[3 * a1 + c]);
+        }
+        const float s01 = du[1] + du[3], s02 = du[2] + du[6], s12 = du[5] + du[7];
+        const float gamma = sqrtf(2.0f * du[0] * du[0] + 2.0f * du[4] * du[4] + 2.0f * du[8] * du[8] + s01 * s01 +
+                                  s02 * s02 + s12 * s12);
+        float lawv;
+        if (cy2) {
+            const float *c = L.prm;
+            const float y = powf(1.0f + powf(c[0] * gamma, c[4]), e_eta);
+            lawv = c[3] + (c[2] - c[3]) * y;
+        } else {
+            lawv = gn_eta(L, gamma);
+        }
+        const float ew = lawv * rules.w5[q];
+        const float T0 = ew * (2.0f * du[0]), T1 = ew * (2.0f * du[4]), T2 = ew * (2.0f * du[8]);
+        const float T3 = ew * s01, T4 = ew * s02, T5 = ew * s12;
+#pragma unroll
+        for (int b = 0; b < 10; b++) {
+            const float gx = g[3 * b], gy = g[3 * b + 1], gz = g[3 * b + 2];
+            r[3 * b] = fmaf(gx, T0, fmaf(gy, T3, fmaf(gz, T4, r[3 * b])));
+            r[3 * b + 1] = fmaf(gx, T3, fmaf(gy, T1, fmaf(gz, T5, r[3 * b + 1])));
+            r[3 * b + 2] = fmaf(gx, T4, fmaf(gy, T5, fmaf(gz, T2, r[3 * b + 2])));
+        }
+    }
+    float4 *S = reinterpret_cast<float4 *>(res + e * 32);
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+        S[k] = make_float4(r[4 * k] * adet, r[4 * k + 1] * adet, r[4 * k + 2] * adet, r[4 * k + 3] * adet);
+    S[7] = make_float4(r[28] * adet, r[29] * adet, 0.0f, 0.0f);
+}
+
 // dense element matrices: adds the viscous part to the Navier-Stokes element
 // matrices (34 x 34, velocity rows/columns first) of elements [first, first+count)
 __global__ void k_gn_dense_add(const float *__restrict__ stage, int64_t first, int64_t count, double *Ke, double *re,
@@ -302,6 +367,11 @@ GNTab make_gn_tables() {
         for (int a = 0; a < 10; a++)
             for (int c = 0; c < 3; c++) t.d15[q][a][c] = (float)d[3 * a + c];
     }
+    return t;
+}
+
+const GNTab &gn_rules() {
+    static const GNTab t = make_gn_tables();
     return t;
 }
 
@@ -355,7 +425,8 @@ __device__ __forceinline__ void p2_basis_at(float x, float y, float z, float *ph
 
 __global__ void __launch_bounds__(128) k_gn_outflow(const double *__restrict__ xyz, const int32_t *__restrict__ conn,
                                                     int64_t ne, const double *__restrict__ u, ViscLaw L, GNOutflow of,
-                                                    float *stage, int64_t e_begin, int64_t e_end) {
+                                                    float *stage, int res_off, int stride, int64_t e_begin,
+                                                    int64_t e_end) {
     const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (k >= of.n) return;  // warp-uniform
@@ -453,8 +524,8 @@ __global__ void __launch_bounds__(128) k_gn_outflow(const double *__restrict__ x
         }
     }
     if (lane < 30) {
-        float *st = stage + e * kGNStride;
-        st[kGNRes + lane] += res;
+        float *st = stage + e * stride;
+        st[res_off + lane] += res;
         if (of.matrix)
 #pragma unroll
             for (int t = 0; t < 30; t++) st[32 * t + lane] += col[t];
@@ -466,16 +537,31 @@ __global__ void __launch_bounds__(128) k_gn_outflow(const double *__restrict__ x
 void launch_gn_elem(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
                     int newton, float *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin,
                     int64_t e_end, const GNOutflow &outflow) {
-    static const GNTab rules = make_gn_tables();
     if (e_end < 0) e_end = ne;
     if (e_end <= e_begin) return;
     k_gn_elem<<<(unsigned)ceil_div(e_end - e_begin, 32 * kGNWarps), 32 * kGNWarps, 0, s>>>(
-        geo, conn, ne, u, law, newton, stage, d_err, e_begin, e_end, rules);
+        geo, conn, ne, u, law, newton, stage, d_err, e_begin, e_end, gn_rules());
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
     if (outflow.n > 0) {
         k_gn_outflow<<<(unsigned)ceil_div(outflow.n * 32, 128), 128, 0, s>>>(xyz, conn, ne, u, law, outflow, stage,
-                                                                             e_begin, e_end);
+                                                                             kGNRes, kGNStride, e_begin, e_end);
+        FEDD_CUDA(cudaGetLastError());
+        lc.n++;
+    }
+}
+
+void launch_gn_residual(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u,
+                        const ViscLaw &law, float *gn_res, int *d_err, cudaStream_t s, LaunchCounter &lc,
+                        const GNOutflow &outflow) {
+    if (ne == 0) return;
+    k_gn_residual<<<ceil_div(ne, 128), 128, 0, s>>>(geo, conn, ne, u, law, gn_res, d_err, gn_rules());
+    FEDD_CUDA(cudaGetLastError());
+    lc.n++;
+    if (outflow.n > 0) {
+        GNOutflow of = outflow;
+        of.matrix = 0;
+        k_gn_outflow<<<(unsigned)ceil_div(of.n * 32, 128), 128, 0, s>>>(xyz, conn, ne, u, law, of, gn_res, 0, 32, 0, ne);
         FEDD_CUDA(cudaGetLastError());
         lc.n++;
     }

@@ -672,6 +672,151 @@ __global__ void k_hyper_invariants(const float *__restrict__ geo, const int32_t 
     }
 }
 
+// ---- the residual alone -------------------------------------------------
+// A call for the residual alone (FEDDLib's "Rhs" call, a line search) needs
+// no tangents: one thread per element takes the element kernel's residual
+// operations in the same order, so the values are those of the call that
+// assembles both, and one thread per node adds the node's entries in the row
+// kernel's order.  Bound by the gathers of connectivity and displacements and
+// by latency (168 registers, 12 warps per SM): 48 and 18 us at 41 x 29 x 35 x 6
+// tets in file order, 5 points, against 394 and 285 us of the matrix stages.
+constexpr int kHyperRes = 40;  // floats per element: (r_a, 0) of local node a as one 16-byte word
+
+template <int LAW>
+__global__ void __launch_bounds__(128) k_hyper_residual(const float *__restrict__ geo, const int32_t *__restrict__ conn,
+                                                        int64_t ne, const double *__restrict__ u, LawParams L,
+                                                        const QPDerivs *__restrict__ qpd,
+                                                        const uint8_t *__restrict__ qpfb, float *__restrict__ stage,
+                                                        int *err, const __grid_constant__ HyperTables tab) {
+    constexpr bool kFibre = LAW == kLawAniso || LAW == kLawMLP;
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= ne) return;
+    float Bi[9];
+    float det = load_geometry(geo, ne, e, Bi);
+    det = L.escale ? det * L.escale[e] : det;
+    if (!(det > 0.0f) && !(det < 0.0f)) set_dev_error(err, kDevBadDet);
+    float r[30];
+#pragma unroll
+    for (int k = 0; k < 30; k++) r[k] = 0.0f;
+    if (u) {
+        float ue[30];
+#pragma unroll
+        for (int n = 0; n < 10; n++) {
+            const double *up = u + 3 * (int64_t)conn[(int64_t)n * ne + e];
+#pragma unroll
+            for (int i = 0; i < 3; i++) ue[3 * n + i] = d2f_rn(up[i]);
+        }
+        const int nq = tab.nq;
+#pragma unroll 1
+        for (int q = 0; q < nq; q++) {
+            float H[9], F[9], C[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) H[k] = 0.0f;
+#pragma unroll
+            for (int n = 0; n < 10; n++)
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) H[3 * i + c] = fmaf(ue[3 * n + i], tab.dphi[q][n][c], H[3 * i + c]);
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    F[3 * i + k] = (i == k ? 1.0f : 0.0f) + H[3 * i] * Bi[k] + H[3 * i + 1] * Bi[3 + k] +
+                                   H[3 * i + 2] * Bi[6 + k];
+            cof3(F, C);
+            const float J = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
+            if (!(J > 0.0f)) set_dev_error(err, kDevBadDet);
+            float Fa1[3] = {0.0f, 0.0f, 0.0f}, Fa2[3] = {0.0f, 0.0f, 0.0f}, inv[4];
+            inv[0] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 9; k++) inv[0] = fmaf(F[k], F[k], inv[0]);
+            inv[1] = J;
+            inv[2] = inv[3] = 1.0f;
+            if (kFibre) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    Fa1[i] = F[3 * i] * L.a1[0] + F[3 * i + 1] * L.a1[1] + F[3 * i + 2] * L.a1[2];
+                    Fa2[i] = F[3 * i] * L.a2[0] + F[3 * i + 1] * L.a2[1] + F[3 * i + 2] * L.a2[2];
+                }
+                inv[2] = Fa1[0] * Fa1[0] + Fa1[1] * Fa1[1] + Fa1[2] * Fa1[2];
+                inv[3] = Fa2[0] * Fa2[0] + Fa2[1] * Fa2[1] + Fa2[2] * Fa2[2];
+            }
+            QPDerivs d;
+            if (LAW == kLawMLP && !qpfb[e * nq + q]) {
+                QPDerivs m;
+                nh_matrix(kLawSKR1, L.mu, L.lam, J, m);
+#pragma unroll
+                for (int k = 0; k < 4; k++) d.d1[k] = qpd[e * nq + q].d1[k];
+                d.d1[0] += m.d1[0];
+                d.d1[1] += m.d1[1];
+            } else {
+                law_plain(L, inv, d);
+            }
+            const float s = tab.w[q] * det;
+            const float4 rs = make_float4(-2.0f * s * d.d1[0], -s * d.d1[1], -2.0f * s * d.d1[2], -2.0f * s * d.d1[3]);
+#pragma unroll
+            for (int a = 0; a < 10; a++) {
+                const float g0 = tab.dphi[q][a][0], g1 = tab.dphi[q][a][1], g2 = tab.dphi[q][a][2];
+                float G[3], x[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) G[k] = Bi[k] * g0 + Bi[3 + k] * g1 + Bi[6 + k] * g2;
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const float c = C[3 * i] * G[0] + C[3 * i + 1] * G[1] + C[3 * i + 2] * G[2];
+                    const float f = F[3 * i] * G[0] + F[3 * i + 1] * G[1] + F[3 * i + 2] * G[2];
+                    x[i] = __fmaf_rn(rs.x, f, __fmul_rn(rs.y, c));  // rounded as in the element kernel
+                }
+                if (kFibre) {
+                    const float ag1 = L.a1[0] * G[0] + L.a1[1] * G[1] + L.a1[2] * G[2];
+                    const float ag2 = L.a2[0] * G[0] + L.a2[1] * G[1] + L.a2[2] * G[2];
+                    const float h1 = rs.z * ag1, h2 = rs.w * ag2;
+#pragma unroll
+                    for (int i = 0; i < 3; i++) x[i] += h1 * Fa1[i] + h2 * Fa2[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 3; i++) r[3 * a + i] = __fadd_rn(r[3 * a + i], x[i]);  // not contracted
+            }
+        }
+    }
+    float4 *S = reinterpret_cast<float4 *>(stage + e * kHyperRes);
+#pragma unroll
+    for (int a = 0; a < 10; a++) S[a] = make_float4(r[3 * a], r[3 * a + 1], r[3 * a + 2], 0.0f);
+}
+
+// one thread per node: its element entries summed in incidence order
+__global__ void __launch_bounds__(128) k_hyper_residual_rows(const int64_t *__restrict__ inc_ptr,
+                                                             const uint32_t *__restrict__ inc,
+                                                             const float *__restrict__ stage, int64_t nnodes,
+                                                             double *__restrict__ res) {
+    const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (n >= nnodes) return;
+    const int64_t i0 = inc_ptr[n];
+    const int m = (int)(inc_ptr[n + 1] - i0);
+    const float4 *S = reinterpret_cast<const float4 *>(stage);
+    float x = 0.0f, y = 0.0f, z = 0.0f;
+    // eight entries in flight
+    for (int t0 = 0; t0 < m; t0 += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (t0 + k < m) {
+                const uint32_t ea = __ldg(inc + i0 + t0 + k);
+                v[k] = __ldg(S + (int64_t)(ea >> 4) * 10 + (ea & 15u));
+            }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (t0 + k < m) {
+                x += v[k].x;
+                y += v[k].y;
+                z += v[k].z;
+            }
+    }
+    res[3 * n] = f2d_exact(x);
+    res[3 * n + 1] = f2d_exact(y);
+    res[3 * n + 2] = f2d_exact(z);
+}
+
 // plain law as a stand-alone QP kernel (same I/O as the surrogate kernel)
 __global__ void k_law_qp_plain(LawParams L, const float *__restrict__ inv, int64_t nqp, QPDerivs *out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -849,6 +994,33 @@ void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr
     lc.n++;
 }
 
+
+void launch_hyper_residual(const Graph &g, const float *geo, const int32_t *conn, int64_t ne, const double *u,
+                           const LawParams &law, const HyperTables &tab, const QPDerivs *qpd,
+                           const uint8_t *qp_fallback, float *stage, double *res, int *d_err, cudaStream_t s,
+                           LaunchCounter &lc) {
+    if (ne > 0) {
+        const unsigned grid = ceil_div(ne, 128);
+#define FEDD_HYPER_RES(LAWK) \
+    k_hyper_residual<LAWK><<<grid, 128, 0, s>>>(geo, conn, ne, u, law, qpd, qp_fallback, stage, d_err, tab)
+        switch (law.kind) {
+        case kLawSKR2: FEDD_HYPER_RES(kLawSKR2); break;
+        case kLawSKR3: FEDD_HYPER_RES(kLawSKR3); break;
+        case kLawAniso: FEDD_HYPER_RES(kLawAniso); break;
+        case kLawMLP: FEDD_HYPER_RES(kLawMLP); break;
+        default: FEDD_HYPER_RES(kLawSKR1); break;
+        }
+#undef FEDD_HYPER_RES
+        FEDD_CUDA(cudaGetLastError());
+        lc.n++;
+    }
+    if (g.nrow_nodes > 0) {
+        k_hyper_residual_rows<<<ceil_div(g.nrow_nodes, 128), 128, 0, s>>>(g.inc_ptr.p, g.inc.p, stage, g.nrow_nodes,
+                                                                          res);
+        FEDD_CUDA(cudaGetLastError());
+        lc.n++;
+    }
+}
 
 void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, const double *u,
                              const LawParams &law, const HyperTables &tab, float *inv, int *d_err, cudaStream_t s,

@@ -33,6 +33,10 @@ constexpr int kRecUT = 84;   // uT[c][12] = |det B| (B^-1 u_k)_c   (k < 10)
 constexpr int kRecGS = 120;  // Gs[6]
 constexpr int kRecNA = 128;  // NA[a][b] = nu rho A_ab + rho N_ab (100 floats)
 static_assert(kNSRecord == kRecNA + 100, "record size");
+// the residual alone reads Bs, p, u and NA, in 16-byte words: Bs[d][4] | p[4] |
+// u[30], two unused | NA in rows of 12
+constexpr int kResRecP = 12, kResRecU = 16, kResRecNA = 48;
+static_assert(kNSResRecord == kResRecNA + 120, "residual record layout");
 
 // device table layout (floats)
 // T is stored per row node a and chunk of four k as [a][kc][lane][4] with
@@ -87,7 +91,8 @@ constexpr int kRecBarOff = kRecAOff + kRecGroups * 2 * kNABytesA;
 constexpr size_t kRecSmem = (size_t)kRecBarOff + 8 * kRecGroups + 16;
 constexpr uint32_t kNAWaitPolls = 1u << 20;  // bounded wait for the MMAs (each poll sleeps ~32 ns)
 static_assert(kRecGS == kRecUT + 36 && kRecNA == kRecGS + 8, "uT, Gs and NA are laid out back to back");
-static_assert(kRecWarpBytes >= 32 * 17 * 16 && kRecWarpBytes >= 32 * 68 * 4, "per-warp staging fits");
+static_assert(kRecWarpBytes >= 32 * 17 * 16 && kRecWarpBytes >= 32 * 68 * 4 && kRecWarpBytes >= 32 * 65 * 4,
+              "per-warp staging fits");
 static_assert(kRecSmem <= 227 * 1024 && kRecGroups * 128 <= 512, "one CTA per SM: shared memory and TMEM");
 
 // byte offset of (row, k) in a K-major, unswizzled operand: 8-row x 16-byte
@@ -109,7 +114,40 @@ __device__ __forceinline__ bool group_sync_or(int g, bool v) {
     return r != 0;
 }
 
-// elements [e_begin, e_end)
+// The warp's 32 rows of NA (100 columns from TMEM) into the residual records:
+// row a of 10 values at 12 a.  Two halves of 50 columns (five rows a) through
+// the warp's staging in padded form (rows of 64 floats, 60 used, as 15 words),
+// then contiguous runs of 240 bytes.
+__device__ __forceinline__ void na_rows_padded(float *sN, uint32_t trow, int lane, float *dst, int64_t ew0, int64_t e_end) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int ch = 0; ch < 4; ch++) {
+            // columns 48 h + 16 ch ...: of these [50 h, 50 h + 50) are wanted
+            float v[16];
+            tc::tmem_ld16(trow + 48 * h + 16 * ch, v);
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const int c = 48 * h + 16 * ch + i - 50 * h;  // column within the half
+                if (c >= 0 && c < 50) sN[lane * 65 + 12 * (c / 10) + c % 10] = v[i];
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 5; a++) sN[lane * 65 + 12 * a + 10] = sN[lane * 65 + 12 * a + 11] = 0.0f;
+        __syncwarp();
+#pragma unroll 4
+        for (int k = lane; k < 32 * 15; k += 32) {
+            const int rr = k / 15, c = k - 15 * rr;
+            const float *s = sN + rr * 65 + 4 * c;
+            if (ew0 + rr < e_end)
+                reinterpret_cast<float4 *>(dst + (ew0 + rr) * kNSResRecord + 60 * h)[c] = make_float4(s[0], s[1], s[2], s[3]);
+        }
+        __syncwarp();
+    }
+}
+
+// elements [e_begin, e_end); RES: the residual's record
+template <bool RES>
 __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__restrict__ geo, const int32_t *__restrict__ conn2,
                                                              const int32_t *__restrict__ conn1, int64_t ne,
                                                              const double *__restrict__ u, const double *__restrict__ p,
@@ -219,8 +257,26 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__res
         // chunks keep the 16-byte shared stores conflict-free
         float4 *sRec = reinterpret_cast<float4 *>(sW);
         const int64_t ew0 = e_lane - lane;
+        if (RES) {  // twelve chunks per record, rows of 13
+            float4 *mine = sRec + lane * 13;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+            for (int k = 0; k < 3; k++)
+                mine[k] = make_float4(R[kRecBS + 4 * k], R[kRecBS + 4 * k + 1], R[kRecBS + 4 * k + 2], 0.0f);
+            mine[3] = make_float4(R[kRecP], R[kRecP + 1], R[kRecP + 2], R[kRecP + 3]);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                mine[4 + k] = make_float4(R[kRecU + 4 * k], R[kRecU + 4 * k + 1], k < 7 ? R[kRecU + 4 * k + 2] : 0.0f,
+                                          k < 7 ? R[kRecU + 4 * k + 3] : 0.0f);
+            __syncwarp();
+#pragma unroll 4
+            for (int k = lane; k < 32 * 12; k += 32) {
+                const int rr = k / 12, c = k - 12 * rr;
+                if (ew0 + rr < e_end) reinterpret_cast<float4 *>(rec + (ew0 + rr) * kNSResRecord)[c] = sRec[rr * 13 + c];
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int h = 0; h < (RES ? 0 : 2); h++) {
 #pragma unroll
             for (int k = 0; k < 16; k++)
                 sRec[lane * 17 + k] = make_float4(R[64 * h + 4 * k], R[64 * h + 4 * k + 1], R[64 * h + 4 * k + 2],
@@ -271,44 +327,50 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__res
             break;
         }
         tc::fence_after_sync();
+        if (RES) {
+            // NA rows padded to 12 floats, four passes of 32 columns: the
+            // staging takes rows of 36 floats
+            na_rows_padded(reinterpret_cast<float *>(sW), trow, lane, rec + kResRecNA, ew0, e_end);
+        } else {
         // NA rows out through the warp's staging: columns 0-63 (rows of 68
-        // floats), then 64-99 (rows of 36); each store instruction writes
-        // whole 256-byte (two rows) or 144-byte (three rows) runs of records
-        float *sN = reinterpret_cast<float *>(sW);
+            // floats), then 64-99 (rows of 36); each store instruction writes
+            // whole 256-byte (two rows) or 144-byte (three rows) runs of records
+            float *sN = reinterpret_cast<float *>(sW);
 #pragma unroll
-        for (int ch = 0; ch < 4; ch++) {
-            float v[16];
-            tc::tmem_ld16(trow + 16 * ch, v);
+            for (int ch = 0; ch < 4; ch++) {
+                float v[16];
+                tc::tmem_ld16(trow + 16 * ch, v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 4)
-                *reinterpret_cast<float4 *>(sN + lane * 68 + 16 * ch + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        }
-        __syncwarp();
+                for (int i = 0; i < 16; i += 4)
+                    *reinterpret_cast<float4 *>(sN + lane * 68 + 16 * ch + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+            __syncwarp();
 #pragma unroll 4
-        for (int r = 0; r < 32; r += 2) {
-            const int rr = r + (lane >> 4);
-            const int64_t er = ew0 + rr;
-            if (er < e_end)
-                reinterpret_cast<float4 *>(rec + er * kNSRecord + kRecNA)[lane & 15] =
-                    *reinterpret_cast<const float4 *>(sN + rr * 68 + 4 * (lane & 15));
-        }
-        __syncwarp();
+            for (int r = 0; r < 32; r += 2) {
+                const int rr = r + (lane >> 4);
+                const int64_t er = ew0 + rr;
+                if (er < e_end)
+                    reinterpret_cast<float4 *>(rec + er * kNSRecord + kRecNA)[lane & 15] =
+                        *reinterpret_cast<const float4 *>(sN + rr * 68 + 4 * (lane & 15));
+            }
+            __syncwarp();
 #pragma unroll
-        for (int ch = 4; ch < 7; ch++) {
-            float v[16];
-            tc::tmem_ld16(trow + 16 * ch, v);
+            for (int ch = 4; ch < 7; ch++) {
+                float v[16];
+                tc::tmem_ld16(trow + 16 * ch, v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 4)
-                if (16 * ch + i < 100)
-                    *reinterpret_cast<float4 *>(sN + lane * 36 + 16 * (ch - 4) + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        }
-        __syncwarp();
-        for (int r = 0; r < 32; r += 3) {
-            const int rr = r + lane / 9, c4 = lane % 9;
-            const int64_t er = ew0 + rr;
-            if (lane < 27 && rr < 32 && er < e_end)
-                reinterpret_cast<float4 *>(rec + er * kNSRecord + kRecNA + 64)[c4] =
-                    *reinterpret_cast<const float4 *>(sN + rr * 36 + 4 * c4);
+                for (int i = 0; i < 16; i += 4)
+                    if (16 * ch + i < 100)
+                        *reinterpret_cast<float4 *>(sN + lane * 36 + 16 * (ch - 4) + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+            __syncwarp();
+            for (int r = 0; r < 32; r += 3) {
+                const int rr = r + lane / 9, c4 = lane % 9;
+                const int64_t er = ew0 + rr;
+                if (lane < 27 && rr < 32 && er < e_end)
+                    reinterpret_cast<float4 *>(rec + er * kNSRecord + kRecNA + 64)[c4] =
+                        *reinterpret_cast<const float4 *>(sN + rr * 36 + 4 * c4);
+            }
         }
         tc::fence_before_sync();
         group_sync(gi);
@@ -442,6 +504,29 @@ __device__ __forceinline__ void stage_vel(float *dst_lane, int slot, int t, int 
         }
     }
     cp_async_commit();
+}
+
+// velocity residual of node n: row (a, i) sums rj over the lanes 3 b + i and
+// rb over the lanes 4 i + p (strided tree sums leave them in lanes i = 0..2
+// and 4 i); rg, in lane i, is the viscous residual of a generalized-Newtonian
+// fluid.  uu (N(u) u + viscous) + up (-B^T p), with the residual's block factors
+template <bool GN>
+__device__ __forceinline__ void vel_residual_out(float rj, float rb, float rg, int64_t n, int lane, const NSCoeff &co,
+                                                 double *res_u) {
+    float x = lane < 30 ? rj : 0.0f, z = lane < 12 ? rb : 0.0f;
+#pragma unroll
+    for (int d = 3; d < 32; d *= 2) {
+        const float y = __shfl_down_sync(0xffffffffu, x, d);
+        if (lane + d < 32) x += y;
+    }
+#pragma unroll
+    for (int d = 1; d < 4; d *= 2) {
+        const float y = __shfl_down_sync(0xffffffffu, z, d);
+        if (lane + d < 32) z += y;
+    }
+    z = __shfl_sync(0xffffffffu, z, lane < 3 ? 4 * lane : 0);
+    const float cuu = (float)co.uu, s = fmaf(cuu, x, (float)co.up * z);
+    if (lane < 3) res_u[3 * n + lane] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
 }
 
 template <bool GN>
@@ -596,23 +681,7 @@ __global__ void __launch_bounds__(512, 2) k_ns_vel_rows(const int4 *__restrict__
             }
         }
         if (res_u) {
-            // row (a, i) sums rj over the lanes 3 b + i and rb over the lanes
-            // 4 i + p: strided tree sums leave them in lanes i = 0..2 and 4 i
-            float x = lw ? rj : 0.0f, z = lb ? rb : 0.0f;
-#pragma unroll
-            for (int d = 3; d < 32; d *= 2) {
-                const float y = __shfl_down_sync(0xffffffffu, x, d);
-                if (lane + d < 32) x += y;
-            }
-#pragma unroll
-            for (int d = 1; d < 4; d *= 2) {
-                const float y = __shfl_down_sync(0xffffffffu, z, d);
-                if (lane + d < 32) z += y;
-            }
-            z = __shfl_sync(0xffffffffu, z, lane < 3 ? 4 * lane : 0);
-            // uu (N(u) u + viscous) + up (-B^T p), with the residual's block factors
-            const float cuu = (float)co.uu, s = fmaf(cuu, x, (float)co.up * z);
-            if (lane < 3) res_u[3 * n + lane] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
+            vel_residual_out<GN>(rj, rb, rg, n, lane, co, res_u);
         }
         if (qp >= 0) {
             if (vals10) {
@@ -712,6 +781,137 @@ __global__ void __launch_bounds__(256) k_ns_pres_rows(const int64_t *__restrict_
     }
 }
 
+// ---- the residual alone -------------------------------------------------
+// One thread per node with the sums of k_ns_vel_rows' lanes in registers, each
+// in that kernel's order, and the lanes' tree sums at the end: the values are
+// those of the call that assembles both.  Per incidence a thread reads 240
+// bytes of the element's record as 16-byte words, and these scattered reads
+// bound it (l1tex 89 % of its peak).  At 40^3 x 6 tets it takes 220 us and the
+// smaller records 102, against 741 and 122 us of the matrix stages.  One warp
+// per node with a lane per sum, as in the row kernels, spends about fifty warp
+// instructions on each incidence for some thirty products: 353 us.
+constexpr int kResY = 20;  // row stride of -Y[a][p][4]: the lanes' rows a start in different bank groups
+
+template <bool GN>
+__device__ __forceinline__ void vel_residual_node(const float *sY, int64_t n, const int4 *__restrict__ ninfo,
+                                                  const uint32_t *__restrict__ inc, const float *__restrict__ rec,
+                                                  const float *__restrict__ gn_res, double *__restrict__ res_u,
+                                                  const NSCoeff &co) {
+    const int4 inf = ninfo[n];
+    const int m = node_m(inf);
+    const uint32_t *il = inc + node_i0(inf);
+    float rj[30], rb[12], rg[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < 30; k++) rj[k] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 12; k++) rb[k] = 0.0f;
+    uint32_t next = m > 0 ? __ldg(il) : 0u;
+#pragma unroll 1
+    for (int t = 0; t < m; t++) {
+        const uint32_t ea = next;
+        if (t + 1 < m) next = __ldg(il + t + 1);
+        const int a = (int)(ea & 15u);
+        const float4 *r = reinterpret_cast<const float4 *>(rec + (size_t)(ea >> 4) * kNSResRecord);
+        float u[32], na[12];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float4 v = __ldg(r + kResRecNA / 4 + 3 * a + k);
+            na[4 * k] = v.x; na[4 * k + 1] = v.y; na[4 * k + 2] = v.z; na[4 * k + 3] = v.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 v = __ldg(r + kResRecU / 4 + k);
+            u[4 * k] = v.x; u[4 * k + 1] = v.y; u[4 * k + 2] = v.z; u[4 * k + 3] = v.w;
+        }
+        const float4 pv = __ldg(r + kResRecP / 4);
+        const float pp[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const float4 bs = __ldg(r + i);
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                const float4 y = lds4(sY + kResY * a + 4 * p);
+                const float bt = fmaf(bs.z, y.z, fmaf(bs.y, y.y, bs.x * y.x));
+                rb[4 * i + p] = fmaf(bt, pp[p], rb[4 * i + p]);
+            }
+            if (GN) rg[i] += __ldg(gn_res + (size_t)(ea >> 4) * 32 + 3 * a + i);
+        }
+#pragma unroll
+        for (int b = 0; b < 10; b++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) rj[3 * b + j] = fmaf(na[b], u[3 * b + j], rj[3 * b + j]);
+    }
+    const float cuu = (float)co.uu;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        // vel_residual_out's strided tree over the lanes 3 b + i and 4 i + p
+        const float x = (((rj[i] + rj[3 + i]) + (rj[6 + i] + rj[9 + i])) + ((rj[12 + i] + rj[15 + i]) + (rj[18 + i] + rj[21 + i]))) +
+                        (rj[24 + i] + rj[27 + i]);
+        const float z = (rb[4 * i] + rb[4 * i + 1]) + (rb[4 * i + 2] + rb[4 * i + 3]);
+        const float s = fmaf(cuu, x, (float)co.up * z);
+        res_u[3 * n + i] = f2d_exact(GN ? fmaf(cuu, rg[i], s) : s);
+    }
+}
+
+// the pressure residual: one thread per pressure node, the sums of the lanes
+// (b, j) in registers and their pairwise (xor) tree at the end
+__device__ __forceinline__ void pres_residual_node(const float *sY, int64_t n, const int64_t *__restrict__ inc_ptr,
+                                                   const uint32_t *__restrict__ inc, const float *__restrict__ rec,
+                                                   double *__restrict__ res_p, float cpu) {
+    const int64_t i0 = inc_ptr[n];
+    const int m = (int)(inc_ptr[n + 1] - i0);
+    float s[32];
+#pragma unroll
+    for (int k = 0; k < 32; k++) s[k] = 0.0f;
+#pragma unroll 1
+    for (int t = 0; t < m; t++) {
+        const uint32_t ea = __ldg(inc + i0 + t);
+        const int q = (int)(ea & 15u);
+        const float4 *r = reinterpret_cast<const float4 *>(rec + (size_t)(ea >> 4) * kNSResRecord);
+        float u[32];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 v = __ldg(r + kResRecU / 4 + k);
+            u[4 * k] = v.x; u[4 * k + 1] = v.y; u[4 * k + 2] = v.z; u[4 * k + 3] = v.w;
+        }
+        const float4 b0 = __ldg(r), b1 = __ldg(r + 1), b2 = __ldg(r + 2);
+#pragma unroll
+        for (int b = 0; b < 10; b++) {
+            const float4 y = lds4(sY + kResY * b + 4 * q);
+            s[3 * b] = fmaf(fmaf(b0.z, y.z, fmaf(b0.y, y.y, b0.x * y.x)), u[3 * b], s[3 * b]);
+            s[3 * b + 1] = fmaf(fmaf(b1.z, y.z, fmaf(b1.y, y.y, b1.x * y.x)), u[3 * b + 1], s[3 * b + 1]);
+            s[3 * b + 2] = fmaf(fmaf(b2.z, y.z, fmaf(b2.y, y.y, b2.x * y.x)), u[3 * b + 2], s[3 * b + 2]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (k < o) s[k] += s[k + o];
+    res_p[n] = f2d_exact(cpu * s[0]);
+}
+
+// blocks [0, pblocks) take the pressure nodes (24 incidences each on the
+// structured meshes: the long threads start first), the rest the velocity nodes
+template <bool GN>
+__global__ void __launch_bounds__(128) k_ns_residual(const int4 *__restrict__ ninfo, const uint32_t *__restrict__ inc,
+                                                     const int64_t *__restrict__ pinc_ptr,
+                                                     const uint32_t *__restrict__ pinc, const float *__restrict__ rec,
+                                                     const float *__restrict__ gtab, const float *__restrict__ gn_res,
+                                                     int64_t nnodes, int64_t pnodes, unsigned pblocks,
+                                                     double *__restrict__ res_u, double *__restrict__ res_p, NSCoeff co) {
+    __shared__ __align__(16) float sY[10 * kResY];  // -Y[a][p][4]
+    for (int t = threadIdx.x; t < 160; t += blockDim.x) sY[kResY * (t >> 4) + (t & 15)] = -gtab[kTabY + t];
+    __syncthreads();
+    if (blockIdx.x < pblocks) {
+        const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+        if (n < pnodes) pres_residual_node(sY, n, pinc_ptr, pinc, rec, res_p, (float)co.pu);
+    } else {
+        const int64_t n = (blockIdx.x - pblocks) * (int64_t)blockDim.x + threadIdx.x;
+        if (n < nnodes) vel_residual_node<GN>(sY, n, ninfo, inc, rec, gn_res, res_u, co);
+    }
+}
+
 // dense 34x34 element matrices and element residuals (AssembleFE view)
 __global__ void k_ns_dense(const float *__restrict__ rec, const float *__restrict__ gtab, int64_t first, int64_t count,
                            float visc_dens, float dens, int newton, double *Ke, double *re, NSCoeff co) {
@@ -799,15 +999,16 @@ void ns_upload_tables(float *d_tables, cudaStream_t s) {
 
 void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
                       const double *p, const float *d_tables, float visc_dens, float dens, float *rec, int *d_err,
-                      cudaStream_t s, LaunchCounter &lc, int64_t e_begin, int64_t e_end) {
+                      cudaStream_t s, LaunchCounter &lc, int64_t e_begin, int64_t e_end, bool residual_only) {
     if (e_end < 0) e_end = ne;
     const int64_t count = e_end - e_begin;
     if (count <= 0) return;
     // persistent CTAs, one per SM (shared memory, all 512 TMEM columns)
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)kRecTile * kRecGroups), (int64_t)sm_count_ns());
-    FEDD_CUDA(cudaFuncSetAttribute(k_ns_record, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmem));
-    k_ns_record<<<grid, kRecThreads, kRecSmem, s>>>(geo, conn2, conn1, ne, u, p, rec, d_err, e_begin, e_end, d_tables,
-                                                  visc_dens, dens);
+    auto kern = residual_only ? k_ns_record<true> : k_ns_record<false>;
+    FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmem));
+    kern<<<grid, kRecThreads, kRecSmem, s>>>(geo, conn2, conn1, ne, u, p, rec, d_err, e_begin, e_end, d_tables, visc_dens,
+                                             dens);
     FEDD_CUDA(cudaGetLastError());
     lc.n += 1;
 }
@@ -866,6 +1067,19 @@ void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_table
     k_ns_pres_rows<<<grid, 32 * warps, smem, s>>>(gp.inc_ptr.p, gp.inc.p, gp.slots.p, gp.adj_ptr.p, rec, d_tables,
                                                   rowptr10, want_jac ? vals10 : nullptr, res_p, nn, max_adj,
                                                   (float)co.pu);
+    FEDD_CUDA(cudaGetLastError());
+    lc.n++;
+}
+
+void launch_ns_residual(const Graph &g, const Graph &gp, const int4 *ninfo, const float *rec, const float *d_tables,
+                        const float *gn_res, double *res_u, double *res_p, cudaStream_t s, LaunchCounter &lc,
+                        const NSCoeff &co) {
+    const int64_t nn = g.nrow_nodes, np = gp.nrow_nodes;
+    const unsigned pb = ceil_div(np, 128), vb = ceil_div(nn, 128);
+    if (pb + vb == 0) return;
+    auto kern = gn_res ? k_ns_residual<true> : k_ns_residual<false>;
+    kern<<<pb + vb, 128, 0, s>>>(ninfo, g.inc.p, gp.inc_ptr.p, gp.inc.p, rec, d_tables, gn_res, nn, np, pb, res_u, res_p,
+                                 co);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

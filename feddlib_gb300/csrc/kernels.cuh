@@ -77,6 +77,7 @@ constexpr int kGNRes = 960;        // offset of the residual row
 constexpr int kNSRecord = 228;     // floats per element record (Navier-Stokes): 128 + NA[10][10]
 constexpr int kNSTab = 5000;      // floats of the Navier-Stokes device tables
 constexpr int kLapTab = 610;      // doubles of the Laplace device tables
+constexpr int kNSResRecord = 168; // floats per element record when only the residual is assembled
 constexpr int kLapStrideP1 = 16;   // doubles: 10 packed K + 4 load + pad
 constexpr int kLapStrideP2 = 72;   // doubles: 55 packed K + 10 load + pad
 
@@ -99,6 +100,12 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
 void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr, double *vals, double *res,
                        int64_t nnodes, cudaStream_t s, LaunchCounter &lc,
                        int64_t n_begin = 0);
+// the residual alone, same values: element residuals (40 floats per element in
+// stage), then the per-node sums
+void launch_hyper_residual(const Graph &g, const float *geo, const int32_t *conn, int64_t ne, const double *u,
+                           const LawParams &law, const HyperTables &tab, const QPDerivs *qpd,
+                           const uint8_t *qp_fallback, float *stage, double *res, int *d_err, cudaStream_t s,
+                           LaunchCounter &lc);
 void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, const double *u,
                              const LawParams &law, const HyperTables &tab, float *inv, int *d_err, cudaStream_t s,
                              LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);
@@ -115,7 +122,8 @@ void launch_hyper_dense(const float *stage, int64_t first, int64_t count, double
 void ns_upload_tables(float *d_tables, cudaStream_t s);
 void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *conn1, int64_t ne, const double *u,
                       const double *p, const float *d_tables, float visc_dens, float dens, float *rec, int *d_err,
-                      cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);
+                      cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1,
+                      bool residual_only = false);
 // per velocity-row node: first incidence, vertex P1 node, neighbour and
 // incidence counts (one int4; built once per mesh)
 void launch_ns_node_info(const Graph &g, const int64_t *padj_ptr, const int32_t *vmap, int4 *info, cudaStream_t s);
@@ -136,6 +144,11 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
 void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_tables, const int64_t *rowptr10,
                          double *vals10, double *res_p, int want_jac, int max_adj, cudaStream_t s,
                          LaunchCounter &lc, const NSCoeff &co = NSCoeff{});
+// the residual alone, same values, from records written with residual_only;
+// gn_res: the viscous residual rows (32 floats per element) or null
+void launch_ns_residual(const Graph &g, const Graph &gp, const int4 *ninfo, const float *rec, const float *d_tables,
+                        const float *gn_res, double *res_u, double *res_p, cudaStream_t s, LaunchCounter &lc,
+                        const NSCoeff &co);
 void launch_ns_dense(const float *rec, const float *d_tables, int64_t first, int64_t count, float visc_dens,
                      float dens, int newton, double *Ke, double *re, cudaStream_t s, const NSCoeff &co = NSCoeff{});
 
@@ -195,6 +208,10 @@ struct GNOutflow {
 void launch_gn_elem(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u, const ViscLaw &law,
                     int newton, float *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                     int64_t e_end = -1, const GNOutflow &outflow = GNOutflow{});
+// the viscous residual rows alone (32 floats per element), same values
+void launch_gn_residual(const double *xyz, const float *geo, const int32_t *conn, int64_t ne, const double *u,
+                        const ViscLaw &law, float *gn_res, int *d_err, cudaStream_t s, LaunchCounter &lc,
+                        const GNOutflow &outflow);
 void launch_gn_dense(const float *stage, int64_t first, int64_t count, double *Ke, double *re, cudaStream_t s,
                      double coeff_uu = 1.0);
 
