@@ -472,8 +472,7 @@ __global__ void k_colsum(const float *__restrict__ in, int64_t rows, int cols, f
 }
 
 struct TrainParams {
-    const float *W1, *b1, *W2, *b2, *w3;
-    float b3;
+    const float *W1, *b1, *W2, *b2, *w3, *b3;
 };
 
 // forward layer 1: X1 = [H1; DH1_0..3] (5B x H), caches S1, T1
@@ -508,7 +507,7 @@ __global__ void k_tr_l2(TrainParams P, int H, const float *__restrict__ Z2, cons
         yp = fmaf(P.w3[j], z > 20.0f ? z : log1pf(expf(z)), yp);
         for (int k = 0; k < 4; k++) gp[k] = fmaf(P.w3[j] * sg, Z2[((1 + k) * B + s) * H + j], gp[k]);
     }
-    const float y = warp_sum(yp) + P.b3;
+    const float y = warp_sum(yp) + *P.b3;
     float g[4];
     for (int k = 0; k < 4; k++) g[k] = warp_sum(gp[k]);
     const int64_t si = idx[s];
@@ -561,6 +560,332 @@ __global__ void k_tr_l1b(TrainParams P, int H, const float *__restrict__ X, cons
     o[4 * H + i] = dz;
 }
 
+// ---- width 64: one kernel for the forward and backward passes -------------
+// The network's 5 channels (h and its four input derivatives) of a sample meet
+// three 64 x 64 products: Z2 = X1 W2^T, DX1 = D W2 and gW2 = D^T X1.  As
+// separate kernels they moved the five-channel matrices X1, Z2, D and DX1
+// through memory nine times (84 MB each at a batch of 65,536), and the last
+// one ran on 80 of the blocks the chip holds.  Here a CTA takes tiles of 16
+// samples and keeps them in shared memory: thread (s, c) of the 256 owns
+// hidden units 4 c .. 4 c + 3 of sample s in all five channels, so the layer
+// formulas between the products run on registers, and a 4 x 4 block of gW2,
+// which stays in registers over all tiles of the CTA, as do the thread's sums
+// of the other gradients.  Each CTA writes one partial sum of every gradient;
+// k_tr_update adds them in a fixed order and takes the Adam step.  FP32
+// throughout; bound by the FP32 pipe (3 x 20,480 multiply-adds per sample) and
+// shared-memory reads: 213 us for a batch of 65,536 (38 TFLOP/s) and 8 us for
+// k_tr_update, against 1,590 us of separate kernels.
+constexpr int kTS = 16;                  // samples per tile
+constexpr int kTThreads = 256;
+constexpr int kTSample = 5 * kH + 4;     // floats per sample: five channels, and 4 so that two samples' rows differ in banks
+constexpr int kTPar = 4 * kH + kH + kH * kH + kH + kH + 2;  // gradients in the parameters' order, then the loss
+constexpr size_t kTSmem = (size_t)(2 * kH * kH + 2 * kTS * kTSample + 4 * kH + 3 * kH) * sizeof(float);
+
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void st4(float *p, const float *v) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// acc[c] += x w for the four columns of w
+__device__ __forceinline__ void fma4(float *acc, float x, const float4 &w) {
+    acc[0] = fmaf(x, w.x, acc[0]);
+    acc[1] = fmaf(x, w.y, acc[1]);
+    acc[2] = fmaf(x, w.z, acc[2]);
+    acc[3] = fmaf(x, w.w, acc[3]);
+}
+// acc[ch][c] = sum_i rows[ch][i] W[i][u0 + c] over 64 i
+__device__ __forceinline__ void tile_product(float acc[5][4], const float *rows, const float *W, int u0) {
+#pragma unroll
+    for (int ch = 0; ch < 5; ch++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[ch][c] = 0.0f;
+#pragma unroll 2
+    for (int i = 0; i < kH; i += 4) {
+        float4 x[5];
+#pragma unroll
+        for (int ch = 0; ch < 5; ch++) x[ch] = ld4(rows + kH * ch + i);
+        const float4 w0 = ld4(W + i * kH + u0), w1 = ld4(W + (i + 1) * kH + u0), w2 = ld4(W + (i + 2) * kH + u0),
+                     w3 = ld4(W + (i + 3) * kH + u0);
+#pragma unroll
+        for (int ch = 0; ch < 5; ch++) {
+            fma4(acc[ch], x[ch].x, w0);
+            fma4(acc[ch], x[ch].y, w1);
+            fma4(acc[ch], x[ch].z, w2);
+            fma4(acc[ch], x[ch].w, w3);
+        }
+    }
+}
+
+// samples idx[0..B) (null: 0..B) in tiles; part: gridDim.x x kTPar
+__global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const float *__restrict__ X,
+                                                          const float *__restrict__ ty, const float *__restrict__ tgr,
+                                                          const int64_t *__restrict__ idx, int64_t B, float wpsi,
+                                                          float wgrad, float *__restrict__ part) {
+    extern __shared__ __align__(16) float sm[];
+    float *sW = sm, *sWT = sW + kH * kH;               // W2[j][i] and W2[j][i] at [i][j]
+    float *sX = sWT + kH * kH, *sD = sX + kTS * kTSample;
+    float *sW1 = sD + kTS * kTSample, *sb1 = sW1 + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
+    const int tid = threadIdx.x, s = tid >> 4, u0 = 4 * (tid & 15), j0 = 4 * (tid >> 4);
+    for (int t = tid; t < kH * kH; t += kTThreads) {
+        const float w = P.W2[t];
+        sW[t] = w;
+        sWT[(t & (kH - 1)) * kH + (t >> 6)] = w;
+    }
+    sW1[tid] = P.W1[tid];  // 4 kH = 256 values
+    if (tid < kH) {
+        sb1[tid] = P.b1[tid];
+        sb2[tid] = P.b2[tid];
+        sw3[tid] = P.w3[tid];
+    }
+    const float b3 = *P.b3;
+    __syncthreads();
+    float *xrow = sX + s * kTSample, *drow = sD + s * kTSample;
+    float gW2[4][4], gW1[4][4], gb1[4], gb2[4], gw3[4], gb3 = 0.0f, loss = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        gb1[a] = gb2[a] = gw3[a] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < 4; b++) gW2[a][b] = gW1[a][b] = 0.0f;
+    }
+    const int64_t ntiles = (B + kTS - 1) / kTS;
+    auto sample = [&](int64_t tile) {
+        const int64_t q = tile * kTS + s;
+        return q < B ? (idx ? idx[q] : q) : (int64_t)-1;
+    };
+    int64_t id = blockIdx.x < ntiles ? sample(blockIdx.x) : -1;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const bool valid = id >= 0;
+        const int64_t si = valid ? id : 0;
+        const float4 x4 = ld4(X + 4 * si), t4 = ld4(tgr + 4 * si);
+        const float tyv = ty[si];
+        if (tile + gridDim.x < ntiles) id = sample(tile + gridDim.x);
+        const float x[4] = {x4.x, x4.y, x4.z, x4.w}, tg[4] = {t4.x, t4.y, t4.z, t4.w};
+        float s1[4], t1[4];
+        {  // layer 1
+            float v[5][4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float4 w = ld4(sW1 + 4 * (u0 + u));
+                const float z = fmaf(w.w, x[3], fmaf(w.z, x[2], fmaf(w.y, x[1], fmaf(w.x, x[0], sb1[u0 + u]))));
+                const float sg = 1.0f / (1.0f + expf(-z));
+                s1[u] = sg;
+                t1[u] = sg * (1.0f - sg);
+                v[0][u] = z > 20.0f ? z : log1pf(expf(z));
+                v[1][u] = sg * w.x;
+                v[2][u] = sg * w.y;
+                v[3][u] = sg * w.z;
+                v[4][u] = sg * w.w;
+            }
+#pragma unroll
+            for (int ch = 0; ch < 5; ch++) st4(xrow + kH * ch + u0, v[ch]);
+        }
+        __syncwarp();  // a sample's rows are written and read by the same half warp
+        float acc[5][4];
+        tile_product(acc, xrow, sWT, u0);
+        // layer 2, the sample's output, gradient and loss, and the backward rows D
+        float sg[4], hv[4], yp = 0.0f, gp[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float z = acc[0][u] + sb2[u0 + u], w3 = sw3[u0 + u];
+            sg[u] = 1.0f / (1.0f + expf(-z));
+            hv[u] = z > 20.0f ? z : log1pf(expf(z));
+            yp = fmaf(w3, hv[u], yp);
+#pragma unroll
+            for (int k = 0; k < 4; k++) gp[k] = fmaf(w3 * sg[u], acc[1 + k][u], gp[k]);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            yp += __shfl_xor_sync(0xffffffffu, yp, o);
+#pragma unroll
+            for (int k = 0; k < 4; k++) gp[k] += __shfl_xor_sync(0xffffffffu, gp[k], o);
+        }
+        const float dy = yp + b3 - tyv, ey = valid ? 2.0f * wpsi * dy : 0.0f;
+        float eg[4], l = wpsi * dy * dy;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float dk = gp[k] - tg[k];
+            eg[k] = valid ? 2.0f * wgrad * dk : 0.0f;
+            l += wgrad * dk * dk;
+        }
+        gb3 += ey;
+        loss += valid ? l : 0.0f;
+        {
+            float d[5][4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float w3 = sw3[u0 + u], tg2 = sg[u] * (1.0f - sg[u]);
+                float dz2 = ey * w3 * sg[u], gw = ey * hv[u];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    dz2 = fmaf(eg[k] * w3 * tg2, acc[1 + k][u], dz2);
+                    gw = fmaf(eg[k] * sg[u], acc[1 + k][u], gw);
+                    d[1 + k][u] = eg[k] * w3 * sg[u];
+                }
+                d[0][u] = dz2;
+                gb2[u] += dz2;
+                gw3[u] += gw;
+            }
+#pragma unroll
+            for (int ch = 0; ch < 5; ch++) st4(drow + kH * ch + u0, d[ch]);
+        }
+        __syncthreads();
+        // gW2 block of the tile's 80 rows
+#pragma unroll 2
+        for (int q = 0; q < kTS; q++)
+#pragma unroll
+            for (int ch = 0; ch < 5; ch++) {
+                const float4 d = ld4(sD + q * kTSample + kH * ch + j0), v = ld4(sX + q * kTSample + kH * ch + u0);
+                fma4(gW2[0], d.x, v);
+                fma4(gW2[1], d.y, v);
+                fma4(gW2[2], d.z, v);
+                fma4(gW2[3], d.w, v);
+            }
+        // backward through layer 2's product and layer 1
+        tile_product(acc, drow, sW, u0);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float4 w = ld4(sW1 + 4 * (u0 + u));
+            const float wk[4] = {w.x, w.y, w.z, w.w};
+            float dz = acc[0][u] * s1[u];
+#pragma unroll
+            for (int k = 0; k < 4; k++) dz = fmaf(acc[1 + k][u] * t1[u], wk[k], dz);
+#pragma unroll
+            for (int k = 0; k < 4; k++) gW1[u][k] += fmaf(dz, x[k], acc[1 + k][u] * s1[u]);
+            gb1[u] += dz;
+        }
+        __syncthreads();  // the next tile overwrites the rows
+    }
+    // the CTA's partial sums: gW2 by its owners, the others summed over the 16
+    // sample groups through shared memory
+    float *out = part + (int64_t)blockIdx.x * kTPar;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) out[5 * kH + (j0 + a) * kH + u0 + b] = gW2[a][b];
+    constexpr int kSmall = 7 * kH;  // gW1 (4 per unit), gb1, gb2, gw3
+    float *red = sX;                // 16 x 448 floats in the rows' place
+    static_assert(kTS * kSmall + 2 * kTS <= 2 * kTS * kTSample, "the partial sums fit the rows");
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) red[s * kSmall + 4 * (u0 + u) + k] = gW1[u][k];
+        red[s * kSmall + 4 * kH + u0 + u] = gb1[u];
+        red[s * kSmall + 5 * kH + u0 + u] = gb2[u];
+        red[s * kSmall + 6 * kH + u0 + u] = gw3[u];
+    }
+    if (u0 == 0) {
+        red[kTS * kSmall + s] = gb3;
+        red[kTS * kSmall + kTS + s] = loss;
+    }
+    __syncthreads();
+    for (int t = tid; t < kSmall + 2; t += kTThreads) {
+        float v = 0.0f;
+        for (int q = 0; q < kTS; q++) v += t < kSmall ? red[q * kSmall + t] : red[kTS * kSmall + kTS * (t - kSmall) + q];
+        // gW1 | gb1 at the front, gb2 | gw3 | gb3 | loss behind gW2
+        out[t < 5 * kH ? t : t + kH * kH] = v;
+    }
+}
+
+// one gradient (or the loss) per lane, eight warps sharing its partial sums;
+// with adam the parameter's Adam step, otherwise the sum into grad
+__global__ void __launch_bounds__(256) k_tr_update(const float *__restrict__ part, int nparts, int adam, float *grad,
+                                                   float *lsum, float *p, float *m1, float *m2, float lr, float b1,
+                                                   float b2, float eps, float c1, float c2, float scale) {
+    __shared__ float red[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    float v = 0.0f;
+    if (i < kTPar)
+        for (int q = w; q < nparts; q += 8) v += part[(int64_t)q * kTPar + i];
+    red[w][lane] = v;
+    __syncthreads();
+    if (w != 0 || i >= kTPar) return;
+#pragma unroll
+    for (int q = 1; q < 8; q++) v += red[q][lane];
+    if (i == kTPar - 1) {
+        *lsum = v;
+    } else if (adam) {
+        const float gi = v * scale;
+        m1[i] = b1 * m1[i] + (1.0f - b1) * gi;
+        m2[i] = b2 * m2[i] + (1.0f - b2) * gi * gi;
+        p[i] -= lr * (m1[i] / c1) / (sqrtf(m2[i] / c2) + eps);
+    } else {
+        grad[i] = v;
+    }
+}
+
+// ---- the seeded shuffle on the device ---------------------------------------
+// The sequential shuffle  for i = n - 1 .. 1: swap(perm[i], perm[j_i]),  with
+// j_i = draw(n - 1 - i) mod (i + 1), evaluated for all i at once.  Position p
+// is written by the steps k > p with j_k = p, which run in descending order,
+// so before step k the value at position k is that of position L_k[0] before
+// its own step, where L_p lists the steps k > p with j_k = p in ascending
+// order, or perm[k] if L_k is empty: V(k) = V(L_k[0]) or perm[k].  The result is
+//     out[i] = V(i)                      if j_i = i (and for i = 0)
+//            = V(k) or perm[j_i]         with k the successor of i in L_{j_i}.
+// Lists and chains have about log n entries.  On the host a shuffle of 200,000
+// samples took 1,140 us; these seven launches take 45 us.
+__host__ __device__ inline uint64_t sm64_mix(uint64_t z) {
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+    return z ^ (z >> 31);
+}
+
+__global__ void k_fy_targets(uint64_t seed, int64_t n, int64_t *target, int64_t *count) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t j = i == 0 ? 0 : (int64_t)(sm64_mix(seed + (uint64_t)(n - i) * 0x9E3779B97F4A7C15ULL) % (uint64_t)(i + 1));
+    target[i] = j;
+    if (j < i) atomicAdd(reinterpret_cast<unsigned long long *>(count + j), 1ull);
+}
+
+// counts the lists' cursors down
+__global__ void k_fy_fill(const int64_t *__restrict__ target, int64_t n, const int64_t *__restrict__ off, int64_t *count,
+                          int64_t *list) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t j = target[i];
+    if (j < i) list[off[j] + (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(count + j), ~0ull) - 1] = i;
+}
+
+__global__ void k_fy_sort(int64_t n, const int64_t *__restrict__ off, int64_t *list) {
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int64_t a = off[p], b = off[p + 1];
+    for (int64_t x = a + 1; x < b; x++) {
+        const int64_t v = list[x];
+        int64_t y = x;
+        for (; y > a && list[y - 1] > v; y--) list[y] = list[y - 1];
+        list[y] = v;
+    }
+}
+
+__global__ void k_fy_resolve(int64_t n, const int64_t *__restrict__ target, const int64_t *__restrict__ off,
+                             const int64_t *__restrict__ list, const int64_t *__restrict__ perm, int64_t *out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t j = target[i];
+    int64_t k = i;
+    bool chain = true;
+    if (j < i) {
+        int64_t x = off[j];
+        const int64_t b = off[j + 1];
+        while (x < b && list[x] != i) x++;
+        chain = x + 1 < b;
+        k = chain ? list[x + 1] : j;
+    }
+    if (chain)
+        for (;;) {  // strictly ascending
+            const int64_t a = off[k];
+            if (a == off[k + 1]) break;
+            k = list[a];
+        }
+    out[i] = perm[k];
+}
+
+__global__ void k_iota(int64_t *p, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) p[i] = i;
+}
+
 __global__ void k_adam(float *p, const float *g, float *m1, float *m2, int n, float lr, float b1, float b2, float eps,
                        float c1, float c2, float scale) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -579,16 +904,21 @@ using namespace fedd;
 struct fedd_trainer {
     int device = 0, H = 64;
     int64_t n = 0;
+    Arena mem;  // the data set, the parameters and their Adam state, the loss
     DBuf<float> X, ty, tg;
     // parameters (flat): W1 (4H) | b1 (H) | W2 (HH) | b2 (H) | w3 (H) | b3 (1)
     DBuf<float> par, grad, m1, m2;
     int64_t step = 0;
-    // workspace for a batch
+    // partial gradients of the width-64 kernel, one set per CTA
+    DBuf<float> partials;
+    // the sample order (from the first run on) and the shuffle's workspace
+    Arena order;
+    int64_t *perm = nullptr, *perm_next = nullptr, *fy_target = nullptr, *fy_count = nullptr, *fy_off = nullptr,
+            *fy_list = nullptr;
+    // workspace for a batch of the general path
     int64_t B = 0;
-    DBuf<int64_t> idx;
     DBuf<float> X1, S1, T1, Z2, D, DX1, GW3, G1, lossv, ey, part;
-    DBuf<float> lsum;  // the batch's summed loss (one float, allocated once)
-    std::vector<int64_t> perm;
+    DBuf<float> lsum;  // the batch's summed loss
     uint64_t rng = 0;
     int64_t cursor = 0;
     std::string err;
@@ -600,7 +930,7 @@ struct fedd_trainer {
         t.W2 = par.p + 5 * H;
         t.b2 = par.p + 5 * H + H * H;
         t.w3 = par.p + 6 * H + H * H;
-        t.b3 = 0.0f;
+        t.b3 = par.p + 7 * H + H * H;
         return t;
     }
 };
@@ -611,7 +941,6 @@ void tr_workspace(fedd_trainer *t, int64_t B) {
     if (t->B == B) return;
     const int H = t->H;
     t->B = B;
-    t->idx.alloc(B);
     t->X1.alloc(5 * B * H);
     t->S1.alloc(B * H);
     t->T1.alloc(B * H);
@@ -624,18 +953,18 @@ void tr_workspace(fedd_trainer *t, int64_t B) {
     t->ey.alloc(B);
 }
 
-// loss and gradient (sum over the batch, not yet divided by B) into t->grad
-float tr_forward_backward(fedd_trainer *t, int64_t B, float wpsi, float wgrad, float b3) {
+// general width: loss and gradient (sums over the batch, not yet divided by B)
+// of the samples idx into t->lsum and t->grad
+void tr_forward_backward(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float wgrad) {
     const int H = t->H;
     cudaStream_t s = 0;
-    TrainParams P = t->tp();
-    P.b3 = b3;
-    k_tr_l1<<<ceil_div(B * H, 256), 256, 0, s>>>(P, H, t->X.p, t->idx.p, B, t->X1.p, t->S1.p, t->T1.p);
+    const TrainParams P = t->tp();
+    k_tr_l1<<<ceil_div(B * H, 256), 256, 0, s>>>(P, H, t->X.p, idx, B, t->X1.p, t->S1.p, t->T1.p);
     {  // Z2 (5B x H) = X1 (5B x H) . W2^T
         dim3 grid(ceil_div(H, 64), ceil_div(5 * B, 64), 1);
         k_sgemm<false, true><<<grid, 256, 0, s>>>(t->X1.p, P.W2, t->Z2.p, (int)(5 * B), H, H, H);
     }
-    k_tr_l2<<<ceil_div(B * 32, 256), 256, 0, s>>>(P, H, t->Z2.p, t->ty.p, t->tg.p, t->idx.p, B, wpsi, wgrad, t->D.p,
+    k_tr_l2<<<ceil_div(B * 32, 256), 256, 0, s>>>(P, H, t->Z2.p, t->ty.p, t->tg.p, idx, B, wpsi, wgrad, t->D.p,
                                                   t->GW3.p, t->lossv.p, t->ey.p);
     float *g = t->grad.p;
     // gradient layout: W1 (4 H) | b1 (H) | W2 (H H) | b2 (H) | w3 (H) | b3; b1's
@@ -656,18 +985,58 @@ float tr_forward_backward(fedd_trainer *t, int64_t B, float wpsi, float wgrad, f
         dim3 grid(ceil_div(H, 64), ceil_div(5 * B, 64), 1);
         k_sgemm<false, false><<<grid, 256, 0, s>>>(t->D.p, P.W2, t->DX1.p, (int)(5 * B), H, H, H);
     }
-    k_tr_l1b<<<ceil_div(B * H, 256), 256, 0, s>>>(P, H, t->X.p, t->idx.p, B, t->DX1.p, t->S1.p, t->T1.p, t->G1.p);
+    k_tr_l1b<<<ceil_div(B * H, 256), 256, 0, s>>>(P, H, t->X.p, idx, B, t->DX1.p, t->S1.p, t->T1.p, t->G1.p);
     k_colsum<<<5 * H, 256, 0, s>>>(t->G1.p, B, 5 * H, gW1);  // gW1 | gb1 contiguous
     k_colsum<<<H, 256, 0, s>>>(t->D.p, B, H, gb2);
     k_colsum<<<H, 256, 0, s>>>(t->GW3.p, B, H, gw3);
     k_colsum<<<1, 256, 0, s>>>(t->ey.p, B, 1, gb3);
     FEDD_CUDA(cudaGetLastError());
-    if (!t->lsum.p) t->lsum.alloc(1);
     k_colsum<<<1, 256, 0, s>>>(t->lossv.p, B, 1, t->lsum.p);
-    float L = 0;
-    FEDD_CUDA(cudaMemcpyAsync(&L, t->lsum.p, sizeof L, cudaMemcpyDeviceToHost, s));
-    FEDD_CUDA(cudaStreamSynchronize(s));
-    return L;
+    FEDD_CUDA(cudaGetLastError());
+}
+
+// width 64: the same, then the Adam step when adam is set (idx null: samples 0..B)
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2, scale;
+};
+void tr_fused(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float wgrad, const AdamStep *adam) {
+    cudaStream_t s = 0;
+    // two CTAs per SM (registers)
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(B, kTS), (int64_t)sms() * 2);
+    if (t->partials.n < (size_t)grid * kTPar) t->partials.alloc((size_t)grid * kTPar);
+    FEDD_CUDA(cudaFuncSetAttribute(k_tr_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem));
+    k_tr_fused<<<grid, kTThreads, kTSmem, s>>>(t->tp(), t->X.p, t->ty.p, t->tg.p, idx, B, wpsi, wgrad, t->partials.p);
+    const AdamStep a = adam ? *adam : AdamStep{};
+    k_tr_update<<<ceil_div(kTPar, 32), 256, 0, s>>>(t->partials.p, (int)grid, adam != nullptr, t->grad.p, t->lsum.p,
+                                                    t->par.p, t->m1.p, t->m2.p, a.lr, a.b1, a.b2, a.eps, a.c1, a.c2,
+                                                    a.scale);
+    FEDD_CUDA(cudaGetLastError());
+}
+
+// the sample order and the shuffle's workspace
+void tr_order(fedd_trainer *t) {
+    if (t->perm) return;
+    const int64_t n = t->n;
+    t->order.reserve(6 * Arena::bytes<int64_t>(n + 1) + scan_scratch(n + 1));
+    t->perm_next = t->order.take<int64_t>(n + 1);
+    t->fy_target = t->order.take<int64_t>(n + 1);
+    t->fy_count = t->order.take<int64_t>(n + 1);
+    t->fy_off = t->order.take<int64_t>(n + 1);
+    t->fy_list = t->order.take<int64_t>(n + 1);
+    t->perm = t->order.take<int64_t>(n + 1);
+    FEDD_CUDA(cudaMemsetAsync(t->fy_count, 0, (n + 1) * sizeof(int64_t), 0));  // k_fy_fill counts it back to zero
+}
+
+void tr_shuffle(fedd_trainer *t, uint64_t seed) {
+    const int64_t n = t->n;
+    const unsigned nb = ceil_div(n, 256);
+    k_fy_targets<<<nb, 256>>>(seed, n, t->fy_target, t->fy_count);
+    exclusive_scan_i64(t->fy_count, t->fy_off, n + 1, t->order, 0);
+    k_fy_fill<<<nb, 256>>>(t->fy_target, n, t->fy_off, t->fy_count, t->fy_list);
+    k_fy_sort<<<nb, 256>>>(n, t->fy_off, t->fy_list);
+    k_fy_resolve<<<nb, 256>>>(n, t->fy_target, t->fy_off, t->fy_list, t->perm, t->perm_next);
+    FEDD_CUDA(cudaGetLastError());
+    std::swap(t->perm, t->perm_next);
 }
 
 template <class F> fedd_status tguard(fedd_trainer *t, F &&f) {
@@ -685,13 +1054,6 @@ template <class F> fedd_status tguard(fedd_trainer *t, F &&f) {
     }
 }
 
-uint64_t sm64(uint64_t &s) {
-    uint64_t z = (s += 0x9E3779B97F4A7C15ULL);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
-}
-
 }  // namespace
 
 extern "C" {
@@ -706,14 +1068,18 @@ fedd_status fedd_trainer_create(int32_t hidden, int64_t n, const float *x, const
         t->device = device;
         t->H = hidden;
         t->n = n;
-        t->X.upload(x, n * 4);
-        t->ty.upload(tpsi, n);
-        t->tg.upload(tgrad, n * 4);
         const int np = t->nparams();
-        t->par.alloc(np);
-        t->grad.alloc(np);
-        t->m1.alloc(np);
-        t->m2.alloc(np);
+        t->mem.reserve(2 * Arena::bytes<float>(n * 4) + Arena::bytes<float>(n) + 4 * Arena::bytes<float>(np) +
+                       Arena::bytes<float>(1));
+        auto put = [&](DBuf<float> &b, int64_t count) { b.view(t->mem.take<float>((size_t)count), (size_t)count); };
+        put(t->X, n * 4);
+        put(t->ty, n);
+        put(t->tg, n * 4);
+        for (DBuf<float> *b : {&t->par, &t->grad, &t->m1, &t->m2}) put(*b, np);
+        put(t->lsum, 1);
+        FEDD_CUDA(cudaMemcpyAsync(t->X.p, x, n * 4 * sizeof(float), cudaMemcpyHostToDevice, 0));
+        FEDD_CUDA(cudaMemcpyAsync(t->ty.p, tpsi, n * sizeof(float), cudaMemcpyHostToDevice, 0));
+        FEDD_CUDA(cudaMemcpyAsync(t->tg.p, tgrad, n * 4 * sizeof(float), cudaMemcpyHostToDevice, 0));
         t->par.zero();
         t->m1.zero();
         t->m2.zero();
@@ -770,13 +1136,17 @@ fedd_status fedd_trainer_grad(fedd_trainer *t, float wpsi, float wgrad, float *l
     return tguard(t, [&] {
         FEDD_CUDA(cudaSetDevice(t->device));
         const int H = t->H;
-        tr_workspace(t, t->n);
-        std::vector<int64_t> id(t->n);
-        for (int64_t i = 0; i < t->n; i++) id[i] = i;
-        FEDD_CUDA(cudaMemcpy(t->idx.p, id.data(), t->n * sizeof(int64_t), cudaMemcpyHostToDevice));
-        float b3 = 0;
-        FEDD_CUDA(cudaMemcpy(&b3, t->par.p + 7 * H + H * H, sizeof b3, cudaMemcpyDeviceToHost));
-        float L = tr_forward_backward(t, t->n, wpsi, wgrad, b3);
+        if (H == kH) {
+            tr_fused(t, nullptr, t->n, wpsi, wgrad, nullptr);
+        } else {
+            tr_workspace(t, t->n);
+            DBuf<int64_t> id;  // every sample in order
+            id.alloc(t->n);
+            k_iota<<<ceil_div(t->n, 256), 256>>>(id.p, t->n);
+            tr_forward_backward(t, id.p, t->n, wpsi, wgrad);
+        }
+        float L = 0;
+        FEDD_CUDA(cudaMemcpy(&L, t->lsum.p, sizeof L, cudaMemcpyDeviceToHost));
         *loss = L / (float)t->n;
         std::vector<float> g(t->nparams());
         FEDD_CUDA(cudaMemcpy(g.data(), t->grad.p, g.size() * sizeof(float), cudaMemcpyDeviceToHost));
@@ -797,37 +1167,43 @@ fedd_status fedd_trainer_run(fedd_trainer *t, int32_t steps, int64_t batch, floa
     return tguard(t, [&] {
         FEDD_CUDA(cudaSetDevice(t->device));
         const int H = t->H;
-        tr_workspace(t, batch);
-        if (t->perm.size() != (size_t)t->n || t->rng != seed) {
-            t->perm.resize(t->n);
-            for (int64_t i = 0; i < t->n; i++) t->perm[i] = i;
+        if (H != kH) tr_workspace(t, batch);
+        if (!t->perm || t->rng != seed) {
+            tr_order(t);
+            k_iota<<<ceil_div(t->n, 256), 256>>>(t->perm, t->n);
+            FEDD_CUDA(cudaGetLastError());
             t->rng = seed;
             t->cursor = t->n;
         }
-        float L = 0;
         for (int it = 0; it < steps; it++) {
             if (t->cursor + batch > t->n) {  // reshuffle (Fisher-Yates, seeded)
-                uint64_t st = t->rng ^ (0x5851F42D4C957F2DULL * (uint64_t)(t->step + 1));
-                for (int64_t i = t->n - 1; i > 0; i--) {
-                    int64_t j = (int64_t)(sm64(st) % (uint64_t)(i + 1));
-                    std::swap(t->perm[i], t->perm[j]);
-                }
+                tr_shuffle(t, t->rng ^ (0x5851F42D4C957F2DULL * (uint64_t)(t->step + 1)));
                 t->cursor = 0;
             }
-            FEDD_CUDA(cudaMemcpy(t->idx.p, t->perm.data() + t->cursor, batch * sizeof(int64_t),
-                                 cudaMemcpyHostToDevice));
+            const int64_t *idx = t->perm + t->cursor;
             t->cursor += batch;
-            float b3 = 0;
-            FEDD_CUDA(cudaMemcpy(&b3, t->par.p + 7 * H + H * H, sizeof b3, cudaMemcpyDeviceToHost));
-            L = tr_forward_backward(t, batch, wpsi, wgrad, b3) / (float)batch;
             t->step++;
-            const float b1 = 0.9f, b2 = 0.999f;
-            const float c1 = 1.0f - std::pow(b1, (float)t->step), c2 = 1.0f - std::pow(b2, (float)t->step);
-            const int np = t->nparams();
-            k_adam<<<ceil_div(np, 256), 256>>>(t->par.p, t->grad.p, t->m1.p, t->m2.p, np, lr, b1, b2, 1e-8f, c1, c2,
-                                               1.0f / (float)batch);
-            FEDD_CUDA(cudaGetLastError());
+            AdamStep a;
+            a.lr = lr;
+            a.b1 = 0.9f;
+            a.b2 = 0.999f;
+            a.eps = 1e-8f;
+            a.c1 = 1.0f - std::pow(a.b1, (float)t->step);
+            a.c2 = 1.0f - std::pow(a.b2, (float)t->step);
+            a.scale = 1.0f / (float)batch;
+            if (H == kH) {
+                tr_fused(t, idx, batch, wpsi, wgrad, &a);
+            } else {
+                tr_forward_backward(t, idx, batch, wpsi, wgrad);
+                const int np = t->nparams();
+                k_adam<<<ceil_div(np, 256), 256>>>(t->par.p, t->grad.p, t->m1.p, t->m2.p, np, a.lr, a.b1, a.b2, a.eps,
+                                                   a.c1, a.c2, a.scale);
+                FEDD_CUDA(cudaGetLastError());
+            }
         }
+        float L = 0;
+        if (steps > 0) FEDD_CUDA(cudaMemcpy(&L, t->lsum.p, sizeof L, cudaMemcpyDeviceToHost));
+        L /= (float)batch;
         FEDD_CUDA(cudaDeviceSynchronize());
         if (last_loss) *last_loss = L;
     });
