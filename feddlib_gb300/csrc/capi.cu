@@ -242,7 +242,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
                               res && d_u != nullptr, h->d_err.p, s, lc);
         });
         stage(h, "hyper_rows", s, [&] {
-            launch_hyper_rows(h->g, h->stage_f.p, h->csr[0].rowptr.p, jac ? v00 : nullptr, res ? ru : nullptr, h->nn,
+            launch_hyper_rows(h->g, h->stage_f.p, jac ? v00 : nullptr, res ? ru : nullptr, h->nn,
                               s, lc);
         });
         break;
@@ -679,7 +679,7 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
                                dv[2], res ? drp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, n0, n1,
                                nullptr, h->coeff);
         } else
-            launch_hyper_rows(h->g, h->stage_f.p, h->csr[0].rowptr.p, dv[0], res ? dru : nullptr, n1, s, lc, n0);
+            launch_hyper_rows(h->g, h->stage_f.p, dv[0], res ? dru : nullptr, n1, s, lc, n0);
         FEDD_CUDA(cudaEventRecord(h->chunk_ev[k], s));
         FEDD_CUDA(cudaStreamWaitEvent(cs, h->chunk_ev[k], 0));
         const int64_t a0 = h->off00[k], a1 = h->off00[k + 1];

@@ -542,53 +542,68 @@ constexpr int kHStage = 100;  // floats per ring slot: three rows of 32 (values,
 constexpr int kHSlots = 96;
 
 // stage incidence t (of m) of a node into ring slot `slot` (a constant after
-// unrolling): lanes 0-23 the three rows 3 a + i of the element matrix (row
-// i = lane / 8, chunk lane % 8; column 30 of each row carries its residual
-// entry), lane 24 the slot map; each lane's destination is ring slot + 4 lane.
-// Every call commits one group, empty past the node's last incidence, so the
-// wait counts hold.
+// unrolling): lanes 0-23 the three rows 3 a + i of the element matrix (96
+// contiguous floats; column 30 of each row carries its residual entry), lane
+// 24 the slot map; each lane's destination is ring slot + 4 lane.  Every call
+// commits one group, empty past the node's last incidence, so the wait counts
+// hold.
 __device__ __forceinline__ void hyper_stage(float *dst_lane, int slot, int t, int m, const IncList &il,
                                             const uint8_t *__restrict__ slots_node,
-                                            const float *__restrict__ stage, int lane) {
+                                            const float *__restrict__ stage_lane, int lane) {
     if (t < m) {  // warp-uniform: every lane takes part in the shuffle
-        const uint32_t ea = incidence_at(il, t);
-        const int a = (int)(ea & 15u);
-        const float *Ke = stage + (size_t)(ea >> 4) * kElemStride;
-        const void *src = lane < 24 ? static_cast<const void *>(Ke + 32 * (3 * a + (lane >> 3)) + 4 * (lane & 7))
+        const uint32_t ea = m <= 32 ? __shfl_sync(0xffffffffu, il.lo, t & 31) : incidence_at(il, t);
+        const void *src = lane < 24 ? static_cast<const void *>(stage_lane + (size_t)(ea >> 4) * kElemStride + 96 * (ea & 15u))
                                     : static_cast<const void *>(slots_node + t * kSlotStride);
         if (lane < 25) cp_async16(dst_lane + slot * kHStage, src);
     }
     cp_async_commit();
 }
 
-// Accumulators: three planes (row components i) of stride 3 max_adj + 1, the
-// last word of each a scratch word that lanes 30 and 31 write.
-__global__ void __launch_bounds__(256) k_hyper_rows(const int64_t *__restrict__ inc_ptr,
+// The node's accumulators are one run of 9 K floats in the order of its CSR
+// values (three rows of 3 K), so the write-out is a linear copy: pairs of
+// values as 16-byte stores, the run shifted by one word when the values start
+// at an odd multiple of 8 bytes.  Behind it lane 30 keeps the node's residual
+// (column 30 of the element's rows), which the same updates accumulate, and
+// lane 31 a scratch word.  The kernel is bound by latency and the shared-memory
+// pipe (76 %) together: 1,915 us at 64^3 x 6 tets and 257 us at 32^3 x 6 (75 %
+// of the copy bandwidth in DRAM bytes), against 2,160 and 285 us with three
+// planes of fixed stride, 8-byte stores, a separate residual sum and eight
+// warps per CTA.  Slower: reading the rows straight into registers without the
+// ring (334 us at 32^3), a ring running on across the nodes of a warp's run
+// (298), the hardware FP32 -> FP64 conversion in place of f2d_exact (294).
+constexpr int kHPad = 8;  // words besides the 9 K
+__global__ void __launch_bounds__(128) k_hyper_rows(const int64_t *__restrict__ inc_ptr,
                                                     const uint32_t *__restrict__ inc,
                                                     const uint8_t *__restrict__ slots,
                                                     const int64_t *__restrict__ adj_ptr,
-                                                    const float *__restrict__ stage, const int64_t *__restrict__ rowptr,
-                                                    double *vals, double *res, int64_t nnodes, int max_adj,
+                                                    const float *__restrict__ stage,
+                                                    double *vals, double *res, int64_t nnodes, int words,
                                                     int64_t n_begin) {
     extern __shared__ __align__(16) float sacc[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int ps = 3 * max_adj + 1;
-    float *ring = sacc + (size_t)w * (kHRing * kHStage + ((3 * ps + 3) & ~3));
-    float *acc = ring + kHRing * kHStage;
+    float *ring = sacc + (size_t)w * (kHRing * kHStage + words);
+    float *mem = ring + kHRing * kHStage;
     const bool lw = lane < 30;
     const int b = lw ? lane / 3 : 0, j = lw ? lane - 3 * (lane / 3) : 0;
     float *dst_lane = ring + 4 * lane;
     const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kHSlots) + b;
+    const float *pV = ring + lane, *stage_lane = stage + 4 * lane;
     for (int64_t n = n_begin + (int64_t)blockIdx.x * nw + w; n < nnodes; n += (int64_t)gridDim.x * nw) {
         const int64_t i0 = inc_ptr[n], i1 = inc_ptr[n + 1];
         const int m = (int)(i1 - i0);
         const IncList il = load_incidences(inc, i0, m, lane);
         const uint8_t *slots_node = slots + i0 * kSlotStride;
 #pragma unroll
-        for (int t = 0; t < kHRing - 1; t++) hyper_stage(dst_lane, t, t, m, il, slots_node, stage, lane);
-        const int K = (int)(adj_ptr[n + 1] - adj_ptr[n]);
-        for (int c = lane; c < 3 * K; c += 32) acc[c] = acc[ps + c] = acc[2 * ps + c] = 0.0f;
-        float r = 0.0f;
+        for (int t = 0; t < kHRing - 1; t++) hyper_stage(dst_lane, t, t, m, il, slots_node, stage_lane, lane);
+        const int64_t a0 = adj_ptr[n];
+        const int K = (int)(adj_ptr[n + 1] - a0), len = 9 * K;
+        double *out = vals + 9 * a0;
+        const int shift = (int)((reinterpret_cast<uintptr_t>(out) >> 3) & 1);
+        float *acc = mem + shift;
+        for (int c = 4 * lane; c < len + kHPad; c += 128)
+            *reinterpret_cast<float4 *>(mem + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int st = lw ? 3 * K : (lane == 30 ? 1 : 0), mul = lw ? 3 : 0;
+        float *d0 = acc + (lw ? j : (lane == 30 ? len : len + 3));
         for (int t0 = 0; t0 < m; t0 += kHRing) {
 #pragma unroll
             for (int rs = 0; rs < kHRing; rs++) {
@@ -598,24 +613,25 @@ __global__ void __launch_bounds__(256) k_hyper_rows(const int64_t *__restrict__ 
                 // the slot's copies are visible to the warp, and every lane is
                 // done with the slot consumed in the previous step, refilled next
                 __syncwarp();
-                hyper_stage(dst_lane, (rs + kHRing - 1) % kHRing, t + kHRing - 1, m, il, slots_node, stage, lane);
-                const float *S = ring + rs * kHStage;
-                float *dst = acc + (lw ? 3 * pS[4 * rs * kHStage] + j : ps - 1);
-                dst[0] += S[lane];
-                dst[ps] += S[32 + lane];
-                dst[2 * ps] += S[64 + lane];
-                r += S[32 * (lane < 3 ? lane : 0) + kElemResCol];  // row i = lane's residual entry
+                hyper_stage(dst_lane, (rs + kHRing - 1) % kHRing, t + kHRing - 1, m, il, slots_node, stage_lane, lane);
+                float *dst = d0 + mul * pS[4 * rs * kHStage];
+                dst[0] += pV[rs * kHStage];
+                dst[st] += pV[rs * kHStage + 32];
+                dst[2 * st] += pV[rs * kHStage + 64];
             }
         }
         cp_async_wait<0>();
         __syncwarp();
-        if (vals) {
-            double *out = vals + rowptr[3 * n];
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-                for (int c = lane; c < 3 * K; c += 32) st_cs(out + i * 3 * K + c, f2d_exact(acc[i * ps + c]));
+        if (vals && len > 0) {
+            if (shift && lane == 31) st_cs(out, f2d_exact(acc[0]));
+            const int pairs = (len - shift) >> 1;
+            for (int c = lane; c < pairs; c += 32) {
+                const float2 x = *reinterpret_cast<const float2 *>(mem + 2 * shift + 2 * c);
+                __stcs(reinterpret_cast<double2 *>(out + shift) + c, make_double2(f2d_exact(x.x), f2d_exact(x.y)));
+            }
+            if (((len - shift) & 1) && lane == 30) st_cs(out + len - 1, f2d_exact(acc[len - 1]));
         }
-        if (res && lane < 3) res[3 * n + lane] = f2d_exact(r);
+        if (res && lane < 3) res[3 * n + lane] = f2d_exact(acc[len + lane]);
         __syncwarp();
     }
 }
@@ -979,21 +995,23 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
     lc.n++;
 }
 
-void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr, double *vals, double *res,
-                       int64_t nnodes, cudaStream_t s, LaunchCounter &lc, int64_t n_begin) {
-    const int warps = 8;
-    const int acc_words = (3 * (3 * g.max_adj + 1) + 3) & ~3;
-    size_t smem = (size_t)warps * (kHRing * kHStage + acc_words) * sizeof(float);
+void launch_hyper_rows(const Graph &g, const float *stage, double *vals, double *res, int64_t nnodes, cudaStream_t s,
+                       LaunchCounter &lc, int64_t n_begin) {
+    const int warps = 4;
+    const int words = (9 * g.max_adj + kHPad + 3) & ~3;
+    const size_t smem = (size_t)warps * (kHRing * kHStage + words) * sizeof(float);
     if (smem > 48 * 1024)
         FEDD_CUDA(cudaFuncSetAttribute(k_hyper_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    unsigned grid = (unsigned)std::min<int64_t>((nnodes - n_begin + warps - 1) / warps, (int64_t)sm_count() * 64);
+    // about six nodes per warp (3.5 to 7 measured alike; one or fourteen cost
+    // 5 %), or all the chip's warps on a small mesh
+    const int64_t nodes = nnodes - n_begin, ctas = (nodes + warps - 1) / warps;
+    const unsigned grid = (unsigned)std::min<int64_t>(ctas, std::max<int64_t>((ctas + 5) / 6, (int64_t)sm_count() * 16));
     if (grid == 0) return;
-    k_hyper_rows<<<grid, 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage, rowptr, vals,
-                                                  res, nnodes, g.max_adj, n_begin);
+    k_hyper_rows<<<grid, 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage, vals, res, nnodes,
+                                                words, n_begin);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }
-
 
 void launch_hyper_residual(const Graph &g, const float *geo, const int32_t *conn, int64_t ne, const double *u,
                            const LawParams &law, const HyperTables &tab, const QPDerivs *qpd,

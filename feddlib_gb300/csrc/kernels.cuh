@@ -97,9 +97,9 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
                        const HyperTables &tab, const QPDerivs *qpd, const uint8_t *qp_fallback, float *stage,
                        int want_res, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                        int64_t e_end = -1);
-void launch_hyper_rows(const Graph &g, const float *stage, const int64_t *rowptr, double *vals, double *res,
-                       int64_t nnodes, cudaStream_t s, LaunchCounter &lc,
-                       int64_t n_begin = 0);
+// vals: the values of block (0,0), whose node n starts at 9 adj_ptr[n]
+void launch_hyper_rows(const Graph &g, const float *stage, double *vals, double *res, int64_t nnodes, cudaStream_t s,
+                       LaunchCounter &lc, int64_t n_begin = 0);
 // the residual alone, same values: element residuals (40 floats per element in
 // stage), then the per-node sums
 void launch_hyper_residual(const Graph &g, const float *geo, const int32_t *conn, int64_t ne, const double *u,
