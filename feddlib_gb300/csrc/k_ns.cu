@@ -46,7 +46,8 @@ constexpr int kTabT = 0;        // T[a][kc][lane][4]  3840
 constexpr int kTabKS = 3840;    // KS[a][b][6]        600
 constexpr int kTabR = 4440;     // R[a][b][4]         400
 constexpr int kTabY = 4840;     // Y[b][p][4] (c < 3) 160
-static_assert(kTabY + 160 == kNSTab, "table size");
+constexpr int kTabB = 5000;     // T and KS as the B operand of the NA product, in na_off's word order: 4480
+static_assert(kTabY + 160 == kTabB && kTabB + 4480 == kNSTab, "table size");
 constexpr int kVelTab = 560;    // floats of tables the velocity-row kernel keeps in shared memory (R, Y)
 
 // reference P2 gradients at the vertices, d_c phi_k at vertex m: with the
@@ -98,7 +99,7 @@ static_assert(kRecSmem <= 227 * 1024 && kRecGroups * 128 <= 512, "one CTA per SM
 // byte offset of (row, k) in a K-major, unswizzled operand: 8-row x 16-byte
 // core matrices, the two of one K step 128 B apart (LBO), row groups 256 B
 // apart (SBO), K steps `step` bytes apart
-__device__ __forceinline__ int na_off(int row, int k, int step) {
+__host__ __device__ __forceinline__ int na_off(int row, int k, int step) {
     return (k >> 3) * step + (row >> 3) * 256 + ((k >> 2) & 1) * 128 + (row & 7) * 16 + (k & 3) * 4;
 }
 
@@ -160,24 +161,15 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__res
     uint64_t *mbar = reinterpret_cast<uint64_t *>(rs + kRecBarOff) + gi;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(rs + kRecBarOff + 8 * kRecGroups);
     uint8_t *sW = sAh + wl * kRecWarpBytes;  // this warp's staging, between the MMAs
-    // B = Y^T: row n, column kk
+    // B = Y^T: row n, column kk; the table holds T and KS in the operand's word
+    // order (na_off), zero padded
+#pragma unroll 3
     for (int t = tid; t < kNAN * kNAK; t += kRecThreads) {
-        const int n = t / kNAK, kk = t - kNAK * (t / kNAK);
-        float y = 0.0f;
-        if (n < 100) {
-            const int a = n / 10, b = n % 10;
-            if (kk < 30) {
-                const int c = kk / 10, k = kk % 10;
-                // T[a][kc][lane = 3 b + c][k % 4] in the device table
-                y = dens * gtab[kTabT + ((a * 3 + k / 4) * 32 + 3 * b + c) * 4 + k % 4];
-            } else if (kk < 36) {
-                y = visc_dens * gtab[kTabKS + (a * 10 + b) * 6 + (kk - 30)];
-            }
-        }
+        const int r = t % (kNAN * 8), kk = t / (kNAN * 8) * 8 + ((r >> 5) & 1) * 4 + (r & 3);
+        const float y = (kk < 30 ? dens : visc_dens) * gtab[kTabB + t];
         const uint32_t h = to_tf32(y);
-        const int o = na_off(n, kk, kNAStepB);
-        *reinterpret_cast<uint32_t *>(sBh + o) = h;
-        *reinterpret_cast<uint32_t *>(sBl + o) = to_tf32(y - __uint_as_float(h));
+        reinterpret_cast<uint32_t *>(sBh)[t] = h;
+        reinterpret_cast<uint32_t *>(sBl)[t] = to_tf32(y - __uint_as_float(h));
     }
     if (tid < 32) tc::tmem_alloc(tslot, 128 * kRecGroups);
     if (gt == 0) tc::mbar_init(mbar, 1);
@@ -191,7 +183,9 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__res
     const int64_t ntiles = (e_end - e_begin + kRecTile - 1) / kRecTile;
     uint32_t phase = 0;
     bool ok = true;
-    for (int64_t tile = (int64_t)blockIdx.x * kRecGroups + gi; tile < ntiles; tile += (int64_t)gridDim.x * kRecGroups) {
+    // tiles go to the CTAs first and to their groups then, so that few tiles
+    // spread over as many SMs
+    for (int64_t tile = blockIdx.x + (int64_t)gridDim.x * gi; tile < ntiles; tile += (int64_t)gridDim.x * kRecGroups) {
         // every thread stays for the collective steps; threads past the range
         // recompute the last element and store nothing
         const int64_t e_lane = e_begin + tile * kRecTile + gt;
@@ -992,6 +986,10 @@ void ns_upload_tables(float *d_tables, cudaStream_t s) {
         for (int b = 0; b < 10; b++)
             for (int p = 0; p < 4; p++)
                 for (int c = 0; c < 3; c++) h[kTabY + (b * 4 + p) * 4 + c] = t.Y[c][p][b];
+        for (int ab = 0; ab < 100; ab++)
+            for (int kk = 0; kk < 36; kk++)
+                h[kTabB + na_off(ab, kk, kNAStepB) / 4] =
+                    kk < 30 ? t.T[kk / 10][ab / 10][ab % 10][kk % 10] : t.KS[ab / 10][ab % 10][kk - 30];
         return h;
     }();
     FEDD_CUDA(cudaMemcpyAsync(d_tables, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -1004,7 +1002,7 @@ void launch_ns_record(const float *geo, const int32_t *conn2, const int32_t *con
     const int64_t count = e_end - e_begin;
     if (count <= 0) return;
     // persistent CTAs, one per SM (shared memory, all 512 TMEM columns)
-    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)kRecTile * kRecGroups), (int64_t)sm_count_ns());
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)kRecTile), (int64_t)sm_count_ns());
     auto kern = residual_only ? k_ns_record<true> : k_ns_record<false>;
     FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRecSmem));
     kern<<<grid, kRecThreads, kRecSmem, s>>>(geo, conn2, conn1, ne, u, p, rec, d_err, e_begin, e_end, d_tables, visc_dens,

@@ -75,7 +75,7 @@ constexpr int kElemResCol = 30;    // column of each row holding its residual en
 constexpr int kGNStride = 992;     // floats per element
 constexpr int kGNRes = 960;        // offset of the residual row
 constexpr int kNSRecord = 228;     // floats per element record (Navier-Stokes): 128 + NA[10][10]
-constexpr int kNSTab = 5000;      // floats of the Navier-Stokes device tables
+constexpr int kNSTab = 9480;      // floats of the Navier-Stokes device tables
 constexpr int kLapTab = 610;      // doubles of the Laplace device tables
 constexpr int kNSResRecord = 168; // floats per element record when only the residual is assembled
 constexpr int kLapStrideP1 = 16;   // doubles: 10 packed K + 4 load + pad
