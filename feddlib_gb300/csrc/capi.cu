@@ -282,8 +282,8 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         // assemble the pressure rows as well
         stage(h, "ns_vel_rows", s, [&] {
             launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab.p, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
-                               v00, v01, res ? ru : nullptr, vd, dn, h->prm.linearization, jac, h->g.max_adj,
-                               h->max_padj, h->ns_fused ? h->vmap.p : nullptr, h->csr[2].rowptr.p, v10,
+                               v00, v01, res ? ru : nullptr, dn, h->prm.linearization, h->g.max_adj,
+                               h->max_padj, h->ns_fused, h->csr[2].rowptr.p, v10,
                                res ? rp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, 0, -1, h->work.p,
                                h->coeff);
         });
@@ -674,8 +674,8 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
         }
         if (ns) {
             launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab.p, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
-                               dv[0], dv[1], res ? dru : nullptr, vd_ns, (float)h->prm.density, h->prm.linearization,
-                               1, h->g.max_adj, h->max_padj, h->ns_fused ? h->vmap.p : nullptr, h->csr[2].rowptr.p,
+                               dv[0], dv[1], res ? dru : nullptr, (float)h->prm.density, h->prm.linearization,
+                               h->g.max_adj, h->max_padj, h->ns_fused, h->csr[2].rowptr.p,
                                dv[2], res ? drp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, n0, n1,
                                nullptr, h->coeff);
         } else

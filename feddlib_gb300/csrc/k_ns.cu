@@ -446,248 +446,319 @@ __global__ void k_ns_node_info(const int64_t *__restrict__ inc_ptr, const int64_
                         K | (Kp << 8) | (m << 16));
 }
 
-// velocity rows: block (0,0) and (0,1) values and the velocity residual.
-// One warp per row node a.  Each incidence's record head (g, Bs, u, p), the
-// 48-byte window holding NA[a][:] and its slot map are staged into a ring of
-// kVRing shared-memory slots, kVRing - 1 incidences ahead, by one 16-byte
-// cp.async per lane (lanes 0-20 the head, 21-23 the NA window, 24 the slot
-// map): 400 bytes instead of the whole 912-byte record.
-// Shared-memory accumulators form three planes, one per row component i,
-// each holding (column slot, j) at 3 slot + j and the pressure columns after
-// the 3 K velocity ones; a lane's update of an incidence is three 4-byte
-// read-modify-writes (32-bit shared accesses run at twice the bytes per clock
-// of 16-byte ones on this part, and no padding word is moved).
-// The incidence loop is unrolled by the ring size so every ring offset is an
-// immediate; idle lanes write a scratch word instead of branching.
+// velocity rows: block (0,0) and (0,1) values and the velocity residual, and
+// at the vertices of a mesh with a verified vertex map the pressure row too.
+// A warp works on two row nodes at a time, one per half warp, an incidence of
+// each per step: with lanes (p, j) of 15 the half's lane owns the columns
+// (b, j) of the two nodes b = 2 p and 2 p + 1, so every value that the ten
+// nodes share (the gradient rows g[j], Bs, the wait, the staging) is read or
+// done once for two incidences.  Warps claim eight consecutive nodes and pair
+// them by their number of incidences, so that the halves end together (on a
+// lattice vertices, 24 incidences, and edge nodes, 4 or 6, alternate).
+// Each incidence's record head (g, Bs, u, p), the 48-byte window holding
+// NA[a][:] and its slot map (25 chunks of 16 bytes) are copied by cp.async
+// into the half's ring of kVRing shared-memory slots, kVRing - 1 incidences
+// ahead.  Each half accumulates in three runs in the order of the CSR
+// values: the 9 K velocity values, the 3 Kp of block (0,1) and the 3 K of the
+// pressure row, so the write-out is a linear copy, pairs of values as 16-byte
+// stores; each run is shifted by one word when its values start at an odd
+// multiple of 8 bytes.  Lanes without work update a scratch word.
 // With a generalized-Newtonian viscous stage (the dense element matrix with
 // rows padded to 32 floats, kGNStride floats per element) each slot also
-// holds the element's three rows 3 a + i (lanes 0-23, second copy) and an
-// 8-float window holding its residual entries 3 a .. 3 a + 2 (lanes 24-25),
-// which the lanes fold into the same accumulation: no separate pass re-reads
-// and re-writes the rows.
+// holds the element's three rows 3 a + i and an 8-float window holding its
+// residual entries 3 a .. 3 a + 2 (26 more chunks), which the lanes fold into
+// the same accumulation: no separate pass re-reads and re-writes the rows.
+// Bound by the shared-memory pipe (about 53 wavefronts per incidence, most of
+// them the accumulators' scattered updates and the broadcast 16-byte reads).
+// At 48^3 x 6 tets 1,299 us, against 1,480 us with one node per warp, three
+// planes of accumulators and 8-byte stores; without the Newton term, whose
+// reads and products the Picard form leaves out, 197 us against 240 at
+// 27 x 19 x 33 x 6 tets in file order; with the viscous rows 494 us against 522
+// at 32^3 x 6.  Groups of four nodes 1,319 us, rings of three or six slots
+// 1,389 and 1,423, eleven warps per CTA (80 registers, spills) 1,461.
 constexpr int kVRing = 4;
 constexpr int kVStage = 100;  // floats per ring slot: record head 84 | NA window 12 | slot map 16 B
 constexpr int kVNA = kRecVel, kVSlots = kRecVel + 12;
 constexpr int kVGn = kVStage, kVGnRes = kVStage + 96, kVStageGn = kVStage + 104;
-static_assert(kVSlots + 4 == kVStage && kRecVel % 4 == 0, "ring slot layout: lane L copies floats [4 L, 4 L + 4)");
+static_assert(kVSlots + 4 == kVStage && kRecVel % 4 == 0, "ring slot layout: chunk c holds floats [4 c, 4 c + 4)");
+// the ring and the accumulators of a half are 16 mod 32 words, so the halves'
+// accesses to the same place of theirs differ in banks
+static_assert(kVRing * kVStage % 32 == 16 && kVRing * kVStageGn % 32 == 16, "half-warp bank offset");
+// warps per CTA at most, two CTAs per SM (shared memory: about 10.3 KB per warp
+// on the structured meshes, 13.6 with the viscous rows)
+__host__ __device__ constexpr int vel_warps(bool gn) { return gn ? 8 : 10; }
 
-// stage incidence t (of m) into ring slot `slot` (a constant after unrolling);
-// every call commits one group, empty past the node's last incidence, so the
-// wait counts hold.  src_lane = 4 lane floats into the record for head lanes,
-// kRecNA + 4 (lane - 21) for NA-window lanes; dst_lane = ring + 4 lane.
-template <bool GN>
-__device__ __forceinline__ void stage_vel(float *dst_lane, int slot, int t, int m, const IncList &il,
-                                          const float *__restrict__ rec, int src_lane, int kind,
-                                          const uint8_t *__restrict__ slots_node, const float *__restrict__ gstage,
-                                          int lane) {
-    constexpr int kStg = GN ? kVStageGn : kVStage;
-    if (t < m) {
-        // one shuffle when the node's list fits the low word (warp-uniform)
-        const uint32_t ea = m <= 32 ? __shfl_sync(0xffffffffu, il.lo, t & 31) : incidence_at(il, t);
-        const int a = (int)(ea & 15u);
-        // NA[a][0..9] starts 8 bytes into a 16-byte boundary when a is odd
-        const float *r = rec + (size_t)(ea >> 4) * kNSRecord + src_lane + (kind == 1 ? 10 * a - 2 * (a & 1) : 0);
-        const void *src = kind == 2 ? static_cast<const void *>(slots_node + t * kSlotStride) : static_cast<const void *>(r);
-        if (kind < 3) cp_async16(dst_lane + slot * kStg, src);
-        if (GN && lane < 26) {
-            const float *Ke = gstage + (size_t)(ea >> 4) * kGNStride;
-            // lane < 24: row 3 a + (lane >> 3), chunk lane & 7; lanes 24, 25: the residual window
-            const float *g = lane < 24 ? Ke + 32 * (3 * a + (lane >> 3)) + 4 * (lane & 7)
-                                       : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (lane - 24);
-            cp_async16(dst_lane - 4 * lane + slot * kStg + (lane < 24 ? kVGn + 4 * lane : kVGnRes + 4 * (lane - 24)), g);
-        }
-    }
-    cp_async_commit();
+// words of one half's accumulators: the three runs, each with its shift and
+// padding to 16 bytes, 32 words of the pressure residual's sum, the scratch word
+__host__ __device__ __forceinline__ int vel_run_words(int len) { return (len + 1 + 3) & ~3; }
+__host__ __device__ __forceinline__ int vel_acc_words(int max_adj, int max_padj, bool pres) {
+    const int w = vel_run_words(9 * max_adj) + vel_run_words(3 * max_padj) + (pres ? vel_run_words(3 * max_adj) : 0) + 36;
+    return (w + 31) & ~31;
 }
 
-// velocity residual of node n: row (a, i) sums rj over the lanes 3 b + i and
-// rb over the lanes 4 i + p (strided tree sums leave them in lanes i = 0..2
-// and 4 i); rg, in lane i, is the viscous residual of a generalized-Newtonian
-// fluid.  uu (N(u) u + viscous) + up (-B^T p), with the residual's block factors
+// len values of one half warp's run (mem + shift) out as FP64
+__device__ __forceinline__ void vel_write(const float *mem, int shift, int len, double *out, int hl) {
+    if (shift && len > 0 && hl == 15) st_cs(out, f2d_exact(mem[1]));
+    const int pairs = len > 0 ? (len - shift) >> 1 : 0;
+    for (int c = hl; c < pairs; c += 16) {
+        const float2 x = *reinterpret_cast<const float2 *>(mem + 2 * shift + 2 * c);
+        __stcs(reinterpret_cast<double2 *>(out + shift) + c, make_double2(f2d_exact(x.x), f2d_exact(x.y)));
+    }
+    if (len > 0 && ((len - shift) & 1) && hl == 14) st_cs(out + len - 1, f2d_exact(mem[shift + len - 1]));
+}
+__device__ __forceinline__ int odd8(const void *p) { return (int)((reinterpret_cast<uintptr_t>(p) >> 3) & 1); }
+
+// velocity residual of the half's node n: row (a, i) sums rj over the lanes
+// (p, i), the nodes b = 2 p and 2 p + 1, and rb over the lanes 4 i + q by
+// strided trees (in b: (((0+1)+(2+3))+((4+5)+(6+7)))+(8+9)); rg, in lane i, is
+// the viscous residual of a generalized-Newtonian fluid.
+// uu (N(u) u + viscous) + up (-B^T p), with the residual's block factors
 template <bool GN>
-__device__ __forceinline__ void vel_residual_out(float rj, float rb, float rg, int64_t n, int lane, const NSCoeff &co,
-                                                 double *res_u) {
-    float x = lane < 30 ? rj : 0.0f, z = lane < 12 ? rb : 0.0f;
-#pragma unroll
-    for (int d = 3; d < 32; d *= 2) {
-        const float y = __shfl_down_sync(0xffffffffu, x, d);
-        if (lane + d < 32) x += y;
-    }
-#pragma unroll
-    for (int d = 1; d < 4; d *= 2) {
-        const float y = __shfl_down_sync(0xffffffffu, z, d);
-        if (lane + d < 32) z += y;
-    }
-    z = __shfl_sync(0xffffffffu, z, lane < 3 ? 4 * lane : 0);
-    const float cuu = (float)co.uu, s = fmaf(cuu, x, (float)co.up * z);
-    if (lane < 3) res_u[3 * n + lane] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
+__device__ __forceinline__ void vel_residual_out(float rj0, float rj1, float rb, float rg, int64_t n, int hl, bool node,
+                                                 const NSCoeff &co, double *res_u) {
+    const float x = hl < 15 ? rj0 + rj1 : 0.0f;
+    float z = hl < 12 ? rb : 0.0f;
+    const float x2 = x + __shfl_down_sync(0xffffffffu, x, 3, 16);
+    const float x4 = x2 + __shfl_down_sync(0xffffffffu, x2, 6, 16);
+    const float xs = x4 + __shfl_down_sync(0xffffffffu, x, 12, 16);
+    z += __shfl_down_sync(0xffffffffu, z, 1, 16);
+    z += __shfl_down_sync(0xffffffffu, z, 2, 16);
+    z = __shfl_sync(0xffffffffu, z, hl < 3 ? 4 * hl : 0, 16);
+    const float cuu = (float)co.uu, s = fmaf(cuu, xs, (float)co.up * z);
+    if (node && hl < 3) res_u[3 * n + hl] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
 }
 
-template <bool GN>
-__global__ void __launch_bounds__(512, 2) k_ns_vel_rows(const int4 *__restrict__ ninfo, const uint32_t *__restrict__ inc,
-                                                        const uint8_t *__restrict__ slots, const float *__restrict__ rec,
-                                                        const float *__restrict__ gtab, const int64_t *__restrict__ rowptr00,
-                                                        const int64_t *__restrict__ rowptr01, double *vals00, double *vals01,
-                                                        double *res_u, int64_t nnodes, float dens, int newton, int max_adj,
-                                                        int max_padj, int64_t n_begin, int fused,
-                                                        const int64_t *__restrict__ rowptr10, double *vals10, double *res_p,
-                                                        const float *__restrict__ gstage, unsigned long long *work,
-                                                        NSCoeff co) {
+template <bool GN, bool NEWTON>
+__global__ void __launch_bounds__(32 * vel_warps(GN), 2)
+    k_ns_vel_rows(const int4 *__restrict__ ninfo, const uint32_t *__restrict__ inc, const uint8_t *__restrict__ slots,
+                  const float *__restrict__ rec, const float *__restrict__ gtab, const int64_t *__restrict__ rowptr00,
+                  const int64_t *__restrict__ rowptr01, double *vals00, double *vals01, double *res_u, int64_t nnodes,
+                  float dens, int group, int acc_words, int64_t n_begin, const int64_t *__restrict__ rowptr10,
+                  double *vals10, double *res_p, const float *__restrict__ gstage, unsigned long long *work, NSCoeff co) {
     constexpr int kStg = GN ? kVStageGn : kVStage;
     extern __shared__ __align__(16) float smem[];
-    // the W table scaled by the Newton weight (rho, or 0 for the Picard form)
-    // and the B^T table negated: sR = wn R[a][b][4], sY = -Y[a][p][4]; the
-    // diagonal part NA comes with each record
+    // the W table scaled by the Newton weight rho and the B^T table negated:
+    // sR = rho R[a][b][4], sY = -Y[a][p][4]; the diagonal part NA comes with
+    // each record (and is all of the Picard form)
     float *sR = smem, *sY = smem + 400;
     static_assert(kTabY == kTabR + 400 && kVelTab == 560, "R and Y are adjacent");
-    const float wn = newton ? dens : 0.0f;
-    for (int t = threadIdx.x; t < kVelTab; t += blockDim.x) smem[t] = t < 400 ? wn * gtab[kTabR + t] : -gtab[kTabR + t];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int ps = 3 * max_adj + max_padj + 1;  // plane stride: + one scratch word that idle lanes write
-    // with a vertex map a fourth plane holds the vertex's pressure row (1,0)
-    const int planes = fused ? 4 : 3;
-    float *ring = smem + kVelTab + (size_t)w * (kVRing * kStg + ((planes * ps + 3) & ~3));
-    float *acc = ring + kVRing * kStg;
+    for (int t = threadIdx.x; t < kVelTab; t += blockDim.x) smem[t] = t < 400 ? dens * gtab[kTabR + t] : -gtab[kTabR + t];
     __syncthreads();
-    // lane roles: (b, j) of the NA / W part for lane < 30, (i, p) = (bi, bp) of the B^T part for lane < 12
-    const bool lw = lane < 30, lb = lane < 12;
-    const int b = lw ? lane / 3 : 0, j = lw ? lane - 3 * (lane / 3) : 0;
-    const int bi = lane >> 2, bp = lane & 3;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15, nw = blockDim.x >> 5;
+    float *ring = smem + kVelTab + (size_t)(2 * w + h) * (kVRing * kStg + acc_words);
+    float *mem = ring + kVRing * kStg;
+    float *sum32 = mem + acc_words - 36, *scratch = mem + acc_words - 4;
+    // lane roles in the half: (p, j) of the NA / W part for hl < 15, (i, q) = (bi, bq) of the B^T part for hl < 12
+    const bool lw = hl < 15, lb = hl < 12;
+    const int p = lw ? hl / 3 : 0, j = lw ? hl - 3 * (hl / 3) : 0;
+    const int bi = hl >> 2, bq = hl & 3;
     const float e0 = j == 0 ? 1.0f : 0.0f, e1 = j == 1 ? 1.0f : 0.0f, e2 = j == 2 ? 1.0f : 0.0f;
     // lane-constant addresses in ring slot 0 and in the tables
     const float *pG = ring + kRecG + 12 * j;
-    const float *pU = ring + kRecU + 3 * b + j;
-    const float *pNA = ring + kVNA + b;
-    const float *pBS = ring + kRecBS + 4 * bi;
+    const float *pU = ring + kRecU + 6 * p + j;
+    const float *pNA = ring + kVNA + 2 * p;
+    const float *pBS = ring + kRecBS + 4 * (lb ? bi : 0);
     const float *pBSj = ring + kRecBS + 4 * j;
-    const float *pP = ring + kRecP + bp;
-    const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kVSlots) + b;
-    const uint8_t *pLoc = reinterpret_cast<const uint8_t *>(ring + kVSlots) + kSlotLocal;
-    const uint8_t *pSp = reinterpret_cast<const uint8_t *>(ring + kVSlots) + 10 + bp;
-    const float *pR = sR + 4 * b;
-    const float *pY = sY + 4 * bp;
-    const float *pYb = sY + 16 * b;
-    // staging roles: 0 record head, 1 NA window, 2 slot map, 3 idle
-    const int kind = lane < kRecVel / 4 ? 0 : (lane < kRecVel / 4 + 3 ? 1 : (lane == kRecVel / 4 + 3 ? 2 : 3));
-    const int src_lane = kind == 0 ? 4 * lane : kRecNA + 4 * (lane - kRecVel / 4);
-    float *dst_lane = ring + 4 * lane;
-    // with `work`, nodes come from a global counter, one per warp step, so
+    const float *pP = ring + kRecP + bq;
+    const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kVSlots);
+    const float *pR = sR + 8 * p, *pY = sY + 4 * bq, *pYb = sY + 32 * p;
+    // chunk hl, and chunk 16 + hl for hl < 9: record head (to 20), NA window (21-23), slot map (24)
+    const char *src1 = reinterpret_cast<const char *>(rec + 4 * hl);
+    const char *src2 = reinterpret_cast<const char *>(hl < 5 ? rec + 64 + 4 * hl : rec + kRecNA + 4 * (hl - 5));
+    float *dst_lane = ring + 4 * hl;
+    // with `work`, nodes come from a global counter, a group per warp step, so
     // all warps stay on one sharp front of the sweep and the ten readers of
-    // an element's record come close in time (a fixed stride gives each warp
-    // nodes of one lattice parity: vertex-heavy warps fall behind, the front
-    // smears, and at 64^3 x 6 the records were read five times from DRAM)
-    for (int64_t it = n_begin + (int64_t)blockIdx.x * nw + w;; it += (int64_t)gridDim.x * nw) {
+    // an element's record come close in time
+    for (int64_t it = n_begin + group * ((int64_t)blockIdx.x * nw + w);; it += group * (int64_t)gridDim.x * nw) {
         if (work) {
             unsigned long long k = 0;
-            if (lane == 0) k = atomicAdd(work, 1ull);
+            if (lane == 0) k = atomicAdd(work, (unsigned long long)group);
             it = n_begin + (int64_t)__shfl_sync(0xffffffffu, k, 0);
         }
         if (it >= nnodes) break;
-        const int64_t n = it;
-        const int4 inf = ninfo[n];
-        const int64_t i0 = node_i0(inf);
-        const int m = node_m(inf);
-        const IncList il = load_incidences(inc, i0, m, lane);
-        const uint8_t *slots_node = slots + i0 * kSlotStride;
+        // lane k < group: node it + k; rank 0 has the most incidences
+        const bool member = (lane & 7) < group && it + (lane & 7) < nnodes;
+        const int4 inf4 = member ? ninfo[it + (lane & 7)] : make_int4(0, 0, -1, 0);
+        const int m4 = node_m(inf4);
+        int rank = 0;
 #pragma unroll
-        for (int t = 0; t < kVRing - 1; t++)
-            stage_vel<GN>(dst_lane, t, t, m, il, rec, src_lane, kind, slots_node, gstage, lane);
-        const int K = node_k(inf), Kp = node_kp(inf);
-        // the P1 node at this vertex, whose pressure row this warp assembles too
-        const int qp = inf.z;
-        for (int c = lane; c < 3 * K + Kp; c += 32) acc[c] = acc[ps + c] = acc[2 * ps + c] = 0.0f;
-        if (qp >= 0)
-            for (int c = lane; c < 3 * K; c += 32) acc[3 * ps + c] = 0.0f;
-        float rj = 0.0f, rb = 0.0f, rq = 0.0f, rg = 0.0f;
-        // the table rows of the current local index a; incidences come sorted
-        // by a, so they reload only when a run of equal a ends
-        int a_cur = -1;
-        float4 rr = make_float4(0.f, 0.f, 0.f, 0.f), y = rr, yq = rr;
-        for (int t0 = 0; t0 < m; t0 += kVRing) {
-#pragma unroll
-            for (int r = 0; r < kVRing; r++) {
-                const int t = t0 + r;
-                if (t >= m) break;
+        for (int k = 0; k < 8; k++) {
+            const int mk = __shfl_sync(0xffffffffu, m4, k);
+            rank += mk > m4 || (mk == m4 && k < (lane & 7));
+        }
+#pragma unroll 1
+        for (int pair = 0; 2 * pair < group; pair++) {
+            const unsigned f0 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair);
+            const unsigned f1 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair + 1);
+            const int k = __ffs(h ? f1 : f0) - 1;
+            int4 inf;
+            inf.x = __shfl_sync(0xffffffffu, inf4.x, k);
+            inf.y = __shfl_sync(0xffffffffu, inf4.y, k);
+            inf.z = __shfl_sync(0xffffffffu, inf4.z, k);
+            inf.w = __shfl_sync(0xffffffffu, inf4.w, k);
+            const int64_t n = it + k;
+            const bool node = k < group && n < nnodes;
+            const int m = node_m(inf), K = node_k(inf), Kp = node_kp(inf);
+            const int qp = inf.z;  // the P1 node at this vertex, whose pressure row this half assembles too
+            const int mm = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            const int64_t i0 = node_i0(inf);
+            const uint32_t *il = inc + i0;
+            if (hl == 8) src2 = reinterpret_cast<const char *>(slots + i0 * kSlotStride);
+            // the half's list, a window of 16 entries at a time
+            uint32_t lst = hl < m ? __ldg(il + hl) : 0u, lst_next = 16 + hl < m ? __ldg(il + 16 + hl) : 0u;
+            // incidence t of the half's node into its ring slot; every call
+            // commits one group, empty past the end, so the wait counts hold
+            auto stage = [&](int slot, int t) {
+                if (t > 0 && (t & 15) == 0) {  // warp-uniform
+                    lst = lst_next;
+                    lst_next = t + 16 + hl < m ? __ldg(il + t + 16 + hl) : 0u;
+                }
+                const uint32_t ea = __shfl_sync(0xffffffffu, lst, t & 15, 16);
+                if (t < m) {
+                    const uint32_t a = ea & 15u;
+                    const size_t eo = (size_t)(ea >> 4) * (kNSRecord * sizeof(float));
+                    cp_async16(dst_lane + slot * kStg, src1 + eo);
+                    // NA[a][0..9] starts 8 bytes into a 16-byte boundary when a is odd
+                    const size_t o2 = hl == 8 ? (size_t)(t * kSlotStride) : eo + (hl < 5 ? 0u : 40u * a - 8u * (a & 1u));
+                    if (hl < 9) cp_async16(dst_lane + slot * kStg + 64, src2 + o2);
+                    if (GN) {
+                        const float *Ke = gstage + (size_t)(ea >> 4) * kGNStride;
+                        cp_async16(dst_lane + slot * kStg + kVGn, Ke + 96 * a + 4 * hl);
+                        if (hl < 10)
+                            cp_async16(dst_lane + slot * kStg + kVGn + 64,
+                                       hl < 8 ? Ke + 96 * a + 64 + 4 * hl : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (hl - 8));
+                    }
+                }
+                cp_async_commit();
+            };
+#pragma unroll 1
+            for (int t = 0; t < kVRing - 1; t++) stage(t, t);
+            double *out00 = node ? vals00 + rowptr00[3 * n] : nullptr, *out01 = node ? vals01 + rowptr01[3 * n] : nullptr;
+            double *out10 = qp >= 0 ? vals10 + rowptr10[qp] : nullptr;
+            const int s00 = odd8(out00), s01 = odd8(out01), s10 = odd8(out10);
+            const int o01 = vel_run_words(9 * K), o10 = o01 + vel_run_words(3 * Kp);
+            const int used = o10 + (qp >= 0 ? vel_run_words(3 * K) : 0);
+            for (int c = 4 * hl; c < used; c += 64) *reinterpret_cast<float4 *>(mem + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            float *acc = mem + s00, *acc1 = mem + o01 + s01, *acc2 = mem + o10 + s10;
+            const int st = 3 * K;
+            float rj0 = 0.0f, rj1 = 0.0f, rb = 0.0f, rq0 = 0.0f, rq1 = 0.0f, rg = 0.0f;
+            // the table rows of the current local index a; incidences come sorted
+            // by a, so they reload only when a run of equal a ends
+            int a_cur = -1;
+            float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rc = ra, y = ra, ya = ra, yc = ra;
+#pragma unroll 1
+            for (int t = 0; t < mm; t++) {
+                const int r = t & (kVRing - 1);
                 cp_async_wait<kVRing - 2>();
                 // the slot's copies are visible to the warp, and every lane is
                 // done with the slot consumed in the previous step, which is
                 // refilled next
                 __syncwarp();
-                stage_vel<GN>(dst_lane, (r + kVRing - 1) % kVRing, t + kVRing - 1, m, il, rec, src_lane, kind,
-                              slots_node, gstage, lane);
+                stage((r + kVRing - 1) & (kVRing - 1), t + kVRing - 1);
+                if (t >= m) continue;  // this half's node is done
                 const int off = r * kStg;
-                const int a = pLoc[4 * off];  // the staged slot map's local-index byte (broadcast)
-                if (a != a_cur) {  // warp-uniform
+                const int a = pS[4 * off + kSlotLocal];  // the staged slot map's local-index byte (broadcast)
+                if (a != a_cur) {
                     a_cur = a;
-                    rr = lds4(pR + 40 * a);
+                    if (NEWTON) {
+                        ra = lds4(pR + 40 * a);
+                        rc = lds4(pR + 40 * a + 4);
+                    }
                     y = lds4(pY + 16 * a);
-                    if (qp >= 0 && a < 4) yq = lds4(pYb + 4 * a);
+                    if (qp >= 0 && a < 4) {
+                        ya = lds4(pYb + 4 * a);
+                        yc = lds4(pYb + 16 + 4 * a);
+                    }
                 }
                 // NA_ab on the diagonal (i = j) plus wn W_(ai)(bj), i = 0..2
-                const float4 g0 = lds4(pG + off), g1 = lds4(pG + off + 4), g2 = lds4(pG + off + 8);
-                const float an = pNA[off + 2 * (a & 1)];
-                const int idx = lw ? 3 * pS[4 * off] + j : ps - 1;
-                float *dst = acc + idx;
-                // g[j][m*3+i]: m0 = (g0.x,g0.y,g0.z) m1 = (g0.w,g1.x,g1.y) m2 = (g1.z,g1.w,g2.x) m3 = (g2.y,g2.z,g2.w)
-                float v0 = dst[0], v1 = dst[ps], v2 = dst[2 * ps];
-                if (GN) {
-                    // the viscous rows (a, i), column (b, j) = lane, and the viscous residual of row (a, lane)
-                    v0 += ring[off + kVGn + lane];
-                    v1 += ring[off + kVGn + 32 + lane];
-                    v2 += ring[off + kVGn + 64 + lane];
-                    rg += ring[off + kVGnRes + ((3 * a) & 3) + (lane & 3)];
+                float4 g0, g1, g2;
+                if (NEWTON) {
+                    g0 = lds4(pG + off);
+                    g1 = lds4(pG + off + 4);
+                    g2 = lds4(pG + off + 8);
                 }
-                dst[0] = fmaf(g2.y, rr.w, fmaf(g1.z, rr.z, fmaf(g0.w, rr.y, fmaf(g0.x, rr.x, fmaf(e0, an, v0)))));
-                dst[ps] = fmaf(g2.z, rr.w, fmaf(g1.w, rr.z, fmaf(g1.x, rr.y, fmaf(g0.y, rr.x, fmaf(e1, an, v1)))));
-                dst[2 * ps] = fmaf(g2.w, rr.w, fmaf(g2.x, rr.z, fmaf(g1.y, rr.y, fmaf(g0.z, rr.x, fmaf(e2, an, v2)))));
-                const float ub = pU[off];
-                rj = fmaf(an, ub, rj);
-                // -Bd_p(a, i): the (0,1) entry of velocity row (a, i), pressure column p
+                const float2 an = *reinterpret_cast<const float2 *>(pNA + off + 2 * (a & 1));
+                const uint32_t ss = *reinterpret_cast<const uint16_t *>(pS + 4 * off + 2 * p);
+                float *dA = lw ? acc + 3 * (ss & 255u) + j : scratch, *dB = lw ? acc + 3 * (ss >> 8) + j : scratch;
+                const int sl = lw ? st : 0;
+                // g[j][m*3+i]: m0 = (g0.x,g0.y,g0.z) m1 = (g0.w,g1.x,g1.y) m2 = (g1.z,g1.w,g2.x) m3 = (g2.y,g2.z,g2.w)
+                {
+                    float v0 = dA[0], v1 = dA[sl], v2 = dA[2 * sl], w0 = dB[0], w1 = dB[sl], w2 = dB[2 * sl];
+                    if (GN) {
+                        // the viscous rows (a, i), columns (b, j), and the viscous residual of row (a, hl)
+                        const float *V = ring + off + kVGn + 6 * p + j;
+                        v0 += V[0];
+                        v1 += V[32];
+                        v2 += V[64];
+                        w0 += V[3];
+                        w1 += V[35];
+                        w2 += V[67];
+                        rg += ring[off + kVGnRes + ((3 * a) & 3) + (hl & 3)];
+                    }
+                    v0 = fmaf(e0, an.x, v0);
+                    v1 = fmaf(e1, an.x, v1);
+                    v2 = fmaf(e2, an.x, v2);
+                    w0 = fmaf(e0, an.y, w0);
+                    w1 = fmaf(e1, an.y, w1);
+                    w2 = fmaf(e2, an.y, w2);
+                    if (NEWTON) {
+                        v0 = fmaf(g2.y, ra.w, fmaf(g1.z, ra.z, fmaf(g0.w, ra.y, fmaf(g0.x, ra.x, v0))));
+                        v1 = fmaf(g2.z, ra.w, fmaf(g1.w, ra.z, fmaf(g1.x, ra.y, fmaf(g0.y, ra.x, v1))));
+                        v2 = fmaf(g2.w, ra.w, fmaf(g2.x, ra.z, fmaf(g1.y, ra.y, fmaf(g0.z, ra.x, v2))));
+                        w0 = fmaf(g2.y, rc.w, fmaf(g1.z, rc.z, fmaf(g0.w, rc.y, fmaf(g0.x, rc.x, w0))));
+                        w1 = fmaf(g2.z, rc.w, fmaf(g1.w, rc.z, fmaf(g1.x, rc.y, fmaf(g0.y, rc.x, w1))));
+                        w2 = fmaf(g2.w, rc.w, fmaf(g2.x, rc.z, fmaf(g1.y, rc.y, fmaf(g0.z, rc.x, w2))));
+                    }
+                    dA[0] = v0;
+                    dA[sl] = v1;
+                    dA[2 * sl] = v2;
+                    dB[0] = w0;
+                    dB[sl] = w1;
+                    dB[2 * sl] = w2;
+                }
+                const float ua = pU[off], ub = pU[off + 3];
+                rj0 = fmaf(an.x, ua, rj0);
+                rj1 = fmaf(an.y, ub, rj1);
+                // -Bd_q(a, i): the (0,1) entry of velocity row (a, i), pressure column q
                 const float4 bs = lds4(pBS + off);
                 const float bt = fmaf(bs.z, y.z, fmaf(bs.y, y.y, bs.x * y.x));
-                float *dp = acc + (lb ? bi * ps + 3 * K + pSp[4 * off] : ps - 1);
+                float *dp = lb ? acc1 + bi * Kp + pS[4 * off + 10 + bq] : scratch;
                 *dp += bt;
                 rb = fmaf(bt, pP[off], rb);
                 if (qp >= 0 && a < 4) {
-                    // -Bd_q(b j): the (1,0) entry of pressure row q = this vertex, column (b, j)
+                    // -Bd_q(b j): the (1,0) entries of pressure row q = this vertex, columns (b, j)
                     const float4 bj = lds4(pBSj + off);
-                    const float pv = fmaf(bj.z, yq.z, fmaf(bj.y, yq.y, bj.x * yq.x));
-                    acc[3 * ps + idx] += pv;
-                    rq = fmaf(pv, ub, rq);
+                    const float pa = fmaf(bj.z, ya.z, fmaf(bj.y, ya.y, bj.x * ya.x));
+                    const float pc = fmaf(bj.z, yc.z, fmaf(bj.y, yc.y, bj.x * yc.x));
+                    float *qa = lw ? acc2 + 3 * (ss & 255u) + j : scratch, *qc = lw ? acc2 + 3 * (ss >> 8) + j : scratch;
+                    *qa += pa;
+                    *qc += pc;
+                    rq0 = fmaf(pa, ua, rq0);
+                    rq1 = fmaf(pc, ub, rq1);
                 }
             }
-        }
-        cp_async_wait<0>();
-        __syncwarp();
-        if (vals00) {
-            double *out = vals00 + rowptr00[3 * n];
-            for (int c = lane; c < 3 * K; c += 32) {
-                st_cs(out + c, f2d_exact(acc[c]));
-                st_cs(out + 3 * K + c, f2d_exact(acc[ps + c]));
-                st_cs(out + 6 * K + c, f2d_exact(acc[2 * ps + c]));
+            cp_async_wait<0>();
+            __syncwarp();
+            vel_write(mem, s00, 9 * K, out00, hl);
+            vel_write(mem + o01, s01, 3 * Kp, out01, hl);
+            if (res_u) vel_residual_out<GN>(rj0, rj1, rb, rg, n, hl, node, co, res_u);
+            if (qp >= 0) vel_write(mem + o10, s10, 3 * K, out10, hl);
+            if (res_p && __any_sync(0xffffffffu, qp >= 0)) {
+                // the pressure residual: the pairwise (xor) tree over 32 words, (b, j) at 3 b + j
+                if (lw) {
+                    sum32[6 * p + j] = rq0;
+                    sum32[6 * p + 3 + j] = rq1;
+                } else {
+                    sum32[30] = sum32[31] = 0.0f;
+                }
+                __syncwarp();
+                float v = sum32[hl] + sum32[hl + 16];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (qp >= 0 && hl == 0) res_p[qp] = f2d_exact((float)co.pu * v);
             }
-            double *out1 = vals01 + rowptr01[3 * n];
-            const float *accp = acc + 3 * K;
-            for (int c = lane; c < Kp; c += 32) {
-                st_cs(out1 + c, f2d_exact(accp[c]));
-                st_cs(out1 + Kp + c, f2d_exact(accp[ps + c]));
-                st_cs(out1 + 2 * Kp + c, f2d_exact(accp[2 * ps + c]));
-            }
+            __syncwarp();
         }
-        if (res_u) {
-            vel_residual_out<GN>(rj, rb, rg, n, lane, co, res_u);
-        }
-        if (qp >= 0) {
-            if (vals10) {
-                double *out = vals10 + rowptr10[qp];
-                for (int c = lane; c < 3 * K; c += 32) st_cs(out + c, f2d_exact(acc[3 * ps + c]));
-            }
-            if (res_p) {
-                const float v = warp_sum(lw ? rq : 0.0f);
-                if (lane == 0) res_p[qp] = f2d_exact((float)co.pu * v);
-            }
-        }
-        __syncwarp();
     }
 }
 
@@ -838,7 +909,7 @@ __device__ __forceinline__ void vel_residual_node(const float *sY, int64_t n, co
     const float cuu = (float)co.uu;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        // vel_residual_out's strided tree over the lanes 3 b + i and 4 i + p
+        // vel_residual_out's trees
         const float x = (((rj[i] + rj[3 + i]) + (rj[6 + i] + rj[9 + i])) + ((rj[12 + i] + rj[15 + i]) + (rj[18 + i] + rj[21 + i]))) +
                         (rj[24 + i] + rj[27 + i]);
         const float z = (rb[4 * i] + rb[4 * i + 1]) + (rb[4 * i + 2] + rb[4 * i + 3]);
@@ -1020,34 +1091,41 @@ void launch_ns_node_info(const Graph &g, const int64_t *padj_ptr, const int32_t 
 
 void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, const float *d_tables,
                         const int64_t *rowptr00, const int64_t *rowptr01, double *vals00, double *vals01, double *res_u,
-                        float visc_dens, float dens, int newton, int want_jac, int max_adj, int max_padj,
-                        const int32_t *vmap, const int64_t *rowptr10, double *vals10, double *res_p,
-                        const float *gstage, cudaStream_t s, LaunchCounter &lc, int64_t n_begin, int64_t n_end,
-                        unsigned long long *work, const NSCoeff &co) {
-    (void)visc_dens;  // nu rho enters through NA, which the record kernels wrote
-    // up to 16 warps share one copy of the tables; two CTAs fit an SM at the
-    // structured meshes' adjacency, fewer warps where the accumulators are larger
+                        float dens, int newton, int max_adj, int max_padj, bool vmap, const int64_t *rowptr10,
+                        double *vals10, double *res_p, const float *gstage, cudaStream_t s, LaunchCounter &lc,
+                        int64_t n_begin, int64_t n_end, unsigned long long *work, const NSCoeff &co) {
     const bool gn = gstage != nullptr;
-    const int planes = vmap ? 4 : 3;
-    const int acc_words = (planes * (3 * max_adj + max_padj + 1) + 3) & ~3;
-    const size_t per_warp = (size_t)(kVRing * (gn ? kVStageGn : kVStage) + acc_words) * sizeof(float);
-    const int warps = (int)std::max<size_t>(1, std::min<size_t>(16, (227 * 1024 - kVelTab * sizeof(float)) / per_warp));
-    size_t smem = kVelTab * sizeof(float) + (size_t)warps * per_warp;
-    auto kern = gn ? k_ns_vel_rows<true> : k_ns_vel_rows<false>;
+    const int acc_words = vel_acc_words(max_adj, max_padj, vmap);
+    const size_t tables = kVelTab * sizeof(float);
+    const size_t per_warp = 2 * (size_t)(kVRing * (gn ? kVStageGn : kVStage) + acc_words) * sizeof(float);
+    // two CTAs per SM share its shared memory; one where the rows are so long
+    // that two would leave few warps
+    int warps = (int)std::min<size_t>(vel_warps(gn), (113 * 1024 - tables) / per_warp);
+    if (warps < 4) warps = (int)std::max<size_t>(1, std::min<size_t>(vel_warps(gn), (227 * 1024 - tables) / per_warp));
+    // groups of eight nodes, or single pairs spread over all SMs where the mesh
+    // does not keep the chip's warps busy for several groups
+    const int64_t nn = n_end < 0 ? g.nrow_nodes : n_end, sms = sm_count_ns();
+    int group = 8;
+    if (nn - n_begin < sms * 2 * warps * 16) {
+        group = 2;
+        work = nullptr;  // every warp takes one pair or a few: fixed positions
+        warps = (int)std::min<int64_t>(warps, std::max<int64_t>(2, ceil_div((nn - n_begin + 1) / 2, 2 * sms)));
+    }
+    const size_t smem = tables + (size_t)warps * per_warp;
+    auto kern = gn ? (newton ? k_ns_vel_rows<true, true> : k_ns_vel_rows<true, false>)
+                   : (newton ? k_ns_vel_rows<false, true> : k_ns_vel_rows<false, false>);
     FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t nn = n_end < 0 ? g.nrow_nodes : n_end;
-    unsigned grid = (unsigned)std::min<int64_t>((nn - n_begin + warps - 1) / warps, (int64_t)sm_count_ns() * 4);
+    unsigned grid = (unsigned)std::min<int64_t>((nn - n_begin + group * warps - 1) / (group * warps), sms * 4);
     if (work) {  // dynamic positions: exactly the CTAs that fit
         int per_sm = 0;
         FEDD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
-        grid = (unsigned)std::min<int64_t>(grid, (int64_t)sm_count_ns() * std::max(per_sm, 1));
+        grid = (unsigned)std::min<int64_t>(grid, sms * std::max(per_sm, 1));
         FEDD_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), s));
     }
     if (grid == 0) return;
-    kern<<<grid, 32 * warps, smem, s>>>(ninfo, g.inc.p, g.slots.p, rec, d_tables, rowptr00, rowptr01,
-                                        want_jac ? vals00 : nullptr, want_jac ? vals01 : nullptr, res_u, nn, dens,
-                                        newton, max_adj, max_padj, n_begin, vmap ? 1 : 0, rowptr10,
-                                        want_jac ? vals10 : nullptr, res_p, gstage, work, co);
+    kern<<<grid, 32 * warps, smem, s>>>(ninfo, g.inc.p, g.slots.p, rec, d_tables, rowptr00, rowptr01, vals00, vals01,
+                                        res_u, nn, dens, group, acc_words, n_begin, rowptr10, vals10, res_p, gstage,
+                                        work, co);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

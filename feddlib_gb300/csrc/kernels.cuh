@@ -134,11 +134,11 @@ void launch_ns_node_info(const Graph &g, const int64_t *padj_ptr, const int32_t 
 struct NSCoeff {
     double uu = 1.0, up = 1.0, pu = 1.0;
 };
+// vmap: ninfo holds a verified vertex map (block (1,0) and res_p come along)
 void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, const float *d_tables,
-                        const int64_t *rowptr00, const int64_t *rowptr01, double *vals00, double *vals01,
-                        double *res_u, float visc_dens, float dens, int newton, int want_jac, int max_adj,
-                        int max_padj, const int32_t *vmap, const int64_t *rowptr10, double *vals10, double *res_p,
-                        const float *gstage, cudaStream_t s, LaunchCounter &lc,
+                        const int64_t *rowptr00, const int64_t *rowptr01, double *vals00, double *vals01, double *res_u,
+                        float dens, int newton, int max_adj, int max_padj, bool vmap, const int64_t *rowptr10,
+                        double *vals10, double *res_p, const float *gstage, cudaStream_t s, LaunchCounter &lc,
                         int64_t n_begin = 0, int64_t n_end = -1, unsigned long long *work = nullptr,
                         const NSCoeff &co = NSCoeff{});
 void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_tables, const int64_t *rowptr10,

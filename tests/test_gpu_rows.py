@@ -30,3 +30,33 @@ def test_value_arrays_at_any_offset(M):
         b, x = buf.cpu().numpy(), res.cpu().numpy()
         assert np.array_equal(b[offset:offset + nnz], v) and np.array_equal(x[offset & 1:][:a.n_u], r)
         assert (b[:offset] == -7.0).all() and (b[offset + nnz:] == -7.0).all()
+
+
+@pytest.mark.parametrize("newton,gn", [(True, False), (False, False), (True, True)])
+@pytest.mark.parametrize("M", [1, 3])
+def test_navier_stokes_blocks_at_any_offset(M, newton, gn):
+    """The three blocks' runs of a node are written the same way; odd node
+    counts leave half of the last pair of nodes empty."""
+    import torch
+    import feddlib_gb300 as F
+    xyz2, el2 = F.structured_mesh(M, 2, seed=80 + M)
+    xyz1, el1 = F.structured_mesh(M, 1, seed=80 + M)
+    u, p = 0.5 * F.fourier_field(xyz2, seed=80), F.uniform_field(80, xyz1.shape[0])
+    a = F.Assembler(F.NAVIER_STOKES, xyz2, el2, elements_p=el1, num_nodes_p=xyz1.shape[0], viscosity=0.01, density=1.3,
+                    newton=newton)
+    if gn:
+        a.set_viscosity_law(0, [1.902, 0.22, 0.056, 0.00345, 1.25], gamma_min=1e-12)
+    want, ru, rp = a.assemble(u=u, p=p)
+    du, dp = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    for offset in range(4):
+        offs = [offset & 1, offset >> 1, (offset + 1) & 1]
+        bufs = [torch.full((w.size + 4,), -7.0, dtype=torch.float64, device="cuda") for w in want]
+        dru = torch.zeros(a.n_u, dtype=torch.float64, device="cuda")
+        drp = torch.zeros(a.n_p, dtype=torch.float64, device="cuda")
+        a.assemble_device(du.data_ptr(), dp.data_ptr(), [b.data_ptr() + 8 * o for b, o in zip(bufs, offs)],
+                          dru.data_ptr(), drp.data_ptr())
+        torch.cuda.synchronize()
+        for b, o, w in zip(bufs, offs, want):
+            x = b.cpu().numpy()
+            assert np.array_equal(x[o:o + w.size], w) and (x[:o] == -7.0).all() and (x[o + w.size:] == -7.0).all()
+        assert np.array_equal(dru.cpu().numpy(), ru) and np.array_equal(drp.cpu().numpy(), rp)
