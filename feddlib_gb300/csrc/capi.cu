@@ -201,12 +201,11 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
     switch (h->prm.problem) {
     case FEDD_LAPLACE:
         stage(h, "lap_elem", s, [&] {
-            launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, h->stage_d.p,
+            launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, jac, h->stage_d.p,
                             h->d_err.p, s, lc);
         });
         stage(h, "lap_rows", s, [&] {
-            launch_lap_rows(h->g, h->stage_d.p, h->order, h->csr[0].rowptr.p, jac ? v00 : nullptr,
-                            res ? ru : nullptr, h->nn, s, lc);
+            launch_lap_rows(h->g, h->stage_d.p, h->order, jac ? v00 : nullptr, res ? ru : nullptr, h->nn, s, lc);
         });
         break;
     case FEDD_LINEAR_ELASTICITY:
@@ -850,7 +849,7 @@ fedd_status fedd_element_matrices(fedd_assembler *h, const double *u, const doub
         int nd = 0;
         if (prob == FEDD_LAPLACE) {
             nd = h->npe;
-            launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, h->stage_d.p,
+            launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, true, h->stage_d.p,
                             h->d_err.p, s, lc);
         } else if (prob == FEDD_NAVIER_STOKES) {
             nd = 34;
@@ -1252,7 +1251,7 @@ extern "C" fedd_status fedd_element_matrices_noalloc(fedd_assembler *h, const do
         if (count > 0) {
             // the element stage of the requested elements only
             if (prob == FEDD_LAPLACE) {
-                launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, h->stage_d.p,
+                launch_lap_elem(h->xyz.p, h->conn.p, h->ne, h->order, h->lap_tab.p, h->prm.source, true, h->stage_d.p,
                                 h->d_err.p, s, lc, e0, e1);
             } else if (prob == FEDD_NAVIER_STOKES) {
                 launch_ns_record(h->geo.p, h->conn.p, h->conn_p.p, h->ne, du, dp, h->ns_tab.p,

@@ -4,9 +4,23 @@
 //     K_ab = |det B| sum_q w_q grad phi_a . grad phi_b
 // FE::assemblyRHS with a constant source (FE_def.hpp:7303-7400):
 //     b_a  = |det B| f sum_q w_q phi_a(q)
-// For affine elements K_ab = sum_s Gs_s KS[a][b][s] with Gs = |det B| B^-1 B^-T
-// and exact reference integrals KS; the load factors m_a = sum_q w_q phi_a
-// are exact for the reference's rules (1 point for P1, 5 points for P2).
+// For affine elements both orders' integrals are combinations of the products
+//     D_ij = V L_i . L_j = C_i . C_j / (6 |det B|)
+// of the barycentric gradients L_i = C_i / det B (C_1..C_3 the cofactor columns,
+// C_0 = -(C_1 + C_2 + C_3), V = |det B| / 6): P1 K_ij = D_ij, and with
+// int lambda_i lambda_j = V (1 + d_ij) / 20 for P2
+//     vertices i, j:           3/5 D_ii, -1/5 D_ij
+//     vertex i, edge (j, k):   (4/5 d_ij - 1/5) D_ik + (4/5 d_ik - 1/5) D_ij
+//     edges (i, j), (k, l):    4/5 ((1 + d_ik) D_jl + (1 + d_il) D_jk
+//                                   + (1 + d_jk) D_il + (1 + d_jl) D_ik).
+// The load factors m_a = sum_q w_q phi_a are exact for the reference's rules (1
+// point for P1, 5 points for P2).
+//
+// The FP64 pipe takes 20 cycles per warp instruction, whatever the number of
+// active lanes, so what counts is FP64 warp instructions: the element kernel
+// forms its entries in few of them, and the row kernel adds an incidence's
+// entries and load for several nodes at once (a warp's 32 lanes hold six P1 or
+// two P2 nodes).
 #include "kernels.cuh"
 
 namespace fedd {
@@ -18,10 +32,16 @@ __device__ __forceinline__ int lap_packed(int n, int a, int b) {
     return a * n - (a * (a - 1)) / 2 + (b - a);
 }
 
-template <int NPE>
-__global__ void k_lap_elem(const double *__restrict__ xyz, const int32_t *__restrict__ conn, int64_t ne, double f,
-                           const double *__restrict__ ks2, const double *__restrict__ mfac, double *stage, int *err,
-                           int64_t e_begin, int64_t e_end) {
+__host__ __device__ constexpr int lap_edge(int a, int end) {  // vertices of P2 node 4 + a: 01 12 02 03 13 23
+    constexpr int E[6][2] = {{0, 1}, {1, 2}, {0, 2}, {0, 3}, {1, 3}, {2, 3}};
+    return E[a][end];
+}
+
+// WANT_K: the stiffness (packed upper triangle); the load always
+template <int NPE, bool WANT_K>
+__global__ void __launch_bounds__(64) k_lap_elem(const double *__restrict__ xyz, const int32_t *__restrict__ conn,
+                                                 int64_t ne, double f, const double *__restrict__ mfac, double *stage,
+                                                 int *err, int64_t e_begin, int64_t e_end) {
     constexpr int STRIDE = NPE == 4 ? kLapStrideP1 : kLapStrideP2;
     constexpr int NK = NPE * (NPE + 1) / 2;
     int64_t e = e_begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -33,86 +53,128 @@ __global__ void k_lap_elem(const double *__restrict__ xyz, const int32_t *__rest
                    xyz[3 * (int64_t)n1 + 2] - z0, xyz[3 * (int64_t)n2 + 2] - z0, xyz[3 * (int64_t)n3 + 2] - z0};
     double C[9];
     C[0] = B[4] * B[8] - B[5] * B[7]; C[1] = B[5] * B[6] - B[3] * B[8]; C[2] = B[3] * B[7] - B[4] * B[6];
-    C[3] = B[2] * B[7] - B[1] * B[8]; C[4] = B[0] * B[8] - B[2] * B[6]; C[5] = B[1] * B[6] - B[0] * B[7];
-    C[6] = B[1] * B[5] - B[2] * B[4]; C[7] = B[2] * B[3] - B[0] * B[5]; C[8] = B[0] * B[4] - B[1] * B[3];
+    if (WANT_K) {
+        C[3] = B[2] * B[7] - B[1] * B[8]; C[4] = B[0] * B[8] - B[2] * B[6]; C[5] = B[1] * B[6] - B[0] * B[7];
+        C[6] = B[1] * B[5] - B[2] * B[4]; C[7] = B[2] * B[3] - B[0] * B[5]; C[8] = B[0] * B[4] - B[1] * B[3];
+    }
     const double det = B[0] * C[0] + B[1] * C[1] + B[2] * C[2];
     if (det == 0.0) set_dev_error(err, kDevBadDet);
-    const double ad = fabs(det), rd = 1.0 / det;
-    double Bi[9];  // Bi[i][j] = C[j][i] / det
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) Bi[3 * i + j] = C[3 * j + i] * rd;
+    const double ad = fabs(det);
     double *S = stage + e * STRIDE;
-    if (NPE == 4) {
-        // grad phi_a = B^-T grad_ref phi_a, one-point rule (weight 1/6)
-        double G[4][3];
+    if (WANT_K) {
+        double G[4][3], D[4][4];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            G[1][k] = Bi[k];
-            G[2][k] = Bi[3 + k];
-            G[3][k] = Bi[6 + k];
+            G[1][k] = C[3 * k];
+            G[2][k] = C[3 * k + 1];
+            G[3][k] = C[3 * k + 2];
             G[0][k] = -(G[1][k] + G[2][k] + G[3][k]);
+        }
+        // P2: a fifth of D
+        const double w = (NPE == 4 ? 1.0 : 0.2) / (6.0 * ad);
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+            const double g0 = w * G[a][0], g1 = w * G[a][1], g2 = w * G[a][2];
+#pragma unroll
+            for (int b = a; b < 4; b++) D[a][b] = D[b][a] = g0 * G[b][0] + g1 * G[b][1] + g2 * G[b][2];
         }
         int t = 0;
 #pragma unroll
-        for (int a = 0; a < 4; a++)
+        for (int a = 0; a < NPE; a++)
 #pragma unroll
-            for (int b = a; b < 4; b++, t++)
-                S[t] = ad * (1.0 / 6.0) * (G[a][0] * G[b][0] + G[a][1] * G[b][1] + G[a][2] * G[b][2]);
-    } else {
-        const int SC[6] = {0, 1, 2, 0, 0, 1}, SD[6] = {0, 1, 2, 1, 2, 2};
-        double Gs[6];
-#pragma unroll
-        for (int s = 0; s < 6; s++)
-            Gs[s] = ad * (Bi[3 * SC[s]] * Bi[3 * SD[s]] + Bi[3 * SC[s] + 1] * Bi[3 * SD[s] + 1] +
-                          Bi[3 * SC[s] + 2] * Bi[3 * SD[s] + 2]);
-        int t = 0;
-        for (int a = 0; a < 10; a++)
-            for (int b = a; b < 10; b++, t++) {
-                double v = 0.0;
-#pragma unroll
-                for (int s = 0; s < 6; s++) v += Gs[s] * ks2[(a * 10 + b) * 6 + s];
+            for (int b = a; b < NPE; b++, t++) {
+                double v;
+                if (NPE == 4) {
+                    v = D[a & 3][b & 3];
+                } else if (b < 4) {
+                    v = a == b ? 3.0 * D[a & 3][a & 3] : -D[a & 3][b & 3];
+                } else if (a < 4) {
+                    const int j = lap_edge(b >= 4 ? b - 4 : 0, 0), k = lap_edge(b >= 4 ? b - 4 : 0, 1);
+                    v = a == j ? 3.0 * D[a & 3][k] - D[a & 3][j]
+                               : (a == k ? 3.0 * D[a & 3][j] - D[a & 3][k] : -(D[a & 3][j] + D[a & 3][k]));
+                } else {
+                    const int i = lap_edge(a >= 4 ? a - 4 : 0, 0), j = lap_edge(a >= 4 ? a - 4 : 0, 1);
+                    const int k = lap_edge(b >= 4 ? b - 4 : 0, 0), l = lap_edge(b >= 4 ? b - 4 : 0, 1);
+                    double s = (i == k ? 2.0 : 1.0) * D[j][l] + (j == l ? 2.0 : 1.0) * D[i][k];
+                    s += (i == l ? 2.0 : 1.0) * D[j][k] + (j == k ? 2.0 : 1.0) * D[i][l];
+                    v = 4.0 * s;
+                }
                 S[t] = v;
             }
     }
+    const double fa = ad * f;
 #pragma unroll
-    for (int a = 0; a < NPE; a++) S[NK + a] = ad * f * mfac[a];
+    for (int a = 0; a < NPE; a++) S[NK + a] = fa * mfac[a];
 }
 
-// one warp per node; FP64 accumulation in shared memory (this problem is
-// small and its configuration asks for FP64 end to end)
+// Several nodes per warp, NPE + 1 lanes each: lane b < NPE adds column b of the
+// node's row of each incidence, lane NPE its load (to the word behind the
+// columns), four incidences read ahead; FP64 accumulation in shared memory, in
+// incidence order.
 template <int NPE>
-__global__ void k_lap_rows(const int64_t *__restrict__ inc_ptr, const uint32_t *__restrict__ inc,
-                           const uint8_t *__restrict__ slots, const int64_t *__restrict__ adj_ptr,
-                           const double *__restrict__ stage, const int64_t *__restrict__ rowptr, double *vals,
-                           double *load, int64_t nnodes, int max_adj) {
+__global__ void __launch_bounds__(128) k_lap_rows(const int64_t *__restrict__ inc_ptr, const uint32_t *__restrict__ inc,
+                                                  const uint8_t *__restrict__ slots, const int64_t *__restrict__ adj_ptr,
+                                                  const double *__restrict__ stage, double *vals, double *load,
+                                                  int64_t nnodes, int max_adj) {
+    constexpr int STRIDE = NPE == 4 ? kLapStrideP1 : kLapStrideP2;
+    constexpr int NK = NPE * (NPE + 1) / 2, W = NPE + 1, NODES = 32 / W, AHEAD = 4;
+    extern __shared__ double dacc[];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, s = lane / W, b = lane - W * s;
+    const int64_t n = (blockIdx.x * (int64_t)(blockDim.x >> 5) + w) * NODES + s;
+    const bool in = s < NODES && n < nnodes;
+    double *acc = dacc + (size_t)(w * (NODES + 1) + s) * (max_adj + 1);  // the last one: lanes without a node
+    const int64_t a0 = in ? adj_ptr[n] : 0, i0 = in ? inc_ptr[n] : 0;
+    const int K = in ? (int)(adj_ptr[n + 1] - a0) : 0, m = in ? (int)(inc_ptr[n + 1] - i0) : 0;
+    for (int c = b; c <= K; c += W) acc[c] = 0.0;
+    int mm = m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    __syncwarp();
+    for (int t0 = 0; t0 < mm; t0 += AHEAD) {
+        double v[AHEAD];
+        int at[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            v[k] = 0.0;
+            at[k] = 0;
+            if (t0 + k < m) {
+                const int64_t i = i0 + t0 + k;
+                const uint32_t ea = __ldg(inc + i);
+                const int a = (int)(ea & 15u);
+                v[k] = __ldg(stage + (int64_t)(ea >> 4) * STRIDE + (b < NPE ? lap_packed(NPE, a, b) : NK + a));
+                at[k] = b < NPE ? __ldg(slots + i * kSlotStride + b) : K;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            if (t0 + k < mm) {
+                if (t0 + k < m) acc[at[k]] += v[k];
+                __syncwarp();
+            }
+        }
+    }
+    if (!in) return;
+    if (vals)
+        for (int c = b; c < K; c += W) vals[a0 + c] = acc[c];
+    if (load && b == NPE) load[n] = acc[K];
+}
+
+// the load alone: one thread per node, its entries in incidence order
+template <int NPE>
+__global__ void __launch_bounds__(128) k_lap_load(const int64_t *__restrict__ inc_ptr, const uint32_t *__restrict__ inc,
+                                                  const double *__restrict__ stage, double *load, int64_t nnodes) {
     constexpr int STRIDE = NPE == 4 ? kLapStrideP1 : kLapStrideP2;
     constexpr int NK = NPE * (NPE + 1) / 2;
-    extern __shared__ double dacc[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    double *acc = dacc + (size_t)w * max_adj;
-    for (int64_t n = (int64_t)blockIdx.x * nw + w; n < nnodes; n += (int64_t)gridDim.x * nw) {
-        const int K = (int)(adj_ptr[n + 1] - adj_ptr[n]);
-        for (int c = lane; c < K; c += 32) acc[c] = 0.0;
-        double r = 0.0;
-        __syncwarp();
-        for (int64_t ii = inc_ptr[n]; ii < inc_ptr[n + 1]; ii++) {
-            const uint32_t ea = inc[ii];
-            const int64_t e = ea >> 4;
-            const int a = ea & 15;
-            const double *S = stage + e * STRIDE;
-            if (lane < NPE) acc[slots[ii * kSlotStride + lane]] += S[lap_packed(NPE, a, lane)];
-            if (lane == 0) r += S[NK + a];
-            __syncwarp();
-        }
-        if (vals) {
-            double *out = vals + rowptr[n];
-            for (int c = lane; c < K; c += 32) out[c] = acc[c];
-        }
-        if (load && lane == 0) load[n] = r;
-        __syncwarp();
+    const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (n >= nnodes) return;
+    const int64_t i1 = inc_ptr[n + 1];
+    double r = 0.0;
+#pragma unroll 4
+    for (int64_t i = inc_ptr[n]; i < i1; i++) {
+        const uint32_t ea = __ldg(inc + i);
+        r += __ldg(stage + (int64_t)(ea >> 4) * STRIDE + NK + (ea & 15u));
     }
+    load[n] = r;
 }
 
 template <int NPE>
@@ -132,68 +194,48 @@ __global__ void k_lap_dense(const double *__restrict__ stage, int64_t first, int
 
 }  // namespace
 
-// Host FP64 tables for the Laplace stage: ks2[a][b][s] (P2 reference
-// stiffness integrals, 600 values) followed by the load factors m[10].
+// Host FP64 table for the Laplace stage: the load factors m[10].
 void lap_make_tables(int order, std::vector<double> &out) {
-    out.assign(610, 0.0);
-    double *m = out.data() + 600;
+    out.assign(kLapTab, 0.0);
     if (order == 1) {
-        for (int a = 0; a < 4; a++) m[a] = (1.0 / 6.0) * 0.25;  // one point, phi = 1/4
+        for (int a = 0; a < 4; a++) out[a] = (1.0 / 6.0) * 0.25;  // one point, phi = 1/4
         return;
     }
     Rule r = make_rule(5);
     for (int q = 0; q < r.n; q++) {
         double ph[10];
         basis_phi(2, r.pts[q], ph);
-        for (int a = 0; a < 10; a++) m[a] += r.w[q] * ph[a];
+        for (int a = 0; a < 10; a++) out[a] += r.w[q] * ph[a];
     }
-    Rule r15 = make_rule(15);
-    const int SC[6] = {0, 1, 2, 0, 0, 1}, SD[6] = {0, 1, 2, 1, 2, 2};
-    for (int a = 0; a < 10; a++)
-        for (int b = 0; b < 10; b++)
-            for (int sidx = 0; sidx < 6; sidx++) {
-                double v = 0;
-                for (int q = 0; q < r15.n; q++) {
-                    double g[10][3];
-                    basis_dphi(2, r15.pts[q], &g[0][0]);
-                    double x = g[a][SC[sidx]] * g[b][SD[sidx]];
-                    if (SC[sidx] != SD[sidx]) x += g[a][SD[sidx]] * g[b][SC[sidx]];
-                    v += r15.w[q] * x;
-                }
-                out[(a * 10 + b) * 6 + sidx] = v;
-            }
 }
 
 void launch_lap_elem(const double *xyz, const int32_t *conn, int64_t ne, int order, const double *d_tables, double f,
-                     double *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin, int64_t e_end) {
+                     bool want_k, double *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin,
+                     int64_t e_end) {
     if (e_end < 0) e_end = ne;
     const int64_t count = e_end - e_begin;
     if (count <= 0) return;
-    if (order == 1)
-        k_lap_elem<4><<<ceil_div(count, 128), 128, 0, s>>>(xyz, conn, ne, f, d_tables, d_tables + 600, stage, d_err,
-                                                           e_begin, e_end);
-    else
-        k_lap_elem<10><<<ceil_div(count, 128), 128, 0, s>>>(xyz, conn, ne, f, d_tables, d_tables + 600, stage, d_err,
-                                                            e_begin, e_end);
+    auto kern = order == 1 ? (want_k ? k_lap_elem<4, true> : k_lap_elem<4, false>)
+                           : (want_k ? k_lap_elem<10, true> : k_lap_elem<10, false>);
+    kern<<<ceil_div(count, 64), 64, 0, s>>>(xyz, conn, ne, f, d_tables, stage, d_err, e_begin, e_end);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }
 
-void launch_lap_rows(const Graph &g, const double *stage, int order, const int64_t *rowptr, double *vals,
-                     double *load, int64_t nnodes, cudaStream_t s, LaunchCounter &lc) {
-    const int warps = 8;
-    size_t smem = (size_t)warps * g.max_adj * sizeof(double);
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    unsigned grid = (unsigned)std::min<int64_t>((nnodes + warps - 1) / warps, (int64_t)(sms > 0 ? sms : 1) * 16);
-    if (grid == 0) return;
-    if (order == 1)
-        k_lap_rows<4><<<grid, 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage, rowptr, vals,
-                                                     load, nnodes, g.max_adj);
-    else
-        k_lap_rows<10><<<grid, 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage, rowptr,
-                                                      vals, load, nnodes, g.max_adj);
+void launch_lap_rows(const Graph &g, const double *stage, int order, double *vals, double *load, int64_t nnodes,
+                     cudaStream_t s, LaunchCounter &lc) {
+    if (nnodes <= 0) return;
+    if (!vals) {
+        auto kern = order == 1 ? k_lap_load<4> : k_lap_load<10>;
+        kern<<<ceil_div(nnodes, 128), 128, 0, s>>>(g.inc_ptr.p, g.inc.p, stage, load, nnodes);
+    } else {
+        const int warps = 4, nodes = order == 1 ? 32 / 5 : 32 / 11;
+        const size_t smem = (size_t)warps * (nodes + 1) * (g.max_adj + 1) * sizeof(double);
+        auto kern = order == 1 ? k_lap_rows<4> : k_lap_rows<10>;
+        if (smem > 48 * 1024) FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<ceil_div(nnodes, warps * nodes), 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage,
+                                                                      vals, load, nnodes, g.max_adj);
+    }
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

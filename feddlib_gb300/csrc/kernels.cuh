@@ -76,7 +76,7 @@ constexpr int kGNStride = 992;     // floats per element
 constexpr int kGNRes = 960;        // offset of the residual row
 constexpr int kNSRecord = 228;     // floats per element record (Navier-Stokes): 128 + NA[10][10]
 constexpr int kNSTab = 9480;      // floats of the Navier-Stokes device tables
-constexpr int kLapTab = 610;      // doubles of the Laplace device tables
+constexpr int kLapTab = 10;       // doubles of the Laplace device table
 constexpr int kNSResRecord = 168; // floats per element record when only the residual is assembled
 constexpr int kLapStrideP1 = 16;   // doubles: 10 packed K + 4 load + pad
 constexpr int kLapStrideP2 = 72;   // doubles: 55 packed K + 10 load + pad
@@ -171,10 +171,11 @@ void launch_rhs_assemble(const Graph &g, const double *xyz, const int32_t *conn,
 // Laplace (FP64)
 void lap_make_tables(int order, std::vector<double> &out);
 void launch_lap_elem(const double *xyz, const int32_t *conn, int64_t ne, int order, const double *d_tables, double f,
-                     double *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
+                     bool want_k, double *stage, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                      int64_t e_end = -1);
-void launch_lap_rows(const Graph &g, const double *stage, int order, const int64_t *rowptr, double *vals,
-                     double *load, int64_t nnodes, cudaStream_t s, LaunchCounter &lc);
+// vals null: the load alone
+void launch_lap_rows(const Graph &g, const double *stage, int order, double *vals, double *load, int64_t nnodes,
+                     cudaStream_t s, LaunchCounter &lc);
 void launch_lap_dense(const double *stage, int order, int64_t first, int64_t count, double *Ke, double *re,
                       cudaStream_t s);
 
