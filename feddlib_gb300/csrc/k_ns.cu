@@ -448,8 +448,8 @@ __global__ void k_ns_node_info(const int64_t *__restrict__ inc_ptr, const int64_
 
 // velocity rows: block (0,0) and (0,1) values and the velocity residual, and
 // at the vertices of a mesh with a verified vertex map the pressure row too.
-// A warp works on two row nodes at a time, one per half warp, an incidence of
-// each per step: with lanes (p, j) of 15 the half's lane owns the columns
+// A warp works on two row nodes at a time (NPW = 2), one per half warp, an
+// incidence of each per step: with lanes (p, j) of 15 the half's lane owns the columns
 // (b, j) of the two nodes b = 2 p and 2 p + 1, so every value that the ten
 // nodes share (the gradient rows g[j], Bs, the wait, the staging) is read or
 // done once for two incidences.  Warps claim eight consecutive nodes and pair
@@ -484,11 +484,16 @@ static_assert(kVSlots + 4 == kVStage && kRecVel % 4 == 0, "ring slot layout: chu
 // the ring and the accumulators of a half are 16 mod 32 words, so the halves'
 // accesses to the same place of theirs differ in banks
 static_assert(kVRing * kVStage % 32 == 16 && kVRing * kVStageGn % 32 == 16, "half-warp bank offset");
-// warps per CTA at most, two CTAs per SM (shared memory: about 10.3 KB per warp
-// on the structured meshes, 13.6 with the viscous rows)
-__host__ __device__ constexpr int vel_warps(bool gn) { return gn ? 8 : 10; }
+// Small meshes take one node per warp (NPW = 1: lane (b, j) of 30 owns one
+// column): a warp then has a node or a few, the time is that of the longest
+// chain of steps, and a step of 30 lanes with a column each is shorter than one
+// of 15 with two (2,197 nodes 20.4 us against 22.9, 9,261 nodes 34 against
+// 38 us; from 24,000 nodes on the pairs are faster, 57 us against 61).
+// warps per CTA at most, two CTAs per SM (shared memory: about 10.3 KB per pair
+// of nodes on the structured meshes, 13.6 with the viscous rows)
+__host__ __device__ constexpr int vel_warps(bool gn, int npw) { return npw == 1 ? 12 : gn ? 8 : 10; }
 
-// words of one half's accumulators: the three runs, each with its shift and
+// words of one node's accumulators: the three runs, each with its shift and
 // padding to 16 bytes, 32 words of the pressure residual's sum, the scratch word
 __host__ __device__ __forceinline__ int vel_run_words(int len) { return (len + 1 + 3) & ~3; }
 __host__ __device__ __forceinline__ int vel_acc_words(int max_adj, int max_padj, bool pres) {
@@ -496,46 +501,51 @@ __host__ __device__ __forceinline__ int vel_acc_words(int max_adj, int max_padj,
     return (w + 31) & ~31;
 }
 
-// len values of one half warp's run (mem + shift) out as FP64
+// len values of a run (mem + shift) out as FP64 by W lanes
+template <int W>
 __device__ __forceinline__ void vel_write(const float *mem, int shift, int len, double *out, int hl) {
-    if (shift && len > 0 && hl == 15) st_cs(out, f2d_exact(mem[1]));
+    if (shift && len > 0 && hl == W - 1) st_cs(out, f2d_exact(mem[1]));
     const int pairs = len > 0 ? (len - shift) >> 1 : 0;
-    for (int c = hl; c < pairs; c += 16) {
+    for (int c = hl; c < pairs; c += W) {
         const float2 x = *reinterpret_cast<const float2 *>(mem + 2 * shift + 2 * c);
         __stcs(reinterpret_cast<double2 *>(out + shift) + c, make_double2(f2d_exact(x.x), f2d_exact(x.y)));
     }
-    if (len > 0 && ((len - shift) & 1) && hl == 14) st_cs(out + len - 1, f2d_exact(mem[shift + len - 1]));
+    if (len > 0 && ((len - shift) & 1) && hl == W - 2) st_cs(out + len - 1, f2d_exact(mem[shift + len - 1]));
 }
 __device__ __forceinline__ int odd8(const void *p) { return (int)((reinterpret_cast<uintptr_t>(p) >> 3) & 1); }
 
-// velocity residual of the half's node n: row (a, i) sums rj over the lanes
-// (p, i), the nodes b = 2 p and 2 p + 1, and rb over the lanes 4 i + q by
-// strided trees (in b: (((0+1)+(2+3))+((4+5)+(6+7)))+(8+9)); rg, in lane i, is
-// the viscous residual of a generalized-Newtonian fluid.
+// velocity residual of the node n of W lanes: row (a, i) sums rj over the lanes
+// (p, i), the nodes b = 2 p and 2 p + 1 with 16 lanes, b = p with 32, and rb
+// over the lanes 4 i + q by strided trees
+// (in b: (((0+1)+(2+3))+((4+5)+(6+7)))+(8+9)); rg, in lane i, is the viscous
+// residual of a generalized-Newtonian fluid.
 // uu (N(u) u + viscous) + up (-B^T p), with the residual's block factors
-template <bool GN>
+template <bool GN, int W>
 __device__ __forceinline__ void vel_residual_out(float rj0, float rj1, float rb, float rg, int64_t n, int hl, bool node,
                                                  const NSCoeff &co, double *res_u) {
-    const float x = hl < 15 ? rj0 + rj1 : 0.0f;
+    float x = W == 16 ? rj0 + rj1 : rj0 + __shfl_down_sync(0xffffffffu, rj0, 3);
+    constexpr int D = W == 16 ? 3 : 6;  // lanes from one pair of nodes b to the next
+    if (hl >= 30 * W / 32) x = 0.0f;
     float z = hl < 12 ? rb : 0.0f;
-    const float x2 = x + __shfl_down_sync(0xffffffffu, x, 3, 16);
-    const float x4 = x2 + __shfl_down_sync(0xffffffffu, x2, 6, 16);
-    const float xs = x4 + __shfl_down_sync(0xffffffffu, x, 12, 16);
-    z += __shfl_down_sync(0xffffffffu, z, 1, 16);
-    z += __shfl_down_sync(0xffffffffu, z, 2, 16);
-    z = __shfl_sync(0xffffffffu, z, hl < 3 ? 4 * hl : 0, 16);
+    const float x2 = x + __shfl_down_sync(0xffffffffu, x, D, W);
+    const float x4 = x2 + __shfl_down_sync(0xffffffffu, x2, 2 * D, W);
+    const float xs = x4 + __shfl_down_sync(0xffffffffu, x, 4 * D, W);
+    z += __shfl_down_sync(0xffffffffu, z, 1, W);
+    z += __shfl_down_sync(0xffffffffu, z, 2, W);
+    z = __shfl_sync(0xffffffffu, z, hl < 3 ? 4 * hl : 0, W);
     const float cuu = (float)co.uu, s = fmaf(cuu, xs, (float)co.up * z);
     if (node && hl < 3) res_u[3 * n + hl] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
 }
 
-template <bool GN, bool NEWTON>
-__global__ void __launch_bounds__(32 * vel_warps(GN), 2)
+template <bool GN, bool NEWTON, int NPW>
+__global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
     k_ns_vel_rows(const int4 *__restrict__ ninfo, const uint32_t *__restrict__ inc, const uint8_t *__restrict__ slots,
                   const float *__restrict__ rec, const float *__restrict__ gtab, const int64_t *__restrict__ rowptr00,
                   const int64_t *__restrict__ rowptr01, double *vals00, double *vals01, double *res_u, int64_t nnodes,
                   float dens, int group, int acc_words, int64_t n_begin, const int64_t *__restrict__ rowptr10,
                   double *vals10, double *res_p, const float *__restrict__ gstage, unsigned long long *work, NSCoeff co) {
     constexpr int kStg = GN ? kVStageGn : kVStage;
+    constexpr int W = 32 / NPW;  // lanes per node, each with the columns of NPW nodes b
     extern __shared__ __align__(16) float smem[];
     // the W table scaled by the Newton weight rho and the B^T table negated:
     // sR = rho R[a][b][4], sY = -Y[a][p][4]; the diagonal part NA comes with
@@ -544,28 +554,30 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
     static_assert(kTabY == kTabR + 400 && kVelTab == 560, "R and Y are adjacent");
     for (int t = threadIdx.x; t < kVelTab; t += blockDim.x) smem[t] = t < 400 ? dens * gtab[kTabR + t] : -gtab[kTabR + t];
     __syncthreads();
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15, nw = blockDim.x >> 5;
-    float *ring = smem + kVelTab + (size_t)(2 * w + h) * (kVRing * kStg + acc_words);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = lane / W, hl = lane % W, nw = blockDim.x >> 5;
+    float *ring = smem + kVelTab + (size_t)(NPW * w + h) * (kVRing * kStg + acc_words);
     float *mem = ring + kVRing * kStg;
     float *sum32 = mem + acc_words - 36, *scratch = mem + acc_words - 4;
-    // lane roles in the half: (p, j) of the NA / W part for hl < 15, (i, q) = (bi, bq) of the B^T part for hl < 12
-    const bool lw = hl < 15, lb = hl < 12;
+    // lane roles: (p, j) of the NA / W part for hl < 30 / NPW, (i, q) = (bi, bq) of the B^T part for hl < 12
+    const bool lw = hl < 30 / NPW, lb = hl < 12;
     const int p = lw ? hl / 3 : 0, j = lw ? hl - 3 * (hl / 3) : 0;
     const int bi = hl >> 2, bq = hl & 3;
     const float e0 = j == 0 ? 1.0f : 0.0f, e1 = j == 1 ? 1.0f : 0.0f, e2 = j == 2 ? 1.0f : 0.0f;
     // lane-constant addresses in ring slot 0 and in the tables
     const float *pG = ring + kRecG + 12 * j;
-    const float *pU = ring + kRecU + 6 * p + j;
-    const float *pNA = ring + kVNA + 2 * p;
+    const float *pU = ring + kRecU + 3 * NPW * p + j;
+    const float *pNA = ring + kVNA + NPW * p;
     const float *pBS = ring + kRecBS + 4 * (lb ? bi : 0);
     const float *pBSj = ring + kRecBS + 4 * j;
     const float *pP = ring + kRecP + bq;
     const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kVSlots);
-    const float *pR = sR + 8 * p, *pY = sY + 4 * bq, *pYb = sY + 32 * p;
-    // chunk hl, and chunk 16 + hl for hl < 9: record head (to 20), NA window (21-23), slot map (24)
+    const float *pR = sR + 4 * NPW * p, *pY = sY + 4 * bq, *pYb = sY + 16 * NPW * p;
+    // chunks of 16 bytes: record head (to 20), NA window (21-23), slot map (24).  Two nodes per warp: chunk hl,
+    // and c2 = 16 + hl for hl < 9; one: c2 = hl < 25 alone
+    const int c2 = NPW == 2 ? 16 + hl : hl;
     const char *src1 = reinterpret_cast<const char *>(rec + 4 * hl);
-    const char *src2 = reinterpret_cast<const char *>(hl < 5 ? rec + 64 + 4 * hl : rec + kRecNA + 4 * (hl - 5));
-    float *dst_lane = ring + 4 * hl;
+    const char *src2 = reinterpret_cast<const char *>(c2 < 21 ? rec + 4 * c2 : rec + kRecNA + 4 * (c2 - 21));
+    float *dst_lane = ring + 4 * hl, *dst2 = ring + 4 * c2;
     // with `work`, nodes come from a global counter, a group per warp step, so
     // all warps stay on one sharp front of the sweep and the ten readers of
     // an element's record come close in time
@@ -577,56 +589,61 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
         }
         if (it >= nnodes) break;
         // lane k < group: node it + k; rank 0 has the most incidences
-        const bool member = (lane & 7) < group && it + (lane & 7) < nnodes;
-        const int4 inf4 = member ? ninfo[it + (lane & 7)] : make_int4(0, 0, -1, 0);
-        const int m4 = node_m(inf4);
+        const bool member = NPW == 1 || ((lane & 7) < group && it + (lane & 7) < nnodes);
+        const int4 inf4 = member ? ninfo[it + (NPW == 1 ? 0 : lane & 7)] : make_int4(0, 0, -1, 0);
         int rank = 0;
+        if (NPW == 2) {
+            const int m4 = node_m(inf4);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int mk = __shfl_sync(0xffffffffu, m4, k);
-            rank += mk > m4 || (mk == m4 && k < (lane & 7));
+            for (int k = 0; k < 8; k++) {
+                const int mk = __shfl_sync(0xffffffffu, m4, k);
+                rank += mk > m4 || (mk == m4 && k < (lane & 7));
+            }
         }
 #pragma unroll 1
-        for (int pair = 0; 2 * pair < group; pair++) {
-            const unsigned f0 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair);
-            const unsigned f1 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair + 1);
-            const int k = __ffs(h ? f1 : f0) - 1;
-            int4 inf;
-            inf.x = __shfl_sync(0xffffffffu, inf4.x, k);
-            inf.y = __shfl_sync(0xffffffffu, inf4.y, k);
-            inf.z = __shfl_sync(0xffffffffu, inf4.z, k);
-            inf.w = __shfl_sync(0xffffffffu, inf4.w, k);
+        for (int pair = 0; NPW * pair < group; pair++) {
+            int k = 0;
+            int4 inf = inf4;
+            if (NPW == 2) {
+                const unsigned f0 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair);
+                const unsigned f1 = __ballot_sync(0xffffffffu, lane < 8 && rank == 2 * pair + 1);
+                k = __ffs(h ? f1 : f0) - 1;
+                inf.x = __shfl_sync(0xffffffffu, inf4.x, k);
+                inf.y = __shfl_sync(0xffffffffu, inf4.y, k);
+                inf.z = __shfl_sync(0xffffffffu, inf4.z, k);
+                inf.w = __shfl_sync(0xffffffffu, inf4.w, k);
+            }
             const int64_t n = it + k;
             const bool node = k < group && n < nnodes;
             const int m = node_m(inf), K = node_k(inf), Kp = node_kp(inf);
             const int qp = inf.z;  // the P1 node at this vertex, whose pressure row this half assembles too
-            const int mm = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            const int mm = NPW == 2 ? max(m, __shfl_xor_sync(0xffffffffu, m, 16)) : m;
             const int64_t i0 = node_i0(inf);
             const uint32_t *il = inc + i0;
-            if (hl == 8) src2 = reinterpret_cast<const char *>(slots + i0 * kSlotStride);
-            // the half's list, a window of 16 entries at a time
-            uint32_t lst = hl < m ? __ldg(il + hl) : 0u, lst_next = 16 + hl < m ? __ldg(il + 16 + hl) : 0u;
-            // incidence t of the half's node into its ring slot; every call
+            if (c2 == 24) src2 = reinterpret_cast<const char *>(slots + i0 * kSlotStride);
+            // the node's list, a window of W entries at a time
+            uint32_t lst = hl < m ? __ldg(il + hl) : 0u, lst_next = W + hl < m ? __ldg(il + W + hl) : 0u;
+            // incidence t of the node into its ring slot; every call
             // commits one group, empty past the end, so the wait counts hold
             auto stage = [&](int slot, int t) {
-                if (t > 0 && (t & 15) == 0) {  // warp-uniform
+                if (t > 0 && t % W == 0) {  // warp-uniform
                     lst = lst_next;
-                    lst_next = t + 16 + hl < m ? __ldg(il + t + 16 + hl) : 0u;
+                    lst_next = t + W + hl < m ? __ldg(il + t + W + hl) : 0u;
                 }
-                const uint32_t ea = __shfl_sync(0xffffffffu, lst, t & 15, 16);
+                const uint32_t ea = __shfl_sync(0xffffffffu, lst, t % W, W);
                 if (t < m) {
                     const uint32_t a = ea & 15u;
                     const size_t eo = (size_t)(ea >> 4) * (kNSRecord * sizeof(float));
-                    cp_async16(dst_lane + slot * kStg, src1 + eo);
+                    if (NPW == 2) cp_async16(dst_lane + slot * kStg, src1 + eo);
                     // NA[a][0..9] starts 8 bytes into a 16-byte boundary when a is odd
-                    const size_t o2 = hl == 8 ? (size_t)(t * kSlotStride) : eo + (hl < 5 ? 0u : 40u * a - 8u * (a & 1u));
-                    if (hl < 9) cp_async16(dst_lane + slot * kStg + 64, src2 + o2);
+                    const size_t o2 = c2 == 24 ? (size_t)(t * kSlotStride) : eo + (c2 < 21 ? 0u : 40u * a - 8u * (a & 1u));
+                    if (c2 < 25) cp_async16(dst2 + slot * kStg, src2 + o2);
                     if (GN) {
                         const float *Ke = gstage + (size_t)(ea >> 4) * kGNStride;
-                        cp_async16(dst_lane + slot * kStg + kVGn, Ke + 96 * a + 4 * hl);
-                        if (hl < 10)
-                            cp_async16(dst_lane + slot * kStg + kVGn + 64,
-                                       hl < 8 ? Ke + 96 * a + 64 + 4 * hl : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (hl - 8));
+                        if (NPW == 2) cp_async16(dst_lane + slot * kStg + kVGn, Ke + 96 * a + 4 * hl);
+                        if (c2 < 26)
+                            cp_async16(dst2 + slot * kStg + kVGn,
+                                       c2 < 24 ? Ke + 96 * a + 4 * c2 : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (c2 - 24));
                     }
                 }
                 cp_async_commit();
@@ -638,7 +655,7 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
             const int s00 = odd8(out00), s01 = odd8(out01), s10 = odd8(out10);
             const int o01 = vel_run_words(9 * K), o10 = o01 + vel_run_words(3 * Kp);
             const int used = o10 + (qp >= 0 ? vel_run_words(3 * K) : 0);
-            for (int c = 4 * hl; c < used; c += 64) *reinterpret_cast<float4 *>(mem + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 4 * hl; c < used; c += 4 * W) *reinterpret_cast<float4 *>(mem + c) = make_float4(0.f, 0.f, 0.f, 0.f);
             float *acc = mem + s00, *acc1 = mem + o01 + s01, *acc2 = mem + o10 + s10;
             const int st = 3 * K;
             float rj0 = 0.0f, rj1 = 0.0f, rb = 0.0f, rq0 = 0.0f, rq1 = 0.0f, rg = 0.0f;
@@ -655,19 +672,19 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
                 // refilled next
                 __syncwarp();
                 stage((r + kVRing - 1) & (kVRing - 1), t + kVRing - 1);
-                if (t >= m) continue;  // this half's node is done
+                if (NPW == 2 && t >= m) continue;  // this half's node is done
                 const int off = r * kStg;
                 const int a = pS[4 * off + kSlotLocal];  // the staged slot map's local-index byte (broadcast)
                 if (a != a_cur) {
                     a_cur = a;
                     if (NEWTON) {
                         ra = lds4(pR + 40 * a);
-                        rc = lds4(pR + 40 * a + 4);
+                        if (NPW == 2) rc = lds4(pR + 40 * a + 4);
                     }
                     y = lds4(pY + 16 * a);
                     if (qp >= 0 && a < 4) {
                         ya = lds4(pYb + 4 * a);
-                        yc = lds4(pYb + 16 + 4 * a);
+                        if (NPW == 2) yc = lds4(pYb + 16 + 4 * a);
                     }
                 }
                 // NA_ab on the diagonal (i = j) plus wn W_(ai)(bj), i = 0..2
@@ -677,48 +694,62 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
                     g1 = lds4(pG + off + 4);
                     g2 = lds4(pG + off + 8);
                 }
-                const float2 an = *reinterpret_cast<const float2 *>(pNA + off + 2 * (a & 1));
-                const uint32_t ss = *reinterpret_cast<const uint16_t *>(pS + 4 * off + 2 * p);
+                float2 an;
+                uint32_t ss;
+                if (NPW == 2) {
+                    an = *reinterpret_cast<const float2 *>(pNA + off + 2 * (a & 1));
+                    ss = *reinterpret_cast<const uint16_t *>(pS + 4 * off + 2 * p);
+                } else {
+                    an = make_float2(pNA[off + 2 * (a & 1)], 0.0f);
+                    ss = pS[4 * off + p];
+                }
                 float *dA = lw ? acc + 3 * (ss & 255u) + j : scratch, *dB = lw ? acc + 3 * (ss >> 8) + j : scratch;
                 const int sl = lw ? st : 0;
                 // g[j][m*3+i]: m0 = (g0.x,g0.y,g0.z) m1 = (g0.w,g1.x,g1.y) m2 = (g1.z,g1.w,g2.x) m3 = (g2.y,g2.z,g2.w)
                 {
-                    float v0 = dA[0], v1 = dA[sl], v2 = dA[2 * sl], w0 = dB[0], w1 = dB[sl], w2 = dB[2 * sl];
+                    float v0 = dA[0], v1 = dA[sl], v2 = dA[2 * sl];
+                    // the viscous rows (a, i), columns (b, j), and the viscous residual of row (a, hl)
+                    const float *V = ring + off + kVGn + 3 * NPW * p + j;
                     if (GN) {
-                        // the viscous rows (a, i), columns (b, j), and the viscous residual of row (a, hl)
-                        const float *V = ring + off + kVGn + 6 * p + j;
                         v0 += V[0];
                         v1 += V[32];
                         v2 += V[64];
-                        w0 += V[3];
-                        w1 += V[35];
-                        w2 += V[67];
                         rg += ring[off + kVGnRes + ((3 * a) & 3) + (hl & 3)];
                     }
                     v0 = fmaf(e0, an.x, v0);
                     v1 = fmaf(e1, an.x, v1);
                     v2 = fmaf(e2, an.x, v2);
-                    w0 = fmaf(e0, an.y, w0);
-                    w1 = fmaf(e1, an.y, w1);
-                    w2 = fmaf(e2, an.y, w2);
                     if (NEWTON) {
                         v0 = fmaf(g2.y, ra.w, fmaf(g1.z, ra.z, fmaf(g0.w, ra.y, fmaf(g0.x, ra.x, v0))));
                         v1 = fmaf(g2.z, ra.w, fmaf(g1.w, ra.z, fmaf(g1.x, ra.y, fmaf(g0.y, ra.x, v1))));
                         v2 = fmaf(g2.w, ra.w, fmaf(g2.x, ra.z, fmaf(g1.y, ra.y, fmaf(g0.z, ra.x, v2))));
-                        w0 = fmaf(g2.y, rc.w, fmaf(g1.z, rc.z, fmaf(g0.w, rc.y, fmaf(g0.x, rc.x, w0))));
-                        w1 = fmaf(g2.z, rc.w, fmaf(g1.w, rc.z, fmaf(g1.x, rc.y, fmaf(g0.y, rc.x, w1))));
-                        w2 = fmaf(g2.w, rc.w, fmaf(g2.x, rc.z, fmaf(g1.y, rc.y, fmaf(g0.z, rc.x, w2))));
+                    }
+                    if (NPW == 2) {
+                        float w0 = dB[0], w1 = dB[sl], w2 = dB[2 * sl];
+                        if (GN) {
+                            w0 += V[3];
+                            w1 += V[35];
+                            w2 += V[67];
+                        }
+                        w0 = fmaf(e0, an.y, w0);
+                        w1 = fmaf(e1, an.y, w1);
+                        w2 = fmaf(e2, an.y, w2);
+                        if (NEWTON) {
+                            w0 = fmaf(g2.y, rc.w, fmaf(g1.z, rc.z, fmaf(g0.w, rc.y, fmaf(g0.x, rc.x, w0))));
+                            w1 = fmaf(g2.z, rc.w, fmaf(g1.w, rc.z, fmaf(g1.x, rc.y, fmaf(g0.y, rc.x, w1))));
+                            w2 = fmaf(g2.w, rc.w, fmaf(g2.x, rc.z, fmaf(g1.y, rc.y, fmaf(g0.z, rc.x, w2))));
+                        }
+                        dB[0] = w0;
+                        dB[sl] = w1;
+                        dB[2 * sl] = w2;
                     }
                     dA[0] = v0;
                     dA[sl] = v1;
                     dA[2 * sl] = v2;
-                    dB[0] = w0;
-                    dB[sl] = w1;
-                    dB[2 * sl] = w2;
                 }
-                const float ua = pU[off], ub = pU[off + 3];
+                const float ua = pU[off], ub = NPW == 2 ? pU[off + 3] : 0.0f;
                 rj0 = fmaf(an.x, ua, rj0);
-                rj1 = fmaf(an.y, ub, rj1);
+                if (NPW == 2) rj1 = fmaf(an.y, ub, rj1);
                 // -Bd_q(a, i): the (0,1) entry of velocity row (a, i), pressure column q
                 const float4 bs = lds4(pBS + off);
                 const float bt = fmaf(bs.z, y.z, fmaf(bs.y, y.y, bs.x * y.x));
@@ -729,30 +760,39 @@ __global__ void __launch_bounds__(32 * vel_warps(GN), 2)
                     // -Bd_q(b j): the (1,0) entries of pressure row q = this vertex, columns (b, j)
                     const float4 bj = lds4(pBSj + off);
                     const float pa = fmaf(bj.z, ya.z, fmaf(bj.y, ya.y, bj.x * ya.x));
-                    const float pc = fmaf(bj.z, yc.z, fmaf(bj.y, yc.y, bj.x * yc.x));
-                    float *qa = lw ? acc2 + 3 * (ss & 255u) + j : scratch, *qc = lw ? acc2 + 3 * (ss >> 8) + j : scratch;
+                    float *qa = lw ? acc2 + 3 * (ss & 255u) + j : scratch;
                     *qa += pa;
-                    *qc += pc;
                     rq0 = fmaf(pa, ua, rq0);
-                    rq1 = fmaf(pc, ub, rq1);
+                    if (NPW == 2) {
+                        const float pc = fmaf(bj.z, yc.z, fmaf(bj.y, yc.y, bj.x * yc.x));
+                        float *qc = lw ? acc2 + 3 * (ss >> 8) + j : scratch;
+                        *qc += pc;
+                        rq1 = fmaf(pc, ub, rq1);
+                    }
                 }
             }
             cp_async_wait<0>();
             __syncwarp();
-            vel_write(mem, s00, 9 * K, out00, hl);
-            vel_write(mem + o01, s01, 3 * Kp, out01, hl);
-            if (res_u) vel_residual_out<GN>(rj0, rj1, rb, rg, n, hl, node, co, res_u);
-            if (qp >= 0) vel_write(mem + o10, s10, 3 * K, out10, hl);
+            vel_write<W>(mem, s00, 9 * K, out00, hl);
+            vel_write<W>(mem + o01, s01, 3 * Kp, out01, hl);
+            if (res_u) vel_residual_out<GN, W>(rj0, rj1, rb, rg, n, hl, node, co, res_u);
+            if (qp >= 0) vel_write<W>(mem + o10, s10, 3 * K, out10, hl);
             if (res_p && __any_sync(0xffffffffu, qp >= 0)) {
                 // the pressure residual: the pairwise (xor) tree over 32 words, (b, j) at 3 b + j
-                if (lw) {
-                    sum32[6 * p + j] = rq0;
-                    sum32[6 * p + 3 + j] = rq1;
+                float v;
+                if (NPW == 2) {
+                    if (lw) {
+                        sum32[6 * p + j] = rq0;
+                        sum32[6 * p + 3 + j] = rq1;
+                    } else {
+                        sum32[30] = sum32[31] = 0.0f;
+                    }
+                    __syncwarp();
+                    v = sum32[hl] + sum32[hl + 16];
                 } else {
-                    sum32[30] = sum32[31] = 0.0f;
+                    v = lw ? rq0 : 0.0f;
+                    v += __shfl_xor_sync(0xffffffffu, v, 16);
                 }
-                __syncwarp();
-                float v = sum32[hl] + sum32[hl + 16];
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 if (qp >= 0 && hl == 0) res_p[qp] = f2d_exact((float)co.pu * v);
@@ -1097,25 +1137,35 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
     const bool gn = gstage != nullptr;
     const int acc_words = vel_acc_words(max_adj, max_padj, vmap);
     const size_t tables = kVelTab * sizeof(float);
-    const size_t per_warp = 2 * (size_t)(kVRing * (gn ? kVStageGn : kVStage) + acc_words) * sizeof(float);
+    const size_t per_node = (size_t)(kVRing * (gn ? kVStageGn : kVStage) + acc_words) * sizeof(float);
+    const int64_t nn = n_end < 0 ? g.nrow_nodes : n_end, count = nn - n_begin, sms = sm_count_ns();
+    // one node per warp below six nodes for each of the chip's warps (24,389
+    // nodes: pairs 57 us, 66 with the viscous rows, one per warp 61 and 73;
+    // 9,261 nodes 38 and 38 against 34 and 39)
+    const int npw = count < 6 * 2 * sms * vel_warps(gn, 1) ? 1 : 2;
     // two CTAs per SM share its shared memory; one where the rows are so long
     // that two would leave few warps
-    int warps = (int)std::min<size_t>(vel_warps(gn), (113 * 1024 - tables) / per_warp);
-    if (warps < 4) warps = (int)std::max<size_t>(1, std::min<size_t>(vel_warps(gn), (227 * 1024 - tables) / per_warp));
-    // groups of eight nodes, or single pairs spread over all SMs where the mesh
-    // does not keep the chip's warps busy for several groups
-    const int64_t nn = n_end < 0 ? g.nrow_nodes : n_end, sms = sm_count_ns();
-    int group = 8;
-    if (nn - n_begin < sms * 2 * warps * 16) {
-        group = 2;
-        work = nullptr;  // every warp takes one pair or a few: fixed positions
-        warps = (int)std::min<int64_t>(warps, std::max<int64_t>(2, ceil_div((nn - n_begin + 1) / 2, 2 * sms)));
+    const size_t per_warp = npw * per_node;
+    const int most = vel_warps(gn, npw);
+    int warps = (int)std::min<size_t>(most, (113 * 1024 - tables) / per_warp);
+    if (warps < 4) warps = (int)std::max<size_t>(1, std::min<size_t>(most, (227 * 1024 - tables) / per_warp));
+    // pairs come from groups of eight nodes, of four below 64 nodes per warp,
+    // where the last groups would leave warps idle (50,653 nodes 92 us against
+    // 107, 185,193 nodes 304 against 300, 912,673 nodes 1,319 against 1,299)
+    const int group = npw == 1 ? 1 : count < 64 * 2 * sms * warps ? 4 : 8;
+    if (npw == 1 && count <= 2 * sms * warps) {
+        work = nullptr;  // a node per warp at most, spread over all SMs
+        warps = (int)std::min<int64_t>(warps, std::max<int64_t>(2, ceil_div(count, 2 * sms)));
     }
     const size_t smem = tables + (size_t)warps * per_warp;
-    auto kern = gn ? (newton ? k_ns_vel_rows<true, true> : k_ns_vel_rows<true, false>)
-                   : (newton ? k_ns_vel_rows<false, true> : k_ns_vel_rows<false, false>);
+    using Kern = decltype(&k_ns_vel_rows<true, true, 1>);
+    const Kern kerns[2][2][2] = {{{k_ns_vel_rows<false, false, 1>, k_ns_vel_rows<false, false, 2>},
+                                  {k_ns_vel_rows<false, true, 1>, k_ns_vel_rows<false, true, 2>}},
+                                 {{k_ns_vel_rows<true, false, 1>, k_ns_vel_rows<true, false, 2>},
+                                  {k_ns_vel_rows<true, true, 1>, k_ns_vel_rows<true, true, 2>}}};
+    const Kern kern = kerns[gn][newton != 0][npw - 1];
     FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    unsigned grid = (unsigned)std::min<int64_t>((nn - n_begin + group * warps - 1) / (group * warps), sms * 4);
+    unsigned grid = (unsigned)std::min<int64_t>((count + group * warps - 1) / (group * warps), sms * 4);
     if (work) {  // dynamic positions: exactly the CTAs that fit
         int per_sm = 0;
         FEDD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));

@@ -60,3 +60,31 @@ def test_navier_stokes_blocks_at_any_offset(M, newton, gn):
             x = b.cpu().numpy()
             assert np.array_equal(x[o:o + w.size], w) and (x[:o] == -7.0).all() and (x[o + w.size:] == -7.0).all()
         assert np.array_equal(dru.cpu().numpy(), ru) and np.array_equal(drp.cpu().numpy(), rp)
+
+
+@pytest.mark.parametrize("M,newton,gn", [(12, True, False), (12, False, True), (14, True, True), (14, False, False),
+                                         (29, True, False)])
+def test_navier_stokes_rows_of_every_mesh_size(M, newton, gn):
+    """How the velocity rows' nodes are given to the warps depends on their
+    number: one node per warp (15,625 nodes), pairs of groups of four (24,389)
+    or of eight (205,379).  The host-buffer call works in node ranges, which
+    take another of these forms than the whole mesh: the same values."""
+    import torch
+    import feddlib_gb300 as F
+    xyz2, el2 = F.structured_mesh(M, 2, seed=90 + M)
+    xyz1, el1 = F.structured_mesh(M, 1, seed=90 + M)
+    u, p = 0.5 * F.fourier_field(xyz2, seed=90), F.uniform_field(90, xyz1.shape[0])
+    a = F.Assembler(F.NAVIER_STOKES, xyz2, el2, elements_p=el1, num_nodes_p=xyz1.shape[0], viscosity=0.01, density=1.3,
+                    newton=newton)
+    if gn:
+        a.set_viscosity_law(0, [1.902, 0.22, 0.056, 0.00345, 1.25], gamma_min=1e-12)
+    want, ru, rp = a.assemble(u=u, p=p)
+    du, dp = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    bufs = [torch.empty(w.size, dtype=torch.float64, device="cuda") for w in want]
+    dru = torch.empty(a.n_u, dtype=torch.float64, device="cuda")
+    drp = torch.empty(a.n_p, dtype=torch.float64, device="cuda")
+    a.assemble_device(du.data_ptr(), dp.data_ptr(), [b.data_ptr() for b in bufs], dru.data_ptr(), drp.data_ptr())
+    torch.cuda.synchronize()
+    for b, w in zip(bufs, want):
+        assert w.any() and np.array_equal(b.cpu().numpy(), w)
+    assert np.array_equal(dru.cpu().numpy(), ru) and np.array_equal(drp.cpu().numpy(), rp)
