@@ -26,6 +26,31 @@ namespace {
 
 constexpr int kWarps = 4;
 
+// Staged element rows, 32 floats each: word elem_col(a, c) of the rows 3 a + i
+// holds column c; columns 0-29 are (b, j) = 3 b + j, 30 the row's residual entry,
+// 31 zero.  The nodes b are in the order 0-5, 8, 9, 6, 7 (elem_node), and a
+// row's eight 16-byte chunks are rotated by elem_rot(a): with these two the
+// 8-byte stores of the element kernel's tiles, (A, B) and transposed, fall on
+// sixteen different bank pairs.
+__device__ __forceinline__ int elem_node(int b) { return b < 6 ? b : b ^ 14; }
+constexpr unsigned kElemRot = 06273375140;  // three bits per node
+__device__ __forceinline__ int elem_rot(int a) { return (int)(kElemRot >> (3 * a)) & 7; }
+__device__ __forceinline__ int elem_col(int a, int c) {
+    const int k = c < 30 ? 3 * elem_node(c / 3) + c % 3 : c;
+    return 4 * (((k >> 2) + elem_rot(a)) & 7) + (k & 3);
+}
+
+// shared to global memory by the bulk copy engine (16-byte multiples), one thread's groups
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(__cvta_generic_to_global(dst)),
+                 "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ---- laws ----------------------------------------------------------------
 __device__ __forceinline__ void nh_matrix(int kind, float mu, float lam, float J, QPDerivs &d) {
     float iJ = 1.0f / J;
@@ -101,43 +126,52 @@ __device__ __forceinline__ void cof3(const float *F, float *C) {
 }
 
 // ---- element stage ----------------------------------------------------
-// One warp per element, elements taken in batches of 32 per warp:
+// A warp takes a batch of consecutive elements, two at a time:
 //   phase 1  the geometry table's entries, one element of the batch per lane;
-// then for each element of the batch:
-//   phase Q  lane q < nq: F_q, cof F_q and the law's derivatives at F_q,
-//            folded with the weight w_q det B into the scalars below;
-//   phase V  one lane per (node a, point q): G = B^-T grad phi_a(q),
+// then for each pair of elements:
+//   phase Q  lane (element, q < nq): F_q, cof F_q and the law's derivatives at
+//            F_q, folded with the weight w_q det B into the scalars below;
+//   phase V  one lane per (element, point q, node a): G = B^-T grad phi_a(q),
 //            c = cof(F_q) G, f = F_q G, the fibre projections a_f . G and
 //            node a's residual contribution at q;
-//   phase K  one lane per 3 x 3 block (a, b), a <= b (55 blocks in two
-//            passes), summing over q in registers
+//   phase K  a half warp per element, one lane per 2 x 2 tile of node pairs
+//            (2 A + x, 2 B + y), A <= B (15 tiles), so a record read from
+//            shared memory serves two blocks; each 3 x 3 block sums over q in
+//            registers
 //              K_(ai)(bj) += gamma G_a.G_b d_ij + alpha c_ai c_bj
 //                            - beta c_bi c_aj + (law-specific terms)
 //            with gamma = 2 s psi_1, beta = s psi_J / J,
 //            alpha = s (psi_JJ + psi_J / J), s = w_q det B;
-//   epilogue both triangles into a shared-memory image of the element's
-//            rows, then 16-byte coalesced stores.
-// The pass of each block (c_pair_lane) is chosen so that within a pass the
-// block stores and the transposed block stores into the image (row stride
-// kSRow) put at most two lanes on one bank.
-constexpr int kSRow = 44;  // floats per row of the shared element image
+//   epilogue both triangles into a shared-memory image of the elements' rows,
+//            which one bulk copy takes to the stage.
 constexpr int kQS = 52;    // floats per quadrature-point record: 13 chunks of 16 B, so the records
                            // of q = 0..4 start in different bank groups
-constexpr int kVS = 12;    // floats per (point, node) record: c0 c1 c2 G0 | G1 G2 f0 f1 | f2 g1 g2 -
 // quadrature-point record: F 0-8, cof F 9-17, (gamma alpha beta kappa) 20,
 // (phi1 phi2 chi1 chi2) 24, F a1 28, F a2 32, s psi_kl 36-45, residual
 // scalars (-2 s psi_1, -s psi_J, -2 s psi_4a, -2 s psi_4b) 48
 constexpr int kQScal = 20, kQFib = 24, kQFa1 = 28, kQFa2 = 32, kQHess = 36, kQRes = 48;
-constexpr int kImage = 30 * kSRow;  // element image: 30 rows (column 30: the row's residual entry)
-constexpr int kPhaseWords = 5 * kQS + 5 * 10 * kVS + 5 * 32;
-static_assert(kPhaseWords <= kImage, "the phase buffers alias the element image");
+// node records of a point: planes of the ten nodes' 16-byte chunks
+// c0 c1 c2 G0 | G1 G2 (g1 g2 with fibres) | f0 f1 f2 - (where the law's blocks
+// have f), the even nodes before the odd ones: the five records that a load's
+// lanes read lie in different bank groups
+constexpr int kVPlane = 40;  // words of a plane of 16-byte chunks
+__device__ __forceinline__ int node_pos(int a) { return (a >> 1) + 5 * (a & 1); }
+constexpr int kImage = kElemStride;  // floats of an element's image
+constexpr int kPairWords = 2 * kImage + 16 + 5 * kQS;
+// words between the points' node records and between their residual
+// contributions, by the banks of phase V's stores (ch: planes; fibre: 16-byte
+// chunks in the second plane, else 8-byte ones)
+__host__ __device__ constexpr int vpoint(bool fibre, int ch, int nq) {
+    return nq == 4 ? (ch == 2 ? 80 : 144) : (fibre ? 92 : 76) + (ch == 2 ? 0 : 32);
+}
+__host__ __device__ constexpr int rpoint(int nq) { return nq == 4 ? 44 : 33; }
+static_assert(5 * kQS + 8 * (vpoint(true, 3, 4) + rpoint(4)) <= 2 * kImage &&
+                  5 * kQS + 10 * (vpoint(true, 3, 5) + rpoint(5)) <= 2 * kImage,
+              "the phase buffers alias the images");
 
-// lane -> block (a << 4 | b) of pass 0 (entries 0-31) and pass 1 (32-54)
-__constant__ uint8_t c_pair_lane[64] = {
-    0x02, 0x03, 0x04, 0x05, 0x06, 0x08, 0x09, 0x13, 0x15, 0x17, 0x19, 0x23, 0x24, 0x28, 0x29, 0x33,
-    0x38, 0x39, 0x44, 0x46, 0x49, 0x55, 0x56, 0x57, 0x59, 0x66, 0x68, 0x78, 0x79, 0x88, 0x89, 0x99,
-    0x00, 0x01, 0x07, 0x11, 0x12, 0x14, 0x16, 0x18, 0x22, 0x25, 0x26, 0x27, 0x34, 0x35, 0x36, 0x37,
-    0x45, 0x47, 0x48, 0x58, 0x67, 0x69, 0x77, 0xff, 0xff, 0xff, 0xff, 0xff, 0xff, 0xff, 0xff, 0xff};
+// lane of a half warp -> tile (A << 4 | B); lane 15 repeats lane 14's and stores nothing
+__constant__ uint8_t c_tile_lane[16] = {0x00, 0x01, 0x02, 0x03, 0x04, 0x11, 0x12, 0x13,
+                                        0x14, 0x22, 0x23, 0x24, 0x33, 0x34, 0x44, 0x44};
 
 // the scalars of one quadrature point that every block reads
 template <int LAW>
@@ -171,12 +205,11 @@ struct PointScalars {
 
 // one block (a, b) at one quadrature point: K += the block's integrand
 template <int LAW>
-__device__ __forceinline__ void block_update(float *K, const float *Va, const float *Vb, const PointScalars<LAW> &P) {
+__device__ __forceinline__ void block_update(float *K, const float4 *va, const float4 *vb, const PointScalars<LAW> &P) {
     constexpr bool kFibre = (LAW == kLawAniso || LAW == kLawMLP || LAW == kLawMLPF);
     constexpr bool kFullHess = (LAW == kLawMLP);
     constexpr bool kCross = (LAW == kLawSKR3);
-    const float4 a0 = reinterpret_cast<const float4 *>(Va)[0], a1 = reinterpret_cast<const float4 *>(Va)[1];
-    const float4 b0 = reinterpret_cast<const float4 *>(Vb)[0], b1 = reinterpret_cast<const float4 *>(Vb)[1];
+    const float4 a0 = va[0], a1 = va[1], b0 = vb[0], b1 = vb[1];
     const float ca[3] = {a0.x, a0.y, a0.z}, cb[3] = {b0.x, b0.y, b0.z};
     float dg = P.s.x * (a0.w * b0.w + a1.x * b1.x + a1.y * b1.y);
     float t[3], n[3];
@@ -190,8 +223,12 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
 #pragma unroll
         for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(cb[i], n[j], fmaf(ca[i], t[j], K[3 * i + j]));
     if (kCross || kFibre) {
-        const float4 a2 = reinterpret_cast<const float4 *>(Va)[2], b2 = reinterpret_cast<const float4 *>(Vb)[2];
-        const float fa[3] = {a1.z, a1.w, a2.x}, fb[3] = {b1.z, b1.w, b2.x};
+        float fa[3], fb[3];
+        if (kCross || kFullHess) {
+            const float4 a2 = va[2], b2 = vb[2];
+            fa[0] = a2.x; fa[1] = a2.y; fa[2] = a2.z;
+            fb[0] = b2.x; fb[1] = b2.y; fb[2] = b2.z;
+        }
         if (kCross) {  // psi_1J (D_1 (x) D_J + D_J (x) D_1), D_1 = 2 f
             float kf[3], kc[3];
 #pragma unroll
@@ -205,7 +242,7 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
                 for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(fa[i], kc[j], fmaf(ca[i], kf[j], K[3 * i + j]));
         }
         if (kFibre) {
-            const float g1 = a2.y * b2.y, g2 = a2.z * b2.z;
+            const float g1 = a1.z * b1.z, g2 = a1.w * b1.w;
             dg = fmaf(P.fib.x, g1, fmaf(P.fib.y, g2, dg));
             if (!kFullHess) {  // psi_4f4f D_4f (x) D_4f, D_4f = 2 (a_f . G) F a_f
                 const float x1 = P.fib.z * g1, x2 = P.fib.w * g2;
@@ -216,7 +253,7 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
                     for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(y2, P.fa2[j], fmaf(y1, P.fa1[j], K[3 * i + j]));
                 }
                 if (LAW == kLawMLPF) {  // psi_4a4b (D_4a (x) D_4b + D_4b (x) D_4a), 4 s psi_4a4b in s.w
-                    const float c12 = P.s.w * a2.y * b2.z, c21 = P.s.w * a2.z * b2.y;
+                    const float c12 = P.s.w * a1.z * b1.w, c21 = P.s.w * a1.w * b1.z;
 #pragma unroll
                     for (int i = 0; i < 3; i++) {
                         const float y1 = c12 * P.fa1[i], y2 = c21 * P.fa2[i];
@@ -232,10 +269,10 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
                     Db[0][i] = 2.0f * fb[i];
                     Da[1][i] = ca[i];
                     Db[1][i] = cb[i];
-                    Da[2][i] = 2.0f * a2.y * P.fa1[i];
-                    Db[2][i] = 2.0f * b2.y * P.fa1[i];
-                    Da[3][i] = 2.0f * a2.z * P.fa2[i];
-                    Db[3][i] = 2.0f * b2.z * P.fa2[i];
+                    Da[2][i] = 2.0f * a1.z * P.fa1[i];
+                    Db[2][i] = 2.0f * b1.z * P.fa1[i];
+                    Da[3][i] = 2.0f * a1.w * P.fa2[i];
+                    Db[3][i] = 2.0f * b1.w * P.fa2[i];
                 }
                 const float *h = P.h;
 #pragma unroll
@@ -258,24 +295,30 @@ __device__ __forceinline__ void block_update(float *K, const float *Va, const fl
 
 // LAW: kLawSKR1 / kLawSKR2 / kLawSKR3 / kLawAniso (fused plain law) or
 // kLawMLP (reads per-QP derivatives of the surrogate network, adds the skr1
-// matrix part).  Six CTAs per SM (at most 85 registers; the 33 KB of shared
-// memory allow six) for every law but the full-Hessian surrogate, four for
-// that one; without the bound the register allocation of these instances
-// drifts between 72 and 160 with unrelated edits.
+// matrix part).  Five CTAs per SM (at most 102 registers; the 43 KB of shared
+// memory allow five), four for the full-Hessian surrogate.  Bound by the
+// instruction rate (70 %) and the shared-memory pipe (76 %) together; DRAM takes
+// the rows at 60 to 85 % of the copy bandwidth.  us at 32^3 x 6 tets of linear
+// elasticity, at 64^3 x 6 of skr2 and at 40^3 x 6 of the fibre-block surrogate:
+// 219, 1,941 and 690 with a warp per element, one block per lane and pass, and an
+// image read back by its lanes; 148, 1,564 and 593 with tiles and bulk stores;
+// 125, 1,501 and 576 with conflict-free stores and a point's values read once for
+// its nodes; 125, 1,330 and 558 with the next pair's displacements read ahead.
 template <int LAW, bool HAS_U>
-__global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_elem(const float *__restrict__ geo,
+__global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_elem(const float *__restrict__ geo,
                                                             const int32_t *__restrict__ conn, int64_t ne,
                                                             const double *__restrict__ u, LawParams L,
                                                             const QPDerivs *__restrict__ qpd,
                                                             const uint8_t *__restrict__ qpfb, float *stage,
-                                                            int want_res, int *err, int64_t e_begin, int64_t e_end,
+                                                            int want_res, int *err, int64_t e_begin, int64_t e_end, int batch,
                                                             const __grid_constant__ HyperTables tab) {
     constexpr bool kFibre = (LAW == kLawAniso || LAW == kLawMLP || LAW == kLawMLPF);
+    constexpr int CH = LAW == kLawMLP || LAW == kLawSKR3 ? 3 : 2;  // chunks of a node record
     __shared__ __align__(16) float sdphi[5][36];  // per point: grad_ref phi of the 10 nodes, zero padded
     __shared__ float sw[5];
-    __shared__ float sBi[kWarps][32][11];
+    __shared__ __align__(16) float sBi[kWarps][32][12];  // B^-1, det B
     __shared__ __align__(16) float sU[kWarps][2][36];  // nodal u of the element pair of phase Q
-    __shared__ __align__(16) float sBuf[kWarps][kImage + 5 * kQS];
+    __shared__ __align__(16) float sBuf[kWarps][kPairWords];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nq = tab.nq;
     for (int i = threadIdx.x; i < 5 * 36; i += blockDim.x) {
@@ -286,25 +329,33 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
     if (lane < 12) sU[w][lane / 6][30 + lane % 6] = 0.0f;
     __syncthreads();
 
-    const unsigned p0 = c_pair_lane[lane], p1 = c_pair_lane[32 + lane];
-    const int pa0 = (int)(p0 >> 4), pb0 = (int)(p0 & 15u);
-    const bool two = p1 != 0xFFu;
-    const int pa1 = two ? (int)(p1 >> 4) : 0, pb1 = two ? (int)(p1 & 15u) : 0;
+    const int h = lane >> 4, hl = lane & 15;
+    const int A = c_tile_lane[hl] >> 4, B = c_tile_lane[hl] & 15;
     // per warp: point records of an even element (QA) | V | Rq, aliased by
-    // the element image, then the point records of the odd element after it
-    // (QB), which the even element's image leaves alone: phase Q runs once
-    // per element pair, on 2 nq lanes
-    float *QA = sBuf[w];            // [5][kQS]
-    float *V = QA + 5 * kQS;        // [5][10][kVS]
-    float *Rq = V + 5 * 10 * kVS;   // [5][32]: residual contribution of (node, component) at q
-    float *QB = sBuf[w] + kImage;   // [5][kQS]
-    float *O = sBuf[w];             // element image, aliases QA, V and Rq
+    // the elements' images, then the point records of the odd element (QB)
+    float *QA = sBuf[w];                         // [5][kQS]
+    float *V = QA + 5 * kQS;                     // [2][nq] of CH planes
+    constexpr int P1 = kVPlane, P2 = P1 + (kFibre ? 40 : 20), W1 = kFibre ? 4 : 2;  // the planes, words per chunk of the second
+    const int vp = vpoint(kFibre, CH, nq), rp = rpoint(nq);
+    float *Rq = V + 2 * nq * vp;                 // [2][nq][rp]: residual contributions of (node, component)
+    float *QB = sBuf[w] + 2 * kImage + 16;       // [5][kQS], in other banks than QA
+    float *O = sBuf[w] + h * kImage;             // this half's image
+    // the tile's places in the image: the pairs of columns c of B in the rows of A, and of A in the rows of B
+    // (those of the odd nodes' rows: 16 words on or back)
+    int oAB[3], oBA[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const int cb = 3 * elem_node(2 * B) + 2 * c, ca = 3 * elem_node(2 * A) + 2 * c;
+        oAB[c] = 192 * A + 4 * (((cb >> 2) + elem_rot(2 * A)) & 7) + (cb & 3);
+        oBA[c] = 192 * B + 4 * (((ca >> 2) + elem_rot(2 * B)) & 7) + (ca & 3);
+    }
+    const int rcol = 32 * lane + 4 * ((7 + elem_rot(lane / 3)) & 7) + 2;  // row `lane`, columns 30 and 31
 
-    for (int64_t e0 = e_begin + ((int64_t)blockIdx.x * kWarps + w) * 32; e0 < e_end;
-         e0 += (int64_t)gridDim.x * kWarps * 32) {
+    for (int64_t e0 = e_begin + ((int64_t)blockIdx.x * kWarps + w) * batch; e0 < e_end;
+         e0 += (int64_t)gridDim.x * kWarps * batch) {
         {  // phase 1: geometry, one element per lane
             int64_t e = e0 + lane;
-            if (e < e_end) {
+            if (lane < batch && e < e_end) {
                 float Bi[9];
                 const float det = load_geometry(geo, ne, e, Bi);
 #pragma unroll
@@ -316,28 +367,43 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
             }
         }
         __syncwarp();
-        const int nb = (int)min((int64_t)32, e_end - e0);
-        for (int t = 0; t < nb; t++) {
-            const int64_t el = e0 + t;
-            float *Q = (t & 1) ? QB : QA;  // this element's point records
-            float Bi[9];
+        const int nb = (int)min((int64_t)batch, e_end - e0);
+        // nodal u of a pair of elements, values lane and lane + 32 of its 60: the
+        // next pair's nodes are read before phase Q, their u before phase K
+        int32_t un[2] = {0, 0};
+        double uv[2] = {0.0, 0.0};
+        auto read_nodes = [&](int t) {
 #pragma unroll
-            for (int k = 0; k < 9; k++) Bi[k] = sBi[w][t][k];
-            // phase Q, at even t for the elements t and t + 1: one lane per
-            // (element, quadrature point), lane = ep nq + q
-            if ((t & 1) == 0) {
+            for (int m = 0; m < 2; m++) {
+                const int k = lane + 32 * m, ep = k >= 30 ? 1 : 0;
+                if (k < 60 && t + ep < nb) un[m] = __ldg(conn + (int64_t)((k - 30 * ep) / 3) * ne + e0 + t + ep);
+            }
+        };
+        auto read_u = [&]() {
+#pragma unroll
+            for (int m = 0; m < 2; m++) uv[m] = __ldg(u + 3 * (int64_t)un[m] + (lane + 32 * m) % 3);
+        };
+        if (HAS_U) {
+            read_nodes(0);
+            read_u();
+        }
+        for (int t = 0; t < nb; t += 2) {
+            const int64_t el = e0 + t;
+            const int pair = t + 1 < nb ? 2 : 1;
+            // phase Q: one lane per (element, quadrature point), lane = ep nq + q
+            {
                 if (HAS_U) {
-                    for (int k = lane; k < 60; k += 32) {
-                        const int ep = k >= 30 ? 1 : 0, kk = k - 30 * ep;
-                        if (t + ep < nb) {
-                            const int32_t node = conn[(int64_t)(kk / 3) * ne + el + ep];
-                            sU[w][ep][kk] = d2f_rn(u[3 * (int64_t)node + kk % 3]);
-                        }
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const int k = lane + 32 * m, ep = k >= 30 ? 1 : 0;
+                        if (k < 60) sU[w][ep][k - 30 * ep] = d2f_rn(uv[m]);
                     }
+                    read_nodes(t + 2);
                 }
+                if (lane == 0) bulk_wait_read();  // the previous pair's images have left
                 __syncwarp();
                 const int ep = lane >= nq ? 1 : 0, q = lane - ep * nq;
-                if (lane < 2 * nq && t + ep < nb) {
+                if (lane < pair * nq) {
                 const float *Bq = sBi[w][t + ep];
                 const float detB = Bq[9];
                 float F[9];
@@ -440,20 +506,36 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
                 }
             }
             __syncwarp();
-            // phase V: one lane per (point q, node a)
-            for (int it = lane; it < 10 * nq; it += 32) {
-                const int q = it / 10, a = it - 10 * q;
-                const float *Qq = Q + q * kQS;
-                const float g0 = sdphi[q][3 * a], g1 = sdphi[q][3 * a + 1], g2 = sdphi[q][3 * a + 2];
-                float G[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) G[k] = Bi[k] * g0 + Bi[3 + k] * g1 + Bi[6 + k] * g2;
-                float FC[20];
+            // phase V: a lane works at one (element, point q) on three nodes (four with five points); which
+            // ones, and the strides, put no two of the lanes' stores at four points on one bank
+            {
+                const int parts = nq == 4 ? 4 : 3, qq = lane / parts, ep = qq >= nq ? 1 : 0, q = qq - ep * nq;
+                if (qq < nq * pair) {
+                const float *Qq = (ep ? QB : QA) + q * kQS;
+                float FC[20], Bi[12];
 #pragma unroll
                 for (int m = 0; m < 5; m++) {
                     const float4 x = reinterpret_cast<const float4 *>(Qq)[m];
                     FC[4 * m] = x.x; FC[4 * m + 1] = x.y; FC[4 * m + 2] = x.z; FC[4 * m + 3] = x.w;
                 }
+#pragma unroll
+                for (int m = 0; m < 3; m++) {
+                    const float4 x = reinterpret_cast<const float4 *>(sBi[w][t + ep])[m];
+                    Bi[4 * m] = x.x; Bi[4 * m + 1] = x.y; Bi[4 * m + 2] = x.z; Bi[4 * m + 3] = x.w;
+                }
+                const float4 rs = *reinterpret_cast<const float4 *>(Qq + kQRes);
+                float4 x1, x2;  // F a1, F a2
+                if (kFibre) {
+                    x1 = *reinterpret_cast<const float4 *>(Qq + kQFa1);
+                    x2 = *reinterpret_cast<const float4 *>(Qq + kQFa2);
+                }
+                float *Vq = V + qq * vp, *rq = Rq + qq * rp;
+                const int per = nq == 4 ? 3 : 4, a0 = per * (lane - parts * qq), a1 = min(a0 + per, 10);
+                for (int a = a0; a < a1; a++) {
+                const float g0 = sdphi[q][3 * a], g1 = sdphi[q][3 * a + 1], g2 = sdphi[q][3 * a + 2];
+                float G[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) G[k] = Bi[k] * g0 + Bi[3 + k] * g1 + Bi[6 + k] * g2;
                 float c[3], f[3];
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
@@ -465,69 +547,96 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 6) k_hyper_e
                     ag1 = L.a1[0] * G[0] + L.a1[1] * G[1] + L.a1[2] * G[2];
                     ag2 = L.a2[0] * G[0] + L.a2[1] * G[1] + L.a2[2] * G[2];
                 }
-                float4 *Vr = reinterpret_cast<float4 *>(V + (q * 10 + a) * kVS);
-                Vr[0] = make_float4(c[0], c[1], c[2], G[0]);
-                Vr[1] = make_float4(G[1], G[2], f[0], f[1]);
-                Vr[2] = make_float4(f[2], ag1, ag2, 0.0f);
+                const int at = node_pos(a);
+                *reinterpret_cast<float4 *>(Vq + 4 * at) = make_float4(c[0], c[1], c[2], G[0]);
+                if (kFibre) *reinterpret_cast<float4 *>(Vq + P1 + 4 * at) = make_float4(G[1], G[2], ag1, ag2);
+                else *reinterpret_cast<float2 *>(Vq + P1 + 2 * at) = make_float2(G[1], G[2]);
+                if (CH == 3) *reinterpret_cast<float4 *>(Vq + P2 + 4 * at) = make_float4(f[0], f[1], f[2], 0.0f);
                 if (want_res) {
-                    const float4 rs = *reinterpret_cast<const float4 *>(Qq + kQRes);
                     float r[3];
 #pragma unroll
                     for (int i = 0; i < 3; i++) r[i] = rs.x * f[i] + rs.y * c[i];
                     if (kFibre) {
-                        const float4 x = *reinterpret_cast<const float4 *>(Qq + kQFa1);
-                        const float4 y = *reinterpret_cast<const float4 *>(Qq + kQFa2);
                         const float h1 = rs.z * ag1, h2 = rs.w * ag2;
-                        r[0] += h1 * x.x + h2 * y.x;
-                        r[1] += h1 * x.y + h2 * y.y;
-                        r[2] += h1 * x.z + h2 * y.z;
+                        r[0] += h1 * x1.x + h2 * x2.x;
+                        r[1] += h1 * x1.y + h2 * x2.y;
+                        r[2] += h1 * x1.z + h2 * x2.z;
                     }
 #pragma unroll
-                    for (int i = 0; i < 3; i++) Rq[32 * q + 3 * a + i] = r[i];
+                    for (int i = 0; i < 3; i++) rq[3 * a + i] = r[i];
+                }
+                }
                 }
             }
             __syncwarp();
-            // phase K: the blocks, summed over the points in registers
-            float K0[9], K1[9];
+            if (HAS_U && t + 2 < nb) read_u();
+            // phase K: the tile's four blocks, summed over the points in registers
+            float K[2][2][9];
 #pragma unroll
-            for (int k = 0; k < 9; k++) K0[k] = K1[k] = 0.0f;
+            for (int k = 0; k < 36; k++) (&K[0][0][0])[k] = 0.0f;
+            const float *Qh = h ? QB : QA, *Vh = V + h * nq * vp;
             for (int q = 0; q < nq; q++) {
                 PointScalars<LAW> P;
-                P.load(Q + q * kQS);
-                const float *Vq = V + q * 10 * kVS;
-                block_update<LAW>(K0, Vq + pa0 * kVS, Vq + pb0 * kVS, P);
-                if (two) block_update<LAW>(K1, Vq + pa1 * kVS, Vq + pb1 * kVS, P);
-            }
-            float r = 0.0f;
-            if (want_res && lane < 30)
-                for (int q = 0; q < nq; q++) r += Rq[32 * q + lane];
-            __syncwarp();  // the phase buffers are dead: the element image overwrites them
+                P.load(Qh + q * kQS);
+                const float *Vq = Vh + q * vp;
+                float4 va[2][CH], vb[2][CH];
+                auto record = [&](int at, float4 *v) {
+                    v[0] = *reinterpret_cast<const float4 *>(Vq + 4 * at);
+                    if (kFibre) {
+                        v[1] = *reinterpret_cast<const float4 *>(Vq + P1 + W1 * at);
+                    } else {
+                        const float2 g = *reinterpret_cast<const float2 *>(Vq + P1 + W1 * at);
+                        v[1] = make_float4(g.x, g.y, 0.0f, 0.0f);
+                    }
+                    if (CH == 3) v[2] = *reinterpret_cast<const float4 *>(Vq + P2 + 4 * at);
+                };
 #pragma unroll
-            for (int pp = 0; pp < 2; pp++) {
-                if (pp == 1 && !two) break;
-                const int a = pp ? pa1 : pa0, b = pp ? pb1 : pb0;
-                const float *Kb = pp ? K1 : K0;
+                for (int x = 0; x < 2; x++) {
+                    record(A + 5 * x, va[x]);
+                    record(B + 5 * x, vb[x]);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; x++)
+#pragma unroll
+                    for (int y = 0; y < 2; y++) block_update<LAW>(K[x][y], va[x], vb[y], P);
+            }
+            float r0 = 0.0f, r1 = 0.0f;
+            if (want_res && lane < 30)
+                for (int q = 0; q < nq; q++) {
+                    r0 += Rq[rp * q + lane];
+                    r1 += Rq[rp * (nq + q) + lane];
+                }
+            if (A == B) {  // the lower block of a tile on the diagonal is the upper one transposed
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
-                    for (int j = 0; j < 3; j++) {
-                        O[kSRow * (3 * a + i) + 3 * b + j] = Kb[3 * i + j];
-                        if (a != b) O[kSRow * (3 * b + j) + 3 * a + i] = Kb[3 * i + j];
+                    for (int j = 0; j < 3; j++) K[1][0][3 * i + j] = K[0][1][3 * j + i];
+            }
+            __syncwarp();  // the phase buffers are dead: the images overwrite them
+            if (hl < 15 && h < pair) {
+#pragma unroll
+                for (int r = 0; r < 6; r++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        const int u = 2 * c, v = 2 * c + 1;  // columns of the tile
+                        *reinterpret_cast<float2 *>(O + (r < 3 ? oAB[c] : oAB[c] ^ 16) + 32 * r) =
+                            make_float2(K[r / 3][u / 3][3 * (r % 3) + u % 3], K[r / 3][v / 3][3 * (r % 3) + v % 3]);
+                        if (A != B)
+                            *reinterpret_cast<float2 *>(O + (r < 3 ? oBA[c] : oBA[c] ^ 16) + 32 * r) =
+                                make_float2(K[u / 3][r / 3][3 * (u % 3) + r % 3], K[v / 3][r / 3][3 * (v % 3) + r % 3]);
                     }
             }
-            if (lane < 30) O[kSRow * lane + kElemResCol] = r;  // row 3 a + i = lane
-            __syncwarp();
-            // global layout: rows of 32 floats, column 30 the residual entry, column 31 zero
-            float4 *dst = reinterpret_cast<float4 *>(stage + el * kElemStride);
-            for (int k = lane; k < kElemStride / 4; k += 32) {
-                float4 v = *reinterpret_cast<const float4 *>(O + kSRow * (k >> 3) + 4 * (k & 7));
-                if ((k & 7) == 7) v.w = 0.0f;
-                dst[k] = v;
+            if (lane < 30) {
+                *reinterpret_cast<float2 *>(sBuf[w] + rcol) = make_float2(r0, 0.0f);
+                if (pair == 2) *reinterpret_cast<float2 *>(sBuf[w] + kImage + rcol) = make_float2(r1, 0.0f);
             }
+            fence_async_shared();
             __syncwarp();
+            if (lane == 0) bulk_store(stage + el * kElemStride, sBuf[w], (uint32_t)(pair * kElemStride * sizeof(float)));
         }
         __syncwarp();
     }
+    if (lane == 0) bulk_wait_all();
 }
 
 // ---- row stage ----------------------------------------------------------
@@ -543,16 +652,18 @@ constexpr int kHSlots = 96;
 
 // stage incidence t (of m) of a node into ring slot `slot` (a constant after
 // unrolling): lanes 0-23 the three rows 3 a + i of the element matrix (96
-// contiguous floats; column 30 of each row carries its residual entry), lane
-// 24 the slot map; each lane's destination is ring slot + 4 lane.  Every call
+// contiguous floats, each row's chunks rotated by elem_rot(a)), lane 24 the
+// slot map; each lane's destination is ring slot + 4 lane.  Every call
 // commits one group, empty past the node's last incidence, so the wait counts
 // hold.
 __device__ __forceinline__ void hyper_stage(float *dst_lane, int slot, int t, int m, const IncList &il,
                                             const uint8_t *__restrict__ slots_node,
-                                            const float *__restrict__ stage_lane, int lane) {
+                                            const float *__restrict__ stage_row, int lane) {
     if (t < m) {  // warp-uniform: every lane takes part in the shuffle
         const uint32_t ea = m <= 32 ? __shfl_sync(0xffffffffu, il.lo, t & 31) : incidence_at(il, t);
-        const void *src = lane < 24 ? static_cast<const void *>(stage_lane + (size_t)(ea >> 4) * kElemStride + 96 * (ea & 15u))
+        const int a = (int)(ea & 15u);
+        const void *src = lane < 24 ? static_cast<const void *>(stage_row + (size_t)(ea >> 4) * kElemStride + 96 * a +
+                                                                4 * ((lane + (kElemRot >> (3 * a))) & 7u))
                                     : static_cast<const void *>(slots_node + t * kSlotStride);
         if (lane < 25) cp_async16(dst_lane + slot * kHStage, src);
     }
@@ -568,7 +679,7 @@ __device__ __forceinline__ void hyper_stage(float *dst_lane, int slot, int t, in
 // pipe (76 %) together: 1,915 us at 64^3 x 6 tets and 257 us at 32^3 x 6 (75 %
 // of the copy bandwidth in DRAM bytes), against 2,160 and 285 us with three
 // planes of fixed stride, 8-byte stores, a separate residual sum and eight
-// warps per CTA.  Slower: reading the rows straight into registers without the
+// warps per CTA (1,944 and 265 us since the stage's chunks are rotated).  Slower: reading the rows straight into registers without the
 // ring (334 us at 32^3), a ring running on across the nodes of a warp's run
 // (298), the hardware FP32 -> FP64 conversion in place of f2d_exact (294).
 constexpr int kHPad = 8;  // words besides the 9 K
@@ -587,14 +698,14 @@ __global__ void __launch_bounds__(128) k_hyper_rows(const int64_t *__restrict__ 
     const int b = lw ? lane / 3 : 0, j = lw ? lane - 3 * (lane / 3) : 0;
     float *dst_lane = ring + 4 * lane;
     const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kHSlots) + b;
-    const float *pV = ring + lane, *stage_lane = stage + 4 * lane;
+    const float *pV = ring + (lw ? 3 * elem_node(b) + j : lane), *stage_row = stage + 32 * (lane >> 3);
     for (int64_t n = n_begin + (int64_t)blockIdx.x * nw + w; n < nnodes; n += (int64_t)gridDim.x * nw) {
         const int64_t i0 = inc_ptr[n], i1 = inc_ptr[n + 1];
         const int m = (int)(i1 - i0);
         const IncList il = load_incidences(inc, i0, m, lane);
         const uint8_t *slots_node = slots + i0 * kSlotStride;
 #pragma unroll
-        for (int t = 0; t < kHRing - 1; t++) hyper_stage(dst_lane, t, t, m, il, slots_node, stage_lane, lane);
+        for (int t = 0; t < kHRing - 1; t++) hyper_stage(dst_lane, t, t, m, il, slots_node, stage_row, lane);
         const int64_t a0 = adj_ptr[n];
         const int K = (int)(adj_ptr[n + 1] - a0), len = 9 * K;
         double *out = vals + 9 * a0;
@@ -613,7 +724,7 @@ __global__ void __launch_bounds__(128) k_hyper_rows(const int64_t *__restrict__ 
                 // the slot's copies are visible to the warp, and every lane is
                 // done with the slot consumed in the previous step, refilled next
                 __syncwarp();
-                hyper_stage(dst_lane, (rs + kHRing - 1) % kHRing, t + kHRing - 1, m, il, slots_node, stage_lane, lane);
+                hyper_stage(dst_lane, (rs + kHRing - 1) % kHRing, t + kHRing - 1, m, il, slots_node, stage_row, lane);
                 float *dst = d0 + mul * pS[4 * rs * kHStage];
                 dst[0] += pV[rs * kHStage];
                 dst[st] += pV[rs * kHStage + 32];
@@ -852,9 +963,9 @@ __global__ void k_hyper_dense(const float *__restrict__ stage, int64_t first, in
     const float *S = stage + (first + e) * kElemStride;
     if (k < 900) {
         int p = k / 30, q = k % 30;
-        Ke[e * 900 + k] = (double)S[32 * p + q];
+        Ke[e * 900 + k] = (double)S[32 * p + elem_col(p / 3, q)];
     } else {
-        re[e * 30 + (k - 900)] = (double)S[32 * (k - 900) + kElemResCol];
+        re[e * 30 + (k - 900)] = (double)S[32 * (k - 900) + elem_col((k - 900) / 3, kElemResCol)];
     }
 }
 
@@ -967,18 +1078,22 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
                        int want_res, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin,
                        int64_t e_end) {
     if (e_end < 0) e_end = ne;
-    int64_t warps = (e_end - e_begin + 31) / 32;
-    unsigned grid = (unsigned)std::min<int64_t>((warps + kWarps - 1) / kWarps, (int64_t)sm_count() * 16);
-    if (grid == 0) return;
+    const int64_t count = e_end - e_begin;
+    if (count <= 0) return;
+    // batches of at most 32 elements, even, that give the chip's warps equal
+    // shares in as few rounds as there have to be
+    const int64_t chip = (int64_t)sm_count() * 5 * kWarps, rounds = ceil_div(count, 32 * chip);
+    const int batch = 2 * (int)ceil_div(count, 2 * rounds * chip);
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)batch * kWarps), (int64_t)sm_count() * 16);
     const bool hu = u != nullptr;
 #define FEDD_HYPER(LAWK)                                                                                 \
     do {                                                                                                 \
         if (hu)                                                                                          \
             k_hyper_elem<LAWK, true><<<grid, 32 * kWarps, 0, s>>>(geo, conn, ne, u, law, qpd, qp_fallback, \
-                                                                  stage, want_res, d_err, e_begin, e_end, tab); \
+                                                                  stage, want_res, d_err, e_begin, e_end, batch, tab); \
         else                                                                                             \
             k_hyper_elem<LAWK, false><<<grid, 32 * kWarps, 0, s>>>(geo, conn, ne, u, law, qpd, qp_fallback, \
-                                                                   stage, want_res, d_err, e_begin, e_end, tab); \
+                                                                   stage, want_res, d_err, e_begin, e_end, batch, tab); \
     } while (0)
     switch (law.kind) {
     case kLawSKR2: FEDD_HYPER(kLawSKR2); break;
