@@ -16,7 +16,7 @@
 // element (advection, its Newton term, B and B^T) is the Navier-Stokes
 // element, assembled by k_ns.cu with the Newtonian viscosity set to zero.
 //
-// One warp per element, elements taken in batches of 32 per warp; lane
+// One warp per element, elements taken in batches per warp; lane
 // 3 b + l owns column (b, l) of the dense 30 x 30 matrix and row (b, l) of
 // the residual.  The geometry comes from the mesh's table, formed in FP64; the
 // rest is FP32.
@@ -80,34 +80,73 @@ __device__ float gn_dterm(const ViscLaw &L, float g) {
                    powf(1.0f + (c[0] * g) * (c[0] * g), (c[1] - 3.0f) * 0.5f));
 }
 
-// per-warp scratch: the element's velocities, and per quadrature point (5
-// stress points, then 15 Newton points) the physical basis gradients, the
-// stress points' gradients scaled by w eta and their w eta (du + du^T), and
-// the Newton points' derivative weight, symmetric velocity gradient and row
-// factors
-constexpr int kGNRow = 44;  // 11 chunks of 16 B: the 16-byte stores of lanes q fall in different bank groups
+// per-warp scratch: the element's velocities; per stress point the physical
+// basis gradients, the same scaled by w eta, and w eta (du + du^T); per Newton
+// point the row factors F_a^k and the column factors -2 w c G_b^l.  Node values
+// lie by component, so two nodes' are a packed operand.
 struct __align__(16) GNWarpSmem {
     float su[32];
-    float sg[20][kGNRow];   // sg[q][4 b + c] = d phi_b / d x_c at point q
-    float sgw[5][kGNRow];   // stress points: w eta d phi_b / d x_c at 4 b + c
-    float sT[5][6];         // stress points: w eta (du + du^T), entries 00 11 22 01 02 12
-    float sw[20];           // Newton points (index 5 + q): -2 w c
-    float sm[15][6];        // Newton points: du11, du22, du33, xy, xz, yz
-    float sgeo[32][10];     // the batch's B^-1 (row-major) and |det B|, one row per element
-    float sF[15][36];       // Newton points: F_a^k at index 3 a + k (rows 16-byte aligned)
+    float sg[5][36];     // d phi_b / d x_c at 12 c + b
+    float ss[5][52];     // w eta d phi_a / d x_c at 12 c + a; rows l of w eta (du + du^T) at 36 + 4 l
+    float sF[15][68];    // F_a^k at 10 k + a, column factors at 32 + 10 l + b
+    float sgeo[32][10];  // the batch's B^-1 (row-major) and |det B|, one row per element
 };
+constexpr int kGNd = 34;  // words between the points' reference gradients d phi_a / d xi_j, at 10 j + a
 
-__global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__restrict__ geo,
+// two single-precision fused multiply-adds in one instruction, each rounded as fmaf
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+// N floats from 16-byte aligned shared memory as N / 2 pairs
+template <int N>
+__device__ __forceinline__ void load_pairs(const float *m, float2 *v) {
+#pragma unroll
+    for (int k = 0; k < N / 4; k++) {
+        const float4 x = reinterpret_cast<const float4 *>(m)[k];
+        v[2 * k] = make_float2(x.x, x.y);
+        v[2 * k + 1] = make_float2(x.z, x.w);
+    }
+    if (N % 4) v[N / 2 - 1] = reinterpret_cast<const float2 *>(m)[N / 2 - 1];
+}
+
+// Bound by the shared-memory pipe (the factors that all lanes read: 8 reads of 16
+// bytes per Newton point) and the instruction rate; us at 32^3 x 6 tets, Newton
+// form, Carreau-Yasuda: 660 with scalar arithmetic, node-wise records and batches
+// of 32; 611 with equal batches and packed updates of the Newton part; 509 packed
+// throughout, 479 with the column factors formed once per point instead of in
+// every lane, 443 with four CTAs per SM instead of six (no spills) and the next
+// element's velocities read ahead (three CTAs 465, five 454).
+constexpr int kGNCtas = 4;  // per SM
+__global__ void __launch_bounds__(32 * kGNWarps, kGNCtas) k_gn_elem(const float *__restrict__ geo,
                                                           const int32_t *__restrict__ conn, int64_t ne,
                                                           const double *__restrict__ u, ViscLaw L, int newton,
-                                                          float *stage, int *err, int64_t e_begin, int64_t e_end,
+                                                          float *stage, int *err, int64_t e_begin, int64_t e_end, int batch,
                                                           const __grid_constant__ GNTab rules) {
     __shared__ GNWarpSmem smem[kGNWarps];
     // the rule tables in shared memory: phase 1 reads a different point per
     // lane, which constant memory would serialise
-    __shared__ GNTab tab;
-    for (int t = threadIdx.x; t < (int)(sizeof(GNTab) / sizeof(float)); t += blockDim.x)
-        reinterpret_cast<float *>(&tab)[t] = reinterpret_cast<const float *>(&rules)[t];
+    __shared__ __align__(8) float tabd[20][kGNd];
+    __shared__ float tabw[20];
+    for (int t = threadIdx.x; t < 20 * 30; t += blockDim.x) {
+        const int q = t / 30, k = t - 30 * q, j = k / 10, a = k - 10 * j;
+        tabd[q][k] = q < 5 ? rules.d5[q][a][j] : rules.d15[q - 5][a][j];
+    }
+    if (threadIdx.x < 20) tabw[threadIdx.x] = threadIdx.x < 5 ? rules.w5[threadIdx.x] : rules.w15[threadIdx.x - 5];
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     GNWarpSmem &S = smem[w];
@@ -116,10 +155,10 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
     const bool cy2 = L.model == 0 && abs_int(L.prm[4] - 2.0f) < 2.220446049250313e-16f;
     const float e_eta = (L.prm[1] - 1.0f) / L.prm[4], e_dterm = (L.prm[1] - 1.0f - L.prm[4]) / L.prm[4];
     const float c0a = cy2 ? powf(L.prm[0], L.prm[4]) : 0.0f;
-    for (int64_t e0 = e_begin + ((int64_t)blockIdx.x * kGNWarps + w) * 32; e0 < e_end;
-         e0 += (int64_t)gridDim.x * kGNWarps * 32) {
-        // geometry of a batch of 32 elements, one element per lane
-        if (e0 + lane < e_end) {
+    const int64_t e0 = e_begin + ((int64_t)blockIdx.x * kGNWarps + w) * batch;
+    if (e0 < e_end) {
+        // geometry of the batch, one element per lane
+        if (lane < batch && e0 + lane < e_end) {
             float gB[9];
             const float gdet = fabsf(load_geometry(geo, ne, e0 + lane, gB));
             if (!(gdet > 0.0f) || !isfinite(gdet)) set_dev_error(err, kDevBadDet);
@@ -128,7 +167,12 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
             S.sgeo[lane][9] = gdet;
         }
         __syncwarp();
-        const int nb = (int)min((int64_t)32, e_end - e0);
+        const int nb = (int)min((int64_t)batch, e_end - e0);
+        const int b = lane < 30 ? lane / 3 : 0, l = lane < 30 ? lane - 3 * (lane / 3) : 0;
+        // lane 3 b + l's velocity of the next element, read ahead: its node
+        // before phase 1, the value before phase 2
+        int32_t node = conn[(int64_t)b * ne + e0];
+        double un = u[3 * (int64_t)node + l];
 #pragma unroll 1
         for (int t = 0; t < nb; t++) {
             const int64_t e = e0 + t;
@@ -136,24 +180,32 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
 #pragma unroll
             for (int k = 0; k < 9; k++) Bi[k] = S.sgeo[t][k];
             const float adet = S.sgeo[t][9];
-            const int b = lane < 30 ? lane / 3 : 0, l = lane < 30 ? lane - 3 * (lane / 3) : 0;
-            if (lane < 30) S.su[lane] = d2f_rn(u[3 * (int64_t)conn[(int64_t)b * ne + e] + l]);
+            if (lane < 30) S.su[lane] = d2f_rn(un);
+            if (t + 1 < nb) node = conn[(int64_t)b * ne + e + 1];
             __syncwarp();
             // phase 1: one lane per quadrature point (AssembleFEGeneralizedNewtonian_def.hpp:998-1083)
             const int nq = newton ? 20 : 5;
             if (lane < nq) {
                 const int q = lane < 5 ? lane : lane - 5;
-                const float(*d)[3] = lane < 5 ? tab.d5[q] : tab.d15[q];
-                float g[30], du[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+                float2 g[3][5];  // g[c][m]: nodes 2 m and 2 m + 1
+                float du[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-                for (int k = 0; k < 10; k++) {
+                for (int m = 0; m < 5; m++) {
+                    float2 d[3], u2[3];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) g[3 * k + c] = d[k][0] * Bi[c] + d[k][1] * Bi[3 + c] + d[k][2] * Bi[6 + c];
-                    *reinterpret_cast<float4 *>(&S.sg[lane][4 * k]) = make_float4(g[3 * k], g[3 * k + 1], g[3 * k + 2], 0.0f);
+                    for (int c = 0; c < 3; c++) {
+                        d[c] = *reinterpret_cast<const float2 *>(&tabd[lane][10 * c + 2 * m]);
+                        u2[c] = *reinterpret_cast<const float2 *>(&S.su[6 * m + 2 * c]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                        g[c][m] = fma2(d[2], both(Bi[6 + c]), fma2(d[0], both(Bi[c]), mul2(d[1], both(Bi[3 + c]))));
+                    const float ux[3] = {u2[0].x, u2[0].y, u2[1].x}, uy[3] = {u2[1].y, u2[2].x, u2[2].y};
 #pragma unroll
                     for (int a1 = 0; a1 < 3; a1++)
 #pragma unroll
-                        for (int c = 0; c < 3; c++) du[3 * a1 + c] = fmaf(S.su[3 * k + a1], g[3 * k + c], du[3 * a1 + c]);
+                        for (int c = 0; c < 3; c++)
+                            du[3 * a1 + c] = fmaf(uy[a1], g[c][m].y, fmaf(ux[a1], g[c][m].x, du[3 * a1 + c]));
                 }
                 const float s01 = du[1] + du[3], s02 = du[2] + du[6], s12 = du[5] + du[7];
                 const float gamma = sqrtf(2.0f * du[0] * du[0] + 2.0f * du[4] * du[4] + 2.0f * du[8] * du[8] + s01 * s01 +
@@ -171,90 +223,84 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
                     lawv = lane < 5 ? gn_eta(L, gamma) : gn_dterm(L, gamma);
                 }
                 if (lane < 5) {
-                    const float ew = lawv * tab.w5[q];
+                    const float ew = lawv * tabw[lane];
+                    float *R = S.ss[q];
 #pragma unroll
-                    for (int k = 0; k < 10; k++)
-                        *reinterpret_cast<float4 *>(&S.sgw[q][4 * k]) =
-                            make_float4(ew * g[3 * k], ew * g[3 * k + 1], ew * g[3 * k + 2], 0.0f);
-                    float *T = S.sT[q];
-                    T[0] = ew * (2.0f * du[0]);
-                    T[1] = ew * (2.0f * du[4]);
-                    T[2] = ew * (2.0f * du[8]);
-                    T[3] = ew * s01;
-                    T[4] = ew * s02;
-                    T[5] = ew * s12;
+                    for (int c = 0; c < 3; c++)
+#pragma unroll
+                        for (int m = 0; m < 5; m++) {
+                            *reinterpret_cast<float2 *>(&S.sg[q][12 * c + 2 * m]) = g[c][m];
+                            *reinterpret_cast<float2 *>(R + 12 * c + 2 * m) = mul2(both(ew), g[c][m]);
+                        }
+                    const float T3 = ew * s01, T4 = ew * s02, T5 = ew * s12;
+                    *reinterpret_cast<float4 *>(R + 36) = make_float4(ew * (2.0f * du[0]), T3, T4, 0.0f);
+                    *reinterpret_cast<float4 *>(R + 40) = make_float4(T3, ew * (2.0f * du[4]), T5, 0.0f);
+                    *reinterpret_cast<float4 *>(R + 44) = make_float4(T4, T5, ew * (2.0f * du[8]), 0.0f);
                 } else {
-                    S.sw[lane] = -2.0f * lawv * tab.w15[q];
+                    const float sw = -2.0f * lawv * tabw[lane];
                     const float xy = 0.5f * (du[1] + du[3]), xz = 0.5f * (du[6] + du[2]), yz = 0.5f * (du[7] + du[5]);
-                    float *m = S.sm[q];
-                    m[0] = du[0];
-                    m[1] = du[4];
-                    m[2] = du[8];
-                    m[3] = xy;
-                    m[4] = xz;
-                    m[5] = yz;
+                    float *R = S.sF[q];
+                    const float2 y00 = both(du[0]), y11 = both(du[4]), y22 = both(du[8]);
+                    const float2 y01 = both(xy), y02 = both(xz), y12 = both(yz), c2 = both(sw);
 #pragma unroll
-                    for (int k = 0; k < 10; k++) {
-                        const float g0 = g[3 * k], g1 = g[3 * k + 1], g2 = g[3 * k + 2];
-                        S.sF[q][3 * k] = g0 * du[0] + g1 * xy + g2 * xz;
-                        S.sF[q][3 * k + 1] = g0 * xy + g1 * du[4] + g2 * yz;
-                        S.sF[q][3 * k + 2] = g0 * xz + g1 * yz + g2 * du[8];
+                    for (int m = 0; m < 5; m++) {
+                        // F_a^k = g_a . (row k of the symmetric gradient); G_b^l the same, except that
+                        // for l = 2 the reference's factor takes g_b,3 in place of g_b,1 in the first
+                        // term (and the order of the sum for l = 0)
+                        const float2 x = g[0][m], y = g[1][m], z = g[2][m];
+                        const float2 F0 = fma2(z, y02, fma2(y, y01, mul2(x, y00)));
+                        const float2 F1 = fma2(z, y12, fma2(x, y01, mul2(y, y11)));
+                        const float2 F2 = fma2(z, y22, fma2(x, y02, mul2(y, y12)));
+                        const float2 G0 = fma2(z, y02, fma2(x, y00, mul2(y, y01)));
+                        const float2 G2 = fma2(z, y22, fma2(z, y02, mul2(y, y12)));
+                        float2 *P = reinterpret_cast<float2 *>(R + 2 * m);
+                        P[0] = F0;
+                        P[5] = F1;
+                        P[10] = F2;
+                        P[16] = mul2(c2, G0);
+                        P[21] = mul2(c2, F1);
+                        P[26] = mul2(c2, G2);
                     }
                 }
             }
             __syncwarp();
+            if (t + 1 < nb) un = u[3 * (int64_t)node + l];
             // phase 2: lane 3 b + l accumulates column (b, l) and residual row (b, l);
             // lanes 30 and 31 keep zeros for the rows' two padding columns
-            float acc[30];
+            float2 acc[15];  // 5 k + m: rows (a, k) of the nodes a = 2 m and 2 m + 1
 #pragma unroll
-            for (int p = 0; p < 30; p++) acc[p] = 0.0f;
+            for (int m = 0; m < 15; m++) acc[m] = make_float2(0.0f, 0.0f);
             float r = 0.0f;
             if (lane < 30) {
                 // stress: acc[(a, k)] += (w eta g_a).g_b d_kl + (w eta g_a,l) g_b,k
-                const float e0 = l == 0 ? 1.0f : 0.0f, e1 = l == 1 ? 1.0f : 0.0f, e2 = l == 2 ? 1.0f : 0.0f;
+                const float2 e0 = both(l == 0 ? 1.0f : 0.0f), e1 = both(l == 1 ? 1.0f : 0.0f), e2 = both(l == 2 ? 1.0f : 0.0f);
                 for (int q = 0; q < 5; q++) {
-                    const float4 gb = *reinterpret_cast<const float4 *>(&S.sg[q][4 * b]);
-                    const float4 *sw4 = reinterpret_cast<const float4 *>(S.sgw[q]);
+                    const float gx = S.sg[q][b], gy = S.sg[q][12 + b], gz = S.sg[q][24 + b];
+                    const float *R = S.ss[q];
+                    float2 sx[5], sy[5], sz[5];
+                    load_pairs<10>(R, sx);
+                    load_pairs<10>(R + 12, sy);
+                    load_pairs<10>(R + 24, sz);
 #pragma unroll
-                    for (int a = 0; a < 10; a++) {
-                        const float4 s = sw4[a];
-                        const float dot = s.x * gb.x + s.y * gb.y + s.z * gb.z;
-                        const float sal = l == 0 ? s.x : (l == 1 ? s.y : s.z);
-                        acc[3 * a] = fmaf(e0, dot, fmaf(sal, gb.x, acc[3 * a]));
-                        acc[3 * a + 1] = fmaf(e1, dot, fmaf(sal, gb.y, acc[3 * a + 1]));
-                        acc[3 * a + 2] = fmaf(e2, dot, fmaf(sal, gb.z, acc[3 * a + 2]));
+                    for (int m = 0; m < 5; m++) {
+                        const float2 dot = fma2(sz[m], both(gz), fma2(sx[m], both(gx), mul2(sy[m], both(gy))));
+                        const float2 sl = l == 0 ? sx[m] : (l == 1 ? sy[m] : sz[m]);
+                        acc[m] = fma2(e0, dot, fma2(sl, both(gx), acc[m]));
+                        acc[5 + m] = fma2(e1, dot, fma2(sl, both(gy), acc[5 + m]));
+                        acc[10 + m] = fma2(e2, dot, fma2(sl, both(gz), acc[10 + m]));
                     }
                     // residual row (b, l): g_b . w eta (du + du^T)[l][:]
-                    const float *T = S.sT[q];
-                    const float t0 = l == 0 ? T[0] : (l == 1 ? T[3] : T[4]);
-                    const float t1 = l == 0 ? T[3] : (l == 1 ? T[1] : T[5]);
-                    const float t2 = l == 0 ? T[4] : (l == 1 ? T[5] : T[2]);
-                    r = fmaf(gb.x, t0, fmaf(gb.y, t1, fmaf(gb.z, t2, r)));
+                    const float *T = R + 36 + 4 * l;
+                    r = fmaf(gx, T[0], fmaf(gy, T[1], fmaf(gz, T[2], r)));
                 }
                 if (newton) {
-                    // G_b^l = g_b . (column l of the symmetric gradient: entries
-                    // (0 3 4), (3 1 5), (4 5 2) of sm), except that for l = 2 the
-                    // reference's factor takes g_b,3 in place of g_b,1 in the
-                    // first term; per-lane indices instead of a branch on l
-                    const int ip = l == 0 ? 0x430 : (l == 1 ? 0x513 : 0x254);  // i0 | i1 << 4 | i2 << 8
                     for (int q = 0; q < 15; q++) {
-                        const float *m = S.sm[q];
-                        const float4 gbn = *reinterpret_cast<const float4 *>(&S.sg[5 + q][4 * b]);
-                        const float g0 = l == 2 ? gbn.z : gbn.x, g1 = gbn.y, g2 = gbn.z;
-                        const float G = g0 * m[ip & 15] + g1 * m[(ip >> 4) & 15] + g2 * m[ip >> 8];
-                        const float cg = S.sw[5 + q] * G;
-                        const float4 *F4 = reinterpret_cast<const float4 *>(S.sF[q]);
+                        const float *R = S.sF[q];
+                        const float2 cg = both(R[32 + 10 * l + b]);
+                        float2 f[15];
+                        load_pairs<30>(R, f);
 #pragma unroll
-                        for (int p4 = 0; p4 < 7; p4++) {
-                            const float4 f = F4[p4];
-                            acc[4 * p4] = fmaf(cg, f.x, acc[4 * p4]);
-                            acc[4 * p4 + 1] = fmaf(cg, f.y, acc[4 * p4 + 1]);
-                            acc[4 * p4 + 2] = fmaf(cg, f.z, acc[4 * p4 + 2]);
-                            acc[4 * p4 + 3] = fmaf(cg, f.w, acc[4 * p4 + 3]);
-                        }
-                        const float2 f2 = reinterpret_cast<const float2 *>(S.sF[q])[14];
-                        acc[28] = fmaf(cg, f2.x, acc[28]);
-                        acc[29] = fmaf(cg, f2.y, acc[29]);
+                        for (int m = 0; m < 15; m++) acc[m] = fma2(cg, f[m], acc[m]);
                     }
                 }
             }
@@ -263,7 +309,11 @@ __global__ void __launch_bounds__(32 * kGNWarps, 6) k_gn_elem(const float *__res
             // that L2 would read back from DRAM to merge)
             float *Se = stage + e * kGNStride;
 #pragma unroll
-            for (int p = 0; p < 30; p++) Se[32 * p + lane] = acc[p] * adet;
+            for (int m = 0; m < 15; m++) {
+                const float2 v = mul2(acc[m], both(adet));
+                Se[32 * (6 * (m % 5) + m / 5) + lane] = v.x;
+                Se[32 * (6 * (m % 5) + 3 + m / 5) + lane] = v.y;
+            }
             Se[kGNRes + lane] = r * adet;
             __syncwarp();  // the next element overwrites the scratch
         }
@@ -539,8 +589,16 @@ void launch_gn_elem(const double *xyz, const float *geo, const int32_t *conn, in
                     int64_t e_end, const GNOutflow &outflow) {
     if (e_end < 0) e_end = ne;
     if (e_end <= e_begin) return;
-    k_gn_elem<<<(unsigned)ceil_div(e_end - e_begin, 32 * kGNWarps), 32 * kGNWarps, 0, s>>>(
-        geo, conn, ne, u, law, newton, stage, d_err, e_begin, e_end, gn_rules());
+    // a warp's batch: at most 32 elements, in equal shares over as few rounds of
+    // the chip's warps as there have to be (21,600 elements in batches of 32 use
+    // a quarter of the warps: 151 us, 39 in equal shares)
+    int dev = 0, sms = 0;
+    FEDD_CUDA(cudaGetDevice(&dev));
+    FEDD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t count = e_end - e_begin, chip = (int64_t)sms * kGNCtas * kGNWarps;
+    const int batch = (int)ceil_div(count, ceil_div(count, 32 * chip) * chip);
+    k_gn_elem<<<ceil_div(count, (int64_t)batch * kGNWarps), 32 * kGNWarps, 0, s>>>(
+        geo, conn, ne, u, law, newton, stage, d_err, e_begin, e_end, batch, gn_rules());
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
     if (outflow.n > 0) {

@@ -53,3 +53,28 @@ def test_elements_of_every_batch(F, problem, M, n, field):
         b = F.Assembler(getattr(F, problem), xyz, np.ascontiguousarray(el[1:n // 2]), E=E, poisson_ratio=NU, **extra)
         Kb, rb = b.element_matrices(u=u)
         assert np.array_equal(Kb, K[1:n // 2]) and np.array_equal(rb, r[1:n // 2])
+
+
+@pytest.mark.parametrize("M,n,newton", [(1, 1, True), (1, 5, False), (8, 3071, True), (8, 3071, False)])
+def test_generalized_newtonian_elements_of_every_batch(F, M, n, newton):
+    """The viscous element stage works in batches that follow the mesh too."""
+    xyz2, el2 = F.structured_mesh(M, 2, seed=60 + M)
+    xyz1, el1 = F.structured_mesh(M, 1, seed=60 + M)
+    el2, el1 = np.ascontiguousarray(el2[:n]), np.ascontiguousarray(el1[:n])
+    u, p = 0.5 * F.fourier_field(xyz2, seed=60), F.uniform_field(60, xyz1.shape[0])
+    prm = [1.902, 0.22, 0.056, 0.00345, 1.25]
+    L = O.visc_law(0, prm, 1e-12)
+
+    def matrices(lo, hi):
+        a = F.Assembler(F.NAVIER_STOKES, xyz2, el2[lo:hi], elements_p=el1[lo:hi], num_nodes_p=xyz1.shape[0],
+                        viscosity=0.01, density=1.0, newton=newton)
+        a.set_viscosity_law(0, prm, gamma_min=1e-12)
+        return a.element_matrices(u=u, p=p)
+
+    K, r = matrices(0, n)
+    for e in sorted({0, 1, 2, 3, n // 2, n - 2, n - 1} & set(range(n))):
+        Jo, ro = O.elem_gn(xyz2[el2[e]], u.reshape(-1, 3)[el2[e]].ravel(), p[el1[e]], L, 1.0, newton)
+        assert rel(K[e], Jo) < 2e-6 and rel(r[e], ro) < 2e-6, e
+    if n > 2:
+        Kb, rb = matrices(1, n // 2)
+        assert np.array_equal(Kb, K[1:n // 2]) and np.array_equal(rb, r[1:n // 2])
