@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(64) k_lap_elem(const double *__restrict__ xyz,
     const double det = B[0] * C[0] + B[1] * C[1] + B[2] * C[2];
     if (det == 0.0) set_dev_error(err, kDevBadDet);
     const double ad = fabs(det);
+    const double fa = ad * f;
     double *S = stage + e * STRIDE;
     if (WANT_K) {
         double G[4][3], D[4][4];
@@ -73,11 +74,22 @@ __global__ void __launch_bounds__(64) k_lap_elem(const double *__restrict__ xyz,
         // P2: a fifth of D
         const double w = (NPE == 4 ? 1.0 : 0.2) / (6.0 * ad);
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
+        for (int a = NPE == 4 ? 1 : 0; a < 4; a++) {
             const double g0 = w * G[a][0], g1 = w * G[a][1], g2 = w * G[a][2];
 #pragma unroll
             for (int b = a; b < 4; b++) D[a][b] = D[b][a] = g0 * G[b][0] + g1 * G[b][1] + g2 * G[b][2];
         }
+        if (NPE == 4) {  // the gradients' sum is zero: the first row from the others
+#pragma unroll
+            for (int a = 1; a < 4; a++) D[0][a] = D[a][0] = -(D[a][1] + D[a][2] + D[a][3]);
+            D[0][0] = -(D[0][1] + D[0][2] + D[0][3]);
+        }
+        // values in pairs: the stores of a warp are not contiguous
+        double even = 0.0;
+        auto put = [&](int t, double v) {
+            if (t & 1) *reinterpret_cast<double2 *>(S + t - 1) = make_double2(even, v);
+            else even = v;
+        };
         int t = 0;
 #pragma unroll
         for (int a = 0; a < NPE; a++)
@@ -99,10 +111,13 @@ __global__ void __launch_bounds__(64) k_lap_elem(const double *__restrict__ xyz,
                     s += (i == l ? 2.0 : 1.0) * D[j][k] + (j == k ? 2.0 : 1.0) * D[i][l];
                     v = 4.0 * s;
                 }
-                S[t] = v;
+                put(t, v);
             }
+#pragma unroll
+        for (int a = 0; a < NPE; a++) put(NK + a, fa * mfac[a]);
+        if ((NK + NPE) & 1) S[NK + NPE - 1] = even;
+        return;
     }
-    const double fa = ad * f;
 #pragma unroll
     for (int a = 0; a < NPE; a++) S[NK + a] = fa * mfac[a];
 }
