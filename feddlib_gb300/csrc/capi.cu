@@ -27,7 +27,6 @@ struct fedd_assembler {
     DBuf<float> geo;        // B^-1 and det B of every element (launch_geometry)
     Graph g, gp;
     DBuf<int32_t> vmap;     // Taylor-Hood: P2 vertex -> P1 node (-1 for edge nodes)
-    DBuf<unsigned long long> work;  // the velocity-row kernel's position counter (device path)
     bool ns_fused = false;  // vmap verified: pressure rows come from the velocity-row kernel
     DBuf<int64_t> padj_ptr;
     DBuf<int4> ninfo;       // per velocity node: first incidence, vertex P1 node, counts (k_ns_vel_rows)
@@ -62,7 +61,10 @@ struct fedd_assembler {
     cudaEvent_t chunk_ev[kChunks + 2] = {};
     bool chunks_ready = false;
     int64_t cut[kChunks + 1] = {}, off00[kChunks + 1] = {}, off01[kChunks + 1] = {}, ecut[kChunks + 1] = {};
+    // the error word, and at d_err.p + 2 the velocity-row kernel's position
+    // counter (device path): one memset clears both
     DBuf<int> d_err;
+    unsigned long long *work() { return reinterpret_cast<unsigned long long *>(d_err.p + 2); }
     // generalized-Newtonian viscosity law (fedd_set_viscosity_law)
     bool gn_on = false;
     ViscLaw gn{};
@@ -197,7 +199,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
          double *v10, double *ru, double *rp, cudaStream_t s) {
     LaunchCounter lc;
     const bool jac = what & FEDD_JACOBIAN, res = what & FEDD_RESIDUAL;
-    FEDD_CUDA(cudaMemsetAsync(h->d_err.p, 0, sizeof(int), s));
+    FEDD_CUDA(cudaMemsetAsync(h->d_err.p, 0, 4 * sizeof(int), s));
     switch (h->prm.problem) {
     case FEDD_LAPLACE:
         stage(h, "lap_elem", s, [&] {
@@ -283,7 +285,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
             launch_ns_vel_rows(h->g, h->ninfo.p, h->stage_f.p, h->ns_tab.p, h->csr[0].rowptr.p, h->csr[1].rowptr.p,
                                v00, v01, res ? ru : nullptr, dn, h->prm.linearization, h->g.max_adj,
                                h->max_padj, h->ns_fused, h->csr[2].rowptr.p, v10,
-                               res ? rp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, 0, -1, h->work.p,
+                               res ? rp : nullptr, h->gn_on ? h->stage_gn.p : nullptr, s, lc, 0, -1, h->work(),
                                h->coeff);
         });
         if (!h->ns_fused)
@@ -374,7 +376,7 @@ fedd_status fedd_create(const fedd_mesh *mesh, const fedd_params *params, int de
                 total += Arena::bytes<T>((size_t)count);
         };
         auto lay_out = [&] {
-            put(h->d_err, 1);
+            put(h->d_err, 4);
             put(h->xyz, nn * 3);
             put(h->conn, n_inc);
             put(h->g.inc_ptr, nn + 1);
@@ -401,7 +403,6 @@ fedd_status fedd_create(const fedd_mesh *mesh, const fedd_params *params, int de
                 put(h->csr[3].rowptr, nn1 + 1);
                 put(h->vmap, nn);
                 put(h->ninfo, nn);
-                put(h->work, 1);
                 put(h->ns_tab, kNSTab);
             } else if (prob == FEDD_ANISO_FIBER) {
                 put(h->qp_inv, ne * nq * 4);

@@ -1149,10 +1149,11 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
     const int most = vel_warps(gn, npw);
     int warps = (int)std::min<size_t>(most, (113 * 1024 - tables) / per_warp);
     if (warps < 4) warps = (int)std::max<size_t>(1, std::min<size_t>(most, (227 * 1024 - tables) / per_warp));
-    // pairs come from groups of eight nodes, of four below 64 nodes per warp,
-    // where the last groups would leave warps idle (50,653 nodes 92 us against
-    // 107, 185,193 nodes 304 against 300, 912,673 nodes 1,319 against 1,299)
-    const int group = npw == 1 ? 1 : count < 64 * 2 * sms * warps ? 4 : 8;
+    // pairs come from groups of eight nodes, of four below 40 nodes per warp,
+    // where the last groups would leave warps idle (Newton form, lattice and
+    // shuffled: 50,653 nodes 92 and 92 us against 107 and 119; 91,125 nodes 150
+    // and 157 against 161 and 155; 185,193 nodes 281 and 303 against 291 and 298)
+    const int group = npw == 1 ? 1 : count < 40 * 2 * sms * warps ? 4 : 8;
     if (npw == 1 && count <= 2 * sms * warps) {
         work = nullptr;  // a node per warp at most, spread over all SMs
         warps = (int)std::min<int64_t>(warps, std::max<int64_t>(2, ceil_div(count, 2 * sms)));
@@ -1170,7 +1171,6 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
         int per_sm = 0;
         FEDD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
         grid = (unsigned)std::min<int64_t>(grid, sms * std::max(per_sm, 1));
-        FEDD_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), s));
     }
     if (grid == 0) return;
     kern<<<grid, 32 * warps, smem, s>>>(ninfo, g.inc.p, g.slots.p, rec, d_tables, rowptr00, rowptr01, vals00, vals01,

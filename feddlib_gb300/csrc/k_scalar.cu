@@ -20,7 +20,10 @@
 // active lanes, so what counts is FP64 warp instructions: the element kernel
 // forms its entries in few of them, and the row kernel adds an incidence's
 // entries and load for several nodes at once (a warp's 32 lanes hold six P1 or
-// two P2 nodes).
+// two P2 nodes).  Element and row kernel, us, before (one warp per node, P2 by
+// the reference gradients' integrals) and after: 16^3 x 6 tets P1 10.3 + 19.9
+// and 7.4 + 9.5, P2 35.6 + 45.2 and 15.8 + 19.0; 40^3 x 6 P2 281 + 559 and
+// 168 + 185 (252 with the element's values stored one by one).
 #include "kernels.cuh"
 
 namespace fedd {

@@ -134,7 +134,8 @@ void launch_ns_node_info(const Graph &g, const int64_t *padj_ptr, const int32_t 
 struct NSCoeff {
     double uu = 1.0, up = 1.0, pu = 1.0;
 };
-// vmap: ninfo holds a verified vertex map (block (1,0) and res_p come along)
+// vmap: ninfo holds a verified vertex map (block (1,0) and res_p come along);
+// work: a counter that is zero when the kernel starts, or null
 void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, const float *d_tables,
                         const int64_t *rowptr00, const int64_t *rowptr01, double *vals00, double *vals01, double *res_u,
                         float dens, int newton, int max_adj, int max_padj, bool vmap, const int64_t *rowptr10,
