@@ -565,72 +565,88 @@ __global__ void k_tr_l1b(TrainParams P, int H, const float *__restrict__ X, cons
 // three 64 x 64 products: Z2 = X1 W2^T, DX1 = D W2 and gW2 = D^T X1.  As
 // separate kernels they moved the five-channel matrices X1, Z2, D and DX1
 // through memory nine times (84 MB each at a batch of 65,536), and the last
-// one ran on 80 of the blocks the chip holds.  Here a CTA takes tiles of 16
-// samples and keeps them in shared memory: thread (s, c) of the 256 owns
-// hidden units 4 c .. 4 c + 3 of sample s in all five channels, so the layer
-// formulas between the products run on registers, and a 4 x 4 block of gW2,
-// which stays in registers over all tiles of the CTA, as do the thread's sums
-// of the other gradients.  Each CTA writes one partial sum of every gradient;
-// k_tr_update adds them in a fixed order and takes the Adam step.  FP32
-// throughout; bound by the FP32 pipe (3 x 20,480 multiply-adds per sample) and
-// shared-memory reads: 213 us for a batch of 65,536 (38 TFLOP/s) and 8 us for
-// k_tr_update, against 1,590 us of separate kernels.
-constexpr int kTS = 16;                  // samples per tile
-constexpr int kTThreads = 256;
+// one ran on 80 of the blocks the chip holds.  Here a CTA takes tiles of
+// GROUPS x SPT samples and keeps them in shared memory: thread (s, c) owns
+// hidden units 4 c .. 4 c + 3 of the samples s, s + GROUPS in all five
+// channels, so the layer formulas between the products run on registers, and a
+// block of gW2, which stays in registers over all tiles of the CTA, as do the
+// thread's sums of the other gradients.  Each CTA writes one partial sum of
+// every gradient; k_tr_update adds them in a fixed order and takes the Adam
+// step.  FP32 throughout, two multiply-adds to an instruction in the products
+// (3 x 20,480 per sample).  A 16-byte read that serves one sample's row and
+// four weights is four of the shared-memory pipe's cycles to 20 multiply-adds:
+// with one sample per thread that pipe is the bound (78 %), with two the FP32
+// pipe.  For a batch of 65,536: 1,590 us of separate kernels; 213 us one
+// sample per thread with scalar multiply-adds; 203 packed; 184 two samples and
+// 384 threads (205 with 256: two warps per scheduler are too few); k_tr_update
+// another 8 us.
+constexpr int kTRows = 16;               // samples of a tile that one share of gW2 adds
 constexpr int kTSample = 5 * kH + 4;     // floats per sample: five channels, and 4 so that two samples' rows differ in banks
 constexpr int kTPar = 4 * kH + kH + kH * kH + kH + kH + 2;  // gradients in the parameters' order, then the loss
-constexpr size_t kTSmem = (size_t)(2 * kH * kH + 2 * kTS * kTSample + 4 * kH + 3 * kH) * sizeof(float);
+constexpr size_t tr_smem(int groups, int spt) {
+    return (size_t)(2 * kH * kH + 2 * groups * spt * kTSample + 4 * kH + 3 * kH) * sizeof(float);
+}
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, const float *v) {
     *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
-// acc[c] += x w for the four columns of w
+// acc[c] += x w for the four columns of w, two to an instruction
 __device__ __forceinline__ void fma4(float *acc, float x, const float4 &w) {
-    acc[0] = fmaf(x, w.x, acc[0]);
-    acc[1] = fmaf(x, w.y, acc[1]);
-    acc[2] = fmaf(x, w.z, acc[2]);
-    acc[3] = fmaf(x, w.w, acc[3]);
+    asm("{.reg .b64 x, w, a;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 w, {%3, %4};\n\tmov.b64 a, {%0, %1};\n\t"
+        "fma.rn.f32x2 a, x, w, a;\n\tmov.b64 {%0, %1}, a;}"
+        : "+f"(acc[0]), "+f"(acc[1])
+        : "f"(x), "f"(w.x), "f"(w.y));
+    asm("{.reg .b64 x, w, a;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 w, {%3, %4};\n\tmov.b64 a, {%0, %1};\n\t"
+        "fma.rn.f32x2 a, x, w, a;\n\tmov.b64 {%0, %1}, a;}"
+        : "+f"(acc[2]), "+f"(acc[3])
+        : "f"(x), "f"(w.z), "f"(w.w));
 }
-// acc[ch][c] = sum_i rows[ch][i] W[i][u0 + c] over 64 i
-__device__ __forceinline__ void tile_product(float acc[5][4], const float *rows, const float *W, int u0) {
+// acc[m][ch][c] = sum_i rows[m][ch][i] W[i][u0 + c] over 64 i, samples `apart` floats apart
+template <int SPT>
+__device__ __forceinline__ void tile_product(float acc[SPT][5][4], const float *rows, int apart, const float *W, int u0) {
 #pragma unroll
-    for (int ch = 0; ch < 5; ch++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[ch][c] = 0.0f;
+    for (int k = 0; k < SPT * 20; k++) (&acc[0][0][0])[k] = 0.0f;
 #pragma unroll 2
     for (int i = 0; i < kH; i += 4) {
-        float4 x[5];
-#pragma unroll
-        for (int ch = 0; ch < 5; ch++) x[ch] = ld4(rows + kH * ch + i);
         const float4 w0 = ld4(W + i * kH + u0), w1 = ld4(W + (i + 1) * kH + u0), w2 = ld4(W + (i + 2) * kH + u0),
                      w3 = ld4(W + (i + 3) * kH + u0);
 #pragma unroll
-        for (int ch = 0; ch < 5; ch++) {
-            fma4(acc[ch], x[ch].x, w0);
-            fma4(acc[ch], x[ch].y, w1);
-            fma4(acc[ch], x[ch].z, w2);
-            fma4(acc[ch], x[ch].w, w3);
+        for (int m = 0; m < SPT; m++) {
+            float4 x[5];
+#pragma unroll
+            for (int ch = 0; ch < 5; ch++) x[ch] = ld4(rows + m * apart + kH * ch + i);
+#pragma unroll
+            for (int ch = 0; ch < 5; ch++) {
+                fma4(acc[m][ch], x[ch].x, w0);
+                fma4(acc[m][ch], x[ch].y, w1);
+                fma4(acc[m][ch], x[ch].z, w2);
+                fma4(acc[m][ch], x[ch].w, w3);
+            }
         }
     }
 }
 
-// samples idx[0..B) (null: 0..B) in tiles; part: gridDim.x x kTPar
-__global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const float *__restrict__ X,
-                                                          const float *__restrict__ ty, const float *__restrict__ tgr,
-                                                          const int64_t *__restrict__ idx, int64_t B, float wpsi,
-                                                          float wgrad, float *__restrict__ part) {
+// samples idx[0..B) (null: 0..B) in tiles of GROUPS SPT; part: gridDim.x x kTPar
+template <int GROUPS, int SPT>
+__global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
+    k_tr_fused(TrainParams P, const float *__restrict__ X, const float *__restrict__ ty, const float *__restrict__ tgr,
+               const int64_t *__restrict__ idx, int64_t B, float wpsi, float wgrad, float *__restrict__ part) {
+    constexpr int TS = GROUPS * SPT, THREADS = 16 * GROUPS;
+    // rows of the thread's gW2 block; SHARES threads own one, each adding kTRows samples of a tile
+    constexpr int JB = 4 * SPT, SHARES = TS / kTRows;
     extern __shared__ __align__(16) float sm[];
     float *sW = sm, *sWT = sW + kH * kH;               // W2[j][i] and W2[j][i] at [i][j]
-    float *sX = sWT + kH * kH, *sD = sX + kTS * kTSample;
-    float *sW1 = sD + kTS * kTSample, *sb1 = sW1 + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
-    const int tid = threadIdx.x, s = tid >> 4, u0 = 4 * (tid & 15), j0 = 4 * (tid >> 4);
-    for (int t = tid; t < kH * kH; t += kTThreads) {
+    float *sX = sWT + kH * kH, *sD = sX + TS * kTSample;
+    float *sW1 = sD + TS * kTSample, *sb1 = sW1 + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
+    const int tid = threadIdx.x, s = tid >> 4, u0 = 4 * (tid & 15);
+    const int share = s / (kH / JB), j0 = JB * (s % (kH / JB));
+    for (int t = tid; t < kH * kH; t += THREADS) {
         const float w = P.W2[t];
         sW[t] = w;
         sWT[(t & (kH - 1)) * kH + (t >> 6)] = w;
     }
-    sW1[tid] = P.W1[tid];  // 4 kH = 256 values
+    if (tid < 4 * kH) sW1[tid] = P.W1[tid];
     if (tid < kH) {
         sb1[tid] = P.b1[tid];
         sb2[tid] = P.b2[tid];
@@ -639,36 +655,45 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const 
     const float b3 = *P.b3;
     __syncthreads();
     float *xrow = sX + s * kTSample, *drow = sD + s * kTSample;
-    float gW2[4][4], gW1[4][4], gb1[4], gb2[4], gw3[4], gb3 = 0.0f, loss = 0.0f;
+    float gW2[JB][4], gW1[4][4], gb1[4], gb2[4], gw3[4], gb3 = 0.0f, loss = 0.0f;
 #pragma unroll
     for (int a = 0; a < 4; a++) {
         gb1[a] = gb2[a] = gw3[a] = 0.0f;
 #pragma unroll
-        for (int b = 0; b < 4; b++) gW2[a][b] = gW1[a][b] = 0.0f;
+        for (int b = 0; b < 4; b++) gW1[a][b] = 0.0f;
     }
-    const int64_t ntiles = (B + kTS - 1) / kTS;
-    auto sample = [&](int64_t tile) {
-        const int64_t q = tile * kTS + s;
+#pragma unroll
+    for (int k = 0; k < 4 * JB; k++) (&gW2[0][0])[k] = 0.0f;
+    const int64_t ntiles = (B + TS - 1) / TS;
+    auto sample = [&](int64_t tile, int m) {
+        const int64_t q = tile * TS + m * GROUPS + s;
         return q < B ? (idx ? idx[q] : q) : (int64_t)-1;
     };
-    int64_t id = blockIdx.x < ntiles ? sample(blockIdx.x) : -1;
+    int64_t id[SPT];
+#pragma unroll
+    for (int m = 0; m < SPT; m++) id[m] = blockIdx.x < ntiles ? sample(blockIdx.x, m) : -1;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const bool valid = id >= 0;
-        const int64_t si = valid ? id : 0;
-        const float4 x4 = ld4(X + 4 * si), t4 = ld4(tgr + 4 * si);
-        const float tyv = ty[si];
-        if (tile + gridDim.x < ntiles) id = sample(tile + gridDim.x);
-        const float x[4] = {x4.x, x4.y, x4.z, x4.w}, tg[4] = {t4.x, t4.y, t4.z, t4.w};
-        float s1[4], t1[4];
-        {  // layer 1
+        bool valid[SPT];
+        float x[SPT][4], tg[SPT][4], tyv[SPT], s1[SPT][4];
+#pragma unroll
+        for (int m = 0; m < SPT; m++) {
+            valid[m] = id[m] >= 0;
+            const int64_t si = valid[m] ? id[m] : 0;
+            const float4 x4 = ld4(X + 4 * si), t4 = ld4(tgr + 4 * si);
+            x[m][0] = x4.x; x[m][1] = x4.y; x[m][2] = x4.z; x[m][3] = x4.w;
+            tg[m][0] = t4.x; tg[m][1] = t4.y; tg[m][2] = t4.z; tg[m][3] = t4.w;
+            tyv[m] = ty[si];
+            if (tile + gridDim.x < ntiles) id[m] = sample(tile + gridDim.x, m);
+        }
+#pragma unroll
+        for (int m = 0; m < SPT; m++) {  // layer 1
             float v[5][4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const float4 w = ld4(sW1 + 4 * (u0 + u));
-                const float z = fmaf(w.w, x[3], fmaf(w.z, x[2], fmaf(w.y, x[1], fmaf(w.x, x[0], sb1[u0 + u]))));
+                const float z = fmaf(w.w, x[m][3], fmaf(w.z, x[m][2], fmaf(w.y, x[m][1], fmaf(w.x, x[m][0], sb1[u0 + u]))));
                 const float sg = 1.0f / (1.0f + expf(-z));
-                s1[u] = sg;
-                t1[u] = sg * (1.0f - sg);
+                s1[m][u] = sg;
                 v[0][u] = z > 20.0f ? z : log1pf(expf(z));
                 v[1][u] = sg * w.x;
                 v[2][u] = sg * w.y;
@@ -676,39 +701,40 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const 
                 v[4][u] = sg * w.w;
             }
 #pragma unroll
-            for (int ch = 0; ch < 5; ch++) st4(xrow + kH * ch + u0, v[ch]);
+            for (int ch = 0; ch < 5; ch++) st4(xrow + m * GROUPS * kTSample + kH * ch + u0, v[ch]);
         }
         __syncwarp();  // a sample's rows are written and read by the same half warp
-        float acc[5][4];
-        tile_product(acc, xrow, sWT, u0);
-        // layer 2, the sample's output, gradient and loss, and the backward rows D
-        float sg[4], hv[4], yp = 0.0f, gp[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float acc[SPT][5][4];
+        tile_product<SPT>(acc, xrow, GROUPS * kTSample, sWT, u0);
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const float z = acc[0][u] + sb2[u0 + u], w3 = sw3[u0 + u];
-            sg[u] = 1.0f / (1.0f + expf(-z));
-            hv[u] = z > 20.0f ? z : log1pf(expf(z));
-            yp = fmaf(w3, hv[u], yp);
+        for (int m = 0; m < SPT; m++) {
+            // layer 2, the sample's output, gradient and loss, and the backward rows D
+            float sg[4], hv[4], yp = 0.0f, gp[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int k = 0; k < 4; k++) gp[k] = fmaf(w3 * sg[u], acc[1 + k][u], gp[k]);
-        }
+            for (int u = 0; u < 4; u++) {
+                const float z = acc[m][0][u] + sb2[u0 + u], w3 = sw3[u0 + u];
+                sg[u] = 1.0f / (1.0f + expf(-z));
+                hv[u] = z > 20.0f ? z : log1pf(expf(z));
+                yp = fmaf(w3, hv[u], yp);
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            yp += __shfl_xor_sync(0xffffffffu, yp, o);
+                for (int k = 0; k < 4; k++) gp[k] = fmaf(w3 * sg[u], acc[m][1 + k][u], gp[k]);
+            }
 #pragma unroll
-            for (int k = 0; k < 4; k++) gp[k] += __shfl_xor_sync(0xffffffffu, gp[k], o);
-        }
-        const float dy = yp + b3 - tyv, ey = valid ? 2.0f * wpsi * dy : 0.0f;
-        float eg[4], l = wpsi * dy * dy;
+            for (int o = 8; o > 0; o >>= 1) {
+                yp += __shfl_xor_sync(0xffffffffu, yp, o);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float dk = gp[k] - tg[k];
-            eg[k] = valid ? 2.0f * wgrad * dk : 0.0f;
-            l += wgrad * dk * dk;
-        }
-        gb3 += ey;
-        loss += valid ? l : 0.0f;
-        {
+                for (int k = 0; k < 4; k++) gp[k] += __shfl_xor_sync(0xffffffffu, gp[k], o);
+            }
+            const float dy = yp + b3 - tyv[m], ey = valid[m] ? 2.0f * wpsi * dy : 0.0f;
+            float eg[4], l = wpsi * dy * dy;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float dk = gp[k] - tg[m][k];
+                eg[k] = valid[m] ? 2.0f * wgrad * dk : 0.0f;
+                l += wgrad * dk * dk;
+            }
+            gb3 += ey;
+            loss += valid[m] ? l : 0.0f;
             float d[5][4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -716,8 +742,8 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const 
                 float dz2 = ey * w3 * sg[u], gw = ey * hv[u];
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    dz2 = fmaf(eg[k] * w3 * tg2, acc[1 + k][u], dz2);
-                    gw = fmaf(eg[k] * sg[u], acc[1 + k][u], gw);
+                    dz2 = fmaf(eg[k] * w3 * tg2, acc[m][1 + k][u], dz2);
+                    gw = fmaf(eg[k] * sg[u], acc[m][1 + k][u], gw);
                     d[1 + k][u] = eg[k] * w3 * sg[u];
                 }
                 d[0][u] = dz2;
@@ -725,45 +751,55 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const 
                 gw3[u] += gw;
             }
 #pragma unroll
-            for (int ch = 0; ch < 5; ch++) st4(drow + kH * ch + u0, d[ch]);
+            for (int ch = 0; ch < 5; ch++) st4(drow + m * GROUPS * kTSample + kH * ch + u0, d[ch]);
         }
         __syncthreads();
-        // gW2 block of the tile's 80 rows
+        // gW2 block of the share's samples, five rows each
+        const float *gD = sD + share * kTRows * kTSample + j0, *gX = sX + share * kTRows * kTSample + u0;
 #pragma unroll 2
-        for (int q = 0; q < kTS; q++)
+        for (int q = 0; q < kTRows; q++)
 #pragma unroll
             for (int ch = 0; ch < 5; ch++) {
-                const float4 d = ld4(sD + q * kTSample + kH * ch + j0), v = ld4(sX + q * kTSample + kH * ch + u0);
-                fma4(gW2[0], d.x, v);
-                fma4(gW2[1], d.y, v);
-                fma4(gW2[2], d.z, v);
-                fma4(gW2[3], d.w, v);
+                const float4 v = ld4(gX + q * kTSample + kH * ch);
+#pragma unroll
+                for (int a = 0; a < JB; a += 4) {
+                    const float4 d = ld4(gD + q * kTSample + kH * ch + a);
+                    fma4(gW2[a], d.x, v);
+                    fma4(gW2[a + 1], d.y, v);
+                    fma4(gW2[a + 2], d.z, v);
+                    fma4(gW2[a + 3], d.w, v);
+                }
             }
         // backward through layer 2's product and layer 1
-        tile_product(acc, drow, sW, u0);
+        tile_product<SPT>(acc, drow, GROUPS * kTSample, sW, u0);
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const float4 w = ld4(sW1 + 4 * (u0 + u));
             const float wk[4] = {w.x, w.y, w.z, w.w};
-            float dz = acc[0][u] * s1[u];
 #pragma unroll
-            for (int k = 0; k < 4; k++) dz = fmaf(acc[1 + k][u] * t1[u], wk[k], dz);
+            for (int m = 0; m < SPT; m++) {
+                const float sg = s1[m][u], t1 = sg * (1.0f - sg);
+                float dz = acc[m][0][u] * sg;
 #pragma unroll
-            for (int k = 0; k < 4; k++) gW1[u][k] += fmaf(dz, x[k], acc[1 + k][u] * s1[u]);
-            gb1[u] += dz;
+                for (int k = 0; k < 4; k++) dz = fmaf(acc[m][1 + k][u] * t1, wk[k], dz);
+#pragma unroll
+                for (int k = 0; k < 4; k++) gW1[u][k] += fmaf(dz, x[m][k], acc[m][1 + k][u] * sg);
+                gb1[u] += dz;
+            }
         }
         __syncthreads();  // the next tile overwrites the rows
     }
-    // the CTA's partial sums: gW2 by its owners, the others summed over the 16
-    // sample groups through shared memory
+    // the CTA's partial sums: the shares of gW2, and the others over the
+    // sample groups, through shared memory
     float *out = part + (int64_t)blockIdx.x * kTPar;
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) out[5 * kH + (j0 + a) * kH + u0 + b] = gW2[a][b];
     constexpr int kSmall = 7 * kH;  // gW1 (4 per unit), gb1, gb2, gw3
-    float *red = sX;                // 16 x 448 floats in the rows' place
-    static_assert(kTS * kSmall + 2 * kTS <= 2 * kTS * kTSample, "the partial sums fit the rows");
+    float *red = sX;                // GROUPS x 448 floats in the rows' place, and behind them the other shares of gW2
+    float *red2 = red + GROUPS * kSmall + 2 * GROUPS;
+    static_assert(GROUPS * kSmall + 2 * GROUPS + (SHARES - 1) * kH * kH <= 2 * TS * kTSample, "the partial sums fit the rows");
+    if (share > 0) {
+#pragma unroll
+        for (int a = 0; a < JB; a++) st4(red2 + (share - 1) * kH * kH + (j0 + a) * kH + u0, gW2[a]);
+    }
 #pragma unroll
     for (int u = 0; u < 4; u++) {
 #pragma unroll
@@ -773,13 +809,26 @@ __global__ void __launch_bounds__(kTThreads, 2) k_tr_fused(TrainParams P, const 
         red[s * kSmall + 6 * kH + u0 + u] = gw3[u];
     }
     if (u0 == 0) {
-        red[kTS * kSmall + s] = gb3;
-        red[kTS * kSmall + kTS + s] = loss;
+        red[GROUPS * kSmall + s] = gb3;
+        red[GROUPS * kSmall + GROUPS + s] = loss;
     }
     __syncthreads();
-    for (int t = tid; t < kSmall + 2; t += kTThreads) {
+    if (share == 0) {
+#pragma unroll
+        for (int a = 0; a < JB; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int k = (j0 + a) * kH + u0 + b;
+                float v = gW2[a][b];
+#pragma unroll
+                for (int c = 1; c < SHARES; c++) v += red2[(c - 1) * kH * kH + k];
+                out[5 * kH + k] = v;
+            }
+    }
+    for (int t = tid; t < kSmall + 2; t += THREADS) {
         float v = 0.0f;
-        for (int q = 0; q < kTS; q++) v += t < kSmall ? red[q * kSmall + t] : red[kTS * kSmall + kTS * (t - kSmall) + q];
+        for (int q = 0; q < GROUPS; q++)
+            v += t < kSmall ? red[q * kSmall + t] : red[GROUPS * kSmall + GROUPS * (t - kSmall) + q];
         // gW1 | gb1 at the front, gb2 | gw3 | gb3 | loss behind gW2
         out[t < 5 * kH ? t : t + kH * kH] = v;
     }
@@ -1001,11 +1050,18 @@ struct AdamStep {
 };
 void tr_fused(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float wgrad, const AdamStep *adam) {
     cudaStream_t s = 0;
-    // two CTAs per SM (registers)
-    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(B, kTS), (int64_t)sms() * 2);
+    // tiles of 48 samples, one CTA per SM, or of 16, two per SM: whichever takes
+    // less time over its rounds of tiles (20.4 and 14.6 us a round; a step of
+    // 65,536 samples 203 against 226 us, 20,000 77 and 84, 15,000 76 and 69, 30,000 118 and 114)
+    const int64_t rounds1 = ceil_div(B, 32 * (int64_t)sms()), rounds2 = ceil_div(B, 48 * (int64_t)sms());
+    const int spt = 7 * rounds2 < 5 * rounds1 ? 2 : 1;
+    const int groups = spt == 2 ? 24 : 16;
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(B, groups * spt), (int64_t)sms() * (2 / spt));
+    const size_t smem = tr_smem(groups, spt);
     if (t->partials.n < (size_t)grid * kTPar) t->partials.alloc((size_t)grid * kTPar);
-    FEDD_CUDA(cudaFuncSetAttribute(k_tr_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem));
-    k_tr_fused<<<grid, kTThreads, kTSmem, s>>>(t->tp(), t->X.p, t->ty.p, t->tg.p, idx, B, wpsi, wgrad, t->partials.p);
+    auto kern = spt == 2 ? k_tr_fused<24, 2> : k_tr_fused<16, 1>;
+    FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, 16 * groups, smem, s>>>(t->tp(), t->X.p, t->ty.p, t->tg.p, idx, B, wpsi, wgrad, t->partials.p);
     const AdamStep a = adam ? *adam : AdamStep{};
     k_tr_update<<<ceil_div(kTPar, 32), 256, 0, s>>>(t->partials.p, (int)grid, adam != nullptr, t->grad.p, t->lsum.p,
                                                     t->par.p, t->m1.p, t->m2.p, a.lr, a.b1, a.b2, a.eps, a.c1, a.c2,

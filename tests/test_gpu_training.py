@@ -47,6 +47,12 @@ def test_fused_gradients(F, n):
     assert abs(g["b3"] - go["b3"]) <= 1e-4 * max(1.0, abs(go["b3"]))
 
 
+# one tile of 48 samples per SM instead of two rounds of 16: from 4,865 samples on 152 SMs
+@pytest.mark.parametrize("n", [4865, 4895, 4896, 4897, 7296, 7297, 9740])
+def test_fused_gradients_two_samples_per_thread(F, n):
+    test_fused_gradients(F, n)
+
+
 def shuffle(perm, seed, step):
     mask = (1 << 64) - 1
     s = (seed ^ (0x5851F42D4C957F2D * (step + 1))) & mask
