@@ -131,9 +131,9 @@ __device__ __forceinline__ void cof3(const float *F, float *C) {
 // then for each pair of elements:
 //   phase Q  lane (element, q < nq): F_q, cof F_q and the law's derivatives at
 //            F_q, folded with the weight w_q det B into the scalars below;
-//   phase V  one lane per (element, point q, node a): G = B^-T grad phi_a(q),
-//            c = cof(F_q) G, f = F_q G, the fibre projections a_f . G and
-//            node a's residual contribution at q;
+//   phase V  a lane per (element, point q) and every few pairs of nodes a:
+//            G = B^-T grad phi_a(q), c = cof(F_q) G, f = F_q G, the fibre
+//            projections a_f . G and the nodes' residual contributions at q;
 //   phase K  a half warp per element, one lane per 2 x 2 tile of node pairs
 //            (2 A + x, 2 B + y), A <= B (15 tiles), so a record read from
 //            shared memory serves two blocks; each 3 x 3 block sums over q in
@@ -150,23 +150,20 @@ constexpr int kQS = 52;    // floats per quadrature-point record: 13 chunks of 1
 // (phi1 phi2 chi1 chi2) 24, F a1 28, F a2 32, s psi_kl 36-45, residual
 // scalars (-2 s psi_1, -s psi_J, -2 s psi_4a, -2 s psi_4b) 48
 constexpr int kQScal = 20, kQFib = 24, kQFa1 = 28, kQFa2 = 32, kQHess = 36, kQRes = 48;
-// node records of a point: planes of the ten nodes' 16-byte chunks
-// c0 c1 c2 G0 | G1 G2 (g1 g2 with fibres) | f0 f1 f2 - (where the law's blocks
-// have f), the even nodes before the odd ones: the five records that a load's
-// lanes read lie in different bank groups
-constexpr int kVPlane = 40;  // words of a plane of 16-byte chunks
-__device__ __forceinline__ int node_pos(int a) { return (a >> 1) + 5 * (a & 1); }
+// node records of a point, two nodes 2 m and 2 m + 1 side by side: planes of the
+// five pairs' 16-byte chunks  c0 c0' c1 c1' | c2 c2' G0 G0' | G1 G1' G2 G2' |
+// g1 g1' g2 g2' with fibres | f0 f0' f1 f1' | f2 f2' - - where the law's blocks
+// have f.  So two nodes' values are the operands of one packed instruction.
+constexpr int kVPlane = 20;
 constexpr int kImage = kElemStride;  // floats of an element's image
 constexpr int kPairWords = 2 * kImage + 16 + 5 * kQS;
 // words between the points' node records and between their residual
-// contributions, by the banks of phase V's stores (ch: planes; fibre: 16-byte
-// chunks in the second plane, else 8-byte ones)
-__host__ __device__ constexpr int vpoint(bool fibre, int ch, int nq) {
-    return nq == 4 ? (ch == 2 ? 80 : 144) : (fibre ? 92 : 76) + (ch == 2 ? 0 : 32);
+// contributions, by the banks of phase V's stores (ch planes)
+__host__ __device__ constexpr int vpoint(int ch, int nq) {
+    return nq == 4 ? (ch <= 4 ? 80 : ch == 5 ? 112 : 144) : (ch == 3 ? 76 : ch <= 5 ? 108 : 120);
 }
 __host__ __device__ constexpr int rpoint(int nq) { return nq == 4 ? 44 : 33; }
-static_assert(5 * kQS + 8 * (vpoint(true, 3, 4) + rpoint(4)) <= 2 * kImage &&
-                  5 * kQS + 10 * (vpoint(true, 3, 5) + rpoint(5)) <= 2 * kImage,
+static_assert(5 * kQS + 8 * (vpoint(6, 4) + rpoint(4)) <= 2 * kImage && 5 * kQS + 10 * (vpoint(6, 5) + rpoint(5)) <= 2 * kImage,
               "the phase buffers alias the images");
 
 // lane of a half warp -> tile (A << 4 | B); lane 15 repeats lane 14's and stores nothing
@@ -203,76 +200,83 @@ struct PointScalars {
     }
 };
 
-// one block (a, b) at one quadrature point: K += the block's integrand
-template <int LAW>
-__device__ __forceinline__ void block_update(float *K, const float4 *va, const float4 *vb, const PointScalars<LAW> &P) {
+// a pair of nodes' record at a quadrature point
+struct NodePair {
+    float2 c[3], G[3], g1, g2, f[3];
+};
+
+// the blocks (a, b) and (a, b') of the row node a (record A's component X) and
+// the node pair of B at one quadrature point: K += the blocks' integrands
+template <int LAW, int X>
+__device__ __forceinline__ void block_update(float2 *K, const NodePair &A, const NodePair &B, const PointScalars<LAW> &P) {
     constexpr bool kFibre = (LAW == kLawAniso || LAW == kLawMLP || LAW == kLawMLPF);
     constexpr bool kFullHess = (LAW == kLawMLP);
     constexpr bool kCross = (LAW == kLawSKR3);
-    const float4 a0 = va[0], a1 = va[1], b0 = vb[0], b1 = vb[1];
-    const float ca[3] = {a0.x, a0.y, a0.z}, cb[3] = {b0.x, b0.y, b0.z};
-    float dg = P.s.x * (a0.w * b0.w + a1.x * b1.x + a1.y * b1.y);
-    float t[3], n[3];
+    auto of = [](float2 v) { return X ? v.y : v.x; };
+    const float ca[3] = {of(A.c[0]), of(A.c[1]), of(A.c[2])};
+    const float2 dot = fma2(both(of(A.G[2])), B.G[2], fma2(both(of(A.G[0])), B.G[0], mul2(both(of(A.G[1])), B.G[1])));
+    float2 t[3];
+    float n[3];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-        t[j] = P.s.y * cb[j];
+        t[j] = mul2(both(P.s.y), B.c[j]);
         n[j] = -P.s.z * ca[j];
     }
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(cb[i], n[j], fmaf(ca[i], t[j], K[3 * i + j]));
-    if (kCross || kFibre) {
-        float fa[3], fb[3];
-        if (kCross || kFullHess) {
-            const float4 a2 = va[2], b2 = vb[2];
-            fa[0] = a2.x; fa[1] = a2.y; fa[2] = a2.z;
-            fb[0] = b2.x; fb[1] = b2.y; fb[2] = b2.z;
-        }
-        if (kCross) {  // psi_1J (D_1 (x) D_J + D_J (x) D_1), D_1 = 2 f
-            float kf[3], kc[3];
+        for (int j = 0; j < 3; j++) K[3 * i + j] = fma2(B.c[i], both(n[j]), fma2(both(ca[i]), t[j], K[3 * i + j]));
+    if (kCross) {  // psi_1J (D_1 (x) D_J + D_J (x) D_1), D_1 = 2 f
+        float2 kf[3], kc[3];
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                kf[j] = P.s.w * fb[j];
-                kc[j] = P.s.w * cb[j];
+        for (int j = 0; j < 3; j++) {
+            kf[j] = mul2(both(P.s.w), B.f[j]);
+            kc[j] = mul2(both(P.s.w), B.c[j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+                K[3 * i + j] = fma2(both(of(A.f[i])), kc[j], fma2(both(ca[i]), kf[j], K[3 * i + j]));
+    }
+    if (kFibre) {
+        const float a1 = of(A.g1), a2 = of(A.g2);
+        const float2 g1 = mul2(both(a1), B.g1), g2 = mul2(both(a2), B.g2);
+        const float2 dg = fma2(both(P.fib.x), g1, fma2(both(P.fib.y), g2, mul2(both(P.s.x), dot)));
+        if (!kFullHess) {  // psi_4f4f D_4f (x) D_4f, D_4f = 2 (a_f . G) F a_f
+            const float2 x1 = mul2(both(P.fib.z), g1), x2 = mul2(both(P.fib.w), g2);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float2 y1 = mul2(x1, both(P.fa1[i])), y2 = mul2(x2, both(P.fa2[i]));
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    K[3 * i + j] = fma2(y2, both(P.fa2[j]), fma2(y1, both(P.fa1[j]), K[3 * i + j]));
             }
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(fa[i], kc[j], fmaf(ca[i], kf[j], K[3 * i + j]));
-        }
-        if (kFibre) {
-            const float g1 = a1.z * b1.z, g2 = a1.w * b1.w;
-            dg = fmaf(P.fib.x, g1, fmaf(P.fib.y, g2, dg));
-            if (!kFullHess) {  // psi_4f4f D_4f (x) D_4f, D_4f = 2 (a_f . G) F a_f
-                const float x1 = P.fib.z * g1, x2 = P.fib.w * g2;
+            if (LAW == kLawMLPF) {  // psi_4a4b (D_4a (x) D_4b + D_4b (x) D_4a), 4 s psi_4a4b in s.w
+                const float2 c12 = mul2(both(P.s.w * a1), B.g2), c21 = mul2(both(P.s.w * a2), B.g1);
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
-                    const float y1 = x1 * P.fa1[i], y2 = x2 * P.fa2[i];
+                    const float2 y1 = mul2(c12, both(P.fa1[i])), y2 = mul2(c21, both(P.fa2[i]));
 #pragma unroll
-                    for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(y2, P.fa2[j], fmaf(y1, P.fa1[j], K[3 * i + j]));
+                    for (int j = 0; j < 3; j++)
+                        K[3 * i + j] = fma2(y2, both(P.fa1[j]), fma2(y1, both(P.fa2[j]), K[3 * i + j]));
                 }
-                if (LAW == kLawMLPF) {  // psi_4a4b (D_4a (x) D_4b + D_4b (x) D_4a), 4 s psi_4a4b in s.w
-                    const float c12 = P.s.w * a1.z * b1.w, c21 = P.s.w * a1.w * b1.z;
+            }
+        } else {  // the full Hessian: sum_kl s psi_kl D_k[a] (x) D_l[b]
 #pragma unroll
-                    for (int i = 0; i < 3; i++) {
-                        const float y1 = c12 * P.fa1[i], y2 = c21 * P.fa2[i];
-#pragma unroll
-                        for (int j = 0; j < 3; j++) K[3 * i + j] = fmaf(y2, P.fa1[j], fmaf(y1, P.fa2[j], K[3 * i + j]));
-                    }
-                }
-            } else {  // the full Hessian: sum_kl s psi_kl D_k[a] (x) D_l[b]
+            for (int y = 0; y < 2; y++) {
+                auto ob = [&](float2 v) { return y ? v.y : v.x; };
                 float Da[4][3], Db[4][3];
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
-                    Da[0][i] = 2.0f * fa[i];
-                    Db[0][i] = 2.0f * fb[i];
+                    Da[0][i] = 2.0f * of(A.f[i]);
+                    Db[0][i] = 2.0f * ob(B.f[i]);
                     Da[1][i] = ca[i];
-                    Db[1][i] = cb[i];
-                    Da[2][i] = 2.0f * a1.z * P.fa1[i];
-                    Db[2][i] = 2.0f * b1.z * P.fa1[i];
-                    Da[3][i] = 2.0f * a1.w * P.fa2[i];
-                    Db[3][i] = 2.0f * b1.w * P.fa2[i];
+                    Db[1][i] = ob(B.c[i]);
+                    Da[2][i] = 2.0f * a1 * P.fa1[i];
+                    Db[2][i] = 2.0f * ob(B.g1) * P.fa1[i];
+                    Da[3][i] = 2.0f * a2 * P.fa2[i];
+                    Db[3][i] = 2.0f * ob(B.g2) * P.fa2[i];
                 }
                 const float *h = P.h;
 #pragma unroll
@@ -282,30 +286,37 @@ __device__ __forceinline__ void block_update(float *K, const float4 *va, const f
                     const float E2 = h[2] * Db[0][j] + h[5] * Db[1][j] + h[7] * Db[2][j] + h[8] * Db[3][j];
                     const float E3 = h[3] * Db[0][j] + h[6] * Db[1][j] + h[8] * Db[2][j] + h[9] * Db[3][j];
 #pragma unroll
-                    for (int i = 0; i < 3; i++)
-                        K[3 * i + j] += Da[0][i] * E0 + Da[1][i] * E1 + Da[2][i] * E2 + Da[3][i] * E3;
+                    for (int i = 0; i < 3; i++) {
+                        float &k = y ? K[3 * i + j].y : K[3 * i + j].x;
+                        k += Da[0][i] * E0 + Da[1][i] * E1 + Da[2][i] * E2 + Da[3][i] * E3;
+                    }
                 }
             }
         }
+#pragma unroll
+        for (int k = 0; k < 9; k += 4) K[k] = make_float2(K[k].x + dg.x, K[k].y + dg.y);
     }
-    K[0] += dg;
-    K[4] += dg;
-    K[8] += dg;
+    if (!kFibre) {
+#pragma unroll
+        for (int k = 0; k < 9; k += 4) K[k] = fma2(both(P.s.x), dot, K[k]);
+    }
 }
 
 // LAW: kLawSKR1 / kLawSKR2 / kLawSKR3 / kLawAniso (fused plain law) or
 // kLawMLP (reads per-QP derivatives of the surrogate network, adds the skr1
-// matrix part).  Five CTAs per SM (at most 102 registers; the 43 KB of shared
-// memory allow five), four for the full-Hessian surrogate.  Bound by the
-// instruction rate (70 %) and the shared-memory pipe (76 %) together; DRAM takes
-// the rows at 60 to 85 % of the copy bandwidth.  us at 32^3 x 6 tets of linear
-// elasticity, at 64^3 x 6 of skr2 and at 40^3 x 6 of the fibre-block surrogate:
-// 219, 1,941 and 690 with a warp per element, one block per lane and pass, and an
-// image read back by its lanes; 148, 1,564 and 593 with tiles and bulk stores;
-// 125, 1,501 and 576 with conflict-free stores and a point's values read once for
-// its nodes; 125, 1,330 and 558 with the next pair's displacements read ahead.
+// matrix part).  Bound by the shared-memory pipe (83 %) and latency; DRAM takes
+// the rows at 75 to 90 % of the copy bandwidth.  us at
+// 32^3 x 6 tets of linear elasticity, at 64^3 x 6 of skr2 and at 40^3 x 6 of the
+// fibre-block surrogate: 219, 1,941 and 690 with a warp per element, one block
+// per lane and pass, and an image read back by its lanes; 148, 1,564 and 593 with
+// tiles and bulk stores; 125, 1,501 and 576 with conflict-free stores and a
+// point's values read once for its nodes; 125, 1,330 and 558 with the next pair's
+// displacements read ahead; 122, 1,151 and 479 with two nodes' values to an
+// instruction and four CTAs per SM (128 registers; with five 120, 1,160 and 514,
+// with three 130, 1,250 and 508).
+constexpr int kElemCtas = 4;  // per SM
 template <int LAW, bool HAS_U>
-__global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_elem(const float *__restrict__ geo,
+__global__ void __launch_bounds__(32 * kWarps, kElemCtas) k_hyper_elem(const float *__restrict__ geo,
                                                             const int32_t *__restrict__ conn, int64_t ne,
                                                             const double *__restrict__ u, LawParams L,
                                                             const QPDerivs *__restrict__ qpd,
@@ -313,8 +324,10 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
                                                             int want_res, int *err, int64_t e_begin, int64_t e_end, int batch,
                                                             const __grid_constant__ HyperTables tab) {
     constexpr bool kFibre = (LAW == kLawAniso || LAW == kLawMLP || LAW == kLawMLPF);
-    constexpr int CH = LAW == kLawMLP || LAW == kLawSKR3 ? 3 : 2;  // chunks of a node record
+    constexpr bool kF = LAW == kLawMLP || LAW == kLawSKR3;  // the blocks have f
+    constexpr int CH = 3 + (kFibre ? 1 : 0) + (kF ? 2 : 0), CF = kFibre ? 4 : 3;  // planes, and the first of f
     __shared__ __align__(16) float sdphi[5][36];  // per point: grad_ref phi of the 10 nodes, zero padded
+    __shared__ __align__(8) float sdpair[5][36];  // the same at 10 j + a
     __shared__ float sw[5];
     __shared__ __align__(16) float sBi[kWarps][32][12];  // B^-1, det B
     __shared__ __align__(16) float sU[kWarps][2][36];  // nodal u of the element pair of phase Q
@@ -324,6 +337,7 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
     for (int i = threadIdx.x; i < 5 * 36; i += blockDim.x) {
         const int q = i / 36, k = i - 36 * q;
         (&sdphi[0][0])[i] = (q < nq && k < 30) ? (&tab.dphi[0][0][0])[30 * q + k] : 0.0f;
+        if (q < nq && k < 30) sdpair[q][10 * (k % 3) + k / 3] = (&tab.dphi[0][0][0])[30 * q + k];
     }
     if (threadIdx.x < 5) sw[threadIdx.x] = (int)threadIdx.x < nq ? tab.w[threadIdx.x] : 0.0f;
     if (lane < 12) sU[w][lane / 6][30 + lane % 6] = 0.0f;
@@ -335,8 +349,7 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
     // the elements' images, then the point records of the odd element (QB)
     float *QA = sBuf[w];                         // [5][kQS]
     float *V = QA + 5 * kQS;                     // [2][nq] of CH planes
-    constexpr int P1 = kVPlane, P2 = P1 + (kFibre ? 40 : 20), W1 = kFibre ? 4 : 2;  // the planes, words per chunk of the second
-    const int vp = vpoint(kFibre, CH, nq), rp = rpoint(nq);
+    const int vp = vpoint(CH, nq), rp = rpoint(nq);
     float *Rq = V + 2 * nq * vp;                 // [2][nq][rp]: residual contributions of (node, component)
     float *QB = sBuf[w] + 2 * kImage + 16;       // [5][kQS], in other banks than QA
     float *O = sBuf[w] + h * kImage;             // this half's image
@@ -506,8 +519,8 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
                 }
             }
             __syncwarp();
-            // phase V: a lane works at one (element, point q) on three nodes (four with five points); which
-            // ones, and the strides, put no two of the lanes' stores at four points on one bank
+            // phase V: a lane works at one (element, point q) on every 4th pair of nodes (every 3rd with five
+            // points); the strides put no two of a quarter warp's stores on one bank
             {
                 const int parts = nq == 4 ? 4 : 3, qq = lane / parts, ep = qq >= nq ? 1 : 0, q = qq - ep * nq;
                 if (qq < nq * pair) {
@@ -530,76 +543,90 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
                     x2 = *reinterpret_cast<const float4 *>(Qq + kQFa2);
                 }
                 float *Vq = V + qq * vp, *rq = Rq + qq * rp;
-                const int per = nq == 4 ? 3 : 4, a0 = per * (lane - parts * qq), a1 = min(a0 + per, 10);
-                for (int a = a0; a < a1; a++) {
-                const float g0 = sdphi[q][3 * a], g1 = sdphi[q][3 * a + 1], g2 = sdphi[q][3 * a + 2];
-                float G[3];
+                for (int m = lane - parts * qq; m < 5; m += parts) {
+                    float2 d[3], G[3], c[3], f[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++) G[k] = Bi[k] * g0 + Bi[3 + k] * g1 + Bi[6 + k] * g2;
-                float c[3], f[3];
+                    for (int j = 0; j < 3; j++) d[j] = *reinterpret_cast<const float2 *>(&sdpair[q][10 * j + 2 * m]);
 #pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    c[i] = FC[9 + 3 * i] * G[0] + FC[9 + 3 * i + 1] * G[1] + FC[9 + 3 * i + 2] * G[2];
-                    f[i] = FC[3 * i] * G[0] + FC[3 * i + 1] * G[1] + FC[3 * i + 2] * G[2];
-                }
-                float ag1 = 0.0f, ag2 = 0.0f;
-                if (kFibre) {
-                    ag1 = L.a1[0] * G[0] + L.a1[1] * G[1] + L.a1[2] * G[2];
-                    ag2 = L.a2[0] * G[0] + L.a2[1] * G[1] + L.a2[2] * G[2];
-                }
-                const int at = node_pos(a);
-                *reinterpret_cast<float4 *>(Vq + 4 * at) = make_float4(c[0], c[1], c[2], G[0]);
-                if (kFibre) *reinterpret_cast<float4 *>(Vq + P1 + 4 * at) = make_float4(G[1], G[2], ag1, ag2);
-                else *reinterpret_cast<float2 *>(Vq + P1 + 2 * at) = make_float2(G[1], G[2]);
-                if (CH == 3) *reinterpret_cast<float4 *>(Vq + P2 + 4 * at) = make_float4(f[0], f[1], f[2], 0.0f);
-                if (want_res) {
-                    float r[3];
+                    for (int k = 0; k < 3; k++)
+                        G[k] = fma2(both(Bi[6 + k]), d[2], fma2(both(Bi[k]), d[0], mul2(both(Bi[3 + k]), d[1])));
 #pragma unroll
-                    for (int i = 0; i < 3; i++) r[i] = rs.x * f[i] + rs.y * c[i];
-                    if (kFibre) {
-                        const float h1 = rs.z * ag1, h2 = rs.w * ag2;
-                        r[0] += h1 * x1.x + h2 * x2.x;
-                        r[1] += h1 * x1.y + h2 * x2.y;
-                        r[2] += h1 * x1.z + h2 * x2.z;
+                    for (int i = 0; i < 3; i++) {
+                        c[i] = fma2(both(FC[9 + 3 * i + 2]), G[2], fma2(both(FC[9 + 3 * i]), G[0], mul2(both(FC[9 + 3 * i + 1]), G[1])));
+                        f[i] = fma2(both(FC[3 * i + 2]), G[2], fma2(both(FC[3 * i]), G[0], mul2(both(FC[3 * i + 1]), G[1])));
                     }
+                    float2 ag1 = both(0.0f), ag2 = ag1;
+                    if (kFibre) {
+                        ag1 = fma2(both(L.a1[2]), G[2], fma2(both(L.a1[0]), G[0], mul2(both(L.a1[1]), G[1])));
+                        ag2 = fma2(both(L.a2[2]), G[2], fma2(both(L.a2[0]), G[0], mul2(both(L.a2[1]), G[1])));
+                    }
+                    auto put = [&](int plane, float2 x, float2 y) {
+                        *reinterpret_cast<float4 *>(Vq + kVPlane * plane + 4 * m) = make_float4(x.x, x.y, y.x, y.y);
+                    };
+                    put(0, c[0], c[1]);
+                    put(1, c[2], G[0]);
+                    put(2, G[1], G[2]);
+                    if (kFibre) put(3, ag1, ag2);
+                    if (kF) {
+                        put(CF, f[0], f[1]);
+                        put(CF + 1, f[2], f[2]);
+                    }
+                    if (want_res) {
+                        float2 r[3];
 #pragma unroll
-                    for (int i = 0; i < 3; i++) rq[3 * a + i] = r[i];
-                }
+                        for (int i = 0; i < 3; i++) r[i] = fma2(both(rs.x), f[i], mul2(both(rs.y), c[i]));
+                        if (kFibre) {
+                            const float2 h1 = mul2(both(rs.z), ag1), h2 = mul2(both(rs.w), ag2);
+                            const float z1[3] = {x1.x, x1.y, x1.z}, z2[3] = {x2.x, x2.y, x2.z};
+#pragma unroll
+                            for (int i = 0; i < 3; i++) {
+                                const float2 e = fma2(h1, both(z1[i]), mul2(h2, both(z2[i])));
+                                r[i] = make_float2(r[i].x + e.x, r[i].y + e.y);
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            rq[6 * m + i] = r[i].x;
+                            rq[6 * m + 3 + i] = r[i].y;
+                        }
+                    }
                 }
                 }
             }
             __syncwarp();
             if (HAS_U && t + 2 < nb) read_u();
             // phase K: the tile's four blocks, summed over the points in registers
-            float K[2][2][9];
+            float2 K[2][9];  // [x]: the blocks (2 A + x, 2 B) and (2 A + x, 2 B + 1)
 #pragma unroll
-            for (int k = 0; k < 36; k++) (&K[0][0][0])[k] = 0.0f;
+            for (int k = 0; k < 18; k++) (&K[0][0])[k] = make_float2(0.0f, 0.0f);
             const float *Qh = h ? QB : QA, *Vh = V + h * nq * vp;
+#pragma unroll 1
             for (int q = 0; q < nq; q++) {
                 PointScalars<LAW> P;
                 P.load(Qh + q * kQS);
                 const float *Vq = Vh + q * vp;
-                float4 va[2][CH], vb[2][CH];
-                auto record = [&](int at, float4 *v) {
-                    v[0] = *reinterpret_cast<const float4 *>(Vq + 4 * at);
-                    if (kFibre) {
-                        v[1] = *reinterpret_cast<const float4 *>(Vq + P1 + W1 * at);
-                    } else {
-                        const float2 g = *reinterpret_cast<const float2 *>(Vq + P1 + W1 * at);
-                        v[1] = make_float4(g.x, g.y, 0.0f, 0.0f);
+                auto record = [&](int m, NodePair &R) {
+                    auto get = [&](int plane, float2 &x, float2 &y) {
+                        const float4 v = *reinterpret_cast<const float4 *>(Vq + kVPlane * plane + 4 * m);
+                        x = make_float2(v.x, v.y);
+                        y = make_float2(v.z, v.w);
+                    };
+                    get(0, R.c[0], R.c[1]);
+                    get(1, R.c[2], R.G[0]);
+                    get(2, R.G[1], R.G[2]);
+                    if (kFibre) get(3, R.g1, R.g2);
+                    if (kF) {
+                        get(CF, R.f[0], R.f[1]);
+                        R.f[2] = *reinterpret_cast<const float2 *>(Vq + kVPlane * (CF + 1) + 4 * m);
                     }
-                    if (CH == 3) v[2] = *reinterpret_cast<const float4 *>(Vq + P2 + 4 * at);
                 };
-#pragma unroll
-                for (int x = 0; x < 2; x++) {
-                    record(A + 5 * x, va[x]);
-                    record(B + 5 * x, vb[x]);
-                }
-#pragma unroll
-                for (int x = 0; x < 2; x++)
-#pragma unroll
-                    for (int y = 0; y < 2; y++) block_update<LAW>(K[x][y], va[x], vb[y], P);
+                NodePair ra, rb;
+                record(A, ra);
+                record(B, rb);
+                block_update<LAW, 0>(K[0], ra, rb, P);
+                block_update<LAW, 1>(K[1], ra, rb, P);
             }
+            auto value = [&](int x, int y, int k) { return y ? K[x][k].y : K[x][k].x; };
             float r0 = 0.0f, r1 = 0.0f;
             if (want_res && lane < 30)
                 for (int q = 0; q < nq; q++) {
@@ -610,7 +637,7 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
-                    for (int j = 0; j < 3; j++) K[1][0][3 * i + j] = K[0][1][3 * j + i];
+                    for (int j = 0; j < 3; j++) K[1][3 * i + j].x = K[0][3 * j + i].y;
             }
             __syncwarp();  // the phase buffers are dead: the images overwrite them
             if (hl < 15 && h < pair) {
@@ -620,10 +647,10 @@ __global__ void __launch_bounds__(32 * kWarps, LAW == kLawMLP ? 4 : 5) k_hyper_e
                     for (int c = 0; c < 3; c++) {
                         const int u = 2 * c, v = 2 * c + 1;  // columns of the tile
                         *reinterpret_cast<float2 *>(O + (r < 3 ? oAB[c] : oAB[c] ^ 16) + 32 * r) =
-                            make_float2(K[r / 3][u / 3][3 * (r % 3) + u % 3], K[r / 3][v / 3][3 * (r % 3) + v % 3]);
+                            make_float2(value(r / 3, u / 3, 3 * (r % 3) + u % 3), value(r / 3, v / 3, 3 * (r % 3) + v % 3));
                         if (A != B)
                             *reinterpret_cast<float2 *>(O + (r < 3 ? oBA[c] : oBA[c] ^ 16) + 32 * r) =
-                                make_float2(K[u / 3][r / 3][3 * (u % 3) + r % 3], K[v / 3][r / 3][3 * (v % 3) + r % 3]);
+                                make_float2(value(u / 3, r / 3, 3 * (u % 3) + r % 3), value(v / 3, r / 3, 3 * (v % 3) + r % 3));
                     }
             }
             if (lane < 30) {
@@ -1082,7 +1109,7 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
     if (count <= 0) return;
     // batches of at most 32 elements, even, that give the chip's warps equal
     // shares in as few rounds as there have to be
-    const int64_t chip = (int64_t)sm_count() * 5 * kWarps, rounds = ceil_div(count, 32 * chip);
+    const int64_t chip = (int64_t)sm_count() * kElemCtas * kWarps, rounds = ceil_div(count, 32 * chip);
     const int batch = 2 * (int)ceil_div(count, 2 * rounds * chip);
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, (int64_t)batch * kWarps), (int64_t)sm_count() * 16);
     const bool hu = u != nullptr;
