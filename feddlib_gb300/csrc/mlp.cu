@@ -627,6 +627,18 @@ __device__ __forceinline__ void tile_product(float acc[SPT][5][4], const float *
     }
 }
 
+// a sum with the rounding errors of its additions kept beside it (Knuth's
+// two-sum), for the last levels of the gradients' sums, where many terms cancel
+struct TwoSum {
+    float s = 0.0f, c = 0.0f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = __fadd_rn(s, x), xx = __fsub_rn(t, s);
+        c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, xx)), __fsub_rn(x, xx)));
+        s = t;
+    }
+    __device__ __forceinline__ float value() const { return __fadd_rn(s, c); }
+};
+
 // samples idx[0..B) (null: 0..B) in tiles of GROUPS SPT; part: gridDim.x x kTPar
 template <int GROUPS, int SPT>
 __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
@@ -655,7 +667,8 @@ __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
     const float b3 = *P.b3;
     __syncthreads();
     float *xrow = sX + s * kTSample, *drow = sD + s * kTSample;
-    float gW2[JB][4], gW1[4][4], gb1[4], gb2[4], gw3[4], gb3 = 0.0f, loss = 0.0f;
+    float gW2[JB][4], gW1[4][4], gb1[4], gb2[4], gw3[4];
+    TwoSum gb3, loss;
 #pragma unroll
     for (int a = 0; a < 4; a++) {
         gb1[a] = gb2[a] = gw3[a] = 0.0f;
@@ -733,8 +746,8 @@ __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
                 eg[k] = valid[m] ? 2.0f * wgrad * dk : 0.0f;
                 l += wgrad * dk * dk;
             }
-            gb3 += ey;
-            loss += valid[m] ? l : 0.0f;
+            gb3.add(ey);
+            loss.add(valid[m] ? l : 0.0f);
             float d[5][4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -809,8 +822,8 @@ __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
         red[s * kSmall + 6 * kH + u0 + u] = gw3[u];
     }
     if (u0 == 0) {
-        red[GROUPS * kSmall + s] = gb3;
-        red[GROUPS * kSmall + GROUPS + s] = loss;
+        red[GROUPS * kSmall + s] = gb3.value();
+        red[GROUPS * kSmall + GROUPS + s] = loss.value();
     }
     __syncthreads();
     if (share == 0) {
@@ -826,11 +839,11 @@ __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
             }
     }
     for (int t = tid; t < kSmall + 2; t += THREADS) {
-        float v = 0.0f;
+        TwoSum v;
         for (int q = 0; q < GROUPS; q++)
-            v += t < kSmall ? red[q * kSmall + t] : red[GROUPS * kSmall + GROUPS * (t - kSmall) + q];
+            v.add(t < kSmall ? red[q * kSmall + t] : red[GROUPS * kSmall + GROUPS * (t - kSmall) + q]);
         // gW1 | gb1 at the front, gb2 | gw3 | gb3 | loss behind gW2
-        out[t < 5 * kH ? t : t + kH * kH] = v;
+        out[t < 5 * kH ? t : t + kH * kH] = v.value();
     }
 }
 
@@ -841,14 +854,15 @@ __global__ void __launch_bounds__(256) k_tr_update(const float *__restrict__ par
                                                    float b2, float eps, float c1, float c2, float scale) {
     __shared__ float red[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
-    float v = 0.0f;
+    TwoSum sum;
     if (i < kTPar)
-        for (int q = w; q < nparts; q += 8) v += part[(int64_t)q * kTPar + i];
-    red[w][lane] = v;
+        for (int q = w; q < nparts; q += 8) sum.add(part[(int64_t)q * kTPar + i]);
+    red[w][lane] = sum.value();
     __syncthreads();
     if (w != 0 || i >= kTPar) return;
 #pragma unroll
-    for (int q = 1; q < 8; q++) v += red[q][lane];
+    for (int q = 1; q < 8; q++) sum.add(red[q][lane]);
+    const float v = sum.value();
     if (i == kTPar - 1) {
         *lsum = v;
     } else if (adam) {
