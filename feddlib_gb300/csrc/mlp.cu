@@ -628,7 +628,10 @@ __device__ __forceinline__ void tile_product(float acc[SPT][5][4], const float *
 }
 
 // a sum with the rounding errors of its additions kept beside it (Knuth's
-// two-sum), for the last levels of the gradients' sums, where many terms cancel
+// two-sum), for the last levels of the gradients' sums and for b3's and the
+// loss's, where many terms cancel: b3 after eight steps of 65,536 samples is
+// 4.5e-7 off on average over twelve seeds (1.0e-6 at most), 5.5e-7 (1.6e-6) with
+// plain sums, for 2 us per step
 struct TwoSum {
     float s = 0.0f, c = 0.0f;
     __device__ __forceinline__ void add(float x) {
@@ -1066,7 +1069,7 @@ void tr_fused(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float 
     cudaStream_t s = 0;
     // tiles of 48 samples, one CTA per SM, or of 16, two per SM: whichever takes
     // less time over its rounds of tiles (20.4 and 14.6 us a round; a step of
-    // 65,536 samples 203 against 226 us, 20,000 77 and 84, 15,000 76 and 69, 30,000 118 and 114)
+    // 65,536 samples 205 against 226 us, 20,000 77 and 84, 15,000 76 and 69, 30,000 118 and 114)
     const int64_t rounds1 = ceil_div(B, 32 * (int64_t)sms()), rounds2 = ceil_div(B, 48 * (int64_t)sms());
     const int spt = 7 * rounds2 < 5 * rounds1 ? 2 : 1;
     const int groups = spt == 2 ? 24 : 16;
