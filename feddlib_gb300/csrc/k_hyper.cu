@@ -1,5 +1,5 @@
-// k_hyper.cu -- P2 elasticity / hyperelasticity: element stage (warp per
-// element, FP32) and row stage (warp per node, deterministic gather).
+// k_hyper.cu -- P2 elasticity / hyperelasticity: element stage (two elements
+// per warp, FP32) and row stage (warp per node, deterministic gather).
 //
 // Element math follows the AceGen kernels FEDDLib calls for
 // "LinearElasticity" (skr1, NeoHookQuadraticTets.f, 4-point rule code 18),

@@ -13,7 +13,7 @@
 //   W_(ai)(bj) = sum_m g[j][m][i] R[a][b][m],  g = |det B| grad u at vertex m
 //   Bd_p(bd) = sum_c Bs[d][c] Y[b][p][c],     Bs = |det B| B^-1
 // A record kernel (one thread per element) writes these
-// coefficients; the row kernels (one warp per node) contract them for the
+// coefficients; the row kernels (a warp per node or two) contract them for the
 // node's row and accumulate in shared memory, then write each CSR value once.
 #include "kernels.cuh"
 #include "tcgen05.cuh"
@@ -452,7 +452,7 @@ __global__ void k_ns_node_info(const int64_t *__restrict__ inc_ptr, const int64_
 // incidence of each per step: with lanes (p, j) of 15 the half's lane owns the columns
 // (b, j) of the two nodes b = 2 p and 2 p + 1, so every value that the ten
 // nodes share (the gradient rows g[j], Bs, the wait, the staging) is read or
-// done once for two incidences.  Warps claim eight consecutive nodes and pair
+// done once for two incidences.  Warps claim four or eight consecutive nodes and pair
 // them by their number of incidences, so that the halves end together (on a
 // lattice vertices, 24 incidences, and edge nodes, 4 or 6, alternate).
 // Each incidence's record head (g, Bs, u, p), the 48-byte window holding
