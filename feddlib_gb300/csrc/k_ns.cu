@@ -472,7 +472,8 @@ __global__ void k_ns_node_info(const int64_t *__restrict__ inc_ptr, const int64_
 // them the accumulators' scattered updates and the broadcast 16-byte reads).
 // At 48^3 x 6 tets 1,299 us, against 1,480 us with one node per warp, three
 // planes of accumulators and 8-byte stores; without the Newton term, whose
-// reads and products the Picard form leaves out, 197 us against 240 at
+// reads and products the Picard form leaves out, 197 us against 240 (189 since
+// it leaves the gradients' nine chunks behind) at
 // 27 x 19 x 33 x 6 tets in file order; with the viscous rows 494 us against 522
 // at 32^3 x 6.  Groups of four nodes 1,319 us, rings of three or six slots
 // 1,389 and 1,423, eleven warps per CTA (80 registers, spills) 1,461.
@@ -481,6 +482,8 @@ constexpr int kVStage = 100;  // floats per ring slot: record head 84 | NA windo
 constexpr int kVNA = kRecVel, kVSlots = kRecVel + 12;
 constexpr int kVGn = kVStage, kVGnRes = kVStage + 96, kVStageGn = kVStage + 104;
 static_assert(kVSlots + 4 == kVStage && kRecVel % 4 == 0, "ring slot layout: chunk c holds floats [4 c, 4 c + 4)");
+static_assert(kRecG == 0 && kRecBS == 36 && kRecBS < kRecU && kRecBS < kRecP && kRecVel == 84,
+              "without the gradients at its front the head has twelve chunks");
 // the ring and the accumulators of a half are 16 mod 32 words, so the halves'
 // accesses to the same place of theirs differ in banks
 static_assert(kVRing * kVStage % 32 == 16 && kVRing * kVStageGn % 32 == 16, "half-warp bank offset");
@@ -573,11 +576,12 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
     const uint8_t *pS = reinterpret_cast<const uint8_t *>(ring + kVSlots);
     const float *pR = sR + 4 * NPW * p, *pY = sY + 4 * bq, *pYb = sY + 16 * NPW * p;
     // chunks of 16 bytes: record head (to 20), NA window (21-23), slot map (24).  Two nodes per warp: chunk hl,
-    // and c2 = 16 + hl for hl < 9; one: c2 = hl < 25 alone
-    const int c2 = NPW == 2 ? 16 + hl : hl;
+    // and c2 = 16 + hl for hl < 9; one: c2 = hl < 25 alone.  Without the Newton term the head's nine chunks of
+    // velocity gradients stay behind, and c2 = 9 + hl for hl < 16 is all
+    const int cg = NPW == 2 ? 16 + hl : hl, c2 = NEWTON ? cg : kRecBS / 4 + hl;
     const char *src1 = reinterpret_cast<const char *>(rec + 4 * hl);
     const char *src2 = reinterpret_cast<const char *>(c2 < 21 ? rec + 4 * c2 : rec + kRecNA + 4 * (c2 - 21));
-    float *dst_lane = ring + 4 * hl, *dst2 = ring + 4 * c2;
+    float *dst_lane = ring + 4 * hl, *dst2 = ring + 4 * c2, *dstg = ring + kVGn + 4 * cg;
     // with `work`, nodes come from a global counter, a group per warp step, so
     // all warps stay on one sharp front of the sweep and the ten readers of
     // an element's record come close in time
@@ -634,16 +638,16 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
                 if (t < m) {
                     const uint32_t a = ea & 15u;
                     const size_t eo = (size_t)(ea >> 4) * (kNSRecord * sizeof(float));
-                    if (NPW == 2) cp_async16(dst_lane + slot * kStg, src1 + eo);
+                    if (NPW == 2 && NEWTON) cp_async16(dst_lane + slot * kStg, src1 + eo);
                     // NA[a][0..9] starts 8 bytes into a 16-byte boundary when a is odd
                     const size_t o2 = c2 == 24 ? (size_t)(t * kSlotStride) : eo + (c2 < 21 ? 0u : 40u * a - 8u * (a & 1u));
                     if (c2 < 25) cp_async16(dst2 + slot * kStg, src2 + o2);
                     if (GN) {
                         const float *Ke = gstage + (size_t)(ea >> 4) * kGNStride;
                         if (NPW == 2) cp_async16(dst_lane + slot * kStg + kVGn, Ke + 96 * a + 4 * hl);
-                        if (c2 < 26)
-                            cp_async16(dst2 + slot * kStg + kVGn,
-                                       c2 < 24 ? Ke + 96 * a + 4 * c2 : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (c2 - 24));
+                        if (cg < 26)
+                            cp_async16(dstg + slot * kStg,
+                                       cg < 24 ? Ke + 96 * a + 4 * cg : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (cg - 24));
                     }
                 }
                 cp_async_commit();
