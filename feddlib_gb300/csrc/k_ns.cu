@@ -15,6 +15,8 @@
 // A record kernel (one thread per element) writes these
 // coefficients; the row kernels (a warp per node or two) contract them for the
 // node's row and accumulate in shared memory, then write each CSR value once.
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "tcgen05.cuh"
 
@@ -472,9 +474,10 @@ __global__ void k_ns_node_info(const int64_t *__restrict__ inc_ptr, const int64_
 // them the accumulators' scattered updates and the broadcast 16-byte reads).
 // At 48^3 x 6 tets 1,299 us, against 1,480 us with one node per warp, three
 // planes of accumulators and 8-byte stores; without the Newton term, whose
-// reads and products the Picard form leaves out, 197 us against 240 (189 since
-// it leaves the gradients' nine chunks behind) at
-// 27 x 19 x 33 x 6 tets in file order; with the viscous rows 494 us against 522
+// reads and products the Picard form leaves out, 197 us against 240 at
+// 27 x 19 x 33 x 6 tets in file order, 189 without staging the gradients and 183
+// without the residual (RES), its sums and the chunks of u and p; the Newton
+// form without the residual at 51 x 37 x 39 x 6 886 us for the call against 977; with the viscous rows 494 us against 522
 // at 32^3 x 6.  Groups of four nodes 1,319 us, rings of three or six slots
 // 1,389 and 1,423, eleven warps per CTA (80 registers, spills) 1,461.
 constexpr int kVRing = 4;
@@ -540,7 +543,7 @@ __device__ __forceinline__ void vel_residual_out(float rj0, float rj1, float rb,
     if (node && hl < 3) res_u[3 * n + hl] = f2d_exact(GN ? fmaf(cuu, rg, s) : s);
 }
 
-template <bool GN, bool NEWTON, int NPW>
+template <bool GN, bool NEWTON, int NPW, bool RES>
 __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
     k_ns_vel_rows(const int4 *__restrict__ ninfo, const uint32_t *__restrict__ inc, const uint8_t *__restrict__ slots,
                   const float *__restrict__ rec, const float *__restrict__ gtab, const int64_t *__restrict__ rowptr00,
@@ -577,8 +580,12 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
     const float *pR = sR + 4 * NPW * p, *pY = sY + 4 * bq, *pYb = sY + 16 * NPW * p;
     // chunks of 16 bytes: record head (to 20), NA window (21-23), slot map (24).  Two nodes per warp: chunk hl,
     // and c2 = 16 + hl for hl < 9; one: c2 = hl < 25 alone.  Without the Newton term the head's nine chunks of
-    // velocity gradients stay behind, and c2 = 9 + hl for hl < 16 is all
-    const int cg = NPW == 2 ? 16 + hl : hl, c2 = NEWTON ? cg : kRecBS / 4 + hl;
+    // velocity gradients stay behind, without the residual its nine of u and p, and c2 for hl < 16 is all
+    const int cg = NPW == 2 ? 16 + hl : hl;
+    const int c2 = NEWTON && RES ? cg
+                   : RES         ? kRecBS / 4 + hl
+                   : NEWTON      ? (hl < 12 ? hl : 9 + hl)
+                                 : (hl < 3 ? kRecBS / 4 + hl : hl < 7 ? 18 + hl : 25);
     const char *src1 = reinterpret_cast<const char *>(rec + 4 * hl);
     const char *src2 = reinterpret_cast<const char *>(c2 < 21 ? rec + 4 * c2 : rec + kRecNA + 4 * (c2 - 21));
     float *dst_lane = ring + 4 * hl, *dst2 = ring + 4 * c2, *dstg = ring + kVGn + 4 * cg;
@@ -638,14 +645,14 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
                 if (t < m) {
                     const uint32_t a = ea & 15u;
                     const size_t eo = (size_t)(ea >> 4) * (kNSRecord * sizeof(float));
-                    if (NPW == 2 && NEWTON) cp_async16(dst_lane + slot * kStg, src1 + eo);
+                    if (NPW == 2 && NEWTON && RES) cp_async16(dst_lane + slot * kStg, src1 + eo);
                     // NA[a][0..9] starts 8 bytes into a 16-byte boundary when a is odd
                     const size_t o2 = c2 == 24 ? (size_t)(t * kSlotStride) : eo + (c2 < 21 ? 0u : 40u * a - 8u * (a & 1u));
                     if (c2 < 25) cp_async16(dst2 + slot * kStg, src2 + o2);
                     if (GN) {
                         const float *Ke = gstage + (size_t)(ea >> 4) * kGNStride;
                         if (NPW == 2) cp_async16(dst_lane + slot * kStg + kVGn, Ke + 96 * a + 4 * hl);
-                        if (cg < 26)
+                        if (cg < (RES ? 26 : 24))
                             cp_async16(dstg + slot * kStg,
                                        cg < 24 ? Ke + 96 * a + 4 * cg : Ke + kGNRes + 4 * ((3 * a) >> 2) + 4 * (cg - 24));
                     }
@@ -718,7 +725,7 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
                         v0 += V[0];
                         v1 += V[32];
                         v2 += V[64];
-                        rg += ring[off + kVGnRes + ((3 * a) & 3) + (hl & 3)];
+                        if (RES) rg += ring[off + kVGnRes + ((3 * a) & 3) + (hl & 3)];
                     }
                     v0 = fmaf(e0, an.x, v0);
                     v1 = fmaf(e1, an.x, v1);
@@ -751,27 +758,29 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
                     dA[sl] = v1;
                     dA[2 * sl] = v2;
                 }
-                const float ua = pU[off], ub = NPW == 2 ? pU[off + 3] : 0.0f;
-                rj0 = fmaf(an.x, ua, rj0);
-                if (NPW == 2) rj1 = fmaf(an.y, ub, rj1);
+                const float ua = RES ? pU[off] : 0.0f, ub = RES && NPW == 2 ? pU[off + 3] : 0.0f;
+                if (RES) {
+                    rj0 = fmaf(an.x, ua, rj0);
+                    if (NPW == 2) rj1 = fmaf(an.y, ub, rj1);
+                }
                 // -Bd_q(a, i): the (0,1) entry of velocity row (a, i), pressure column q
                 const float4 bs = lds4(pBS + off);
                 const float bt = fmaf(bs.z, y.z, fmaf(bs.y, y.y, bs.x * y.x));
                 float *dp = lb ? acc1 + bi * Kp + pS[4 * off + 10 + bq] : scratch;
                 *dp += bt;
-                rb = fmaf(bt, pP[off], rb);
+                if (RES) rb = fmaf(bt, pP[off], rb);
                 if (qp >= 0 && a < 4) {
                     // -Bd_q(b j): the (1,0) entries of pressure row q = this vertex, columns (b, j)
                     const float4 bj = lds4(pBSj + off);
                     const float pa = fmaf(bj.z, ya.z, fmaf(bj.y, ya.y, bj.x * ya.x));
                     float *qa = lw ? acc2 + 3 * (ss & 255u) + j : scratch;
                     *qa += pa;
-                    rq0 = fmaf(pa, ua, rq0);
+                    if (RES) rq0 = fmaf(pa, ua, rq0);
                     if (NPW == 2) {
                         const float pc = fmaf(bj.z, yc.z, fmaf(bj.y, yc.y, bj.x * yc.x));
                         float *qc = lw ? acc2 + 3 * (ss >> 8) + j : scratch;
                         *qc += pc;
-                        rq1 = fmaf(pc, ub, rq1);
+                        if (RES) rq1 = fmaf(pc, ub, rq1);
                     }
                 }
             }
@@ -779,9 +788,9 @@ __global__ void __launch_bounds__(32 * vel_warps(GN, NPW), 2)
             __syncwarp();
             vel_write<W>(mem, s00, 9 * K, out00, hl);
             vel_write<W>(mem + o01, s01, 3 * Kp, out01, hl);
-            if (res_u) vel_residual_out<GN, W>(rj0, rj1, rb, rg, n, hl, node, co, res_u);
+            if (RES && res_u) vel_residual_out<GN, W>(rj0, rj1, rb, rg, n, hl, node, co, res_u);
             if (qp >= 0) vel_write<W>(mem + o10, s10, 3 * K, out10, hl);
-            if (res_p && __any_sync(0xffffffffu, qp >= 0)) {
+            if (RES && res_p && __any_sync(0xffffffffu, qp >= 0)) {
                 // the pressure residual: the pairwise (xor) tree over 32 words, (b, j) at 3 b + j
                 float v;
                 if (NPW == 2) {
@@ -1163,12 +1172,16 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
         warps = (int)std::min<int64_t>(warps, std::max<int64_t>(2, ceil_div(count, 2 * sms)));
     }
     const size_t smem = tables + (size_t)warps * per_warp;
-    using Kern = decltype(&k_ns_vel_rows<true, true, 1>);
-    const Kern kerns[2][2][2] = {{{k_ns_vel_rows<false, false, 1>, k_ns_vel_rows<false, false, 2>},
-                                  {k_ns_vel_rows<false, true, 1>, k_ns_vel_rows<false, true, 2>}},
-                                 {{k_ns_vel_rows<true, false, 1>, k_ns_vel_rows<true, false, 2>},
-                                  {k_ns_vel_rows<true, true, 1>, k_ns_vel_rows<true, true, 2>}}};
-    const Kern kern = kerns[gn][newton != 0][npw - 1];
+    const bool res = res_u || res_p;
+    using Kern = decltype(&k_ns_vel_rows<true, true, 1, true>);
+    auto pick = [&](auto GN, auto NEWTON) -> Kern {
+        constexpr bool g = decltype(GN)::value, n = decltype(NEWTON)::value;
+        if (npw == 1) return res ? k_ns_vel_rows<g, n, 1, true> : k_ns_vel_rows<g, n, 1, false>;
+        return res ? k_ns_vel_rows<g, n, 2, true> : k_ns_vel_rows<g, n, 2, false>;
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    const Kern kern = gn ? (newton ? pick(yes, yes) : pick(yes, no)) : (newton ? pick(no, yes) : pick(no, no));
     FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     unsigned grid = (unsigned)std::min<int64_t>((count + group * warps - 1) / (group * warps), sms * 4);
     if (work) {  // dynamic positions: exactly the CTAs that fit

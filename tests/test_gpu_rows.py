@@ -88,3 +88,24 @@ def test_navier_stokes_rows_of_every_mesh_size(M, newton, gn):
     for b, w in zip(bufs, want):
         assert w.any() and np.array_equal(b.cpu().numpy(), w)
     assert np.array_equal(dru.cpu().numpy(), ru) and np.array_equal(drp.cpu().numpy(), rp)
+
+
+@pytest.mark.parametrize("newton,gn", [(True, False), (False, False), (True, True), (False, True)])
+@pytest.mark.parametrize("M", [2, 15])
+def test_navier_stokes_matrix_alone(M, newton, gn):
+    """A call for the matrix alone stages less of each record and sums no
+    residual; the values are those of the call for both."""
+    import feddlib_gb300 as F
+    xyz2, el2 = F.structured_mesh(M, 2, seed=40 + M)
+    xyz1, el1 = F.structured_mesh(M, 1, seed=40 + M)
+    u, p = 0.5 * F.fourier_field(xyz2, seed=40), F.uniform_field(40, xyz1.shape[0])
+    a = F.Assembler(F.NAVIER_STOKES, xyz2, el2, elements_p=el1, num_nodes_p=xyz1.shape[0], viscosity=0.01, density=1.3,
+                    newton=newton)
+    if gn:
+        a.set_viscosity_law(0, [1.902, 0.22, 0.056, 0.00345, 1.25], gamma_min=1e-12)
+    both, ru, _ = a.assemble(u=u, p=p)
+    both = [b.copy() for b in both]
+    alone, none, _ = a.assemble(u=u, p=p, residual=False)
+    assert none is None and ru.any()
+    for b, v in zip(both, alone):
+        assert b.any() and np.array_equal(b, v)
