@@ -630,8 +630,10 @@ __device__ __forceinline__ void tile_product(float acc[SPT][5][4], const float *
 // a sum with the rounding errors of its additions kept beside it (Knuth's
 // two-sum), for the last levels of the gradients' sums and for b3's and the
 // loss's, where many terms cancel: b3 after eight steps of 65,536 samples is
-// 4.5e-7 off on average over twelve seeds (1.0e-6 at most), 5.5e-7 (1.6e-6) with
-// plain sums, for 2 us per step
+// 2.6e-7 off on average over 18 seeds, 2.9e-7 with plain sums over the tiles,
+// 3.6e-7 with plain sums throughout (a trainer's creation on 200,000 samples and
+// the eight steps take 2,207, 2,192 and 2,188 us); the loss, an evaluation at the
+// updated parameters, is 5.6e-7 off in all three
 struct TwoSum {
     float s = 0.0f, c = 0.0f;
     __device__ __forceinline__ void add(float x) {
@@ -1261,8 +1263,12 @@ fedd_status fedd_trainer_run(fedd_trainer *t, int32_t steps, int64_t batch, floa
             a.b1 = 0.9f;
             a.b2 = 0.999f;
             a.eps = 1e-8f;
-            a.c1 = 1.0f - std::pow(a.b1, (float)t->step);
-            a.c2 = 1.0f - std::pow(a.b2, (float)t->step);
+            // in double: 1 - beta^t in FP32 keeps beta^t's rounding, up to 1.5e-5 of
+            // c2 in the early steps, which scales all parameters' moves alike (loss
+            // of eight steps of 65,536 samples off by 2.6e-6 on average over 18
+            // seeds, 5.6e-7 this way)
+            a.c1 = (float)(1.0 - std::pow((double)a.b1, (double)t->step));
+            a.c2 = (float)(1.0 - std::pow((double)a.b2, (double)t->step));
             a.scale = 1.0f / (float)batch;
             if (H == kH) {
                 tr_fused(t, idx, batch, wpsi, wgrad, &a);
