@@ -641,7 +641,11 @@ struct TwoSum {
         c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, xx)), __fsub_rn(x, xx)));
         s = t;
     }
-    __device__ __forceinline__ float value() const { return __fadd_rn(s, c); }
+    // an infinite sum's errors are not numbers: the sum itself
+    __device__ __forceinline__ float value() const {
+        const float v = __fadd_rn(s, c);
+        return isfinite(v) ? v : s;
+    }
 };
 
 // samples idx[0..B) (null: 0..B) in tiles of GROUPS SPT; part: gridDim.x x kTPar

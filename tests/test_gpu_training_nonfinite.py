@@ -1,0 +1,36 @@
+"""Training with values that are not finite: sums that overflow are infinite,
+as FP32 sums are."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from test_gpu_training import KEYS, f64, problem
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def F():
+    import feddlib_gb300 as F
+    return F
+
+
+@pytest.mark.parametrize("H", [64, 16])
+@pytest.mark.parametrize("n", [1, 20, 5001])
+def test_infinite_sums(F, H, n):
+    """A target of 1e25: its squared distance overflows, every gradient is
+    still finite.  Targets of -3e38: b3's gradient overflows too."""
+    X, ty, tg, m = problem(H, n, n)
+    ty[n // 2] = 1e25
+    tr = F.Trainer(H, X, ty, tg)
+    tr.set_params(m)
+    loss, g = tr.grad(wpsi=1.0, wgrad=0.7)
+    _, go = O.mlp_loss({k: f64(v) for k, v in m.items()}, f64(X), f64(ty), f64(tg), 1.0, 0.7)
+    assert loss == np.inf
+    for k in KEYS:  # the bound of the finite case
+        assert np.linalg.norm(f64(g[k]) - go[k]) <= 1e-4 * np.linalg.norm(go[k]), k
+    assert abs(g["b3"] - go["b3"]) <= 1e-4 * abs(go["b3"])
+    tr = F.Trainer(H, X, np.full(n, -3e38, dtype=np.float32), tg)
+    tr.set_params(m)
+    loss, g = tr.grad(wpsi=1.0, wgrad=0.7)
+    assert loss == np.inf and g["b3"] == np.inf
