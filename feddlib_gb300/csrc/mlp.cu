@@ -700,11 +700,13 @@ __global__ void __launch_bounds__(16 * GROUPS, SPT == 1 ? 2 : 1)
 #pragma unroll
         for (int m = 0; m < SPT; m++) {
             valid[m] = id[m] >= 0;
-            const int64_t si = valid[m] ? id[m] : 0;
-            const float4 x4 = ld4(X + 4 * si), t4 = ld4(tgr + 4 * si);
+            // the places behind the last sample hold zeros: their products with the
+            // errors, which are zero, stay zero
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 x4 = valid[m] ? ld4(X + 4 * id[m]) : none, t4 = valid[m] ? ld4(tgr + 4 * id[m]) : none;
             x[m][0] = x4.x; x[m][1] = x4.y; x[m][2] = x4.z; x[m][3] = x4.w;
             tg[m][0] = t4.x; tg[m][1] = t4.y; tg[m][2] = t4.z; tg[m][3] = t4.w;
-            tyv[m] = ty[si];
+            tyv[m] = valid[m] ? ty[id[m]] : 0.0f;
             if (tile + gridDim.x < ntiles) id[m] = sample(tile + gridDim.x, m);
         }
 #pragma unroll
