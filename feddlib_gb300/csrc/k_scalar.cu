@@ -22,7 +22,7 @@
 // entries and load for several nodes at once (a warp's 32 lanes hold six P1 or
 // two P2 nodes).  Element and row kernel, us, before (one warp per node, P2 by
 // the reference gradients' integrals) and after: 16^3 x 6 tets P1 10.3 + 19.9
-// and 7.4 + 9.5, P2 35.6 + 45.2 and 15.8 + 19.0; 40^3 x 6 P2 281 + 559 and
+// and 8.2 + 9.5, P2 35.6 + 45.2 and 15.8 + 19.0; 40^3 x 6 P2 281 + 559 and
 // 168 + 185 (252 with the element's values stored one by one).
 #include "kernels.cuh"
 
@@ -74,18 +74,15 @@ __global__ void __launch_bounds__(64) k_lap_elem(const double *__restrict__ xyz,
             G[3][k] = C[3 * k + 2];
             G[0][k] = -(G[1][k] + G[2][k] + G[3][k]);
         }
-        // P2: a fifth of D
+        // P2: a fifth of D.  Row 0 from G_0 like the others: as minus the sum of their
+        // entries (7.5 us instead of 8.2 at 16^3 x 6 tets P1) it loses the square of
+        // an element's height over its base, 5e-9 of D_00 at 1000
         const double w = (NPE == 4 ? 1.0 : 0.2) / (6.0 * ad);
 #pragma unroll
-        for (int a = NPE == 4 ? 1 : 0; a < 4; a++) {
+        for (int a = 0; a < 4; a++) {
             const double g0 = w * G[a][0], g1 = w * G[a][1], g2 = w * G[a][2];
 #pragma unroll
             for (int b = a; b < 4; b++) D[a][b] = D[b][a] = g0 * G[b][0] + g1 * G[b][1] + g2 * G[b][2];
-        }
-        if (NPE == 4) {  // the gradients' sum is zero: the first row from the others
-#pragma unroll
-            for (int a = 1; a < 4; a++) D[0][a] = D[a][0] = -(D[a][1] + D[a][2] + D[a][3]);
-            D[0][0] = -(D[0][1] + D[0][2] + D[0][3]);
         }
         // values in pairs: the stores of a warp are not contiguous
         double even = 0.0;
