@@ -92,11 +92,14 @@ struct fedd_assembler {
     int64_t n_dir_u = 0, n_dir_p = 0;
     int64_t launches = 0;
     std::string err;
-    // profiling: event pairs per (call, stage)
+    // profiling: event pairs per (call, stage).  What a call records depends on
+    // what it assembles: each recorded call has its own list of stages, as
+    // indexes into stage_names
     static constexpr int kProfCalls = 256, kProfStages = 8;
     bool prof = false;
     int prof_calls = 0, prof_stage = 0;
     std::vector<cudaEvent_t> ev;  // kProfCalls * kProfStages * 2
+    std::vector<int> prof_lists[kProfCalls];
     std::vector<std::string> stage_names;
     ~fedd_assembler() {
         for (auto e : ev) cudaEventDestroy(e);
@@ -189,8 +192,13 @@ template <class Fn> void stage(fedd_assembler *h, const char *name, cudaStream_t
     fn();
     if (on) {
         FEDD_CUDA(cudaEventRecord(e[1], s));
-        if ((int)h->stage_names.size() <= h->prof_stage) h->stage_names.resize(h->prof_stage + 1);
-        h->stage_names[h->prof_stage] = name;
+        if (h->prof_calls == 0 && h->prof_stage == 0) h->stage_names.clear();  // the totals were read, or none recorded
+        auto &names = h->stage_names;
+        auto &list = h->prof_lists[h->prof_calls];
+        const size_t id = std::find(names.begin(), names.end(), name) - names.begin();
+        if (id == names.size()) names.push_back(name);
+        list.resize(h->prof_stage);
+        list.push_back((int)id);
         h->prof_stage++;
     }
 }
@@ -199,6 +207,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
          double *v10, double *ru, double *rp, cudaStream_t s) {
     LaunchCounter lc;
     const bool jac = what & FEDD_JACOBIAN, res = what & FEDD_RESIDUAL;
+    h->prof_stage = 0;  // a call that failed may have left some
     FEDD_CUDA(cudaMemsetAsync(h->d_err.p, 0, 4 * sizeof(int), s));
     switch (h->prm.problem) {
     case FEDD_LAPLACE:
@@ -796,7 +805,7 @@ fedd_status fedd_set_profiling(fedd_assembler *h, int on) {
         }
         h->prof = on != 0;
         h->prof_calls = 0;
-        h->prof_stage = 0;
+        if (on) h->stage_names.clear();
     });
 }
 
@@ -804,15 +813,17 @@ fedd_status fedd_stage_times(fedd_assembler *h, int max_stages, double *ms_total
     if (!h || !ms_total || !nstages || !calls || max_stages <= 0) return FEDD_ERR_ARG;
     return guarded(h, [&] {
         FEDD_CUDA(cudaSetDevice(h->device));
+        if (h->prof_calls == 0) h->stage_names.clear();
         const int ns = std::min<int>((int)h->stage_names.size(), max_stages);
         for (int k = 0; k < ns; k++) ms_total[k] = 0.0;
         for (int c = 0; c < h->prof_calls; c++)
-            for (int k = 0; k < ns; k++) {
+            for (size_t k = 0; k < h->prof_lists[c].size(); k++) {
+                if (h->prof_lists[c][k] >= ns) continue;
                 cudaEvent_t *e = &h->ev[((size_t)c * fedd_assembler::kProfStages + k) * 2];
                 FEDD_CUDA(cudaEventSynchronize(e[1]));
                 float ms = 0.0f;
                 FEDD_CUDA(cudaEventElapsedTime(&ms, e[0], e[1]));
-                ms_total[k] += ms;
+                ms_total[h->prof_lists[c][k]] += ms;
             }
         *nstages = ns;
         *calls = h->prof_calls;

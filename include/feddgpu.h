@@ -305,7 +305,9 @@ fedd_status fedd_launch_count(const fedd_assembler *h, int64_t *launches);
  * FEDDLib counterpart; FEDDLib times its loops on the host with
  * Teuchos::TimeMonitor (feddlib/core/Utils/FEDDUtils.hpp:7-12).
  * fedd_stage_times synchronises, returns per-stage totals in ms over the
- * recorded calls and clears them. */
+ * recorded calls and clears them.  A call's stages depend on what it
+ * assembles (a residual alone has kernels of its own); the totals are by name,
+ * over all recorded calls, in the order in which the names first came up. */
 fedd_status fedd_set_profiling(fedd_assembler *h, int on);
 fedd_status fedd_stage_times(fedd_assembler *h, int max_stages, double *ms_total, int *nstages,
                              int64_t *calls);
