@@ -482,7 +482,7 @@ __global__ void k_tr_l1(TrainParams P, int H, const float *__restrict__ X, const
     if (t >= B * H) return;
     const int64_t s = t / H;
     const int i = (int)(t - s * H);
-    const float *x = X + 4 * idx[s];
+    const float *x = X + 4 * (idx ? idx[s] : s);
     float z = P.b1[i];
     for (int k = 0; k < 4; k++) z = fmaf(P.W1[4 * i + k], x[k], z);
     const float sg = 1.0f / (1.0f + expf(-z)), tg = sg * (1.0f - sg);
@@ -510,7 +510,7 @@ __global__ void k_tr_l2(TrainParams P, int H, const float *__restrict__ Z2, cons
     const float y = warp_sum(yp) + *P.b3;
     float g[4];
     for (int k = 0; k < 4; k++) g[k] = warp_sum(gp[k]);
-    const int64_t si = idx[s];
+    const int64_t si = idx ? idx[s] : s;
     const float ey = 2.0f * wpsi * (y - ty[si]);
     float eg[4], l = wpsi * (y - ty[si]) * (y - ty[si]);
     for (int k = 0; k < 4; k++) {
@@ -546,7 +546,7 @@ __global__ void k_tr_l1b(TrainParams P, int H, const float *__restrict__ X, cons
     if (t >= B * H) return;
     const int64_t s = t / H;
     const int i = (int)(t - s * H);
-    const float *x = X + 4 * idx[s];
+    const float *x = X + 4 * (idx ? idx[s] : s);
     const float sg = S1[s * H + i], tg = T1[s * H + i];
     float dz = DX1[s * H + i] * sg;
     float dd[4];
@@ -1028,7 +1028,7 @@ void tr_workspace(fedd_trainer *t, int64_t B) {
 }
 
 // general width: loss and gradient (sums over the batch, not yet divided by B)
-// of the samples idx into t->lsum and t->grad
+// of the samples idx (null: 0..B) into t->lsum and t->grad
 void tr_forward_backward(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float wgrad) {
     const int H = t->H;
     cudaStream_t s = 0;
@@ -1221,10 +1221,7 @@ fedd_status fedd_trainer_grad(fedd_trainer *t, float wpsi, float wgrad, float *l
             tr_fused(t, nullptr, t->n, wpsi, wgrad, nullptr);
         } else {
             tr_workspace(t, t->n);
-            DBuf<int64_t> id;  // every sample in order
-            id.alloc(t->n);
-            k_iota<<<ceil_div(t->n, 256), 256>>>(id.p, t->n);
-            tr_forward_backward(t, id.p, t->n, wpsi, wgrad);
+            tr_forward_backward(t, nullptr, t->n, wpsi, wgrad);
         }
         float L = 0;
         FEDD_CUDA(cudaMemcpy(&L, t->lsum.p, sizeof L, cudaMemcpyDeviceToHost));
