@@ -263,6 +263,14 @@ struct Arena {
     }
 };
 
+// Lets kern take whatever dynamic shared memory a launch asks for.  The limit
+// belongs to the kernel, not to the launch: one that followed a handle's mesh
+// would be lowered by another thread's handle between the call that sets it and
+// the launch, which is then refused.  For kernels without static shared memory.
+template <class K> void allow_dynamic_smem(K kern) {
+    FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+}
+
 inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
 }  // namespace fedd

@@ -1139,11 +1139,10 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
 
 void launch_hyper_rows(const Graph &g, const float *stage, double *vals, double *res, int64_t nnodes, cudaStream_t s,
                        LaunchCounter &lc, int64_t n_begin) {
-    const int warps = 4;
+    constexpr int warps = 4;
     const int words = (9 * g.max_adj + kHPad + 3) & ~3;
     const size_t smem = (size_t)warps * (kHRing * kHStage + words) * sizeof(float);
-    if (smem > 48 * 1024)
-        FEDD_CUDA(cudaFuncSetAttribute(k_hyper_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static_assert(warps * (kHRing * kHStage + 9 * kMaxAdjacency + kHPad + 3) * sizeof(float) <= 48 * 1024, "no opt-in needed");
     // about six nodes per warp (3.5 to 7 measured alike; one or fourteen cost
     // 5 %), or all the chip's warps on a small mesh
     const int64_t nodes = nnodes - n_begin, ctas = (nodes + warps - 1) / warps;

@@ -1182,7 +1182,7 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
     const std::true_type yes;
     const std::false_type no;
     const Kern kern = gn ? (newton ? pick(yes, yes) : pick(yes, no)) : (newton ? pick(no, yes) : pick(no, no));
-    FEDD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dynamic_smem(kern);
     unsigned grid = (unsigned)std::min<int64_t>((count + group * warps - 1) / (group * warps), sms * 4);
     if (work) {  // dynamic positions: exactly the CTAs that fit
         int per_sm = 0;
@@ -1203,7 +1203,7 @@ void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_table
     const int warps = 8;
     const int acc_words = (3 * max_adj + 1 + 3) & ~3;
     size_t smem = (160 + (size_t)warps * (kPRing * kPStage + acc_words)) * sizeof(float);
-    FEDD_CUDA(cudaFuncSetAttribute(k_ns_pres_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dynamic_smem(k_ns_pres_rows);
     const int64_t nn = gp.nrow_nodes;
     unsigned grid = (unsigned)std::min<int64_t>((nn + warps - 1) / warps, (int64_t)sm_count_ns() * 8);
     if (grid == 0) return;
