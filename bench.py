@@ -812,6 +812,31 @@ def measure(F, name, args, local, dist, world, rank, headline):
     return out
 
 
+def summary(out):
+    """The record as one line of about 3 KB: the headline workload's figures,
+    and of each other workload its rate, time, roofline fraction, end-to-end
+    rate, largest deviation from the oracle and, for the surrogate, its time
+    and errors against the plain law.  Stage rooflines, notes and the other
+    reports are in the whole record, which is eight times as long."""
+    keys = ["metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "step_roofline", "roofline", "stages_ms", "gpu_launches", "clocks",
+            "e2e", "cpu_baseline", "parity"]
+    notes = ("stages_ms_from", "note", "sample")
+    line = {k: {n: v for n, v in out[k].items() if n not in notes} if isinstance(out[k], dict) else out[k]
+            for k in keys if k in out}
+    for name, w in out.get("workloads", {}).items():
+        far = [v for k, v in (w.get("parity") or {}).items() if k in ("00", "01", "10", "load", "res_u", "res_p") and v]
+        sub = {"value": round(w["value"]), "ms_per_step": round(w["ms_per_step"], 4),
+               "frac": round(w["step_roofline"]["frac"], 4), "e2e": round(w["e2e"]["value"])}
+        if far:
+            sub["parity"] = float("%.3g" % max(far))
+        for k in ("speedup_vs_plain", "stress_rel_fro", "tangent_rel_fro"):
+            if k in (w.get("surrogate") or {}):
+                sub[k] = float("%.4g" % w["surrogate"][k])
+        line.setdefault("workloads", {})[name] = sub
+    return line
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -851,7 +876,8 @@ def main():
             subs[name] = measure(F, name, args, local, None, 1, rank, headline=False)
         out["workloads"] = subs
     if rank == 0:
-        print(json.dumps(out))
+        print(json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(summary(out)), flush=True)
     if dist:
         dist.destroy_process_group()
     return 0
