@@ -252,8 +252,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
                               res && d_u != nullptr, h->d_err.p, s, lc);
         });
         stage(h, "hyper_rows", s, [&] {
-            launch_hyper_rows(h->g, h->stage_f.p, jac ? v00 : nullptr, res ? ru : nullptr, h->nn,
-                              s, lc);
+            launch_hyper_rows(h->g, h->stage_f.p, v00, res ? ru : nullptr, h->nn, s, lc);
         });
         break;
     }
@@ -299,7 +298,7 @@ void run(fedd_assembler *h, unsigned what, const double *d_u, const double *d_p,
         });
         if (!h->ns_fused)
             stage(h, "ns_pres_rows", s, [&] {
-                launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, v10, res ? rp : nullptr, jac,
+                launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, v10, res ? rp : nullptr,
                                     h->gp.max_adj, s, lc, h->coeff);
             });
         break;
@@ -703,7 +702,7 @@ bool run_host_pipelined(fedd_assembler *h, unsigned what, const double *du, cons
     }
     if (ns) {
         if (!h->ns_fused)
-            launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, dv[2], res ? drp : nullptr, 1,
+            launch_ns_pres_rows(h->gp, h->stage_f.p, h->ns_tab.p, h->csr[2].rowptr.p, dv[2], res ? drp : nullptr,
                                 h->gp.max_adj, s, lc, h->coeff);
         FEDD_CUDA(cudaEventRecord(h->chunk_ev[K], s));
         FEDD_CUDA(cudaStreamWaitEvent(cs, h->chunk_ev[K], 0));

@@ -114,8 +114,6 @@ __device__ __forceinline__ float load_geometry(const float *__restrict__ geo, in
     return __ldg(geo + 9 * ne + e);
 }
 
-__device__ __forceinline__ float ld_nc(const float *p) { return __ldg(p); }
-
 // streaming (evict-first) store of the write-once CSR values
 __device__ __forceinline__ void st_cs(double *p, double v) { __stcs(p, v); }
 
@@ -124,18 +122,9 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 
 // ---- asynchronous copies (cp.async) and per-node incidence lists ----------
-__device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
@@ -145,24 +134,12 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// ---- TF32 tensor-core products (mma.sync m16n8k8, FP32 accumulate) --------
-// Fragments (g = lane / 4, tq = lane % 4): A row-major 16x8, a0 = A[g][tq],
-// a1 = A[g+8][tq], a2 = A[g][tq+4], a3 = A[g+8][tq+4]; B 8x8, b0 = B[tq][g],
-// b1 = B[tq+4][g]; C/D 16x8, c0 = C[g][2 tq], c1 = C[g][2 tq + 1],
-// c2 = C[g+8][2 tq], c3 = C[g+8][2 tq + 1].  Callers split each operand into
-// TF32 hi + lo parts and sum hi.hi + hi.lo + lo.hi (3xTF32: FP32-level products).
+// to TF32, nearest; products in FP32 accuracy split each operand into hi + lo
+// parts and sum hi.hi + hi.lo + lo.hi
 __device__ __forceinline__ uint32_t to_tf32(float x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return r;
-}
-
-__device__ __forceinline__ void mma_tf32(float *d, const uint32_t *a, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // the node's incidence list, one coalesced load: lane k holds entries k and

@@ -23,17 +23,11 @@ void basis_dphi(int order, const double *p, double *g);   // Helper::gradPhi, 3D
 //   T[c][a][b][k]  = sum_q w_q phi_a phi_k dc phi_b        (advection)
 //   R[a][b][m]     = sum_q w_q lambda_m phi_a phi_b          (Newton term)
 //   Y[c][p][b]     = sum_q5 w_q psi_p dc phi_b               (divergence)
-//   WPHI, DQ, PHIQ = weights x basis, reference gradients and basis at the
-//                    15 points (advection evaluated at the quadrature points)
 struct NSTables {
     float KS[10][10][6];
     float T[3][10][10][10];
     float R[10][10][4];
     float Y[3][4][10];
-    // quadrature-point form of the advection term (15-point rule):
-    float WPHI[10][16];    // w_q phi_a(q)
-    float DQ[10][3][16];   // d_c phi_b(q) (reference gradients)
-    float PHIQ[15][10];    // phi_k(q)
 };
 void make_ns_tables(NSTables *t);
 
@@ -48,7 +42,9 @@ void make_hyper_tables(int npts, HyperTables *t);
 // ------------------------------------------------------------- graph -----
 // Node -> element incidence plus the sorted node adjacency of one block.
 // For a row node n: incidences inc[inc_ptr[n] .. inc_ptr[n+1]) packed as
-// (element << 4) | local_row_index, ascending; per incidence kSlotStride
+// (element << 4) | local_row_index, ordered by local row index first and
+// element second: the order of summation, and the row kernels reload their
+// tables once per local index.  Per incidence kSlotStride
 // bytes: slot (position in adj row of n) of each of the element's column
 // nodes, at byte offset `slot_off`.
 struct Graph {
@@ -118,7 +114,8 @@ void launch_vertex_map(const int32_t *conn2, const int32_t *conn1, int64_t ne, i
 void node_range_max_elem(const Graph &g, const int64_t *bounds, int K, int64_t *out, cudaStream_t s);
 
 // element arrays: num_elements x npe (AoS, as the C ABI takes them) to the
-// npe x num_elements layout the graph build reads, on the device
+// npe x num_elements layout that the element kernels and the vertex map read,
+// on the device (the graph build reads the caller's)
 void device_aos_to_soa(const int32_t *aos, int64_t ne, int npe, int32_t *soa, cudaStream_t s);
 
 // message slot of handle-less C-ABI calls (per host thread)

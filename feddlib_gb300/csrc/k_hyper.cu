@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(128) k_hyper_rows(const int64_t *__restrict__ 
         }
         cp_async_wait<0>();
         __syncwarp();
-        if (vals && len > 0) {
+        if (len > 0) {
             if (shift && lane == 31) st_cs(out, f2d_exact(acc[0]));
             const int pairs = (len - shift) >> 1;
             for (int c = lane; c < pairs; c += 32) {
@@ -971,17 +971,6 @@ __global__ void __launch_bounds__(128) k_hyper_residual_rows(const int64_t *__re
     res[3 * n + 2] = f2d_exact(z);
 }
 
-// plain law as a stand-alone QP kernel (same I/O as the surrogate kernel)
-__global__ void k_law_qp_plain(LawParams L, const float *__restrict__ inv, int64_t nqp, QPDerivs *out) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= nqp) return;
-    float4 v = reinterpret_cast<const float4 *>(inv)[i];
-    float x[4] = {v.x, v.y, v.z, v.w};
-    QPDerivs d;
-    law_plain(L, x, d);
-    out[i] = d;
-}
-
 __global__ void k_hyper_dense(const float *__restrict__ stage, int64_t first, int64_t count, double *Ke, double *re) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= count * 930) return;
@@ -1188,14 +1177,6 @@ void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, 
     if (e_end <= e_begin) return;
     k_hyper_invariants<<<ceil_div(e_end - e_begin, 128), 128, 0, s>>>(geo, conn, ne, u, law, inv, d_err, e_begin,
                                                                         e_end, tab);
-    FEDD_CUDA(cudaGetLastError());
-    lc.n++;
-}
-
-void launch_law_qp_plain(const LawParams &law, const float *inv, int64_t nqp, QPDerivs *out, cudaStream_t s,
-                         LaunchCounter &lc) {
-    if (nqp == 0) return;
-    k_law_qp_plain<<<ceil_div(nqp, 256), 256, 0, s>>>(law, inv, nqp, out);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

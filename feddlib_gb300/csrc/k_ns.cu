@@ -324,11 +324,11 @@ __global__ void __launch_bounds__(kRecThreads, 1) k_ns_record(const float *__res
         }
         tc::fence_after_sync();
         if (RES) {
-            // NA rows padded to 12 floats, four passes of 32 columns: the
-            // staging takes rows of 36 floats
+            // NA rows padded to 12 floats: two halves of 50 columns, staging
+            // rows of 65 floats
             na_rows_padded(reinterpret_cast<float *>(sW), trow, lane, rec + kResRecNA, ew0, e_end);
         } else {
-        // NA rows out through the warp's staging: columns 0-63 (rows of 68
+            // NA rows out through the warp's staging: columns 0-63 (rows of 68
             // floats), then 64-99 (rows of 36); each store instruction writes
             // whole 256-byte (two rows) or 144-byte (three rows) runs of records
             float *sN = reinterpret_cast<float *>(sW);
@@ -887,10 +887,8 @@ __global__ void __launch_bounds__(256) k_ns_pres_rows(const int64_t *__restrict_
         }
         cp_async_wait<0>();
         __syncwarp();
-        if (vals10) {
-            double *out = vals10 + rowptr10[n];
-            for (int c = lane; c < 3 * K; c += 32) st_cs(out + c, f2d_exact(acc[c]));
-        }
+        double *out = vals10 + rowptr10[n];
+        for (int c = lane; c < 3 * K; c += 32) st_cs(out + c, f2d_exact(acc[c]));
         if (res_p) {
             float v = warp_sum(lw ? r : 0.0f);
             if (lane == 0) res_p[n] = f2d_exact(cpu * v);
@@ -1198,8 +1196,7 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
 }
 
 void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_tables, const int64_t *rowptr10,
-                         double *vals10, double *res_p, int want_jac, int max_adj, cudaStream_t s, LaunchCounter &lc,
-                         const NSCoeff &co) {
+                         double *vals10, double *res_p, int max_adj, cudaStream_t s, LaunchCounter &lc, const NSCoeff &co) {
     const int warps = 8;
     const int acc_words = (3 * max_adj + 1 + 3) & ~3;
     size_t smem = (160 + (size_t)warps * (kPRing * kPStage + acc_words)) * sizeof(float);
@@ -1208,8 +1205,7 @@ void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_table
     unsigned grid = (unsigned)std::min<int64_t>((nn + warps - 1) / warps, (int64_t)sm_count_ns() * 8);
     if (grid == 0) return;
     k_ns_pres_rows<<<grid, 32 * warps, smem, s>>>(gp.inc_ptr.p, gp.inc.p, gp.slots.p, gp.adj_ptr.p, rec, d_tables,
-                                                  rowptr10, want_jac ? vals10 : nullptr, res_p, nn, max_adj,
-                                                  (float)co.pu);
+                                                  rowptr10, vals10, res_p, nn, max_adj, (float)co.pu);
     FEDD_CUDA(cudaGetLastError());
     lc.n++;
 }

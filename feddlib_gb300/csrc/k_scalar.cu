@@ -169,8 +169,7 @@ __global__ void __launch_bounds__(128) k_lap_rows(const int64_t *__restrict__ in
         }
     }
     if (!in) return;
-    if (vals)
-        for (int c = b; c < K; c += W) vals[a0 + c] = acc[c];
+    for (int c = b; c < K; c += W) vals[a0 + c] = acc[c];
     if (load && b == NPE) load[n] = acc[K];
 }
 

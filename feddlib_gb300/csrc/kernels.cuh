@@ -97,7 +97,9 @@ void launch_hyper_elem(const float *geo, const int32_t *conn, int64_t ne, const 
                        const HyperTables &tab, const QPDerivs *qpd, const uint8_t *qp_fallback, float *stage,
                        int want_res, int *d_err, cudaStream_t s, LaunchCounter &lc, int64_t e_begin = 0,
                        int64_t e_end = -1);
-// vals: the values of block (0,0), whose node n starts at 9 adj_ptr[n]
+// vals: the values of block (0,0), whose node n starts at 9 adj_ptr[n].  The
+// value arrays of the matrix row launchers are never null (a call for the
+// residual alone has launchers of its own); the residuals may be.
 void launch_hyper_rows(const Graph &g, const float *stage, double *vals, double *res, int64_t nnodes, cudaStream_t s,
                        LaunchCounter &lc, int64_t n_begin = 0);
 // the residual alone, same values: element residuals (40 floats per element in
@@ -111,8 +113,6 @@ void launch_hyper_invariants(const float *geo, const int32_t *conn, int64_t ne, 
                              LaunchCounter &lc, int64_t e_begin = 0, int64_t e_end = -1);
 void launch_mlp_qp(const MLPDev &m, const LawParams &law, const float *inv, int64_t nqp, QPDerivs *out,
                    uint8_t *fallback, int *d_count, int *d_err, cudaStream_t s, LaunchCounter &lc);
-void launch_law_qp_plain(const LawParams &law, const float *inv, int64_t nqp, QPDerivs *out, cudaStream_t s,
-                         LaunchCounter &lc);
 void launch_law_eval(const LawParams &law, const MLPDev *m, int64_t n, const double *F, double *psi, double *P,
                      double *A, cudaStream_t s);
 void launch_hyper_dense(const float *stage, int64_t first, int64_t count, double *Ke, double *re, cudaStream_t s);
@@ -143,8 +143,8 @@ void launch_ns_vel_rows(const Graph &g, const int4 *ninfo, const float *rec, con
                         int64_t n_begin = 0, int64_t n_end = -1, unsigned long long *work = nullptr,
                         const NSCoeff &co = NSCoeff{});
 void launch_ns_pres_rows(const Graph &gp, const float *rec, const float *d_tables, const int64_t *rowptr10,
-                         double *vals10, double *res_p, int want_jac, int max_adj, cudaStream_t s,
-                         LaunchCounter &lc, const NSCoeff &co = NSCoeff{});
+                         double *vals10, double *res_p, int max_adj, cudaStream_t s, LaunchCounter &lc,
+                         const NSCoeff &co = NSCoeff{});
 // the residual alone, same values, from records written with residual_only;
 // gn_res: the viscous residual rows (32 floats per element) or null
 void launch_ns_residual(const Graph &g, const Graph &gp, const int4 *ninfo, const float *rec, const float *d_tables,

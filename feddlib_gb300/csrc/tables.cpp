@@ -132,13 +132,6 @@ void make_ns_tables(NSTables *t) {
                 }
                 t->Y[c][pn][b] = (float)v;
             }
-    for (int a = 0; a < 10; a++)
-        for (int q = 0; q < 16; q++) {
-            t->WPHI[a][q] = q < 15 ? (float)(q15.w[q] * phi[q][a]) : 0.0f;
-            for (int c = 0; c < 3; c++) t->DQ[a][c][q] = q < 15 ? (float)dphi[q][a][c] : 0.0f;
-        }
-    for (int q = 0; q < 15; q++)
-        for (int k = 0; k < 10; k++) t->PHIQ[q][k] = (float)phi[q][k];
 }
 
 void make_hyper_tables(int npts, HyperTables *t) {
