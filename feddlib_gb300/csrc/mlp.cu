@@ -579,7 +579,7 @@ __global__ void k_tr_l1b(TrainParams P, int H, const float *__restrict__ X, cons
 // pipe.  For a batch of 65,536: 1,590 us of separate kernels; 213 us one
 // sample per thread with scalar multiply-adds; 203 packed; 184 two samples and
 // 384 threads (205 with 256: two warps per scheduler are too few); k_tr_update
-// another 8 us.
+// another 7 us.
 constexpr int kTRows = 16;               // samples of a tile that one share of gW2 adds
 constexpr int kTSample = 5 * kH + 4;     // floats per sample: five channels, and 4 so that two samples' rows differ in banks
 constexpr int kTPar = 4 * kH + kH + kH * kH + kH + kH + 2;  // gradients in the parameters' order, then the loss
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(256) k_tr_update(const float *__restrict__ par
 //     out[i] = V(i)                      if j_i = i (and for i = 0)
 //            = V(k) or perm[j_i]         with k the successor of i in L_{j_i}.
 // Lists and chains have about log n entries.  On the host a shuffle of 200,000
-// samples took 1,140 us; these seven launches take 45 us.
+// samples took 1,140 us; these seven launches take 47 us.
 __host__ __device__ inline uint64_t sm64_mix(uint64_t z) {
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
@@ -1076,8 +1076,9 @@ struct AdamStep {
 void tr_fused(fedd_trainer *t, const int64_t *idx, int64_t B, float wpsi, float wgrad, const AdamStep *adam) {
     cudaStream_t s = 0;
     // tiles of 48 samples, one CTA per SM, or of 16, two per SM: whichever takes
-    // less time over its rounds of tiles (20.4 and 14.6 us a round; a step of
-    // 65,536 samples 205 against 226 us, 20,000 77 and 84, 15,000 76 and 69, 30,000 118 and 114)
+    // less time over its rounds of tiles (20.4 and 14.6 us a round; wall time
+    // of a step with its share of the shuffles: 65,536 samples 205 against 226 us, 20,000 77 and
+    // 84, 15,000 76 and 69, 30,000 118 and 114)
     const int64_t rounds1 = ceil_div(B, 32 * (int64_t)sms()), rounds2 = ceil_div(B, 48 * (int64_t)sms());
     const int spt = 7 * rounds2 < 5 * rounds1 ? 2 : 1;
     const int groups = spt == 2 ? 24 : 16;
