@@ -246,7 +246,7 @@ void launch_lap_rows(const Graph &g, const double *stage, int order, double *val
         const int warps = 4, nodes = order == 1 ? 32 / 5 : 32 / 11;
         const size_t smem = (size_t)warps * (nodes + 1) * (g.max_adj + 1) * sizeof(double);
         auto kern = order == 1 ? k_lap_rows<4> : k_lap_rows<10>;
-        allow_dynamic_smem(kern);
+        if (smem > 48 * 1024) allow_dynamic_smem(kern);
         kern<<<ceil_div(nnodes, warps * nodes), 32 * warps, smem, s>>>(g.inc_ptr.p, g.inc.p, g.slots.p, g.adj_ptr.p, stage,
                                                                       vals, load, nnodes, g.max_adj);
     }
